@@ -58,8 +58,8 @@ struct Index {
   DevBuf<uint32_t> xst;      // linear scans: the same, tiled [ceil(N/128)][wp/4][128] x 16 B
   DevBuf<uint32_t> xsl;      // byte samples (kind 4) or CWS codes (kind 10) bit-sliced and tiled
                              // like xst, for the threshold-filter scan (derived, not stored)
-  DevBuf<uint8_t> xse;       // tensor-core sketch scans: sketch bits as E4M3 +-1 rows,
-                             // [ceil(n/256)*256][128 * ceil(words/4)] (derived, not stored)
+  DevBuf<uint8_t> xse;       // tensor-core sketch scans: sketch bits as E2M1 +-1 rows, two
+                             // to a byte, [ceil(n/224)*224][128 * ceil(words/8)] (derived, not stored)
   DevBuf<float> xsf, xsft;   // JL sketches [n][sdim] and their tile layout
   DevBuf<float> sk_planes;   // SimHash planes [32*sketchDim][d] or JL rows [sdim][d]
   DevBuf<uint16_t> sk_split; // SimHash planes split into BF16 [hi | lo | hi] rows for the
@@ -135,7 +135,7 @@ void sketch_queries(Index& idx, float* q, int nq, DevBuf<uint32_t>* qs, DevBuf<f
 int next_pow2(int v);
 
 // Build idx.xst (the linear scans' tiled sketches) from idx.xs, and for Hamming / one-bit
-// Jaccard sketches of at most 1024 bits idx.xse (their E4M3 rows for the tensor cores).
+// Jaccard sketches of at most 1024 bits idx.xse (their E2M1 rows for the tensor cores).
 void tile_sketches(Index& idx, cudaStream_t stream);
 
 // Arrays derived from stored ones at build and at load: the tensor-core scans' FP64 row norms,

@@ -54,6 +54,7 @@ constexpr int F_EPI_WARPS = 16;  // four warpgroups, one 64-column piece each
 
 constexpr int F_SBUF = 8;  // staged survivors a row and warpgroup (flushed with one atomic)
 constexpr int kTauRegs = 80;  // group maxima a lane holds in the register threshold select
+constexpr int kTauRegsFew = 44;  // and its smaller form: 1,408 maxima, what a base of 1.2M points leaves
 
 // Shared-memory layout by operand format.  BF16: a tile row is two 128-byte swizzle rows
 // (64 columns each); E4M3: one (all 128 columns), so tiles are half the size and the
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(F_THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + F_BAR_OFF + 8 * (4 * F_STAGES + 5 + 2 * F_NACC));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform for the compiler too
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -216,45 +217,46 @@ __global__ void __launch_bounds__(F_THREADS, 1)
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    {
+      const uint32_t leader = elect_one();  // the warp stays converged (see elect_one)
       int it = 0, ua = 0;
       bool ok = true;
       for (int u = blockIdx.x; u < U && ok; u += gridDim.x, ++ua) {
         const int c = u / a.QT;
         const int p0 = c * a.CH, p1 = min(a.NP, p0 + a.CH);
         const int ab = ua & 1;
-        if (!mbar_wait(A_FULL(ab), (ua >> 1) & 1, abort_flag)) break;
+        if (!mbar_wait_warp(A_FULL(ab), (ua >> 1) & 1, abort_flag)) break;
         tc_fence_after();
         for (int p = p0; p < p1; ++p) {
           const int b = it % F_NACC, ub = it / F_NACC;
-          if (!mbar_wait(ACC_EMPTY(b), (ub & 1) ^ 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(ACC_EMPTY(b), (ub & 1) ^ 1, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const int st = it % F_STAGES, rd = it / F_STAGES;
-          if (!mbar_wait(FULL(st), rd & 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(FULL(st), rd & 1, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t dt = tmem + (uint32_t)(b * TN), as = s0 + F_A_OFF + ab * A_BYTES;
           const uint32_t bs = s0 + F_B_OFF + st * B_TILE;
           if (F8) {
-            umma_tile_e4m3<TN>(dt, as, bs, a.ksteps);
-            umma_commit(EMPTY(st));
+            umma_tile_e4m3<TN>(dt, as, bs, a.ksteps, leader);
+            umma_commit(EMPTY(st), leader);
           } else if (!SPLIT) {
-            umma_tile<TN>(dt, as, bs, a.ksteps);
-            umma_commit(EMPTY(st));
+            umma_tile<TN>(dt, as, bs, a.ksteps, leader);
+            umma_commit(EMPTY(st), leader);
           } else {
-            umma_steps<TN>(dt, as, bs, 0, min(4, a.ksteps));
-            umma_commit(EMPTY(st));
-            if (!mbar_wait(FULL_HI(st), rd & 1, abort_flag)) { ok = false; break; }
+            umma_steps<TN>(dt, as, bs, 0, min(4, a.ksteps), leader);
+            umma_commit(EMPTY(st), leader);
+            if (!mbar_wait_warp(FULL_HI(st), rd & 1, abort_flag)) { ok = false; break; }
             tc_fence_after();
-            umma_steps<TN>(dt, as, bs, 4, a.ksteps);
-            umma_commit(EMPTY_HI(st));
+            umma_steps<TN>(dt, as, bs, 4, a.ksteps, leader);
+            umma_commit(EMPTY_HI(st), leader);
           }
-          umma_commit(ACC_FULL(b));
+          umma_commit(ACC_FULL(b), leader);
           ++it;
         }
-        umma_commit(A_EMPTY(ab));  // the query tile is free once this unit's MMAs complete
+        umma_commit(A_EMPTY(ab), leader);  // the query tile is free once this unit's MMAs complete
       }
       // drain: all issued MMAs complete before TMEM is released
-      umma_commit(DONE);
+      umma_commit(DONE, leader);
       mbar_wait(DONE, 0, abort_flag, true);
     }
     __syncwarp();
@@ -688,8 +690,8 @@ void launch_filter_scan(const CUtensorMap& ma, const CUtensorMap& mb, const CUte
 void launch_tau_select(const float* gmax, int nq, int M, int rank, float margin, float* tau, cudaStream_t s) {
   ProfScope _ps("tc_tau_select", s);
   // the register slots a lane walks in every bisection step: as few as cover M
-  if (M <= 32 * (kTauRegs / 2) && M % 4 == 0)
-    tau_select_reg_kernel<kTauRegs / 2><<<ceil_div(nq, 8), 256, 0, s>>>(gmax, nq, M, rank, margin, tau);
+  if (M <= 32 * kTauRegsFew && M % 4 == 0)
+    tau_select_reg_kernel<kTauRegsFew><<<ceil_div(nq, 8), 256, 0, s>>>(gmax, nq, M, rank, margin, tau);
   else if (M <= 32 * kTauRegs && M % 4 == 0)
     tau_select_reg_kernel<kTauRegs><<<ceil_div(nq, 8), 256, 0, s>>>(gmax, nq, M, rank, margin, tau);
   else

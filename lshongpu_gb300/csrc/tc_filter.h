@@ -52,8 +52,8 @@ void launch_cand_select(const int* cnt, const uint64_t* cand, int nq, int cap, i
 // top-C of each query.  ok = false: no prepass shape bounds C well (use the popcount scan).
 struct HammingPlan {
   bool ok;
-  int NT;    // 256-point base tiles
-  int GW;    // prepass group width (64 or 8; 0 = no prepass, every point survives)
+  int NT;    // 224-point base tiles
+  int GW;    // prepass group width (56 or 8; 0 = no prepass, every point survives)
   int S;     // prepass samples every S-th tile
   int NS;    // sampled tiles
   int M;     // group maxima a query
@@ -61,13 +61,15 @@ struct HammingPlan {
   int cap;   // survivor slots a query
 };
 HammingPlan plan_hamming(int64_t n, int C);
-// 128-bit chunks of a sketch row of `words` words (rows of 128 * chunks E4M3 bytes).
+// 256-bit chunks of a sketch row of `words` words (rows of 128 * chunks bytes, two E2M1
+// codes a byte), and the base's rows padded to whole tiles.
 int hamming_chunks(int words);
-// Sketch rows [n][wp] (first `words` real) -> E4M3 +-1 rows [rows_pad][128 * chunks].
+int64_t hamming_rows(int64_t n);
+// Sketch rows [n][wp] (first `words` real) -> E2M1 +-1 rows [rows_pad][128 * chunks].
 void launch_expand_bits(const uint32_t* xs, int64_t n, int wp, int words, int64_t rows_pad, uint8_t* out,
                         cudaStream_t s);
-// Top-C keys [nq][C] of each query by (hamming asc, id asc); xse: the base's E4M3 rows
-// (launch_expand_bits, rows padded to 256), xst: the tiled sketches (listed rescans), qs:
+// Top-C keys [nq][C] of each query by (hamming asc, id asc); xse: the base's E2M1 rows
+// (launch_expand_bits, hamming_rows(n) of them), xst: the tiled sketches (listed rescans), qs:
 // query sketches [nq][wp].  op: OP_HAMMING or OP_ONEBIT_JACCARD.
 void launch_tc_hamming(const uint8_t* xse, int64_t n, const uint32_t* xst, int wp, int words, const uint32_t* qs,
                        int nq, int op, int C, uint64_t* out, int* err, cudaStream_t s);

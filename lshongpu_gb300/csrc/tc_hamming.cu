@@ -1,20 +1,21 @@
-// Tensor-core sketch scan: the Hamming distance of bit sketches as a +-1 E4M3 GEMM
+// Tensor-core sketch scan: the Hamming distance of bit sketches as a +-1 E2M1 (FP4) GEMM
 // (implementations 3 and 5 -- SimHash and one-bit weighted MinHash -- in place of the
 // XOR/popcount scan of scan_bits.cu for batches that fill the tensor cores; the
 // reference's scanHammingDistance, sketchedDistanceScanners.cuh:14-100, and its one-bit
 // scanJaccardDistance, :194-274).
 //
-// Bit b of a sketch becomes the E4M3 value 1 - 2b: +1.0 (0x38) or -1.0 (0xB8).  For two
-// sketches of B = 32 * words bits the dot product of those rows is (#equal bits) -
-// (#different bits) = B - 2 * hamming.  Every product is +-1 and every partial sum an
-// integer of magnitude <= B <= 1024, which FP32 holds exactly, so the accumulator gives
-// hamming = (B - dot) / 2 exactly, and the top-C by (hamming, id) equals the popcount
-// scan's.  The one-bit Jaccard distance 1 - (B - hamming) / B orders points the same way.
-// Rows are padded to whole 128-byte chunks with 0x00 (+0.0), which adds nothing.
+// Bit b of a sketch becomes the E2M1 value 1 - 2b: +1.0 (0x2) or -1.0 (0xA), two to a byte.
+// For two sketches of B = 32 * words bits the dot product of those rows is (#equal bits) -
+// (#different bits) = B - 2 * hamming.  Every product is +-1, every block scale 1.0 and
+// every partial sum an integer of magnitude <= B <= 1024, which FP32 holds exactly, so the
+// accumulator gives hamming = (B - dot) / 2 exactly, and the top-C by (hamming, id) equals
+// the popcount scan's.  The one-bit Jaccard distance 1 - (B - hamming) / B orders points the
+// same way.  Rows are padded to whole 128-byte chunks (256 bits) with 0x0 (+0.0), which adds
+// nothing.
 //
 // Selection, as in the threshold-filter scan of tc_filter.cu, in two GEMM passes:
 //   prepass  on every S-th base tile writes each query's group maxima of the score (the
-//            best score of each 64- or 8-point group of a sampled tile); tau[q] = the
+//            best score of each 56- or 8-point group of a sampled tile); tau[q] = the
 //            r-th largest of them (launch_tau_select).  With S = 1, r = C and every point
 //            of the exact top-C scores >= tau.  With S > 1, r = C/S + 4 sqrt(C/S) + 8 -- the
 //            C-th best point of the base would put about C/S points of the sample above
@@ -31,17 +32,32 @@
 //            listed and rescanned exactly by the popcount scan on the device, so the result
 //            is always the exact top-C.
 //
-// tc_hamming_kernel: persistent, one CTA per SM, 640 threads.  A unit is (query tile of 128
-// rows, chunk of up to 32 consecutive base tiles of 256 points), numbered chunk-major so
-// that all SMs stream the same base tiles at a time (each read from HBM about once a batch,
-// then from L2).  The query tile stays in shared memory for the unit (KC chunks of 128 rows
-// x 128 bytes); the base tile streams through a ring of one-chunk stages (256 rows x 128
-// bytes).  Warp 0 issues the TMA copies, warp 1 the MMAs (tcgen05.mma kind::f8f6f4, A and
-// B both E4M3, M = 128, N = 256, K = 32 each; 4 a chunk, 4 * KC a tile), warp 2 owns the
-// 512 TMEM columns (two 256-column FP32 accumulators), warps 4-19 are the epilogue
-// (warpgroup g reads columns [64g, 64g + 64), one query row a thread).  Every mbarrier
-// wait is bounded (2 s); a CTA that times out raises error 2, drains its copies and MMAs,
-// frees TMEM and returns.
+// tc_hamming_kernel: persistent, one CTA per SM, 640 threads, in clusters of CL = 2 CTAs (1
+// for batches of one query tile).  A unit is (CL query tiles of 128 rows, chunk of up to 36
+// consecutive base tiles of 224 points), numbered chunk-major so that all SMs stream the
+// same base tiles at a time (each read from HBM about once a batch, then from L2).  Each CTA
+// keeps its query tile in shared memory for the unit (KC chunks of 128 rows x 128 bytes);
+// the base tile streams through a ring of one-chunk stages (224 rows x 128 bytes), half of
+// each stage loaded by either CTA and multicast to both: a 128 x 224 tile of 1,024 bits is
+// 1,792 cycles of MMA, and fetching its 112 KB for one SM alone would take more than the
+// about 85 KB a microsecond an SM gets from L2.
+// Warp 0 issues the TMA copies, warp 1 the MMAs (tcgen05.mma kind::mxf4 with block scales
+// of 1.0, M = 128, N = 224, K = 64 each; 4 a chunk), warp 2 owns the 512 TMEM columns, warps
+// 4-19 are the epilogue (warpgroup g reads columns [56g, 56g + 56), one query row a thread).
+// N = 224 leaves TMEM columns [224, 256) beside the two accumulators (at 0 and 256) for the
+// scale factors, which are filled once with the UE8M0 code of 1.0 (0x7f), so their layout
+// does not matter.  Every mbarrier wait is bounded (2 s); a CTA that times out raises
+// error 2, drains its copies and MMAs, frees TMEM and returns; the CTAs of a cluster leave
+// together.
+//
+// Measured (filter pass; 10,000 queries): 1.2M points of 1,024 bits 7.52 -> 3.25 ms (7.5
+// PFLOP/s of +-1 products; 2.5 ms is the MMAs alone), 500k points of 256 bits at C = 4,096
+// 4.79 -> 1.77 ms (bounded by the 1.3% survivors: without any the same pass takes 0.67 ms);
+// before: E4M3 rows (twice the bytes, half the MMA rate), a query tile a CTA with its own
+// copy of every base tile, MMAs issued from a diverged warp, branches around each store.
+//
+// tc_signs_kernel: the same pipeline with BF16 operands and one query tile for the SimHash
+// projections (below).
 #include "index.h"
 #include "launch_count.h"
 #include "profile.h"
@@ -61,45 +77,51 @@ namespace tc {
 namespace {
 
 constexpr int H_THREADS = 640;
-constexpr int HN = 256;           // base points a tile (UMMA N)
-constexpr int H_CHUNK = 128;      // bytes of a row in one K chunk (one 128-byte swizzle row)
-constexpr int H_NACC = 2;         // TMEM accumulators of HN columns
-constexpr int H_TMEM_COLS = H_NACC * HN;
+constexpr int HN = 224;           // base points a tile (UMMA N): 4 warpgroups x 7 groups of 8 columns
+constexpr int HW = HN / 4;        // columns a warpgroup reads
+constexpr int H_CHUNK = 128;      // bytes of a row in one K chunk (one 128-byte swizzle row): 256 bits
+constexpr int H_TMEM_COLS = 512;  // accumulators at columns 0 and 256, scale factors at [224, 256)
+constexpr int H_ACC_COL = 256;
+constexpr int H_SF_COL = HN;
+constexpr int H_MAX_CH = 36;      // base tiles a unit: 36 * 224 column offsets fit the staging's 13 bits
 constexpr int H_EPI_WARPS = 16;
 constexpr int H_SEL_MAX = 16384;  // survivors a query the block select sorts at most
-constexpr int kHTauRegs = 80;
+constexpr int PN = 256;           // planes a tile of the projections' GEMM (UMMA N)
+constexpr int P_NACC = 2;         // its TMEM accumulators of PN columns
 
 constexpr int kSmemLimit = 232448;  // dynamic shared memory a CTA may opt into
 
-// Shared-memory layout for rows of KC chunks.  The survivor staging takes what is left
-// (8, 4, 2 or 1 entries a row and warpgroup; none: each survivor takes its own slot).
+// Shared-memory layout for rows of KC chunks: the resident query tile, the ring of base
+// chunks, and the survivor staging (SBUF 4-byte entries a row and warpgroup).
 template <int KC>
 struct HLayout {
-  static constexpr int A_BYTES = KC * BM * H_CHUNK;  // resident query tile
-  static constexpr int B_BYTES = HN * H_CHUNK;       // one chunk of a base tile: 32 KB
-  static constexpr int STAGES = KC <= 4 ? 4 : 3;
+  static constexpr int A_BYTES = KC * BM * H_CHUNK;  // query tile
+  static constexpr int B_BYTES = HN * H_CHUNK;       // one chunk of a base tile: 28 KB
+  static constexpr int STAGES = 4;
   static constexpr int FIXED = A_BYTES + STAGES * B_BYTES + 256 + 1024;  // + barriers + alignment slack
-  static constexpr int ROOM = (kSmemLimit - FIXED) / (4 * BM * 8);
-  static constexpr int SBUF = ROOM >= 8 ? 8 : ROOM >= 4 ? 4 : ROOM >= 2 ? 2 : ROOM >= 1 ? 1 : 0;
+  static constexpr int ROOM = (kSmemLimit - FIXED) / (4 * BM * 4);
+  static constexpr int SBUF = ROOM >= 24 ? 24 : ROOM;
   static constexpr int A_OFF = 0;
   static constexpr int B_OFF = A_BYTES;
-  static constexpr int S_OFF = B_OFF + STAGES * B_BYTES;  // scores then ids, [4][SBUF][BM] each
-  static constexpr int BAR_OFF = S_OFF + 4 * SBUF * BM * 8;
+  static constexpr int S_OFF = B_OFF + STAGES * B_BYTES;  // [4][SBUF][BM] entries
+  static constexpr int BAR_OFF = S_OFF + 4 * SBUF * BM * 4;
   static constexpr int SMEM = BAR_OFF + 256 + 1024;
   static_assert(SMEM <= kSmemLimit, "shared memory per CTA");
-  static_assert(8 * (2 * STAGES + 2 + 2 * H_NACC + 1) + 12 <= 256, "barrier area");
+  static_assert(SBUF >= 8, "staging room");
+  static_assert(8 * (2 * STAGES + 7) + 8 <= 256, "barrier area");
 };
-
-constexpr int MODE_SIGNS = 2;  // SimHash projections: sign bits, uncertain ones listed
+static_assert(H_MAX_CH * HN <= 8192, "column offsets of a unit fit 13 bits");
 
 struct HArgs {
   int nq;
   int64_t n;
   int QT;           // query tiles
+  int QP;           // groups of CL of them
   int NP;           // base positions scanned (base tile = p * dstride)
   int dstride;
   int CH;           // positions a unit
   int NCH;          // chunks of positions
+  int ksteps;       // MMA K steps (64 bits each) that cover a sketch
   float* gmax;      // MODE_GROUPMAX: [nq][M] group maxima
   int M;
   const float* tau; // MODE_FILTER: threshold a query (nullptr: keep every point)
@@ -107,34 +129,319 @@ struct HArgs {
   uint64_t* cand;   // [nq][cap] survivor keys
   int cap;
   int* err;
-  // MODE_SIGNS: rows are points, the "base" is the planes
-  const float* rown;   // point norms
-  const float* pnorm;  // plane norms (padded to whole tiles with zeros)
-  float band;          // a sign is certain when |score| > band * |x| * |r|
-  uint32_t* out32;     // [nq][words] sign bits
-  int words, P;        // words a point, planes (32 * words)
-  uint2* list;         // [grid][list_cap] (point, plane) of the uncertain signs, a segment a CTA
-  int* list_cnt;       // [grid] entries a segment (may exceed list_cap: overflow)
-  int list_cap;
 };
 
-// Out of line: called from every group of the unrolled survivor path, inlined copies would
-// crowd the instruction cache.
-__device__ __noinline__ void h_flush(int* cnt, uint64_t* dst, int cap, const float* ssc, const int* sid, int scnt) {
-  const int base = atomicAdd(cnt, scnt);
-  for (int e = 0; e < scnt; ++e)
-    if (base + e < cap) dst[base + e] = make_key(-ssc[e * BM], sid[e * BM]);
+// Survivor staging: a thread's entries lie BM words apart in its warpgroup's [SBUF][BM]
+// array (lane = bank).  An entry is the score's float bits with the column's offset in the
+// unit in the low 13 bits: scores are integers of magnitude at most 1024, whose mantissas
+// leave the low 14 bits zero.  A push is a compare, an add and two predicated instructions,
+// without a branch: at the one-bit MinHash rates (1.3% of the scores survive, about 25 a
+// warp and tile) branches around each store had made the survivor path five times as long
+// as everything else in the kernel.
+__device__ __forceinline__ void h_push(uint32_t v, float tau, uint32_t& at, uint32_t off) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ge.f32 p, %1, %2;\n\t@p st.shared.u32 [%0], %3;\n\t@p add.u32 %0, %0, %4;\n\t}"
+      : "+r"(at)
+      : "f"(__uint_as_float(v)), "f"(tau), "r"(v + off), "n"(BM * 4)
+      : "memory");
 }
 
-// BF: operands are BF16 (kind::f16, 64 elements a 128-byte chunk) instead of E4M3.
-template <int MODE, int GW, int KC, bool BF = false>
+// Move this thread's `n` > 0 staged entries to its query's candidate array: one atomicAdd
+// reserves the slots.  id0: the base id of offset 0.  Out of line: inlined copies would
+// crowd the instruction cache.
+__device__ __noinline__ void h_flush(int* cnt, uint64_t* dst, int cap, uint32_t at0, int n, int id0) {
+  const int base = atomicAdd(cnt, n);
+  for (int e = 0; e < n; ++e) {
+    uint32_t w;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(at0 + e * (BM * 4)));
+    if (base + e < cap) dst[base + e] = make_key(-__uint_as_float(w & ~0x3fffu), id0 + (int)(w & 0x1fffu));
+  }
+}
+
+template <int MODE, int GW, int KC, int CL>
 __global__ void __launch_bounds__(H_THREADS, 1)
     tc_hamming_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                       const HArgs a) {
   using LY = HLayout<KC>;
   constexpr int STAGES = LY::STAGES, SBUF = LY::SBUF;
-  static_assert(MODE != MODE_FILTER || GW == 64, "the filter reads whole 64-column pieces");
-  static_assert(GW == 64 || GW == 8, "group width");
+  static_assert(MODE != MODE_FILTER || GW == HW, "the filter reads whole pieces");
+  static_assert(GW == HW || GW == 8, "group width");
+  const int U = a.NCH * a.QP;
+  const int cid = blockIdx.x / CL, ncl = gridDim.x / CL;  // cluster, clusters
+  if (cid >= U) return;  // no unit for this cluster: leave before any barrier or TMEM use
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const uint32_t s0 = smem_u32(sm);
+  const uint32_t bar0 = s0 + LY::BAR_OFF;
+  auto FULL = [&](int s) { return bar0 + 8u * s; };
+  auto EMPTY = [&](int s) { return bar0 + 8u * (STAGES + s); };
+  const uint32_t A_FULL = bar0 + 8u * (2 * STAGES);
+  const uint32_t A_EMPTY = bar0 + 8u * (2 * STAGES + 1);
+  auto ACC_FULL = [&](int b) { return bar0 + 8u * (2 * STAGES + 2 + b); };
+  auto ACC_EMPTY = [&](int b) { return bar0 + 8u * (2 * STAGES + 4 + b); };
+  const uint32_t DONE = bar0 + 8u * (2 * STAGES + 6);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + LY::BAR_OFF + 8 * (2 * STAGES + 7));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform for the compiler too
+  const int lane = threadIdx.x & 31;
+  const int rank = CL > 1 ? (int)cluster_rank() : 0;
+  constexpr uint16_t kAll = (uint16_t)((1u << CL) - 1u);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(FULL(s), 1);
+      mbar_init(EMPTY(s), CL);  // every CTA of the cluster has read the stage
+    }
+    mbar_init(A_FULL, 1);
+    mbar_init(A_EMPTY, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(ACC_FULL(b), 1);
+      mbar_init(ACC_EMPTY(b), H_EPI_WARPS);
+    }
+    mbar_init(DONE, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 2) tmem_alloc(smem_u32(tmem_slot), H_TMEM_COLS);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  if (warp >= 4 && warp < 8) {  // scale factors: 1.0 in every byte of every lane
+#pragma unroll
+    for (int c = H_SF_COL; c < H_ACC_COL; c += 8)
+      tmem_fill8(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c, 0x7f7f7f7fu);
+    tmem_wait_st();
+  }
+  tc_fence_before();
+  if (CL > 1) cluster_sync();  // the peer's barriers are initialised before anything arrives on them
+  else __syncthreads();
+  tc_fence_after();
+
+  if (warp == 0) {
+    // ---------------- TMA producer ----------------
+    if (lane == 0) {
+      int it = 0, na = 0;  // base chunks and query tiles issued
+      int have = -1;       // query tile in shared memory
+      bool ok = true;
+      for (int u = cid; u < U && ok; u += ncl) {
+        const int qp = u % a.QP, c = u / a.QP;
+        const int p0 = c * a.CH, p1 = min(a.NP, p0 + a.CH);
+        // The unit's first STAGES base chunks are issued before its query tile: their
+        // stages free up as the previous unit's MMAs consume the ring, so the copies run
+        // while those MMAs finish.  The query tile is reloaded once the previous unit's MMAs
+        // have completed, and kept when the next unit has the same one.  (A tile past the
+        // last one, where the query tiles do not fill the cluster, reads as zeros.)
+        const int total = (p1 - p0) * KC, pre = min(STAGES, total);
+        for (int ci = 0; ci <= total; ++ci) {
+          if (ci == pre && qp != have) {
+            if (!mbar_wait(A_EMPTY, (na & 1) ^ 1, abort_flag)) { ok = false; break; }
+            mbar_expect_tx(A_FULL, LY::A_BYTES);
+#pragma unroll
+            for (int kc = 0; kc < KC; ++kc)
+              tma_load_2d(s0 + LY::A_OFF + kc * BM * H_CHUNK, &mapA, kc * H_CHUNK, (CL * qp + rank) * BM, A_FULL);
+            ++na;
+            have = qp;
+          }
+          if (ci == total) break;
+          const int p = p0 + ci / KC, kc = ci % KC;
+          const int st = it % STAGES, rd = it / STAGES;
+          if (!mbar_wait(EMPTY(st), (rd & 1) ^ 1, abort_flag)) { ok = false; break; }
+          mbar_expect_tx(FULL(st), LY::B_BYTES);
+          // this CTA's share of the stage, to every CTA of the cluster
+          const uint32_t dst = s0 + LY::B_OFF + st * LY::B_BYTES + rank * (LY::B_BYTES / CL);
+          const int row = p * a.dstride * HN + rank * (HN / CL);
+          if (CL > 1) tma_load_2d_multicast(dst, &mapB, kc * H_CHUNK, row, FULL(st), kAll);
+          else tma_load_2d(dst, &mapB, kc * H_CHUNK, row, FULL(st));
+          ++it;
+        }
+      }
+      // drain: every copy into this CTA has landed and every stage has been given back (the
+      // peer's arrivals included) before the CTA may exit
+      for (int j = max(0, it - STAGES); j < it; ++j) {
+        mbar_wait(FULL(j % STAGES), (j / STAGES) & 1, abort_flag, true);
+        mbar_wait(EMPTY(j % STAGES), (j / STAGES) & 1, abort_flag, true);
+      }
+      if (na > 0) mbar_wait(A_FULL, (na - 1) & 1, abort_flag, true);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ---------------- MMA issuer ----------------
+    {
+      const uint32_t leader = elect_one();  // the warp stays converged (see elect_one)
+      constexpr uint32_t idesc = idesc_mxf4(HN);
+      int it = 0, ia = 0, na = 0;
+      int have = -1;
+      bool ok = true;
+      for (int u = cid; u < U && ok; u += ncl) {
+        const int qp = u % a.QP, c = u / a.QP;
+        const int p0 = c * a.CH, p1 = min(a.NP, p0 + a.CH);
+        if (qp != have) {
+          if (!mbar_wait_warp(A_FULL, na & 1, abort_flag)) break;
+          tc_fence_after();
+          ++na;
+          have = qp;
+        }
+        for (int p = p0; p < p1 && ok; ++p) {
+          const int b = ia & 1, ub = ia >> 1;
+          if (!mbar_wait_warp(ACC_EMPTY(b), (ub & 1) ^ 1, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t d_tmem = tmem + (uint32_t)(b * H_ACC_COL);
+          for (int kc = 0; kc < KC; ++kc) {
+            const int st = it % STAGES, rd = it / STAGES;
+            if (!mbar_wait_warp(FULL(st), rd & 1, abort_flag)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t a_base = s0 + LY::A_OFF + kc * BM * H_CHUNK;
+            const uint32_t b_base = s0 + LY::B_OFF + st * LY::B_BYTES;
+            const int steps = min(4, a.ksteps - 4 * kc);
+#pragma unroll
+            for (int kk = 0; kk < H_CHUNK / 32; ++kk)  // 32 bytes a step: K = 64
+              if (kk < steps)
+                umma_mxf4(d_tmem, smem_desc(a_base + kk * 32), smem_desc(b_base + kk * 32), idesc,
+                          tmem + (uint32_t)H_SF_COL, (kc > 0 || kk > 0) ? 1u : 0u, leader);
+            if (CL > 1) umma_commit_multicast(EMPTY(st), kAll, leader);
+            else umma_commit(EMPTY(st), leader);
+            ++it;
+          }
+          if (!ok) break;
+          umma_commit(ACC_FULL(b), leader);
+          ++ia;
+        }
+        // the query tile is free once this unit's MMAs complete
+        if (u + ncl < U && (u + ncl) % a.QP != qp) umma_commit(A_EMPTY, leader);
+      }
+      // drain: all issued MMAs complete before TMEM is released
+      umma_commit(DONE, leader);
+      mbar_wait(DONE, 0, abort_flag, true);
+    }
+    __syncwarp();
+  } else if (warp >= 4) {
+    // ---------------- epilogue ----------------
+    const int g = (warp - 4) >> 2;         // warpgroup: columns [56g, 56g + 56) of every accumulator
+    const int r = (warp & 3) * 32 + lane;  // query row within the tile = TMEM lane
+    const uint32_t tbase = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g * HW);
+    const uint32_t at0 = s0 + LY::S_OFF + (uint32_t)(g * SBUF * BM + r) * 4u;
+    constexpr int GRP = SBUF >= 16 ? 8 : 4;                            // columns pushed between two room checks
+    const uint32_t at_lim = at0 + (uint32_t)(SBUF - GRP) * (BM * 4u);  // beyond: no room for GRP more
+    uint32_t at = at0;
+    int ia = 0;
+    bool ok = true;
+    for (int u = cid; u < U && ok; u += ncl) {
+      const int qp = u % a.QP, c = u / a.QP;
+      const int p0 = c * a.CH, p1 = min(a.NP, p0 + a.CH);
+      const int q = (CL * qp + rank) * BM + r;
+      const int id0 = p0 * HN;  // base id of offset 0 (MODE_FILTER scans every tile; n < 2^31)
+      float tau = INFINITY;
+      if (MODE == MODE_FILTER && q < a.nq) tau = a.tau ? a.tau[q] : -INFINITY;
+      auto flush = [&] {
+        if (at > at0)
+          h_flush(a.cnt + q, a.cand + (int64_t)q * a.cap, a.cap, at0, (int)((at - at0) / (BM * 4u)), id0);
+        at = at0;
+        __syncwarp();
+      };
+      for (int p = p0; p < p1; ++p) {
+        const int b = ia & 1, ub = ia >> 1;
+        // warp-uniform, so that a warp which gives up leaves its votes together
+        if (!mbar_wait_warp(ACC_FULL(b), ub & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        uint32_t v[HW];
+        tmem_ld56(tbase + (uint32_t)(b * H_ACC_COL), v);
+        tmem_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ACC_EMPTY(b));  // scores are in registers: the MMA may reuse the buffer
+        ++ia;
+        const int64_t cbase = (int64_t)p * a.dstride * HN + g * HW;  // base id of v[0]
+        if (cbase + HW > a.n) {  // last base tile: padding rows become NaN, which no maximum or compare takes
+#pragma unroll
+          for (int j = 0; j < HW; ++j)
+            if (cbase + j >= a.n) v[j] = 0x7fc00000u;
+        }
+        float m[7];
+#pragma unroll
+        for (int gg = 0; gg < 7; ++gg) m[gg] = max8(v, gg);
+        const float tm = max3f(max3f(m[0], m[1], m[2]), max3f(m[3], m[4], m[5]), m[6]);
+        if (MODE == MODE_GROUPMAX) {
+          const int piece = 4 * p + g;
+          if (q < a.nq) {  // a group of padding only is NaN: stored as -inf, not a score
+            if (GW == HW) {
+              a.gmax[(int64_t)q * a.M + piece] = fmaxf(tm, -INFINITY);
+            } else {  // 7 groups and an empty slot: rows of 16-byte stores
+              float4* dst = reinterpret_cast<float4*>(a.gmax + (int64_t)q * a.M + 8 * piece);
+              dst[0] = make_float4(fmaxf(m[0], -INFINITY), fmaxf(m[1], -INFINITY), fmaxf(m[2], -INFINITY),
+                                   fmaxf(m[3], -INFINITY));
+              dst[1] = make_float4(fmaxf(m[4], -INFINITY), fmaxf(m[5], -INFINITY), fmaxf(m[6], -INFINITY), -INFINITY);
+            }
+          }
+        } else if (__any_sync(0xffffffffu, tm >= tau)) {
+          const uint32_t off = (uint32_t)((p - p0) * HN + g * HW);
+#pragma unroll
+          for (int gg = 0; gg < 7; ++gg) {
+            if (!__any_sync(0xffffffffu, m[gg] >= tau)) continue;
+#pragma unroll
+            for (int h = 0; h < 8; h += GRP) {
+              if (__any_sync(0xffffffffu, at > at_lim)) flush();
+#pragma unroll
+              for (int jj = h; jj < h + GRP; ++jj) h_push(v[8 * gg + jj], tau, at, off + (uint32_t)(8 * gg + jj));
+            }
+          }
+        }
+      }
+      if (MODE == MODE_FILTER) flush();  // the next unit is another query tile
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 2) {
+    tc_fence_after();
+    tmem_dealloc(tmem, H_TMEM_COLS);
+  }
+  if (threadIdx.x == 0 && *abort_flag) atomicExch(a.err, 2);
+  if (CL > 1) cluster_sync();  // no CTA leaves while its peer may still write into it
+}
+
+// ---- projections kernel (tc_signs_kernel) -------------------------------------------------
+// Shared-memory layout for split-BF16 rows of KC chunks.
+template <int KC>
+struct PLayout {
+  static constexpr int A_BYTES = KC * BM * H_CHUNK;  // resident point tile
+  static constexpr int B_BYTES = PN * H_CHUNK;       // one chunk of a plane tile: 32 KB
+  static constexpr int STAGES = KC <= 4 ? 4 : 3;
+  static constexpr int A_OFF = 0;
+  static constexpr int B_OFF = A_BYTES;
+  static constexpr int BAR_OFF = B_OFF + STAGES * B_BYTES;
+  static constexpr int SMEM = BAR_OFF + 256 + 1024;  // + barriers + alignment slack
+  static_assert(SMEM <= kSmemLimit, "shared memory per CTA");
+  static_assert(8 * (2 * STAGES + 2 + 2 * P_NACC + 1) + 12 <= 256, "barrier area");
+};
+
+struct SignArgs {
+  int n;            // points
+  int QT;           // point tiles
+  int NP;           // plane tiles
+  int CH;           // plane tiles a unit
+  int NCH;          // chunks of them
+  const float* rown;   // point norms
+  const float* pnorm;  // plane norms (padded to whole tiles with zeros)
+  float band;          // a sign is certain when |score| > band * |x| * |r|
+  uint32_t* out32;     // [n][words] sign bits
+  int words, P;        // words a point, planes (32 * words)
+  uint2* list;         // [grid][list_cap] (point, plane) of the uncertain signs, a segment a CTA
+  int* list_cnt;       // [grid] entries a segment (may exceed list_cap: overflow)
+  int list_cap;
+  int* err;
+};
+
+// Operands are BF16 (kind::f16, 64 elements a 128-byte chunk).
+template <int KC>
+__global__ void __launch_bounds__(H_THREADS, 1)
+    tc_signs_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+                      const SignArgs a) {
+  using LY = PLayout<KC>;
+  constexpr int STAGES = LY::STAGES;
   const int U = a.NCH * a.QT;
   if ((int)blockIdx.x >= U) return;  // no unit for this CTA: leave before any barrier or TMEM use
 
@@ -147,12 +454,12 @@ __global__ void __launch_bounds__(H_THREADS, 1)
   const uint32_t A_FULL = bar0 + 8u * (2 * STAGES);
   const uint32_t A_EMPTY = bar0 + 8u * (2 * STAGES + 1);
   auto ACC_FULL = [&](int b) { return bar0 + 8u * (2 * STAGES + 2 + b); };
-  auto ACC_EMPTY = [&](int b) { return bar0 + 8u * (2 * STAGES + 2 + H_NACC + b); };
-  const uint32_t DONE = bar0 + 8u * (2 * STAGES + 2 + 2 * H_NACC);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + LY::BAR_OFF + 8 * (2 * STAGES + 3 + 2 * H_NACC));
+  auto ACC_EMPTY = [&](int b) { return bar0 + 8u * (2 * STAGES + 2 + P_NACC + b); };
+  const uint32_t DONE = bar0 + 8u * (2 * STAGES + 2 + 2 * P_NACC);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + LY::BAR_OFF + 8 * (2 * STAGES + 3 + 2 * P_NACC));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform for the compiler too
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -162,13 +469,13 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     }
     mbar_init(A_FULL, 1);
     mbar_init(A_EMPTY, 1);
-    for (int b = 0; b < H_NACC; ++b) {
+    for (int b = 0; b < P_NACC; ++b) {
       mbar_init(ACC_FULL(b), 1);
       mbar_init(ACC_EMPTY(b), H_EPI_WARPS);
     }
     mbar_init(DONE, 1);
     *abort_flag = 0;
-    *reinterpret_cast<int*>(tmem_slot + 2) = 0;  // MODE_SIGNS list count
+    *reinterpret_cast<int*>(tmem_slot + 2) = 0;  // list count
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) tmem_alloc(smem_u32(tmem_slot), H_TMEM_COLS);
@@ -204,7 +511,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
           const int st = it % STAGES, rd = it / STAGES;
           if (!mbar_wait(EMPTY(st), (rd & 1) ^ 1, abort_flag)) { ok = false; break; }
           mbar_expect_tx(FULL(st), LY::B_BYTES);
-          tma_load_2d(s0 + LY::B_OFF + st * LY::B_BYTES, &mapB, kc * H_CHUNK, p * a.dstride * HN, FULL(st));
+          tma_load_2d(s0 + LY::B_OFF + st * LY::B_BYTES, &mapB, kc * H_CHUNK, p * PN, FULL(st));
           ++it;
         }
       }
@@ -215,46 +522,43 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = BF ? idesc_bf16(BM, HN) : idesc_e4m3(BM, HN);
+    {
+      const uint32_t leader = elect_one();  // the warp stays converged (see elect_one)
+      constexpr uint32_t idesc = idesc_bf16(BM, PN);
       int it = 0, ia = 0, ua = 0;
       bool ok = true;
       for (int u = blockIdx.x; u < U && ok; u += gridDim.x, ++ua) {
         const int c = u / a.QT;
         const int p0 = c * a.CH, p1 = min(a.NP, p0 + a.CH);
-        if (!mbar_wait(A_FULL, ua & 1, abort_flag)) break;
+        if (!mbar_wait_warp(A_FULL, ua & 1, abort_flag)) break;
         tc_fence_after();
         for (int p = p0; p < p1 && ok; ++p) {
-          const int b = ia % H_NACC, ub = ia / H_NACC;
-          if (!mbar_wait(ACC_EMPTY(b), (ub & 1) ^ 1, abort_flag)) { ok = false; break; }
+          const int b = ia % P_NACC, ub = ia / P_NACC;
+          if (!mbar_wait_warp(ACC_EMPTY(b), (ub & 1) ^ 1, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t d_tmem = tmem + (uint32_t)(b * HN);
+          const uint32_t d_tmem = tmem + (uint32_t)(b * PN);
           for (int kc = 0; kc < KC; ++kc) {
             const int st = it % STAGES, rd = it / STAGES;
-            if (!mbar_wait(FULL(st), rd & 1, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_warp(FULL(st), rd & 1, abort_flag)) { ok = false; break; }
             tc_fence_after();
             const uint32_t a_base = s0 + LY::A_OFF + kc * BM * H_CHUNK;
             const uint32_t b_base = s0 + LY::B_OFF + st * LY::B_BYTES;
 #pragma unroll
-            for (int kk = 0; kk < H_CHUNK / 32; ++kk) {  // 32 bytes a step: K = 32 E4M3 or 16 BF16
-              if (BF)
-                umma_bf16(d_tmem, smem_desc(a_base + kk * 32), smem_desc(b_base + kk * 32), idesc,
-                          (kc > 0 || kk > 0) ? 1u : 0u);
-              else
-                umma_e4m3(d_tmem, smem_desc(a_base + kk * 32), smem_desc(b_base + kk * 32), idesc,
-                          (kc > 0 || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < H_CHUNK / 32; ++kk) {  // 32 bytes a step: K = 16
+              umma_bf16(d_tmem, smem_desc(a_base + kk * 32), smem_desc(b_base + kk * 32), idesc,
+                        (kc > 0 || kk > 0) ? 1u : 0u, leader);
             }
-            umma_commit(EMPTY(st));
+            umma_commit(EMPTY(st), leader);
             ++it;
           }
           if (!ok) break;
-          umma_commit(ACC_FULL(b));
+          umma_commit(ACC_FULL(b), leader);
           ++ia;
         }
-        umma_commit(A_EMPTY);  // the query tile is free once this unit's MMAs complete
+        umma_commit(A_EMPTY, leader);  // the query tile is free once this unit's MMAs complete
       }
       // drain: all issued MMAs complete before TMEM is released
-      umma_commit(DONE);
+      umma_commit(DONE, leader);
       mbar_wait(DONE, 0, abort_flag, true);
     }
     __syncwarp();
@@ -263,36 +567,30 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     const int g = (warp - 4) >> 2;         // warpgroup: columns [64g, 64g+64) of every accumulator
     const int r = (warp & 3) * 32 + lane;  // query row within the tile = TMEM lane
     const uint32_t tbase = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g * 64);
-    float* ssc = reinterpret_cast<float*>(sm + LY::S_OFF) + (size_t)g * SBUF * BM + r;
-    int* sid = reinterpret_cast<int*>(sm + LY::S_OFF + 4 * SBUF * BM * 4) + (size_t)g * SBUF * BM + r;
-    int scnt = 0;
     int ia = 0;
     bool ok = true;
-    int* seg_cnt = reinterpret_cast<int*>(tmem_slot + 2);  // MODE_SIGNS: this CTA's list count
-    uint2* seg = MODE == MODE_SIGNS ? a.list + (int64_t)blockIdx.x * a.list_cap : nullptr;
+    int* seg_cnt = reinterpret_cast<int*>(tmem_slot + 2);  // this CTA's list count
+    uint2* seg = a.list + (int64_t)blockIdx.x * a.list_cap;
     for (int u = blockIdx.x; u < U && ok; u += gridDim.x) {
       const int qt = u % a.QT, c = u / a.QT;
       const int p0 = c * a.CH, p1 = min(a.NP, p0 + a.CH);
       const int q = qt * BM + r;
-      float tau = INFINITY;
-      if (MODE == MODE_FILTER && q < a.nq) tau = a.tau ? a.tau[q] : -INFINITY;
       for (int p = p0; p < p1; ++p) {
-        const int b = ia % H_NACC, ub = ia / H_NACC;
+        const int b = ia % P_NACC, ub = ia / P_NACC;
         if (!mbar_wait(ACC_FULL(b), ub & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         uint32_t v[64];
-        tmem_ld64(tbase + (uint32_t)(b * HN), v);
+        tmem_ld64(tbase + (uint32_t)(b * PN), v);
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(ACC_EMPTY(b));  // scores are in registers: the MMA may reuse the buffer
         ++ia;
-        const int64_t cbase = (int64_t)p * a.dstride * HN + g * 64;  // base id of v[0]
-        const int piece = 4 * p + g;
-        if (MODE == MODE_SIGNS) {
+        const int cbase = p * PN + g * 64;  // plane of v[0]
+        {
           // bit = score >= 0, as the reference's sign test; a sign within the split-BF16
           // error bound of zero is listed for the exact recheck
-          if (q < a.nq && cbase < a.P) {
+          if (q < a.n && cbase < a.P) {
             const float bx = a.band * a.rown[q];
             const float4* pn4 = reinterpret_cast<const float4*>(a.pnorm + cbase);
             uint32_t w0 = 0, w1 = 0;
@@ -317,75 +615,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             row[0] = w0;
             if (cbase + 32 < a.P) row[1] = w1;
           }
-        } else if (MODE == MODE_GROUPMAX) {
-          if (cbase + 64 > a.n) {  // last base tile: padding rows are not points
-#pragma unroll
-            for (int j = 0; j < 64; ++j)
-              if (cbase + j >= a.n) v[j] = __float_as_uint(-INFINITY);
-          }
-          if (q < a.nq) {
-            if (GW == 64) {
-              float m[8];
-#pragma unroll
-              for (int gg = 0; gg < 8; ++gg) m[gg] = max8(v, gg);
-              a.gmax[(int64_t)q * a.M + piece] =
-                  max3f(max3f(m[0], m[1], m[2]), max3f(m[3], m[4], m[5]), fmaxf(m[6], m[7]));
-            } else {
-              float4 lo, hi;
-              lo.x = max8(v, 0); lo.y = max8(v, 1); lo.z = max8(v, 2); lo.w = max8(v, 3);
-              hi.x = max8(v, 4); hi.y = max8(v, 5); hi.z = max8(v, 6); hi.w = max8(v, 7);
-              float4* dst = reinterpret_cast<float4*>(a.gmax + (int64_t)q * a.M + 8 * piece);
-              dst[0] = lo;
-              dst[1] = hi;
-            }
-          }
-        } else {
-          if (cbase + 64 > a.n) {  // padding rows become NaN, which never passes
-#pragma unroll
-            for (int j = 0; j < 64; ++j)
-              if (cbase + j >= a.n) v[j] = 0x7fc00000u;
-          }
-          float m[8];
-#pragma unroll
-          for (int gg = 0; gg < 8; ++gg) m[gg] = max8(v, gg);
-          const float tm = max3f(max3f(m[0], m[1], m[2]), max3f(m[3], m[4], m[5]), fmaxf(m[6], m[7]));
-          if (__any_sync(0xffffffffu, tm >= tau)) {
-            const int ibase = (int)cbase;  // ids fit in 32 bits (n < 2^31)
-            int* qcnt = a.cnt + q;
-            uint64_t* qdst = a.cand + (int64_t)q * a.cap;
-#pragma unroll
-            for (int gg = 0; gg < 8; ++gg) {
-              if (!__any_sync(0xffffffffu, m[gg] >= tau)) continue;
-              if (SBUF > 0) {
-                int ng = 0;
-#pragma unroll
-                for (int jj = 0; jj < 8; ++jj) ng += __uint_as_float(v[8 * gg + jj]) >= tau ? 1 : 0;
-                if (scnt + ng > SBUF) {
-                  h_flush(qcnt, qdst, a.cap, ssc, sid, scnt);
-                  scnt = 0;
-                }
-              }
-#pragma unroll
-              for (int jj = 0; jj < 8; ++jj) {
-                const float sc = __uint_as_float(v[8 * gg + jj]);
-                if (sc >= tau) {
-                  if (SBUF >= 8 || (SBUF > 0 && scnt < SBUF)) {  // 8 entries always fit after a flush
-                    ssc[scnt * BM] = sc;
-                    sid[scnt * BM] = ibase + 8 * gg + jj;
-                    ++scnt;
-                  } else {  // no staging room: a slot of its own
-                    const int pos = atomicAdd(qcnt, 1);
-                    if (pos < a.cap) qdst[pos] = make_key(-sc, ibase + 8 * gg + jj);
-                  }
-                }
-              }
-            }
-          }
         }
-      }
-      if (MODE == MODE_FILTER && SBUF > 0 && scnt > 0) {  // the next unit is another query tile
-        h_flush(a.cnt + q, a.cand + (int64_t)q * a.cap, a.cap, ssc, sid, scnt);
-        scnt = 0;
       }
     }
   }
@@ -397,30 +627,30 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     tmem_dealloc(tmem, H_TMEM_COLS);
   }
   if (threadIdx.x == 0 && *abort_flag) atomicExch(a.err, 2);
-  if (MODE == MODE_SIGNS && threadIdx.x == 0) a.list_cnt[blockIdx.x] = *reinterpret_cast<int*>(tmem_slot + 2);
+  if (threadIdx.x == 0) a.list_cnt[blockIdx.x] = *reinterpret_cast<int*>(tmem_slot + 2);
 }
 
-// Sketch rows of wp words (the first `words` real) -> E4M3 rows of kp bytes: bit b of word w
-// (LSB first) -> byte 32w + b = 0x38 (+1) for a 0 bit, 0xB8 (-1) for a 1 bit; bytes past
-// 32 * words and rows past n are 0x00.  One thread writes 16 bytes (half a word).
+// Sketch rows of wp words (the first `words` real) -> E2M1 rows of kp bytes: bit b of word w
+// (LSB first) -> nibble 32w + b (low nibble first) = 0x2 (+1) for a 0 bit, 0xA (-1) for a 1
+// bit; nibbles past 32 * words and rows past n are 0x0.  One thread writes a word's 16 bytes.
 __global__ void expand_bits_kernel(const uint32_t* __restrict__ xs, int64_t n, int wp, int words, int kp,
                                    int64_t rows_pad, uint4* __restrict__ out) {
   const int per_row = kp / 16;
   const int64_t total = rows_pad * per_row;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = t / per_row;
-    const int h = (int)(t - i * per_row);  // 16-byte piece of the row: bits 16h .. 16h + 15
-    const int w = h >> 1;
+    const int w = (int)(t - i * per_row);
     uint4 o = make_uint4(0, 0, 0, 0);
     if (i < n && w < words) {
-      const uint32_t bits = xs[i * wp + w] >> (16 * (h & 1));
+      const uint32_t bits = xs[i * wp + w];
       uint32_t r[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const uint32_t nib = (bits >> (4 * e)) & 0xFu;
-        // bit j of the nibble -> bit 7 of byte j (the sign of +-1.0)
-        const uint32_t spread = (nib & 1u) << 7 | (nib & 2u) << 14 | (nib & 4u) << 21 | (nib & 8u) << 28;
-        r[e] = 0x38383838u | spread;
+        uint32_t b = (bits >> (8 * e)) & 0xFFu;  // bit j of the byte -> bit 3 of nibble j (the sign of +-1.0)
+        b = (b | (b << 12)) & 0x000F000Fu;
+        b = (b | (b << 6)) & 0x03030303u;
+        b = (b | (b << 3)) & 0x11111111u;
+        r[e] = 0x22222222u | (b << 3);
       }
       o = make_uint4(r[0], r[1], r[2], r[3]);
     }
@@ -557,39 +787,67 @@ CUtensorMap map_sketch_rows(const void* base, int64_t rows, int kp, int box_rows
   return make_map_bytes(base, rows, kp, box_rows);
 }
 
-template <int MODE, int GW, int KC, bool BF = false>
-void run_hamming(const CUtensorMap& ma, const CUtensorMap& mb, HArgs a, const char* name, cudaStream_t s,
-                 int* grid_out = nullptr) {
+template <int MODE, int GW, int KC, int CL>
+void run_hamming(const CUtensorMap& ma, const CUtensorMap& mb, HArgs a, const char* name, cudaStream_t s) {
+  // units: long enough to amortise the query tile's reload, at least 8 a cluster
+  const int G = std::max(1, num_sms() / CL);
+  a.QP = ceil_div(a.QT, CL);
+  const int64_t work = (int64_t)a.NP * a.QP;
+  a.CH = (int)std::max<int64_t>(1, std::min<int64_t>(H_MAX_CH, (work + 8 * G - 1) / (8 * G)));
+  a.NCH = ceil_div(a.NP, a.CH);
+  const int grid = CL * std::min(G, a.NCH * a.QP);
+  auto kern = tc_hamming_kernel<MODE, GW, KC, CL>;
+  constexpr int smem = HLayout<KC>::SMEM;
+  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(H_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = CL;
+  at.val.clusterDim.y = 1;
+  at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = CL > 1 ? 1 : 0;
+  ProfScope _ps(name, s);
+  LSHG_CUDA(cudaLaunchKernelEx(&cfg, kern, ma, mb, a));
+  count_launch();
+}
+
+// cl: CTAs a cluster; mb's boxes hold a CTA's share of a base tile (HN / cl rows).
+template <int MODE, int GW>
+void run_hamming_kc(int kc, int cl, const CUtensorMap& ma, const CUtensorMap& mb, const HArgs& a, const char* name,
+                    cudaStream_t s) {
+  switch (kc * 2 + (cl - 1)) {
+    case 2: run_hamming<MODE, GW, 1, 1>(ma, mb, a, name, s); break;
+    case 3: run_hamming<MODE, GW, 1, 2>(ma, mb, a, name, s); break;
+    case 4: run_hamming<MODE, GW, 2, 1>(ma, mb, a, name, s); break;
+    case 5: run_hamming<MODE, GW, 2, 2>(ma, mb, a, name, s); break;
+    case 6: run_hamming<MODE, GW, 3, 1>(ma, mb, a, name, s); break;
+    case 7: run_hamming<MODE, GW, 3, 2>(ma, mb, a, name, s); break;
+    case 8: run_hamming<MODE, GW, 4, 1>(ma, mb, a, name, s); break;
+    case 9: run_hamming<MODE, GW, 4, 2>(ma, mb, a, name, s); break;
+    default: throw Error(LSHG_ERR_INVALID_ARGUMENT, "tensor-core sketch scan: rows of 1..4 chunks of 256 bits");
+  }
+}
+
+template <int KC>
+void run_signs(const CUtensorMap& ma, const CUtensorMap& mb, SignArgs a, cudaStream_t s, int* grid_out) {
   const int G = num_sms();
   const int64_t work = (int64_t)a.NP * a.QT;
   a.CH = (int)std::max<int64_t>(1, std::min<int64_t>(32, (work + 8 * G - 1) / (8 * G)));
   a.NCH = ceil_div(a.NP, a.CH);
-  const int U = a.NCH * a.QT;
-  const int grid = std::min(G, U);
-  if (grid_out) *grid_out = grid;
-  auto kern = tc_hamming_kernel<MODE, GW, KC, BF>;
-  constexpr int smem = HLayout<KC>::SMEM;
+  const int grid = std::min(G, a.NCH * a.QT);
+  *grid_out = grid;
+  auto kern = tc_signs_kernel<KC>;
+  constexpr int smem = PLayout<KC>::SMEM;
   LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  ProfScope _ps(name, s);
+  ProfScope _ps("tc_project_gemm", s);
   kern<<<grid, H_THREADS, smem, s>>>(ma, mb, a);
   count_launch();
   LSHG_CHECK_LAUNCH();
-}
-
-template <int MODE, int GW>
-void run_hamming_kc(int kc, const CUtensorMap& ma, const CUtensorMap& mb, const HArgs& a, const char* name,
-                    cudaStream_t s) {
-  switch (kc) {
-    case 1: run_hamming<MODE, GW, 1>(ma, mb, a, name, s); break;
-    case 2: run_hamming<MODE, GW, 2>(ma, mb, a, name, s); break;
-    case 3: run_hamming<MODE, GW, 3>(ma, mb, a, name, s); break;
-    case 4: run_hamming<MODE, GW, 4>(ma, mb, a, name, s); break;
-    case 5: run_hamming<MODE, GW, 5>(ma, mb, a, name, s); break;
-    case 6: run_hamming<MODE, GW, 6>(ma, mb, a, name, s); break;
-    case 7: run_hamming<MODE, GW, 7>(ma, mb, a, name, s); break;
-    case 8: run_hamming<MODE, GW, 8>(ma, mb, a, name, s); break;
-    default: throw Error(LSHG_ERR_INVALID_ARGUMENT, "tensor-core sketch scan: rows of 1..8 chunks of 128 bits");
-  }
 }
 
 // ---- SimHash projections on the tensor cores ---------------------------------------------
@@ -665,14 +923,14 @@ void launch_tc_signs(const float* x, int64_t n, int d, const uint16_t* planes_sp
   LSHG_REQUIRE(P == 32 * words && P >= 32, "tensor-core projections: whole 32-plane words");
   const int kp = signs_part_cols(d), kc = 3 * kp * 2 / H_CHUNK;
   const int64_t rows_pad = (int64_t)ceil_div(n, BM) * BM;
-  const int64_t ppad = (int64_t)ceil_div(P, HN) * HN;
-  LSHG_REQUIRE(rows_pad / BM * (ppad / HN) < (int64_t)INT_MAX, "tensor-core projections: problem too large");
+  const int64_t ppad = (int64_t)ceil_div(P, PN) * PN;
+  LSHG_REQUIRE(rows_pad / BM * (ppad / PN) < (int64_t)INT_MAX, "tensor-core projections: problem too large");
   ProfScope _ps("tc_project", s);
   DevBuf<uint16_t> xa((size_t)rows_pad * 3 * kp, s);
   DevBuf<float> xn((size_t)rows_pad, s);
   launch_split_bf16(x, n, d, rows_pad, 0, xa.ptr, xn.ptr, s);
   const CUtensorMap ma = map_sketch_rows(xa.ptr, rows_pad, 6 * kp, BM);
-  const CUtensorMap mb = map_sketch_rows(planes_split, ppad, 6 * kp, HN);
+  const CUtensorMap mb = map_sketch_rows(planes_split, ppad, 6 * kp, PN);
   // about 0.1% of the signs of unit points and N(0, 1) planes fall inside the band; each
   // CTA's segment holds 4x its share, and the SIMT projection redoes everything if one
   // overflows
@@ -682,12 +940,10 @@ void launch_tc_signs(const float* x, int64_t n, int d, const uint16_t* planes_sp
   DevBuf<uint2> list((size_t)G * cap, s);
   DevBuf<int> cnt((size_t)G + 1, s);
   LSHG_CUDA(cudaMemsetAsync(cnt.ptr, 0, cnt.bytes(), s));
-  HArgs a{};
-  a.nq = (int)n;
-  a.n = P;
+  SignArgs a{};
+  a.n = (int)n;
   a.QT = (int)(rows_pad / BM);
-  a.NP = (int)(ppad / HN);
-  a.dstride = 1;
+  a.NP = (int)(ppad / PN);
   a.err = err;
   a.rown = xn.ptr;
   a.pnorm = pnorm;
@@ -699,8 +955,8 @@ void launch_tc_signs(const float* x, int64_t n, int d, const uint16_t* planes_sp
   a.list_cnt = cnt.ptr;
   a.list_cap = cap;
   int grid = 0;
-  if (kc == 3) run_hamming<MODE_SIGNS, 64, 3, true>(ma, mb, a, "tc_project_gemm", s, &grid);
-  else run_hamming<MODE_SIGNS, 64, 6, true>(ma, mb, a, "tc_project_gemm", s, &grid);
+  if (kc == 3) run_signs<3>(ma, mb, a, s, &grid);
+  else run_signs<6>(ma, mb, a, s, &grid);
   int* overflow = cnt.ptr + G;
   {
     const int64_t total = (int64_t)grid * cap;
@@ -732,13 +988,14 @@ HammingPlan plan_hamming(int64_t n, int C) {
     const int NS = ceil_div(NT, S);
     const double m = (double)C / S;
     const int r = S == 1 ? C : std::min(C, (int)std::ceil(m + 4.0 * std::sqrt(m) + 8.0));
-    for (int GW : {64, 8}) {
-      const int64_t M = (int64_t)NS * (HN / GW);
-      if (M >= 4 * (int64_t)r) {
+    for (int GW : {HW, 8}) {
+      const int64_t M = (int64_t)NS * (HN / GW);  // maxima
+      // about 4 r of them (28 short: a base keeps its plan when its tiles round differently)
+      if (M + 28 >= 4 * (int64_t)r) {
         p.S = S;
         p.NS = NS;
         p.GW = GW;
-        p.M = (int)M;
+        p.M = GW == HW ? (int)M : NS * 32;  // slots a row: 8-point groups are stored 8 a piece, 7 used
         p.rank = r;
         const int64_t want = 3 * (int64_t)r * S + 2048;
         int64_t cap = 1024;
@@ -754,7 +1011,8 @@ HammingPlan plan_hamming(int64_t n, int C) {
   return p;
 }
 
-int hamming_chunks(int words) { return (words + 3) / 4; }
+int hamming_chunks(int words) { return (words + 7) / 8; }
+int64_t hamming_rows(int64_t n) { return (int64_t)ceil_div(n, HN) * HN; }
 
 void launch_expand_bits(const uint32_t* xs, int64_t n, int wp, int words, int64_t rows_pad, uint8_t* out,
                         cudaStream_t s) {
@@ -790,7 +1048,7 @@ void launch_tc_hamming(const uint8_t* xse, int64_t n, const uint32_t* xst, int w
   const int kc = hamming_chunks(words), kp = kc * H_CHUNK;
   const int64_t qpad = (int64_t)ceil_div(nq, BM) * BM;
   const int QT = (int)(qpad / BM);
-  const int64_t npad = (int64_t)ceil_div(n, HN) * HN;
+  const int64_t npad = hamming_rows(n);
   const HammingPlan plan = plan_hamming(n, C);
   LSHG_REQUIRE(plan.ok, "tensor-core sketch scan: C too large for this base");
   LSHG_REQUIRE((int64_t)QT * plan.NT < (int64_t)INT_MAX, "tensor-core sketch scan: problem too large");
@@ -800,11 +1058,15 @@ void launch_tc_hamming(const uint8_t* xse, int64_t n, const uint32_t* xst, int w
     launch_expand_bits(qs, nq, wp, words, qpad, qe.ptr, s);
   }
   const CUtensorMap ma = map_sketch_rows(qe.ptr, qpad, kp, BM);
-  const CUtensorMap mb = map_sketch_rows(xse, npad, kp, HN);
+  // clusters of two query tiles share each base tile's fetch; one tile alone would leave the
+  // second CTA without work
+  const int cl = QT > 1 ? 2 : 1;
+  const CUtensorMap mb = map_sketch_rows(xse, npad, kp, HN / cl);
   HArgs a{};
   a.nq = nq;
   a.n = n;
   a.QT = QT;
+  a.ksteps = (words + 1) / 2;
   a.err = err;
   DevBuf<float> tau(nq, s);
   if (plan.M > 0) {
@@ -813,8 +1075,8 @@ void launch_tc_hamming(const uint8_t* xse, int64_t n, const uint32_t* xst, int w
     a.dstride = plan.S;
     a.gmax = gmax.ptr;
     a.M = plan.M;
-    if (plan.GW == 64) run_hamming_kc<MODE_GROUPMAX, 64>(kc, ma, mb, a, "tc_hamming_prepass", s);
-    else run_hamming_kc<MODE_GROUPMAX, 8>(kc, ma, mb, a, "tc_hamming_prepass", s);
+    if (plan.GW == HW) run_hamming_kc<MODE_GROUPMAX, HW>(kc, cl, ma, mb, a, "tc_hamming_prepass", s);
+    else run_hamming_kc<MODE_GROUPMAX, 8>(kc, cl, ma, mb, a, "tc_hamming_prepass", s);
     // scores are integers, computed the same way in both passes: no margin
     launch_tau_select(gmax.ptr, nq, plan.M, plan.rank, 0.0f, tau.ptr, s);
   }
@@ -829,7 +1091,7 @@ void launch_tc_hamming(const uint8_t* xse, int64_t n, const uint32_t* xst, int w
   a.cnt = cnt.ptr;
   a.cand = cand.ptr;
   a.cap = plan.cap;
-  run_hamming_kc<MODE_FILTER, 64>(kc, ma, mb, a, "tc_hamming", s);
+  run_hamming_kc<MODE_FILTER, HW>(kc, cl, ma, mb, a, "tc_hamming", s);
   DevBuf<int> ovf((size_t)nq + 1, s);
   LSHG_CUDA(cudaMemsetAsync(ovf.ptr, 0, sizeof(int), s));
   launch_int_select(cnt.ptr, cand.ptr, plan.cap, (int)std::min<int64_t>(C, n), C, 32 * words, nq, out, ovf.ptr, s);

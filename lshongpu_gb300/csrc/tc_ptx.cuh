@@ -77,6 +77,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return mbar_wait_slow(bar, parity, abort_flag, ignore_abort);
 }
 
+// The same wait by a converged warp; its outcome is the warp's.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
 // 1-D bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) from global
 // into this CTA's shared memory, completion counted in bytes on `bar`.
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -94,6 +99,28 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
+// The same load into every CTA of the cluster whose bit is set in `mask`: data and byte count
+// arrive at the same offsets (dst, bar) of each.
+__device__ __forceinline__ void tma_load_2d_multicast(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar,
+                                                      uint16_t mask) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1, "
+      "{%2, %3}], [%4], %5;" ::"r"(dst),
+      "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar), "h"(mask)
+      : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// Every thread of the cluster; orders shared-memory writes before it (barrier inits) and
+// keeps a CTA alive until its peers are done with its shared memory.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 B apart.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
   return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
@@ -105,12 +132,23 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// MMAs and their commits are issued by one thread of a warp that stays converged: `leader`
+// is the thread that elect_one() picked, and the instructions carry it as a predicate.
+// Inside an `if (lane == 0)` the compiler cannot keep descriptors in uniform registers, and
+// the instruction takes nothing else: moving them there cost 72 to 85 cycles an MMA and 50 a
+// commit (measured, of 112 to 128 that the MMA itself takes, and not overlapped with the
+// waits in between), against 30 and 12 this way.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t l;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(l));
+  return l;
+}
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
-                                          uint32_t accumulate) {
+                                          uint32_t accumulate, uint32_t leader) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(
-          tmem_d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, l;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 l, %5, 0;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
 // One 128 x N x (16 * ksteps) product; A is a 128-row tile and B an N-row tile, both
@@ -118,28 +156,30 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t 
 // zero beyond the data dimension d, so ksteps = ceil(d / 16) gives the same FP32 sums as
 // all eight steps (the skipped steps would add exact zeros).
 template <int N>
-__device__ __forceinline__ void umma_tile(uint32_t d_tmem, uint32_t a_base, uint32_t b_base, int ksteps) {
+__device__ __forceinline__ void umma_tile(uint32_t d_tmem, uint32_t a_base, uint32_t b_base, int ksteps,
+                                          uint32_t leader) {
   constexpr uint32_t idesc = idesc_bf16(BM, N);
 #pragma unroll
   for (int kk = 0; kk < KD / 16; ++kk) {
     if (kk < ksteps) {
       const uint32_t koff = (kk & 3) * 32;
       umma_bf16(d_tmem, smem_desc(a_base + (kk >> 2) * HALF_BYTES + koff),
-                smem_desc(b_base + (kk >> 2) * (N * 128) + koff), idesc, kk > 0 ? 1u : 0u);
+                smem_desc(b_base + (kk >> 2) * (N * 128) + koff), idesc, kk > 0 ? 1u : 0u, leader);
     }
   }
 }
 // K steps [k0, k1) of umma_tile: a tile's MMAs issued in pieces, each after its own part
 // of the operands has landed.  Step 0 clears the accumulator.
 template <int N>
-__device__ __forceinline__ void umma_steps(uint32_t d_tmem, uint32_t a_base, uint32_t b_base, int k0, int k1) {
+__device__ __forceinline__ void umma_steps(uint32_t d_tmem, uint32_t a_base, uint32_t b_base, int k0, int k1,
+                                           uint32_t leader) {
   constexpr uint32_t idesc = idesc_bf16(BM, N);
 #pragma unroll
   for (int kk = 0; kk < KD / 16; ++kk) {
     if (kk >= k0 && kk < k1) {
       const uint32_t koff = (kk & 3) * 32;
       umma_bf16(d_tmem, smem_desc(a_base + (kk >> 2) * HALF_BYTES + koff),
-                smem_desc(b_base + (kk >> 2) * (N * 128) + koff), idesc, kk > 0 ? 1u : 0u);
+                smem_desc(b_base + (kk >> 2) * (N * 128) + koff), idesc, kk > 0 ? 1u : 0u, leader);
     }
   }
 }
@@ -151,24 +191,25 @@ __host__ __device__ constexpr uint32_t idesc_e4m3(int M, int N) {
   return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 __device__ __forceinline__ void umma_e4m3(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
-                                          uint32_t accumulate) {
+                                          uint32_t accumulate, uint32_t leader) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(
-          tmem_d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, l;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 l, %5, 0;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
 // One 128 x N x (32 * ksteps) E4M3 product: each step advances 32 bytes (K = 32) along the
 // single 128-byte row of A (128-row tile) and B (N-row tile); as with BF16, rows are zero
 // past d, so ksteps = ceil(d / 32) gives the same sums as all four steps.
 template <int N>
-__device__ __forceinline__ void umma_tile_e4m3(uint32_t d_tmem, uint32_t a_base, uint32_t b_base, int ksteps) {
+__device__ __forceinline__ void umma_tile_e4m3(uint32_t d_tmem, uint32_t a_base, uint32_t b_base, int ksteps,
+                                               uint32_t leader) {
   constexpr uint32_t idesc = idesc_e4m3(BM, N);
 #pragma unroll
   for (int kk = 0; kk < KD / 32; ++kk) {
     if (kk < ksteps) {
       const uint32_t koff = kk * 32;
-      umma_e4m3(d_tmem, smem_desc(a_base + koff), smem_desc(b_base + koff), idesc, kk > 0 ? 1u : 0u);
+      umma_e4m3(d_tmem, smem_desc(a_base + koff), smem_desc(b_base + koff), idesc, kk > 0 ? 1u : 0u, leader);
     }
   }
 }
@@ -176,8 +217,43 @@ __host__ __device__ inline int tc_ksteps_e4m3(int d) { return d <= 0 ? 1 : (d > 
 // E4M3 codes hold unit vectors times this factor: every component (|v| <= 1) stays within
 // the format's range (448) and components down to 2^-14 stay in its normal range.
 constexpr float kE4M3Scale = 256.0f;
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+
+// FP4 operands with block scales: rows of E2M1 codes, two a byte, and one UE8M0 scale a
+// 32-element block held in TMEM.  Instruction descriptor: kind::mxf4, A = B = E2M1 (format
+// 1), UE8M0 scales (bit 23), scale ids 0, dense K = 64, both K-major, M = 128 (bit 27) x N.
+__host__ __device__ constexpr uint32_t idesc_mxf4(int N) {
+  return (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | (1u << 23) | (1u << 27);
+}
+__device__ __forceinline__ void umma_mxf4(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t tmem_sf,
+                                          uint32_t accumulate, uint32_t leader) {
+  asm volatile(
+      "{\n\t.reg .pred p, l;\n\tsetp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 l, %6, 0;\n\t"
+      "@l tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%4], [%4], p;\n\t}" ::"r"(
+          tmem_d),
+      "l"(a), "l"(b), "r"(idesc), "r"(tmem_sf), "r"(accumulate), "r"(leader)
+      : "memory");
+}
+// The same 32-bit value into 8 consecutive TMEM columns of this thread's lane.
+__device__ __forceinline__ void tmem_fill8(uint32_t taddr, uint32_t v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr), "r"(v)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t leader) {
+  asm volatile(
+      "{\n\t.reg .pred l;\n\tsetp.ne.b32 l, %1, 0;\n\t"
+      "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+      "r"(leader)
+      : "memory");
+}
+// The same arrival on the barrier at this offset of every CTA in `mask`.
+__device__ __forceinline__ void umma_commit_multicast(uint32_t bar, uint16_t mask, uint32_t leader) {
+  asm volatile(
+      "{\n\t.reg .pred l;\n\tsetp.ne.b32 l, %2, 0;\n\t"
+      "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(
+          bar),
+      "h"(mask), "r"(leader)
+      : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -210,6 +286,26 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t (&r)[64]) {
       : "r"(taddr));
 }
 
+// 56 consecutive TMEM columns of this thread's lane (issue only; complete with tmem_wait_ld).
+__device__ __forceinline__ void tmem_ld56(uint32_t taddr, uint32_t (&r)[56]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+      "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]),
+        "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47])
+      : "r"(taddr + 32));
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55])
+               : "r"(taddr + 48));
+}
+
 // Three-input maximum (sm_100+ max.f32 with three sources).
 __device__ __forceinline__ float max3f(float a, float b, float c) {
   float r;
@@ -218,7 +314,8 @@ __device__ __forceinline__ float max3f(float a, float b, float c) {
 }
 
 // Maximum of the 8 consecutive scores v[8g .. 8g+7].
-__device__ __forceinline__ float max8(const uint32_t (&v)[64], int g) {
+template <int NV>
+__device__ __forceinline__ float max8(const uint32_t (&v)[NV], int g) {
   return max3f(max3f(__uint_as_float(v[8 * g]), __uint_as_float(v[8 * g + 1]), __uint_as_float(v[8 * g + 2])),
                max3f(__uint_as_float(v[8 * g + 3]), __uint_as_float(v[8 * g + 4]), __uint_as_float(v[8 * g + 5])),
                fmaxf(__uint_as_float(v[8 * g + 6]), __uint_as_float(v[8 * g + 7])));

@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 3 + 2 * NACC);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform for the compiler too
   const int lane = threadIdx.x & 31;
   const int total = QT * NT;
   const int t_begin = blockIdx.x * per;
@@ -229,31 +229,32 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    {
+      const uint32_t leader = elect_one();  // the warp stays converged (see elect_one)
       int cur_qt = -1, a_round = 0, it = 0;
       for (int t = t_begin; t < t_end; ++t) {
         const int qt = t / NT;
         if (qt != cur_qt) {
-          if (!mbar_wait(A_FULL, a_round & 1, abort_flag)) break;
+          if (!mbar_wait_warp(A_FULL, a_round & 1, abort_flag)) break;
           tc_fence_after();
           cur_qt = qt;
           ++a_round;
         }
         const int b = it % NACC, ub = it / NACC;  // ub-th use of accumulator b
-        if (!mbar_wait(ACC_EMPTY(b), (ub & 1) ^ 1, abort_flag)) break;
+        if (!mbar_wait_warp(ACC_EMPTY(b), (ub & 1) ^ 1, abort_flag)) break;
         tc_fence_after();
         const int st = it % STAGES, rd = it / STAGES;
-        if (!mbar_wait(FULL(st), rd & 1, abort_flag)) break;
+        if (!mbar_wait_warp(FULL(st), rd & 1, abort_flag)) break;
         tc_fence_after();
-        umma_tile<BN>(tmem + (uint32_t)(b * BN), s0 + L.a_off, s0 + L.b_off + st * TILE_BYTES, ksteps);
-        umma_commit(EMPTY(st));
-        umma_commit(ACC_FULL(b));
+        umma_tile<BN>(tmem + (uint32_t)(b * BN), s0 + L.a_off, s0 + L.b_off + st * TILE_BYTES, ksteps, leader);
+        umma_commit(EMPTY(st), leader);
+        umma_commit(ACC_FULL(b), leader);
         const bool last_of_qt = (t + 1 == t_end) || ((t + 1) / NT != qt);
-        if (last_of_qt) umma_commit(A_EMPTY);
+        if (last_of_qt) umma_commit(A_EMPTY, leader);
         ++it;
       }
       // drain: all issued MMAs complete before TMEM is released
-      umma_commit(DONE);
+      umma_commit(DONE, leader);
       mbar_wait(DONE, 0, abort_flag, true);
     }
     __syncwarp();

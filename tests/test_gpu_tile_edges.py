@@ -1,0 +1,36 @@
+"""Sizes at the edges of the scan kernels' tiles, on the GPU: base tiles, query tiles, K
+chunks and the selection regimes of the tensor-core scans, each against the general path
+or the CPU oracle.  Sketch distances are integers and distances are the reference's
+single-precision formula on both sides, so everything is compared for equality.
+"""
+import numpy as np
+import pytest
+
+from lshongpu_gb300 import datasets
+
+pytestmark = pytest.mark.gpu
+
+D = 100
+POPCOUNT, TENSOR = 1, 2
+
+
+def data(n, nq, d=D, seed=61, count=40):
+    return datasets.clustered(n, d, seed, count=count), datasets.clustered(nq, d, seed + 1, count=count)
+
+
+@pytest.mark.parametrize("n,nq,words,C", [
+    (224, 1, 1, 32),          # one full base tile, one query, one K step
+    (225, 128, 2, 32),        # one point in the second tile
+    (16352, 129, 8, 256),     # the largest base that keeps every point; a query tile of one row
+    (16353, 257, 9, 256),     # one more: prepass; a cluster with one query tile; a second chunk of one word
+    (50176, 384, 17, 512),    # whole tiles; 3 query tiles; 3 chunks
+    (140001, 100, 25, 4096),  # 4 chunks (the last of one word), 8-point groups, one query tile
+])
+def test_sketch_scan_edges_equal_popcount(engine, n, nq, words, C):
+    """The FP4 sketch scan (base tiles of 224 points, clusters of two 128-row query tiles,
+    chunks of 8 words) returns what the popcount scan returns."""
+    x, q = data(n, nq)
+    res = [engine.Index(x, implementation=3, sketchDim=words,
+                        options=engine.make_options(candidates=C, sketch_scan=mode)).query(q, 32)
+           for mode in (TENSOR, POPCOUNT)]
+    assert np.array_equal(res[0], res[1])
