@@ -20,19 +20,32 @@
 // e.g. duplicated points or a zero query) is listed for the exact per-row list kernel in
 // tc_scan.cu, which runs on the device-side list without a host round trip.
 //
-// Work decomposition of tc_filter_kernel: a unit is (query tile, chunk of CH consecutive
-// base positions); units are numbered chunk-major and dealt round-robin to one CTA per
-// SM.  At any moment the CTAs therefore work on the same one or two chunks for different
-// query tiles, so each base tile is read from HBM about once and served from L2 to the
-// other query tiles; the query tile of a unit is double-buffered in shared memory.
+// Work decomposition of tc_filter_kernel: persistent, one CTA per SM, in clusters of CL = 2
+// CTAs (1 for batches of one query tile).  A unit is (CL query tiles, chunk of CH consecutive
+// base positions); units are numbered chunk-major and dealt round-robin to the clusters.  At
+// any moment the clusters therefore work on the same one or two chunks for different query
+// tiles, so each base tile is read from HBM about once and served from L2.  The two CTAs of a
+// cluster are an MMA pair (tcgen05 cta_group::2): each holds a query tile of its own and half
+// of every base tile, and the even one issues the MMAs of both.  A CTA on its own would read
+// 84 KB of operands from shared memory and write 56 KB of base tile into it for the 896
+// cycles of MMA of a 128 x 256 tile at d = 100 -- 1,094 cycles at 128 bytes a cycle; in a
+// pair it is 56 + 28 KB.  A CTA keeps its query tile, and its staged survivors, when its next
+// unit has the same one.
 //
-// Tiles are 128 queries x 256 base points (tcgen05.mma M = 128, N = 256).  Warp roles (640
-// threads): warp 0 TMA producer, warp 1 MMA issuer (one elected thread), warp 2 TMEM
-// allocator (2 accumulators x 256 columns = 512), warp 3 idle, warps 4-19 the epilogue:
-// warpgroup g (warps 4+4g .. 7+4g) reads TMEM columns [64g, 64g+64) of every accumulator,
-// thread (warp & 3) * 32 + lane owns query row = TMEM lane.  Every mbarrier
-// wait is bounded; a CTA that times out raises the error flag, drains its own copies and
-// MMAs, frees TMEM and returns.
+// Tiles are 128 queries x 256 base points (tcgen05.mma M = 128, N = 256).  A row is KC chunks
+// of 128 bytes -- 64 BF16 columns (KC = 1 for d <= 64, else 2) or 128 E4M3 ones -- and a ring
+// stage one chunk of a base tile (32 KB, or a pair's 16 KB each), given back as soon as its K steps are done.  Warp
+// roles (640 threads): warp 0 TMA producer, warp 1 MMA issuer, warp 2 TMEM allocator (2
+// accumulators x 256 columns = 512), warp 3 idle, warps 4-19 the epilogue: warpgroup g (warps
+// 4+4g .. 7+4g) reads TMEM columns [64g, 64g+64) of every accumulator, thread (warp & 3) *
+// 32 + lane owns query row = TMEM lane.  Every mbarrier wait is bounded; a CTA that times
+// out raises the error flag, drains its own copies and MMAs, frees TMEM and returns; the
+// CTAs of a cluster leave together.
+//
+// Measured (10,000 queries, 1.2M x 100): prepass 128 -> 104 us, filter pass 1.90 -> 1.73 ms.
+// Copies and MMAs alone are MMA-bound in a pair (1.13 ms of MMAs; 1.40 ms in single CTAs);
+// the filter pass is bounded by its epilogue: reading a tile's scores, their maxima and, in
+// 42% of a warp's pieces, a survivor.
 #include "index.h"
 #include "launch_count.h"
 #include "profile.h"
@@ -46,37 +59,40 @@ namespace tc {
 namespace {
 
 constexpr int F_THREADS = 640;
-constexpr int TN = FILTER_TN;                   // base points a tile = UMMA N
-constexpr int B_HALF = TN * KHALF * 2;          // 32 KB: one 64-column half of a BF16 base tile
-constexpr int F_NACC = 2;                       // TMEM accumulators of TN columns
-constexpr int F_TMEM_COLS = F_NACC * TN;        // 512 = all of TMEM (one CTA per SM)
-constexpr int F_EPI_WARPS = 16;  // four warpgroups, one 64-column piece each
-
-constexpr int F_SBUF = 8;  // staged survivors a row and warpgroup (flushed with one atomic)
+constexpr int TN = FILTER_TN;        // base points a tile = UMMA N
+constexpr int F_CHUNK = 128;         // bytes of a row in one K chunk (one 128-byte swizzle row)
+constexpr int F_A_CHUNK = BM * F_CHUNK;  // 16 KB of a query tile
+constexpr int F_NACC = 2;            // TMEM accumulators of TN columns
+constexpr int F_TMEM_COLS = F_NACC * TN;  // 512 = all of TMEM (one CTA per SM)
+constexpr int F_EPI_WARPS = 16;      // four warpgroups, one 64-column piece each
 constexpr int kTauRegs = 80;  // group maxima a lane holds in the register threshold select
 constexpr int kTauRegsFew = 44;  // and its smaller form: 1,408 maxima, what a base of 1.2M points leaves
 
-// Shared-memory layout by operand format.  BF16: a tile row is two 128-byte swizzle rows
-// (64 columns each); E4M3: one (all 128 columns), so tiles are half the size and the
-// base ring has twice the stages.
-template <bool F8>
+// Shared-memory layout of a CTA in a cluster of CL: CL buffers of its query tile (rows of KC
+// chunks; a pair loads its next query tiles while these are in use, a CTA alone has but one
+// query tile), the ring of its shares of base chunks, and the survivor staging (SBUF entries
+// of (score, id) a row and warpgroup).
+template <int KC, int CL>
 struct FLayout {
-  static constexpr int A_BYTES = F8 ? BM * 128 : TILE_BYTES;  // query tile: 16 or 32 KB
-  static constexpr int B_BYTES = F8 ? TN * 128 : 2 * B_HALF;  // base tile: 32 or 64 KB
-  static constexpr int STAGES = F8 ? 4 : 2;
-  static constexpr int A_OFF = 0;                             // two query tiles
-  static constexpr int B_OFF = 2 * A_BYTES;                   // STAGES base tiles
-  static constexpr int S_OFF = B_OFF + STAGES * B_BYTES;      // survivor staging: scores then ids, [4][F_SBUF][BM]
-  static constexpr int BAR_OFF = S_OFF + 4 * F_SBUF * BM * 8;
-  static constexpr int SMEM = BAR_OFF + 256 + 1024;           // + barriers + 1 KB alignment slack
+  static constexpr int AB = CL;
+  static constexpr int A_BYTES = KC * F_A_CHUNK;
+  static constexpr int B_BYTES = TN / CL * F_CHUNK;  // 32 KB, or 16 KB of a pair's
+  static constexpr int STAGES = CL == 2 ? 6 : 4;
+  static constexpr int SBUF = 16;
+  static constexpr int A_OFF = 0;
+  static constexpr int B_OFF = AB * A_BYTES;
+  static constexpr int S_OFF = B_OFF + STAGES * B_BYTES;  // [4][SBUF][BM] entries of 8 bytes
+  static constexpr int BAR_OFF = S_OFF + 4 * SBUF * BM * 8;
+  static constexpr int SMEM = BAR_OFF + 256 + 1024;  // + barriers + 1 KB alignment slack
   static_assert(SMEM <= 232448, "shared memory per CTA");
-  static_assert(8 * (4 * STAGES + 5 + 2 * F_NACC) + 8 <= 256, "barrier area");
+  static_assert(8 * (2 * STAGES + 2 * AB + 2 * F_NACC + 1) + 8 <= 256, "barrier area");
 };
 
 struct FilterArgs {
   int nq;
   int64_t n;
   int QT;        // query tiles
+  int QP;        // groups of CL of them
   int NP;        // base positions scanned (tiles NP of them, base tile = p * dstride)
   int dstride;
   int CH;        // positions per unit
@@ -88,177 +104,188 @@ struct FilterArgs {
   uint64_t* cand;    // [nq][cap] survivor keys
   int cap;
   int ksteps;    // MMA K steps covering the data dimension (K = 16 BF16 or 32 E4M3 a step)
-  int hi_cols;   // columns loaded of the second 64-column half of a base tile
+  int hi_bytes;  // bytes a row loaded of the second chunk of a base tile (what its K steps read)
   int* err;
 };
 
-// Move a row's staged survivors (score, id; stride BM in shared memory) to the query's
-// candidate array: one atomicAdd reserves the slots.
-__device__ __forceinline__ void flush_staged(int* cnt, uint64_t* dst, int cap, const float* ssc, const int* sid,
-                                          int& scnt) {
-  if (scnt > 0) {
-    const int base = atomicAdd(cnt, scnt);
-    for (int e = 0; e < scnt; ++e)
-      if (base + e < cap) dst[base + e] = make_key(-ssc[e * BM], sid[e * BM]);
-    scnt = 0;
+// Move a row's staged survivors to the query's candidate array: one atomicAdd reserves the
+// slots.
+__device__ __forceinline__ void f_flush(int* cnt, uint64_t* dst, int cap, uint32_t at0, uint32_t at) {
+  if (at > at0) {
+    int pos = atomicAdd(cnt, (int)((at - at0) / (BM * 8u)));
+#pragma unroll 1
+    for (uint32_t e = at0; e < at; e += BM * 8u, ++pos) {
+      uint32_t v, id;
+      asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v), "=r"(id) : "r"(e));
+      if (pos < cap) dst[pos] = make_key(-__uint_as_float(v), (int)id);
+    }
   }
 }
 
-// F8: E4M3 operands (kind::f8f6f4); mapBhi is unused.
-template <int MODE, int GW, bool F8>
+// F8: E4M3 operands (kind::f8f6f4), one chunk; otherwise BF16 in KC chunks.  mapB's boxes
+// hold a CTA's share (TN / CL rows) of a chunk, mapBhi's of the trimmed second chunk.
+template <int MODE, int GW, bool F8, int KC, int CL>
 __global__ void __launch_bounds__(F_THREADS, 1)
     tc_filter_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                      const __grid_constant__ CUtensorMap mapBhi, const FilterArgs a) {
-  using LY = FLayout<F8>;
-  constexpr int F_STAGES = LY::STAGES;
-  constexpr int F_A_OFF = LY::A_OFF, F_B_OFF = LY::B_OFF, F_S_OFF = LY::S_OFF, F_BAR_OFF = LY::BAR_OFF;
-  constexpr int A_BYTES = LY::A_BYTES, B_TILE = LY::B_BYTES;
+  using LY = FLayout<KC, CL>;
+  constexpr int SBUF = LY::SBUF, F_STAGES = LY::STAGES, AB = LY::AB;
   static_assert(MODE == MODE_GROUPMAX || GW == 64, "the filter reads whole 64-column pieces");
   static_assert(GW == 64 || GW == 8, "group width");
-  const int U = a.NCH * a.QT;
-  if ((int)blockIdx.x >= U) return;  // no unit for this CTA: leave before any barrier or TMEM use
+  static_assert(!F8 || KC == 1, "an E4M3 row is one chunk");
+  const int U = a.NCH * a.QP;
+  const int cid = blockIdx.x / CL, ncl = gridDim.x / CL;  // cluster, clusters
+  if (cid >= U) return;  // no unit for this cluster: leave before any barrier or TMEM use
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t s0 = smem_u32(sm);
-  const uint32_t bar0 = s0 + F_BAR_OFF;
+  const uint32_t bar0 = s0 + LY::BAR_OFF;
   auto FULL = [&](int s) { return bar0 + 8u * s; };
   auto EMPTY = [&](int s) { return bar0 + 8u * (F_STAGES + s); };
   auto A_FULL = [&](int s) { return bar0 + 8u * (2 * F_STAGES + s); };
-  auto A_EMPTY = [&](int s) { return bar0 + 8u * (2 * F_STAGES + 2 + s); };
-  auto ACC_FULL = [&](int b) { return bar0 + 8u * (2 * F_STAGES + 4 + b); };
-  auto ACC_EMPTY = [&](int b) { return bar0 + 8u * (2 * F_STAGES + 4 + F_NACC + b); };
-  const uint32_t DONE = bar0 + 8u * (2 * F_STAGES + 4 + 2 * F_NACC);
-  // Prepass (BF16): the second 64-column half of a base stage has barriers of its own
-  // (FULL / EMPTY cover the first), so the first half is refilled once its four K steps
-  // are done.  The prepass reads every S-th tile and its epilogue is light, so it waits on
-  // the copies: split, it ran 16% faster at 1.2M x 100.  The filter pass ran 6% slower
-  // split and keeps one pair of barriers a stage.
-  constexpr bool SPLIT = !F8 && MODE == MODE_GROUPMAX;
-  auto FULL_HI = [&](int s) { return bar0 + 8u * (2 * F_STAGES + 5 + 2 * F_NACC + s); };
-  auto EMPTY_HI = [&](int s) { return bar0 + 8u * (3 * F_STAGES + 5 + 2 * F_NACC + s); };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + F_BAR_OFF + 8 * (4 * F_STAGES + 5 + 2 * F_NACC));
+  auto A_EMPTY = [&](int s) { return bar0 + 8u * (2 * F_STAGES + AB + s); };
+  auto ACC_FULL = [&](int b) { return bar0 + 8u * (2 * F_STAGES + 2 * AB + b); };
+  auto ACC_EMPTY = [&](int b) { return bar0 + 8u * (2 * F_STAGES + 2 * AB + F_NACC + b); };
+  const uint32_t DONE = bar0 + 8u * (2 * F_STAGES + 2 * AB + 2 * F_NACC);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + LY::BAR_OFF + 8 * (2 * F_STAGES + 2 * AB + 2 * F_NACC + 1));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform for the compiler too
   const int lane = threadIdx.x & 31;
+  const int rank = CL > 1 ? (int)cluster_rank() : 0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < F_STAGES; ++s) {
       mbar_init(FULL(s), 1);
       mbar_init(EMPTY(s), 1);
-      mbar_init(FULL_HI(s), 1);
-      mbar_init(EMPTY_HI(s), 1);
     }
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < AB; ++s) {
       mbar_init(A_FULL(s), 1);
       mbar_init(A_EMPTY(s), 1);
     }
     for (int b = 0; b < F_NACC; ++b) {
       mbar_init(ACC_FULL(b), 1);
-      mbar_init(ACC_EMPTY(b), F_EPI_WARPS);
+      mbar_init(ACC_EMPTY(b), CL * F_EPI_WARPS);  // a pair's even CTA waits for both
     }
     mbar_init(DONE, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 2) tmem_alloc(smem_u32(tmem_slot), F_TMEM_COLS);
+  if (warp == 2) tmem_alloc<CL>(smem_u32(tmem_slot), F_TMEM_COLS);
   tc_fence_before();
-  __syncthreads();
+  if (CL > 1) cluster_sync();  // the peer's barriers are initialised before anything arrives on them
+  else __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
-      int it = 0, ua = 0;
-      bool ok = true, last_hi = true;  // last_hi: the last tile's second half was issued
-      for (int u = blockIdx.x; u < U && ok; u += gridDim.x, ++ua) {
-        const int qt = u % a.QT, c = u / a.QT;
+      // a pair's bytes are counted on its even CTA's barriers, where the MMAs are issued
+      auto load = [&](uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+        if (CL > 1) tma_load_2d_pair(dst, map, x, y, cluster_addr(bar, 0));
+        else tma_load_2d(dst, map, x, y, bar);
+      };
+      int it = 0, na = 0;  // base chunks and query tiles issued
+      int have = -1;       // group whose query tile was issued last
+      bool ok = true;
+      for (int u = cid; u < U && ok; u += ncl) {
+        const int qp = u % a.QP, c = u / a.QP;
         const int p0 = c * a.CH, p1 = min(a.NP, p0 + a.CH);
-        const int ab = ua & 1;
-        if (!mbar_wait(A_EMPTY(ab), ((ua >> 1) & 1) ^ 1, abort_flag)) break;
-        mbar_expect_tx(A_FULL(ab), A_BYTES);
-        tma_load_2d(s0 + F_A_OFF + ab * A_BYTES, &mapA, 0, qt * BM, A_FULL(ab));
-        if (!F8) tma_load_2d(s0 + F_A_OFF + ab * A_BYTES + HALF_BYTES, &mapA, KHALF, qt * BM, A_FULL(ab));
-        for (int p = p0; p < p1; ++p) {
-          const int st = it % F_STAGES, rd = it / F_STAGES;
-          if (!mbar_wait(EMPTY(st), (rd & 1) ^ 1, abort_flag)) { ok = false; break; }
-          const uint32_t dst = s0 + F_B_OFF + st * B_TILE;
-          const int row = p * a.dstride * TN;
-          if (F8) {
-            mbar_expect_tx(FULL(st), B_TILE);
-            tma_load_2d(dst, &mapB, 0, row, FULL(st));
-          } else if (!SPLIT) {
-            mbar_expect_tx(FULL(st), B_HALF + TN * a.hi_cols * 2);
-            tma_load_2d(dst, &mapB, 0, row, FULL(st));
-            tma_load_2d(dst + B_HALF, &mapBhi, KHALF, row, FULL(st));
-          } else {
-            mbar_expect_tx(FULL(st), B_HALF);
-            tma_load_2d(dst, &mapB, 0, row, FULL(st));
-            if (!mbar_wait(EMPTY_HI(st), (rd & 1) ^ 1, abort_flag)) { ++it; last_hi = false; ok = false; break; }
-            mbar_expect_tx(FULL_HI(st), TN * a.hi_cols * 2);
-            tma_load_2d(dst + B_HALF, &mapBhi, KHALF, row, FULL_HI(st));
+        if (qp != have) {  // (a tile past the last one, where the tiles do not fill the cluster, reads as zeros)
+          const int ab = na % AB;
+          if (!mbar_wait(A_EMPTY(ab), ((na / AB) & 1) ^ 1, abort_flag)) break;
+          if (rank == 0) mbar_expect_tx(A_FULL(ab), CL * LY::A_BYTES);
+#pragma unroll
+          for (int kc = 0; kc < KC; ++kc)
+            load(s0 + LY::A_OFF + ab * LY::A_BYTES + kc * F_A_CHUNK, &mapA, kc * KHALF, (CL * qp + rank) * BM,
+                 A_FULL(ab));
+          ++na;
+          have = qp;
+        }
+        for (int p = p0; p < p1 && ok; ++p) {
+          const int row = p * a.dstride * TN + rank * (TN / CL);  // this CTA's share of the tile
+#pragma unroll
+          for (int kc = 0; kc < KC; ++kc) {
+            const int st = it % F_STAGES, rd = it / F_STAGES;
+            if (!mbar_wait(EMPTY(st), (rd & 1) ^ 1, abort_flag)) { ok = false; break; }
+            if (rank == 0) mbar_expect_tx(FULL(st), TN * (kc == 0 ? F_CHUNK : a.hi_bytes));
+            load(s0 + LY::B_OFF + st * LY::B_BYTES, kc == 0 ? &mapB : &mapBhi, kc * KHALF, row, FULL(st));
+            ++it;
           }
-          ++it;
         }
       }
-      // drain: every issued copy has landed before the CTA may exit -- the last F_STAGES
-      // tiles.  Split stages: the second halves too, except the last tile's when it was
-      // never issued; then the second half of the tile before the window may still be in
-      // flight (only its first half's MMAs had to finish before the last tile was issued)
-      for (int j = max(0, it - F_STAGES - 1); j < it; ++j) {
-        if (j >= it - F_STAGES) mbar_wait(FULL(j % F_STAGES), (j / F_STAGES) & 1, abort_flag, true);
-        if (SPLIT && (last_hi ? j >= it - F_STAGES : j < it - 1))
-          mbar_wait(FULL_HI(j % F_STAGES), (j / F_STAGES) & 1, abort_flag, true);
+      // drain: every copy has landed and every stage has been given back before the CTA may
+      // exit (a pair's odd CTA sees its copies' end only by the stages that come back)
+      for (int j = max(0, it - F_STAGES); j < it; ++j) {
+        if (rank == 0) mbar_wait(FULL(j % F_STAGES), (j / F_STAGES) & 1, abort_flag, true);
+        mbar_wait(EMPTY(j % F_STAGES), (j / F_STAGES) & 1, abort_flag, true);
       }
-      for (int j = max(0, ua - 2); j < ua; ++j) mbar_wait(A_FULL(j & 1), (j >> 1) & 1, abort_flag, true);
+      if (rank == 0)
+        for (int j = max(0, na - AB); j < na; ++j) mbar_wait(A_FULL(j % AB), (j / AB) & 1, abort_flag, true);
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    {
-      const uint32_t leader = elect_one();  // the warp stays converged (see elect_one)
-      int it = 0, ua = 0;
-      bool ok = true;
-      for (int u = blockIdx.x; u < U && ok; u += gridDim.x, ++ua) {
-        const int c = u / a.QT;
-        const int p0 = c * a.CH, p1 = min(a.NP, p0 + a.CH);
-        const int ab = ua & 1;
-        if (!mbar_wait_warp(A_FULL(ab), (ua >> 1) & 1, abort_flag)) break;
+    // ---------------- MMA issuer (a pair's: its even CTA) ----------------
+    const uint32_t leader = elect_one();  // the warp stays converged (see elect_one)
+    constexpr uint32_t idesc = F8 ? idesc_e4m3(CL * BM, TN) : idesc_bf16(CL * BM, TN);
+    auto commit = [&](uint32_t bar) {
+      if (CL > 1) umma_commit_pair(bar, leader);
+      else umma_commit(bar, leader);
+    };
+    // A tile's MMAs take 896 cycles at d = 100 and this warp issues nothing else meanwhile, so
+    // its own time a tile has to stay below that: running stage and parity instead of
+    // divisions, descriptors by 32-bit additions.
+    const uint32_t a_lo0 = smem_desc_lo(s0 + LY::A_OFF), b_lo0 = smem_desc_lo(s0 + LY::B_OFF);
+    int st = 0, na = 0, b = 0;
+    uint32_t ph = 0, acc_ph = 1;
+    int have = -1;
+    bool ok = rank == 0;
+    for (int u = cid; u < U && ok; u += ncl) {
+      const int qp = u % a.QP, c = u / a.QP;
+      const int p0 = c * a.CH, p1 = min(a.NP, p0 + a.CH);
+      if (qp != have) {
+        if (!mbar_wait_warp(A_FULL(na % AB), (na / AB) & 1, abort_flag)) break;
         tc_fence_after();
-        for (int p = p0; p < p1; ++p) {
-          const int b = it % F_NACC, ub = it / F_NACC;
-          if (!mbar_wait_warp(ACC_EMPTY(b), (ub & 1) ^ 1, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          const int st = it % F_STAGES, rd = it / F_STAGES;
-          if (!mbar_wait_warp(FULL(st), rd & 1, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t dt = tmem + (uint32_t)(b * TN), as = s0 + F_A_OFF + ab * A_BYTES;
-          const uint32_t bs = s0 + F_B_OFF + st * B_TILE;
-          if (F8) {
-            umma_tile_e4m3<TN>(dt, as, bs, a.ksteps, leader);
-            umma_commit(EMPTY(st), leader);
-          } else if (!SPLIT) {
-            umma_tile<TN>(dt, as, bs, a.ksteps, leader);
-            umma_commit(EMPTY(st), leader);
-          } else {
-            umma_steps<TN>(dt, as, bs, 0, min(4, a.ksteps), leader);
-            umma_commit(EMPTY(st), leader);
-            if (!mbar_wait_warp(FULL_HI(st), rd & 1, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            umma_steps<TN>(dt, as, bs, 4, a.ksteps, leader);
-            umma_commit(EMPTY_HI(st), leader);
-          }
-          umma_commit(ACC_FULL(b), leader);
-          ++it;
-        }
-        umma_commit(A_EMPTY(ab), leader);  // the query tile is free once this unit's MMAs complete
+        ++na;
+        have = qp;
       }
-      // drain: all issued MMAs complete before TMEM is released
-      umma_commit(DONE, leader);
-      mbar_wait(DONE, 0, abort_flag, true);
+      const int ab = (na - 1) % AB;
+      const uint32_t a_lo = a_lo0 + (uint32_t)ab * (LY::A_BYTES >> 4);
+      for (int p = p0; p < p1; ++p) {
+        if (!mbar_wait_warp(ACC_EMPTY(b), acc_ph, abort_flag)) { ok = false; break; }
+        const uint32_t d_tmem = tmem + (uint32_t)(b * TN);
+#pragma unroll
+        for (int kc = 0; kc < KC; ++kc) {
+          if (!mbar_wait_warp(FULL(st), ph, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t b_lo = b_lo0 + (uint32_t)st * (LY::B_BYTES >> 4);
+          // rows are zero past the data dimension: steps beyond it would add exact zeros
+#pragma unroll
+          for (int kk = 0; kk < F_CHUNK / 32; ++kk) {  // 32 bytes a step
+            const uint64_t ad = smem_desc_of(a_lo + kc * (F_A_CHUNK >> 4) + 2 * kk), bd = smem_desc_of(b_lo + 2 * kk);
+            if (4 * kc + kk >= a.ksteps) continue;
+            if (F8) umma_e4m3<CL>(d_tmem, ad, bd, idesc, (kc > 0 || kk > 0) ? 1u : 0u, leader);
+            else umma_bf16<CL>(d_tmem, ad, bd, idesc, (kc > 0 || kk > 0) ? 1u : 0u, leader);
+          }
+          commit(EMPTY(st));
+          if (++st == F_STAGES) {
+            st = 0;
+            ph ^= 1u;
+          }
+        }
+        if (!ok) break;
+        commit(ACC_FULL(b));
+        b ^= 1;
+        if (b == 0) acc_ph ^= 1u;
+      }
+      // the query tile is free once this unit's MMAs complete
+      if (u + ncl < U && (u + ncl) % a.QP != qp) commit(A_EMPTY(ab));
     }
+    // drain: all issued MMAs complete before TMEM is released
+    if (rank == 0) commit(DONE);
+    mbar_wait(DONE, 0, abort_flag, true);
     __syncwarp();
   } else if (warp >= 4) {
     // ---------------- epilogue ----------------
@@ -266,99 +293,98 @@ __global__ void __launch_bounds__(F_THREADS, 1)
     const int r = (warp & 3) * 32 + lane;        // query row within the tile = TMEM lane
     const uint32_t tbase = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g * 64);
     // Survivors are staged per row in shared memory as (score, id) -- this thread's own
-    // column of the warpgroup's [F_SBUF][BM] arrays, so no synchronisation is needed --
-    // and reach the query's global array in batches: one atomicAdd a flush instead of
-    // one a survivor, and the ordering keys are built only then.
-    float* ssc = reinterpret_cast<float*>(sm + F_S_OFF) + (size_t)g * F_SBUF * BM + r;
-    int* sid = reinterpret_cast<int*>(sm + F_S_OFF + 4 * F_SBUF * BM * 4) + (size_t)g * F_SBUF * BM + r;
-    int scnt = 0;
-    int it = 0;
+    // column of the warpgroup's [SBUF][BM] array, so no synchronisation is needed -- and
+    // reach the query's global array in batches: one atomicAdd a flush instead of one a
+    // survivor, and the ordering keys are built only then.  A warp flushes when one of its
+    // rows runs out of room and when its next unit has another query tile.
+    const uint32_t at0 = s0 + LY::S_OFF + (uint32_t)(g * SBUF * BM + r) * 8u;
+    const uint32_t at_end = at0 + (uint32_t)SBUF * (BM * 8u);
+    uint32_t at = at0;
+    int ia = 0;
     bool ok = true;
-    for (int u = blockIdx.x; u < U && ok; u += gridDim.x) {
-      const int qt = u % a.QT, c = u / a.QT;
+    for (int u = cid; u < U && ok; u += ncl) {
+      const int qp = u % a.QP, c = u / a.QP;
       const int p0 = c * a.CH, p1 = min(a.NP, p0 + a.CH);
-      const int q = qt * BM + r;
+      const int q = (CL * qp + rank) * BM + r;
       float tau = INFINITY;
       if (MODE == MODE_FILTER && q < a.nq) tau = a.tau ? a.tau[q] : -INFINITY;
+      auto flush = [&] {
+        f_flush(a.cnt + q, a.cand + (int64_t)q * a.cap, a.cap, at0, at);
+        at = at0;
+      };
       for (int p = p0; p < p1; ++p) {
-        const int b = it % F_NACC, ub = it / F_NACC;
-        if (!mbar_wait(ACC_FULL(b), ub & 1, abort_flag)) { ok = false; break; }
+        const int b = ia % F_NACC, ub = ia / F_NACC;
+        // warp-uniform, so that a warp which gives up leaves its votes together
+        if (!mbar_wait_warp(ACC_FULL(b), ub & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         uint32_t v[64];
         tmem_ld64(tbase + (uint32_t)(b * TN), v);
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(ACC_EMPTY(b));  // scores are in registers: the MMA may reuse the buffer
-        ++it;
+        if (lane == 0) {  // scores are in registers: the MMA may reuse the buffer
+          if (CL > 1) mbar_arrive_cluster(cluster_addr(ACC_EMPTY(b), 0));
+          else mbar_arrive(ACC_EMPTY(b));
+        }
+        ++ia;
         const int64_t cbase = (int64_t)p * a.dstride * TN + g * 64;  // base id of v[0]
         const int piece = 4 * p + g;  // index of this 64-column piece among the row's sampled pieces
-        if (MODE == MODE_GROUPMAX) {
-          if (cbase + 64 > a.n) {  // last base tile: padding rows are not points
+        if (cbase + 64 > a.n) {  // last base tile: padding rows become NaN, which no maximum or compare takes
 #pragma unroll
-            for (int j = 0; j < 64; ++j)
-              if (cbase + j >= a.n) v[j] = __float_as_uint(-INFINITY);
-          }
+          for (int j = 0; j < 64; ++j)
+            if (cbase + j >= a.n) v[j] = 0x7fc00000u;
+        }
+        float m[8];
+#pragma unroll
+        for (int gg = 0; gg < 8; ++gg) m[gg] = max8(v, gg);
+        const float tm = max3f(max3f(m[0], m[1], m[2]), max3f(m[3], m[4], m[5]), fmaxf(m[6], m[7]));
+        if (MODE == MODE_GROUPMAX) {
           if (q < a.nq) {
             if (GW == 64) {
-              float m[8];
-#pragma unroll
-              for (int gg = 0; gg < 8; ++gg) m[gg] = max8(v, gg);
-              a.gmax[(int64_t)q * a.M + piece] =
-                  max3f(max3f(m[0], m[1], m[2]), max3f(m[3], m[4], m[5]), fmaxf(m[6], m[7]));
+              a.gmax[(int64_t)q * a.M + piece] = tm;
             } else {
-              float4 lo, hi;
-              lo.x = max8(v, 0); lo.y = max8(v, 1); lo.z = max8(v, 2); lo.w = max8(v, 3);
-              hi.x = max8(v, 4); hi.y = max8(v, 5); hi.z = max8(v, 6); hi.w = max8(v, 7);
               float4* dst = reinterpret_cast<float4*>(a.gmax + (int64_t)q * a.M + 8 * piece);
-              dst[0] = lo;
-              dst[1] = hi;
+              dst[0] = make_float4(m[0], m[1], m[2], m[3]);
+              dst[1] = make_float4(m[4], m[5], m[6], m[7]);
             }
           }
-        } else {
-          if (cbase + 64 > a.n) {  // last base tile: padding rows become NaN, which never passes
+        } else if (__any_sync(0xffffffffu, tm >= tau)) {
+          const int ibase = (int)cbase;  // ids fit in 32 bits (n < 2^31)
+          unsigned lm = 0;
 #pragma unroll
-            for (int j = 0; j < 64; ++j)
-              if (cbase + j >= a.n) v[j] = 0x7fc00000u;
-          }
-          float m[8];
+          for (int gg = 0; gg < 8; ++gg) lm |= m[gg] >= tau ? (1u << gg) : 0u;
+          const unsigned hm = __reduce_or_sync(0xffffffffu, lm);
 #pragma unroll
-          for (int gg = 0; gg < 8; ++gg) m[gg] = max8(v, gg);
-          const float tm = max3f(max3f(m[0], m[1], m[2]), max3f(m[3], m[4], m[5]), fmaxf(m[6], m[7]));
-          if (__any_sync(0xffffffffu, tm >= tau)) {
-            const int ibase = (int)cbase;  // ids fit in 32 bits (n < 2^31)
+          for (int gg = 0; gg < 8; ++gg) {
+            if (!(hm & (1u << gg))) continue;
+            int ng = 0;  // this lane's survivors in the group
 #pragma unroll
-            for (int gg = 0; gg < 8; ++gg) {
-              if (!__any_sync(0xffffffffu, m[gg] >= tau)) continue;
-              int ng = 0;  // this lane's survivors in the group
+            for (int jj = 0; jj < 8; ++jj) ng += __uint_as_float(v[8 * gg + jj]) >= tau ? 1 : 0;
+            if (at + (uint32_t)ng * (BM * 8u) > at_end) flush();
 #pragma unroll
-              for (int jj = 0; jj < 8; ++jj) ng += __uint_as_float(v[8 * gg + jj]) >= tau ? 1 : 0;
-              if (scnt + ng > F_SBUF) flush_staged(a.cnt + q, a.cand + (int64_t)q * a.cap, a.cap, ssc, sid, scnt);
-#pragma unroll
-              for (int jj = 0; jj < 8; ++jj) {
-                const float s = __uint_as_float(v[8 * gg + jj]);
-                if (s >= tau) {
-                  ssc[scnt * BM] = s;
-                  sid[scnt * BM] = ibase + 8 * gg + jj;
-                  ++scnt;
-                }
+            for (int jj = 0; jj < 8; ++jj) {
+              const float sc = __uint_as_float(v[8 * gg + jj]);
+              if (sc >= tau) {
+                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(v[8 * gg + jj]), "r"(ibase + 8 * gg + jj) : "memory");
+                at += BM * 8u;
               }
             }
           }
         }
       }
-      if (MODE == MODE_FILTER && scnt > 0)  // the next unit is another query tile
-        flush_staged(a.cnt + q, a.cand + (int64_t)q * a.cap, a.cap, ssc, sid, scnt);
+      if (MODE == MODE_FILTER && (!ok || u + ncl >= U || (u + ncl) % a.QP != qp)) flush();
     }
   }
 
   tc_fence_before();
-  __syncthreads();
+  if (CL > 1) cluster_sync();  // both CTAs are done with TMEM and with each other's barriers
+  else __syncthreads();
   if (warp == 2) {
     tc_fence_after();
-    tmem_dealloc(tmem, F_TMEM_COLS);
+    tmem_dealloc<CL>(tmem, F_TMEM_COLS);
   }
   if (threadIdx.x == 0 && *abort_flag) atomicExch(a.err, 2);
+  if (CL > 1) cluster_sync();  // a pair leaves together
 }
 
 // Descending scan of one warp's 256-bin histogram: digit = the bin where the count of keys
@@ -581,24 +607,52 @@ __global__ void merge_fallback_kernel(const uint64_t* __restrict__ part, const i
   }
 }
 
-template <int MODE, int GW, bool F8>
-void run_filter(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mbhi, FilterArgs a, const char* name,
-                cudaStream_t s) {
+template <int MODE, int GW, bool F8, int KC, int CL>
+void run_filter_as(const FilterMaps& m, FilterArgs a, int clusters, const char* name, cudaStream_t s) {
   // chunk size: long enough to amortise the query-tile switch (at most 32 tiles), short
-  // enough for >= 16 units per CTA so the last unit leaves little imbalance
-  const int G = num_sms();
-  const int64_t work = (int64_t)a.NP * a.QT;
-  a.CH = (int)std::max<int64_t>(1, std::min<int64_t>(32, (work + 16 * G - 1) / (16 * G)));
+  // enough for >= 16 units per cluster so the last unit leaves little imbalance
+  const int64_t work = (int64_t)a.NP * a.QP;
+  a.CH = (int)std::max<int64_t>(1, std::min<int64_t>(32, (work + 16 * clusters - 1) / (16 * clusters)));
   a.NCH = ceil_div(a.NP, a.CH);
-  const int U = a.NCH * a.QT;
-  const int grid = std::min(G, U);
-  auto kern = tc_filter_kernel<MODE, GW, F8>;
-  constexpr int smem = FLayout<F8>::SMEM;
+  const int grid = CL * std::min(clusters, a.NCH * a.QP);
+  auto kern = tc_filter_kernel<MODE, GW, F8, KC, CL>;
+  constexpr int smem = FLayout<KC, CL>::SMEM;
   LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(F_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = CL;
+  at.val.clusterDim.y = 1;
+  at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = CL > 1 ? 1 : 0;
   ProfScope _ps(name, s);
-  kern<<<grid, F_THREADS, smem, s>>>(ma, mb, mbhi, a);
+  LSHG_CUDA(cudaLaunchKernelEx(&cfg, kern, m.a, m.b, m.bhi, a));
   count_launch();
-  LSHG_CHECK_LAUNCH();
+}
+
+template <int MODE, int GW, bool F8, int KC>
+void run_filter(const FilterMaps& m, FilterArgs a, const char* name, cudaStream_t s) {
+  a.QP = ceil_div(a.QT, m.cl);
+  const int G = std::max(1, num_sms() / m.cl);
+  // Clusters in a multiple of the groups keep one query tile each for the whole scan: nothing
+  // is reloaded and the staging is flushed when it is full, not every unit (100k x 100, 1,000
+  // queries: units of two tiles).  Worth up to 6% of the SMs.
+  const int keep = a.QP <= G ? G / a.QP * a.QP : 0;
+  const int clusters = keep * 100 >= G * 94 ? keep : G;
+  if (m.cl == 2) run_filter_as<MODE, GW, F8, KC, 2>(m, a, clusters, name, s);
+  else run_filter_as<MODE, GW, F8, KC, 1>(m, a, clusters, name, s);
+}
+
+template <int MODE, int GW>
+void run_filter_fmt(const FilterMaps& m, const FilterArgs& a, const char* name, cudaStream_t s) {
+  if (m.e4m3) run_filter<MODE, GW, true, 1>(m, a, name, s);
+  else if (a.ksteps <= 4) run_filter<MODE, GW, false, 1>(m, a, name, s);
+  else run_filter<MODE, GW, false, 2>(m, a, name, s);
 }
 
 }  // namespace
@@ -609,9 +663,14 @@ void run_filter(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
 // tau stays at or below that point unless the count exceeds its mean by four standard
 // deviations, and about r * S points survive (CT * S with r = CT).  A query with fewer
 // than CT survivors is rescanned exactly by the list kernel (cand_select lists it), so
-// the rank only trades survivors against fallbacks.  S is the largest that leaves at
-// least 4 r maxima a row, so that the r-th largest is a tight bound.
-FilterPlan plan_filter(int64_t n, int CT) {
+// the rank only trades survivors against fallbacks.  Among the S that leave at least 4 r
+// maxima a row, so that the r-th largest is a tight bound, the plan takes the cheapest, by
+// what each part took at 1.2M x 10,000 and 100k x 1,000: 0.9 us a sampled tile of an SM, 3.2 ps
+// a maximum of the threshold select, 0.12 ns a survivor (its way through the filter and the
+// candidate select).  10,000 queries on 1.2M points: S = 16 prepass, threshold, filter and
+// select 104 + 39 + 1,730 + 60 us, S = 8 199 + 75 + 1,630 + 44; 1,000 on 100k: S = 16 10 +
+// 10 + 48 + 18 us, S = 1 25 + 17 + 33 + 9.
+FilterPlan plan_filter(int64_t n, int CT, int nq) {
   FilterPlan p{};
   const int NT = ceil_div(n, TN);
   p.NT = NT;
@@ -619,13 +678,19 @@ FilterPlan plan_filter(int64_t n, int CT) {
   if (NT >= CT) {  // 64-column maxima: 4 a tile
     p.GW = 64;
     p.S = 1;
-    for (int S : {16, 8, 4, 2}) {
+    const int QT = ceil_div(nq, BM);
+    double best = 0.0;
+    for (int S : {16, 8, 4, 2, 1}) {
       const double m = (double)CT / S;
-      const int r = std::min(CT, (int)std::ceil(m + 4.0 * std::sqrt(m) + 8.0));
-      if (4 * ceil_div(NT, S) >= 4 * r) {
+      const int r = S == 1 ? CT : std::min(CT, (int)std::ceil(m + 4.0 * std::sqrt(m) + 8.0));
+      const int NS = ceil_div(NT, S);
+      if (S > 1 && NS < r) continue;
+      const double cost = 0.9e-6 * ceil_div((int64_t)NS * QT, num_sms()) + 3.2e-12 * (double)nq * 4 * NS +
+                          0.12e-9 * (double)nq * r * S;
+      if (best == 0.0 || cost < best) {
+        best = cost;
         p.S = S;
         p.rank = r;
-        break;
       }
     }
     p.NS = ceil_div(NT, p.S);
@@ -648,15 +713,33 @@ FilterPlan plan_filter(int64_t n, int CT) {
   return p;
 }
 
-void launch_filter_scan(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mbhi, int hi_cols,
-                        const FilterPlan& plan, int nq, int64_t n, int d, int QT, int CT, float* tau, int* cnt,
-                        uint64_t* cand, int* err, bool e4m3, cudaStream_t s) {
+FilterMaps make_filter_maps(const void* q, int64_t qrows, const void* base, int64_t brows, int d, bool e4m3) {
+  FilterMaps m{};
+  m.e4m3 = e4m3;
+  // clusters of two query tiles share each base tile's fetch; one tile alone would leave the
+  // second CTA without work
+  m.cl = qrows > BM ? 2 : 1;
+  m.hi_cols = std::max(8, std::min(KHALF, 16 * tc_ksteps(d) - KHALF));
+  if (e4m3) {
+    m.a = make_map_e4m3(q, qrows, BM);
+    m.b = make_map_e4m3(base, brows, TN / m.cl);
+    m.bhi = m.b;
+  } else {
+    m.a = make_map(q, qrows);
+    m.b = make_map(base, brows, TN / m.cl);
+    m.bhi = make_map(base, brows, TN / m.cl, m.hi_cols);
+  }
+  return m;
+}
+
+void launch_filter_scan(const FilterMaps& m, const FilterPlan& plan, int nq, int64_t n, int d, int QT, float* tau,
+                        int* cnt, uint64_t* cand, int* err, cudaStream_t s) {
   FilterArgs a{};
-  a.hi_cols = hi_cols;
+  a.hi_bytes = m.hi_cols * 2;
   a.nq = nq;
-  a.ksteps = e4m3 ? tc_ksteps_e4m3(d) : tc_ksteps(d);
+  a.ksteps = m.e4m3 ? tc_ksteps_e4m3(d) : tc_ksteps(d);
   // scores of E4M3 codes carry the factor kE4M3Scale^2
-  const float margin = e4m3 ? kTauMargin * kE4M3Scale * kE4M3Scale : kTauMargin;
+  const float margin = m.e4m3 ? kTauMargin * kE4M3Scale * kE4M3Scale : kTauMargin;
   a.n = n;
   a.QT = QT;
   a.err = err;
@@ -666,13 +749,8 @@ void launch_filter_scan(const CUtensorMap& ma, const CUtensorMap& mb, const CUte
     a.dstride = plan.S;
     a.gmax = gmax.ptr;
     a.M = plan.M;
-    if (e4m3) {
-      if (plan.GW == 64) run_filter<MODE_GROUPMAX, 64, true>(ma, mb, mbhi, a, "tc_prepass", s);
-      else run_filter<MODE_GROUPMAX, 8, true>(ma, mb, mbhi, a, "tc_prepass", s);
-    } else {
-      if (plan.GW == 64) run_filter<MODE_GROUPMAX, 64, false>(ma, mb, mbhi, a, "tc_prepass", s);
-      else run_filter<MODE_GROUPMAX, 8, false>(ma, mb, mbhi, a, "tc_prepass", s);
-    }
+    if (plan.GW == 64) run_filter_fmt<MODE_GROUPMAX, 64>(m, a, "tc_prepass", s);
+    else run_filter_fmt<MODE_GROUPMAX, 8>(m, a, "tc_prepass", s);
     launch_tau_select(gmax.ptr, nq, plan.M, plan.rank, margin, tau, s);
   }
   a.gmax = nullptr;
@@ -683,8 +761,7 @@ void launch_filter_scan(const CUtensorMap& ma, const CUtensorMap& mb, const CUte
   a.cnt = cnt;
   a.cand = cand;
   a.cap = plan.cap;
-  if (e4m3) run_filter<MODE_FILTER, 64, true>(ma, mb, mbhi, a, "tc_filter", s);
-  else run_filter<MODE_FILTER, 64, false>(ma, mb, mbhi, a, "tc_filter", s);
+  run_filter_fmt<MODE_FILTER, 64>(m, a, "tc_filter", s);
 }
 
 void launch_tau_select(const float* gmax, int nq, int M, int rank, float margin, float* tau, cudaStream_t s) {

@@ -17,7 +17,8 @@ constexpr int MODE_FILTER = 1;    // main pass: keep scores >= the row's thresho
 // the same instruction sequence, so this only guards against a last-bit difference.
 constexpr float kTauMargin = 1e-6f;
 
-// Parameters of the threshold prepass for a base of n points and CT candidates a query.
+// Parameters of the threshold prepass for a base of n points, CT candidates a query and a batch
+// of nq queries.
 struct FilterPlan {
   int NT;   // 256-point base tiles
   int GW;   // group width of the prepass maxima (64 or 8; 0 = no prepass, keep every point)
@@ -28,16 +29,21 @@ struct FilterPlan {
   int cap;  // survivor slots a query
 };
 
-FilterPlan plan_filter(int64_t n, int CT);
+FilterPlan plan_filter(int64_t n, int CT, int nq);
+
+// Tensor maps of a scan: query rows (padded to 128) and base rows (padded to FILTER_TN), BF16
+// rows of 128 columns or E4M3 rows of 128 bytes.
+struct FilterMaps {
+  CUtensorMap a, b, bhi;  // bhi: the second 64 columns, trimmed to hi_cols (what the K steps read)
+  int hi_cols;
+  int cl;  // CTAs a cluster (2 when there are two query tiles or more); b's boxes hold a CTA's share of a tile
+  bool e4m3;
+};
+FilterMaps make_filter_maps(const void* q, int64_t qrows, const void* base, int64_t brows, int d, bool e4m3);
 
 // Prepass + threshold selection + filter pass: fills cnt[q] and cand[q][0..cap).
-// mb: base tiles (256 rows x 64 columns boxes); mbhi: boxes of the second 64-column half
-// trimmed to hi_cols columns (the K steps past the data dimension are never read).
-// e4m3: operands are E4M3 codes (rows of 128 bytes; mb boxes of 256 rows x 128 bytes, mbhi
-// unused); otherwise BF16 as above.
-void launch_filter_scan(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mbhi, int hi_cols,
-                        const FilterPlan& plan, int nq, int64_t n, int d, int QT, int CT, float* tau, int* cnt,
-                        uint64_t* cand, int* err, bool e4m3, cudaStream_t s);
+void launch_filter_scan(const FilterMaps& m, const FilterPlan& plan, int nq, int64_t n, int d, int QT, float* tau,
+                        int* cnt, uint64_t* cand, int* err, cudaStream_t s);
 
 // tau[q] = a lower bound (within 1/65536 of the row's range) of the rank-th largest of the
 // row's M group maxima, minus margin; -inf when the row holds fewer than rank maxima.

@@ -35,12 +35,13 @@
 // tc_hamming_kernel: persistent, one CTA per SM, 640 threads, in clusters of CL = 2 CTAs (1
 // for batches of one query tile).  A unit is (CL query tiles of 128 rows, chunk of up to 36
 // consecutive base tiles of 224 points), numbered chunk-major so that all SMs stream the
-// same base tiles at a time (each read from HBM about once a batch, then from L2).  Each CTA
-// keeps its query tile in shared memory for the unit (KC chunks of 128 rows x 128 bytes);
-// the base tile streams through a ring of one-chunk stages (224 rows x 128 bytes), half of
-// each stage loaded by either CTA and multicast to both: a 128 x 224 tile of 1,024 bits is
-// 1,792 cycles of MMA, and fetching its 112 KB for one SM alone would take more than the
-// about 85 KB a microsecond an SM gets from L2.
+// same base tiles at a time (each read from HBM about once a batch, then from L2).  The two
+// CTAs of a cluster are an MMA pair (tcgen05 cta_group::2): each keeps its query tile in shared
+// memory for the unit (KC chunks of 128 rows x 128 bytes) and streams its half of the base
+// tile through a ring of one-chunk stages (112 rows x 128 bytes); the even one issues the MMAs
+// of both.  A CTA on its own reads 11 KB of operands from shared memory an MMA of 112 cycles and
+// writes 28 KB of base tile every four -- 160 bytes a cycle of the 128 there are -- and takes
+// 112 KB a tile from L2; in a pair both halve on the base tile's side.
 // Warp 0 issues the TMA copies, warp 1 the MMAs (tcgen05.mma kind::mxf4 with block scales
 // of 1.0, M = 128, N = 224, K = 64 each; 4 a chunk), warp 2 owns the 512 TMEM columns, warps
 // 4-19 are the epilogue (warpgroup g reads columns [56g, 56g + 56), one query row a thread).
@@ -50,11 +51,12 @@
 // error 2, drains its copies and MMAs, frees TMEM and returns; the CTAs of a cluster leave
 // together.
 //
-// Measured (filter pass; 10,000 queries): 1.2M points of 1,024 bits 7.52 -> 3.25 ms (7.5
+// Measured (filter pass; 10,000 queries): 1.2M points of 1,024 bits 7.52 -> 2.96 ms (8.3
 // PFLOP/s of +-1 products; 2.5 ms is the MMAs alone), 500k points of 256 bits at C = 4,096
-// 4.79 -> 1.77 ms (bounded by the 1.3% survivors: without any the same pass takes 0.67 ms);
+// 4.79 -> 1.79 ms (bounded by the 1.3% survivors: without any the same pass takes 0.67 ms);
 // before: E4M3 rows (twice the bytes, half the MMA rate), a query tile a CTA with its own
-// copy of every base tile, MMAs issued from a diverged warp, branches around each store.
+// copy of every base tile, MMAs issued from a diverged warp, branches around each store.  The
+// pair's MMAs against two CTAs that multicast the base tile to each other: 3.25 -> 2.96 ms.
 //
 // tc_signs_kernel: the same pipeline with BF16 operands and one query tile for the SimHash
 // projections (below).
@@ -91,23 +93,21 @@ constexpr int P_NACC = 2;         // its TMEM accumulators of PN columns
 
 constexpr int kSmemLimit = 232448;  // dynamic shared memory a CTA may opt into
 
-// Shared-memory layout for rows of KC chunks: the resident query tile, the ring of base
-// chunks, and the survivor staging (SBUF 4-byte entries a row and warpgroup).
-template <int KC>
+// Shared-memory layout of a CTA in a cluster of CL, for rows of KC chunks: the resident query
+// tile, the ring of its shares of base chunks, and the survivor staging (SBUF 4-byte entries a
+// row and warpgroup).
+template <int KC, int CL>
 struct HLayout {
   static constexpr int A_BYTES = KC * BM * H_CHUNK;  // query tile
-  static constexpr int B_BYTES = HN * H_CHUNK;       // one chunk of a base tile: 28 KB
-  static constexpr int STAGES = 4;
-  static constexpr int FIXED = A_BYTES + STAGES * B_BYTES + 256 + 1024;  // + barriers + alignment slack
-  static constexpr int ROOM = (kSmemLimit - FIXED) / (4 * BM * 4);
-  static constexpr int SBUF = ROOM >= 24 ? 24 : ROOM;
+  static constexpr int B_BYTES = HN / CL * H_CHUNK;  // one chunk of a base tile: 28 KB, or a pair's 14 KB
+  static constexpr int STAGES = CL == 2 ? 7 : 4;
+  static constexpr int SBUF = 24;
   static constexpr int A_OFF = 0;
   static constexpr int B_OFF = A_BYTES;
   static constexpr int S_OFF = B_OFF + STAGES * B_BYTES;  // [4][SBUF][BM] entries
   static constexpr int BAR_OFF = S_OFF + 4 * SBUF * BM * 4;
-  static constexpr int SMEM = BAR_OFF + 256 + 1024;
+  static constexpr int SMEM = BAR_OFF + 256 + 1024;  // + barriers + alignment slack
   static_assert(SMEM <= kSmemLimit, "shared memory per CTA");
-  static_assert(SBUF >= 8, "staging room");
   static_assert(8 * (2 * STAGES + 7) + 8 <= 256, "barrier area");
 };
 static_assert(H_MAX_CH * HN <= 8192, "column offsets of a unit fit 13 bits");
@@ -162,7 +162,7 @@ template <int MODE, int GW, int KC, int CL>
 __global__ void __launch_bounds__(H_THREADS, 1)
     tc_hamming_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                       const HArgs a) {
-  using LY = HLayout<KC>;
+  using LY = HLayout<KC, CL>;
   constexpr int STAGES = LY::STAGES, SBUF = LY::SBUF;
   static_assert(MODE != MODE_FILTER || GW == HW, "the filter reads whole pieces");
   static_assert(GW == HW || GW == 8, "group width");
@@ -187,24 +187,23 @@ __global__ void __launch_bounds__(H_THREADS, 1)
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform for the compiler too
   const int lane = threadIdx.x & 31;
   const int rank = CL > 1 ? (int)cluster_rank() : 0;
-  constexpr uint16_t kAll = (uint16_t)((1u << CL) - 1u);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(FULL(s), 1);
-      mbar_init(EMPTY(s), CL);  // every CTA of the cluster has read the stage
+      mbar_init(EMPTY(s), 1);
     }
     mbar_init(A_FULL, 1);
     mbar_init(A_EMPTY, 1);
     for (int b = 0; b < 2; ++b) {
       mbar_init(ACC_FULL(b), 1);
-      mbar_init(ACC_EMPTY(b), H_EPI_WARPS);
+      mbar_init(ACC_EMPTY(b), CL * H_EPI_WARPS);  // a pair's even CTA waits for both
     }
     mbar_init(DONE, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 2) tmem_alloc(smem_u32(tmem_slot), H_TMEM_COLS);
+  if (warp == 2) tmem_alloc<CL>(smem_u32(tmem_slot), H_TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -223,6 +222,11 @@ __global__ void __launch_bounds__(H_THREADS, 1)
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
+      // a pair's bytes are counted on its even CTA's barriers, where the MMAs are issued
+      auto load = [&](uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+        if (CL > 1) tma_load_2d_pair(dst, map, x, y, cluster_addr(bar, 0));
+        else tma_load_2d(dst, map, x, y, bar);
+      };
       int it = 0, na = 0;  // base chunks and query tiles issued
       int have = -1;       // query tile in shared memory
       bool ok = true;
@@ -238,10 +242,10 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         for (int ci = 0; ci <= total; ++ci) {
           if (ci == pre && qp != have) {
             if (!mbar_wait(A_EMPTY, (na & 1) ^ 1, abort_flag)) { ok = false; break; }
-            mbar_expect_tx(A_FULL, LY::A_BYTES);
+            if (rank == 0) mbar_expect_tx(A_FULL, CL * LY::A_BYTES);
 #pragma unroll
             for (int kc = 0; kc < KC; ++kc)
-              tma_load_2d(s0 + LY::A_OFF + kc * BM * H_CHUNK, &mapA, kc * H_CHUNK, (CL * qp + rank) * BM, A_FULL);
+              load(s0 + LY::A_OFF + kc * BM * H_CHUNK, &mapA, kc * H_CHUNK, (CL * qp + rank) * BM, A_FULL);
             ++na;
             have = qp;
           }
@@ -249,30 +253,35 @@ __global__ void __launch_bounds__(H_THREADS, 1)
           const int p = p0 + ci / KC, kc = ci % KC;
           const int st = it % STAGES, rd = it / STAGES;
           if (!mbar_wait(EMPTY(st), (rd & 1) ^ 1, abort_flag)) { ok = false; break; }
-          mbar_expect_tx(FULL(st), LY::B_BYTES);
-          // this CTA's share of the stage, to every CTA of the cluster
-          const uint32_t dst = s0 + LY::B_OFF + st * LY::B_BYTES + rank * (LY::B_BYTES / CL);
-          const int row = p * a.dstride * HN + rank * (HN / CL);
-          if (CL > 1) tma_load_2d_multicast(dst, &mapB, kc * H_CHUNK, row, FULL(st), kAll);
-          else tma_load_2d(dst, &mapB, kc * H_CHUNK, row, FULL(st));
+          if (rank == 0) mbar_expect_tx(FULL(st), CL * LY::B_BYTES);
+          load(s0 + LY::B_OFF + st * LY::B_BYTES, &mapB, kc * H_CHUNK, p * a.dstride * HN + rank * (HN / CL), FULL(st));
           ++it;
         }
       }
-      // drain: every copy into this CTA has landed and every stage has been given back (the
-      // peer's arrivals included) before the CTA may exit
+      // drain: every copy has landed and every stage has been given back before the CTA may
+      // exit (a pair's odd CTA sees its copies' end only by the stages that come back)
       for (int j = max(0, it - STAGES); j < it; ++j) {
-        mbar_wait(FULL(j % STAGES), (j / STAGES) & 1, abort_flag, true);
+        if (rank == 0) mbar_wait(FULL(j % STAGES), (j / STAGES) & 1, abort_flag, true);
         mbar_wait(EMPTY(j % STAGES), (j / STAGES) & 1, abort_flag, true);
       }
-      if (na > 0) mbar_wait(A_FULL, (na - 1) & 1, abort_flag, true);
+      if (rank == 0 && na > 0) mbar_wait(A_FULL, (na - 1) & 1, abort_flag, true);
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    {
+    // ---------------- MMA issuer (a pair's: its even CTA) ----------------
+    if (rank == 0) {
       const uint32_t leader = elect_one();  // the warp stays converged (see elect_one)
-      constexpr uint32_t idesc = idesc_mxf4(HN);
-      int it = 0, ia = 0, na = 0;
+      constexpr uint32_t idesc = idesc_mxf4(CL * BM, HN);
+      auto commit = [&](uint32_t bar) {
+        if (CL > 1) umma_commit_pair(bar, leader);
+        else umma_commit(bar, leader);
+      };
+      // Running stage and parity, descriptors by 32-bit additions, steps cut off by the
+      // predicate: a tile's MMAs take 448 cycles a chunk, and this warp's own time has to stay
+      // below that.
+      const uint32_t a_lo = smem_desc_lo(s0 + LY::A_OFF), b_lo0 = smem_desc_lo(s0 + LY::B_OFF);
+      int st = 0, na = 0, b = 0;
+      uint32_t ph = 0, acc_ph = 1;
       int have = -1;
       bool ok = true;
       for (int u = cid; u < U && ok; u += ncl) {
@@ -284,38 +293,37 @@ __global__ void __launch_bounds__(H_THREADS, 1)
           ++na;
           have = qp;
         }
-        for (int p = p0; p < p1 && ok; ++p) {
-          const int b = ia & 1, ub = ia >> 1;
-          if (!mbar_wait_warp(ACC_EMPTY(b), (ub & 1) ^ 1, abort_flag)) { ok = false; break; }
-          tc_fence_after();
+        for (int p = p0; p < p1; ++p) {
+          if (!mbar_wait_warp(ACC_EMPTY(b), acc_ph, abort_flag)) { ok = false; break; }
           const uint32_t d_tmem = tmem + (uint32_t)(b * H_ACC_COL);
+#pragma unroll
           for (int kc = 0; kc < KC; ++kc) {
-            const int st = it % STAGES, rd = it / STAGES;
-            if (!mbar_wait_warp(FULL(st), rd & 1, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_warp(FULL(st), ph, abort_flag)) { ok = false; break; }
             tc_fence_after();
-            const uint32_t a_base = s0 + LY::A_OFF + kc * BM * H_CHUNK;
-            const uint32_t b_base = s0 + LY::B_OFF + st * LY::B_BYTES;
-            const int steps = min(4, a.ksteps - 4 * kc);
+            const uint32_t b_lo = b_lo0 + (uint32_t)st * (LY::B_BYTES >> 4);
 #pragma unroll
             for (int kk = 0; kk < H_CHUNK / 32; ++kk)  // 32 bytes a step: K = 64
-              if (kk < steps)
-                umma_mxf4(d_tmem, smem_desc(a_base + kk * 32), smem_desc(b_base + kk * 32), idesc,
-                          tmem + (uint32_t)H_SF_COL, (kc > 0 || kk > 0) ? 1u : 0u, leader);
-            if (CL > 1) umma_commit_multicast(EMPTY(st), kAll, leader);
-            else umma_commit(EMPTY(st), leader);
-            ++it;
+              if (4 * kc + kk < a.ksteps) umma_mxf4<CL>(d_tmem, smem_desc_of(a_lo + kc * (BM * H_CHUNK >> 4) + 2 * kk), smem_desc_of(b_lo + 2 * kk),
+                            idesc, tmem + (uint32_t)H_SF_COL, (kc > 0 || kk > 0) ? 1u : 0u,
+                            leader);
+            commit(EMPTY(st));
+            if (++st == STAGES) {
+              st = 0;
+              ph ^= 1u;
+            }
           }
           if (!ok) break;
-          umma_commit(ACC_FULL(b), leader);
-          ++ia;
+          commit(ACC_FULL(b));
+          b ^= 1;
+          if (b == 0) acc_ph ^= 1u;
         }
         // the query tile is free once this unit's MMAs complete
-        if (u + ncl < U && (u + ncl) % a.QP != qp) umma_commit(A_EMPTY, leader);
+        if (u + ncl < U && (u + ncl) % a.QP != qp) commit(A_EMPTY);
       }
-      // drain: all issued MMAs complete before TMEM is released
-      umma_commit(DONE, leader);
-      mbar_wait(DONE, 0, abort_flag, true);
+      commit(DONE);
     }
+    // drain: all issued MMAs complete before TMEM is released
+    mbar_wait(DONE, 0, abort_flag, true);
     __syncwarp();
   } else if (warp >= 4) {
     // ---------------- epilogue ----------------
@@ -351,7 +359,10 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(ACC_EMPTY(b));  // scores are in registers: the MMA may reuse the buffer
+        if (lane == 0) {  // scores are in registers: the MMA may reuse the buffer
+          if (CL > 1) mbar_arrive_cluster(cluster_addr(ACC_EMPTY(b), 0));
+          else mbar_arrive(ACC_EMPTY(b));
+        }
         ++ia;
         const int64_t cbase = (int64_t)p * a.dstride * HN + g * HW;  // base id of v[0]
         if (cbase + HW > a.n) {  // last base tile: padding rows become NaN, which no maximum or compare takes
@@ -394,13 +405,14 @@ __global__ void __launch_bounds__(H_THREADS, 1)
   }
 
   tc_fence_before();
-  __syncthreads();
+  if (CL > 1) cluster_sync();  // both CTAs are done with TMEM and with each other's barriers
+  else __syncthreads();
   if (warp == 2) {
     tc_fence_after();
-    tmem_dealloc(tmem, H_TMEM_COLS);
+    tmem_dealloc<CL>(tmem, H_TMEM_COLS);
   }
   if (threadIdx.x == 0 && *abort_flag) atomicExch(a.err, 2);
-  if (CL > 1) cluster_sync();  // no CTA leaves while its peer may still write into it
+  if (CL > 1) cluster_sync();  // a pair leaves together
 }
 
 // ---- projections kernel (tc_signs_kernel) -------------------------------------------------
@@ -797,7 +809,7 @@ void run_hamming(const CUtensorMap& ma, const CUtensorMap& mb, HArgs a, const ch
   a.NCH = ceil_div(a.NP, a.CH);
   const int grid = CL * std::min(G, a.NCH * a.QP);
   auto kern = tc_hamming_kernel<MODE, GW, KC, CL>;
-  constexpr int smem = HLayout<KC>::SMEM;
+  constexpr int smem = HLayout<KC, CL>::SMEM;
   LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);

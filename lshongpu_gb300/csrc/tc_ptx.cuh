@@ -99,15 +99,25 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
-// The same load into every CTA of the cluster whose bit is set in `mask`: data and byte count
-// arrive at the same offsets (dst, bar) of each.
-__device__ __forceinline__ void tma_load_2d_multicast(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar,
-                                                      uint16_t mask) {
+// The same load by a CTA of an MMA pair: data into this CTA's shared memory, the byte count to
+// `bar`, a cluster address that may lie in the pair's other CTA.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1, "
-      "{%2, %3}], [%4], %5;" ::"r"(dst),
-      "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar), "h"(mask)
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
+      "[%4];" ::"r"(dst),
+      "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar)
       : "memory");
+}
+// Cluster address of the same shared-memory offset in CTA `rank`, and an arrival there.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// (CTA-scope release: a cluster-scope one would first wait for the thread's global stores, over
+// 1,000 cycles, and what it signals -- TMEM reads -- is ordered by the tcgen05 fence.)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
@@ -127,11 +137,23 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
+// The low word of that descriptor, to which a step of 16 * k bytes along the rows adds k, and
+// the descriptor of such a word: what an issue loop computes a step is one 32-bit addition.
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t addr) { return ((addr >> 4) & 0x3FFFu) | (1u << 16); }
+__device__ __forceinline__ uint64_t smem_desc_of(uint32_t lo) {
+  constexpr uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);
+  return ((uint64_t)hi << 32) | lo;
+}
+
 // Instruction descriptor: kind::f16, A = B = BF16, D = F32, both K-major, M x N.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// CG = 2: the MMA of a CTA pair (tcgen05 cta_group::2), issued by its even CTA: 256 rows, 128
+// from each CTA's A tile and into its own TMEM, against N columns of which each CTA's shared
+// memory holds half.
+//
 // MMAs and their commits are issued by one thread of a warp that stays converged: `leader`
 // is the thread that elect_one() picked, and the instructions carry it as a predicate.
 // Inside an `if (lane == 0)` the compiler cannot keep descriptors in uniform registers, and
@@ -143,13 +165,21 @@ __device__ __forceinline__ uint32_t elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(l));
   return l;
 }
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
-                                          uint32_t accumulate, uint32_t leader) {
-  asm volatile(
-      "{\n\t.reg .pred p, l;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 l, %5, 0;\n\t"
-      "@l tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader)
-      : "memory");
+template <int CG = 1>
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate,
+    uint32_t leader) {
+  if (CG == 2)
+    asm volatile(
+        "{\n\t.reg .pred p, l;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 l, %5, 0;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p, l;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 l, %5, 0;\n\t"
+        "@l tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader)
+        : "memory");
 }
 // One 128 x N x (16 * ksteps) product; A is a 128-row tile and B an N-row tile, both
 // stored as two 64-column swizzled halves (A half = 16 KB, B half = N * 128 B).  Rows are
@@ -168,21 +198,6 @@ __device__ __forceinline__ void umma_tile(uint32_t d_tmem, uint32_t a_base, uint
     }
   }
 }
-// K steps [k0, k1) of umma_tile: a tile's MMAs issued in pieces, each after its own part
-// of the operands has landed.  Step 0 clears the accumulator.
-template <int N>
-__device__ __forceinline__ void umma_steps(uint32_t d_tmem, uint32_t a_base, uint32_t b_base, int k0, int k1,
-                                           uint32_t leader) {
-  constexpr uint32_t idesc = idesc_bf16(BM, N);
-#pragma unroll
-  for (int kk = 0; kk < KD / 16; ++kk) {
-    if (kk >= k0 && kk < k1) {
-      const uint32_t koff = (kk & 3) * 32;
-      umma_bf16(d_tmem, smem_desc(a_base + (kk >> 2) * HALF_BYTES + koff),
-                smem_desc(b_base + (kk >> 2) * (N * 128) + koff), idesc, kk > 0 ? 1u : 0u, leader);
-    }
-  }
-}
 __host__ __device__ inline int tc_ksteps(int d) { return d <= 0 ? 1 : (d > KD ? KD / 16 : (d + 15) / 16); }
 
 // FP8 operands: rows of KD E4M3 bytes (one 128-byte swizzle row holds the whole K).
@@ -190,28 +205,21 @@ __host__ __device__ inline int tc_ksteps(int d) { return d <= 0 ? 1 : (d > KD ? 
 __host__ __device__ constexpr uint32_t idesc_e4m3(int M, int N) {
   return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
-__device__ __forceinline__ void umma_e4m3(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
-                                          uint32_t accumulate, uint32_t leader) {
-  asm volatile(
-      "{\n\t.reg .pred p, l;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 l, %5, 0;\n\t"
-      "@l tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader)
-      : "memory");
-}
-// One 128 x N x (32 * ksteps) E4M3 product: each step advances 32 bytes (K = 32) along the
-// single 128-byte row of A (128-row tile) and B (N-row tile); as with BF16, rows are zero
-// past d, so ksteps = ceil(d / 32) gives the same sums as all four steps.
-template <int N>
-__device__ __forceinline__ void umma_tile_e4m3(uint32_t d_tmem, uint32_t a_base, uint32_t b_base, int ksteps,
-                                               uint32_t leader) {
-  constexpr uint32_t idesc = idesc_e4m3(BM, N);
-#pragma unroll
-  for (int kk = 0; kk < KD / 32; ++kk) {
-    if (kk < ksteps) {
-      const uint32_t koff = kk * 32;
-      umma_e4m3(d_tmem, smem_desc(a_base + koff), smem_desc(b_base + koff), idesc, kk > 0 ? 1u : 0u, leader);
-    }
-  }
+template <int CG = 1>
+__device__ __forceinline__ void umma_e4m3(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate,
+    uint32_t leader) {
+  if (CG == 2)
+    asm volatile(
+        "{\n\t.reg .pred p, l;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 l, %5, 0;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p, l;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 l, %5, 0;\n\t"
+        "@l tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader)
+        : "memory");
 }
 __host__ __device__ inline int tc_ksteps_e4m3(int d) { return d <= 0 ? 1 : (d > KD ? KD / 32 : (d + 31) / 32); }
 // E4M3 codes hold unit vectors times this factor: every component (|v| <= 1) stays within
@@ -220,18 +228,25 @@ constexpr float kE4M3Scale = 256.0f;
 
 // FP4 operands with block scales: rows of E2M1 codes, two a byte, and one UE8M0 scale a
 // 32-element block held in TMEM.  Instruction descriptor: kind::mxf4, A = B = E2M1 (format
-// 1), UE8M0 scales (bit 23), scale ids 0, dense K = 64, both K-major, M = 128 (bit 27) x N.
-__host__ __device__ constexpr uint32_t idesc_mxf4(int N) {
-  return (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | (1u << 23) | (1u << 27);
+// 1), UE8M0 scales (bit 23), scale ids 0, dense K = 64, both K-major, M x N.
+__host__ __device__ constexpr uint32_t idesc_mxf4(int M, int N) {
+  return (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | (1u << 23) | ((uint32_t)(M >> 4) << 24);
 }
-__device__ __forceinline__ void umma_mxf4(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t tmem_sf,
-                                          uint32_t accumulate, uint32_t leader) {
-  asm volatile(
-      "{\n\t.reg .pred p, l;\n\tsetp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 l, %6, 0;\n\t"
-      "@l tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%4], [%4], p;\n\t}" ::"r"(
-          tmem_d),
-      "l"(a), "l"(b), "r"(idesc), "r"(tmem_sf), "r"(accumulate), "r"(leader)
-      : "memory");
+template <int CG = 1>
+__device__ __forceinline__ void umma_mxf4(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t tmem_sf, uint32_t accumulate,
+    uint32_t leader) {
+  if (CG == 2)
+    asm volatile(
+        "{\n\t.reg .pred p, l;\n\tsetp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 l, %6, 0;\n\t"
+        "@l tcgen05.mma.cta_group::2.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%4], [%4], p;\n\t}" ::"r"(tmem_d),
+        "l"(a), "l"(b), "r"(idesc), "r"(tmem_sf), "r"(accumulate), "r"(leader)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p, l;\n\tsetp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 l, %6, 0;\n\t"
+        "@l tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%4], [%4], p;\n\t}" ::"r"(tmem_d),
+        "l"(a), "l"(b), "r"(idesc), "r"(tmem_sf), "r"(accumulate), "r"(leader)
+        : "memory");
 }
 // The same 32-bit value into 8 consecutive TMEM columns of this thread's lane.
 __device__ __forceinline__ void tmem_fill8(uint32_t taddr, uint32_t v) {
@@ -246,25 +261,34 @@ __device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t leader) {
       "r"(leader)
       : "memory");
 }
-// The same arrival on the barrier at this offset of every CTA in `mask`.
-__device__ __forceinline__ void umma_commit_multicast(uint32_t bar, uint16_t mask, uint32_t leader) {
+// A pair's commit: arrives on the barrier at this offset of both CTAs.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint32_t leader) {
   asm volatile(
-      "{\n\t.reg .pred l;\n\tsetp.ne.b32 l, %2, 0;\n\t"
-      "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(
+      "{\n\t.reg .pred l;\n\t.reg .b16 m;\n\tsetp.ne.b32 l, %1, 0;\n\tmov.b16 m, 3;\n\t"
+      "@l tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}" ::"r"(
           bar),
-      "h"(mask), "r"(leader)
+      "r"(leader)
       : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+template <int CG = 1>
 __device__ __forceinline__ void tmem_alloc(uint32_t slot_smem, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(cols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  if (CG == 2) {  // executed by one warp of either CTA of the pair
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
 }
+template <int CG = 1>
 __device__ __forceinline__ void tmem_dealloc(uint32_t tmem, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+  if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+  else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
 }
 
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }

@@ -541,7 +541,7 @@ void launch_tc_scan(Index& I, const float* q, int nq, int k, lshg_point* out, cu
   int* err = I.error_word(s);
   const int64_t qpad = (int64_t)ceil_div(nq, BM) * BM;
   const int QT = (int)(qpad / BM);
-  FilterPlan plan = plan_filter(I.n, CT);
+  FilterPlan plan = plan_filter(I.n, CT, nq);
   // test hook: LSHG_TC_FORCE_FALLBACK=1 sends every query through the list kernel, so
   // tests can compare the two selection paths on the same inputs
   if (const char* e = getenv("LSHG_TC_FORCE_FALLBACK"); e && e[0] == '1') plan.cap = 0;
@@ -549,21 +549,15 @@ void launch_tc_scan(Index& I, const float* q, int nq, int k, lshg_point* out, cu
   LSHG_REQUIRE((int64_t)QT * NT < (int64_t)INT_MAX, "tensor-core scan: problem too large");
   DevBuf<uint16_t> qbf((size_t)qpad * KD, s);
   to_unit_bf16(q, nq, I.d, qpad, qbf.ptr, s);
-  const CUtensorMap ma = make_map(qbf.ptr, qpad);
   const int64_t npad = (int64_t)ceil_div(I.n, FILTER_TN) * FILTER_TN;
-  const CUtensorMap mb = make_map(I.xbf.ptr, npad);                    // list kernel: 128-row boxes
-  const CUtensorMap mb256 = make_map(I.xbf.ptr, npad, FILTER_TN);      // filter: 256-row boxes
-  // the filter's second 64-column half only up to the last K step (columns 64..16*ksteps)
-  const int hi_cols = std::max(8, std::min(KHALF, 16 * tc_ksteps(I.d) - KHALF));
-  const CUtensorMap mb256hi = make_map(I.xbf.ptr, npad, FILTER_TN, hi_cols);
+  const CUtensorMap mb = make_map(I.xbf.ptr, npad);  // list kernel: 128-row boxes
   DevBuf<uint8_t> qf8;
-  CUtensorMap ma8{}, mb8{};
   if (e4m3) {
     qf8.alloc((size_t)qpad * KD, s);
     to_unit_e4m3(q, nq, I.d, qpad, qf8.ptr, s);
-    ma8 = make_map_e4m3(qf8.ptr, qpad, BM);
-    mb8 = make_map_e4m3(I.xf8.ptr, npad, FILTER_TN);
   }
+  const FilterMaps maps = e4m3 ? make_filter_maps(qf8.ptr, qpad, I.xf8.ptr, npad, I.d, true)
+                               : make_filter_maps(qbf.ptr, qpad, I.xbf.ptr, npad, I.d, false);
 
   // 1-2. thresholds and survivors
   DevBuf<float> tau((size_t)nq, s);
@@ -571,12 +565,7 @@ void launch_tc_scan(Index& I, const float* q, int nq, int k, lshg_point* out, cu
   int* ovf = cnt.ptr + nq;
   LSHG_CUDA(cudaMemsetAsync(cnt.ptr, 0, (size_t)(nq + 1) * sizeof(int), s));
   DevBuf<uint64_t> cand((size_t)nq * plan.cap, s);
-  if (e4m3)
-    launch_filter_scan(ma8, mb8, mb8, hi_cols, plan, nq, I.n, I.d, QT, CT, tau.ptr, cnt.ptr, cand.ptr, err, true,
-                       s);
-  else
-    launch_filter_scan(ma, mb256, mb256hi, hi_cols, plan, nq, I.n, I.d, QT, CT, tau.ptr, cnt.ptr, cand.ptr, err,
-                       false, s);
+  launch_filter_scan(maps, plan, nq, I.n, I.d, QT, tau.ptr, cnt.ptr, cand.ptr, err, s);
 
   // 3. top-CT of the survivors
   DevBuf<uint64_t> best((size_t)nq * CT, s);
