@@ -323,7 +323,7 @@ Index::~Index() {
   x.release(); xnorm.release(); xt.release(); xs.release(); xse.release(); xsl.release(); xsf.release(); xsft.release();
   sk_planes.release(); sk_split.release(); sk_pnorm.release();
   keys.release(); offsets.release(); buckets.release(); key_planes.release(); cp_diag.release(); bitmaps.release();
-  xbf.release(); xbf_scale.release(); xf8.release(); xnorm64.release(); xst.release(); qstats.release();
+  xbf.release(); xbf_scale.release(); xf8.release(); ebf.release(); ebf_res.release(); xnorm64.release(); xst.release(); qstats.release();
   cws_tab.release(); cws_rank.release(); cws_key_tab.release();
   for (auto* ops : {&ops_keys, &ops_sketch})
     for (auto& op : *ops)
@@ -533,6 +533,7 @@ std::unique_ptr<Index> build_index(const lshg_index_params& p, DevBuf<float>&& b
   if (p.framework == 0 && impl == 2) {
     I.xt.alloc((size_t)ceil_div(n, 128) * 128 * d, s);
     launch_tile_transpose(X, n, d, I.xt.ptr, s);
+    derive_exact(I, s);
   }
   if (p.framework == 0 && (impl == 8 || impl == 9)) tc_prepare(I, s);
   if (p.framework == 1) I.lsh_grid = lsh_query_grid(1 << 30);
@@ -632,6 +633,7 @@ void query_index(Index& I, float* q, int nq, int k, lshg_point* out, cudaStream_
     return;
   }
   if (impl == 2) {
+    if (query_exact_filtered(I, q, nq, qnorm.ptr, k, out, s)) return;
     const int C = kp;
     int splits = scan_float_splits(I.n, nq, C);
     DevBuf<uint64_t> part((size_t)nq * splits * C, s);

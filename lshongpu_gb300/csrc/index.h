@@ -91,6 +91,13 @@ struct Index {
   DevBuf<double> xnorm64;    // base row norms in double for the FP64 re-check (derived, not stored)
   int dp = 0;
 
+  // Exact angular scan (implementation 2, d <= 128): BF16 unit rows for the tensor-core
+  // candidate filter of scan_exact.cu and the largest residual |x/|x| - row| (derived, not
+  // stored).  Empty when a base row has no bounded score error (zero, non-finite or extreme
+  // norm): such a base takes the FP32 scan.
+  DevBuf<uint16_t> ebf;
+  DevBuf<float> ebf_res;
+
   // Device error words of the query path (a pipeline or row-copy wait that timed out,
   // the weighted-MinHash draw limit), one per stream that has run queries on this index:
   // the kernels of a batch raise the word of the stream they run on, and a sync on a
@@ -142,6 +149,13 @@ void tile_sketches(Index& idx, cudaStream_t stream);
 // and the split SimHash planes of the tensor-core projection.
 void derive_tc(Index& idx, cudaStream_t stream);
 void derive_simhash(Index& idx, cudaStream_t stream);
+// The exact angular scan's BF16 rows (Index::ebf); waits for the stream.
+void derive_exact(Index& idx, cudaStream_t stream);
+// Exact angular top-k through the tensor-core filter (scan_exact.cu): the ids and distances of
+// the FP32 scan.  False when the index, k or the batch is not one it serves, or its
+// temporaries do not fit: nothing has been written to `out` then.
+bool query_exact_filtered(Index& idx, const float* q, int nq, const float* qnorm, int k, lshg_point* out,
+                          cudaStream_t stream);
 
 // Persistence (persist.cpp): checksummed binary image of a built index.
 void save_index(const Index& idx, const char* path);

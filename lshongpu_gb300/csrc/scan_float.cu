@@ -13,6 +13,8 @@
 // (distanceFunctions.cuh:23-40), and generalized Jaccard is 1 - sum(min)/sum(max)
 // (distanceFunctions.cuh:10-21).  Exact-scan distances are therefore bit-identical to
 // the reference's; only the selection order differs (ties by lower index).
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "launch_count.h"
@@ -300,10 +302,13 @@ __device__ __noinline__ uint64_t merge_candidates(uint64_t* list, uint64_t k0, u
   return __shfl_sync(0xffffffffu, best[EC - 1], 31);
 }
 
+// The scan of query block q0 .. q0 + 63 over the tiles of one split.  rows: the queries' rows of
+// q (nullptr: themselves).
 template <int DIST, int EC>
-__global__ void __launch_bounds__(256, 2) scan_float_reg_kernel(
+__device__ __forceinline__ void scan_reg_block(
     const float* __restrict__ xt, int64_t n, int d, const float* __restrict__ xnorm, const float* __restrict__ q,
-    int nq, const float* __restrict__ qnorm, int tiles_per_split, int splits, int nbuf, uint64_t* __restrict__ out) {
+    int nq, const float* __restrict__ qnorm, int tiles_per_split, int splits, int nbuf, uint64_t* __restrict__ out,
+    int q0, int split, const int* __restrict__ rows) {
   constexpr int C = 32 * EC;
   extern __shared__ __align__(16) unsigned char smem[];
   size_t off = 0;
@@ -314,8 +319,6 @@ __global__ void __launch_bounds__(256, 2) scan_float_reg_kernel(
   uint64_t* scratch = reinterpret_cast<uint64_t*>(smem + smem_take(off, (size_t)8 * 32 * 8));
   uint64_t* cbuf = reinterpret_cast<uint64_t*>(smem + smem_take(off, (size_t)kRegQB * kRegBuf * 8));
 
-  const int q0 = blockIdx.x * kRegQB;
-  const int split = blockIdx.y;
   const int ntiles = (int)((n + kTile - 1) / kTile);
   const int t_begin = split * tiles_per_split;
   const int t_end = min(ntiles, t_begin + tiles_per_split);
@@ -323,10 +326,10 @@ __global__ void __launch_bounds__(256, 2) scan_float_reg_kernel(
 
   for (int i = threadIdx.x; i < kRegQB * d; i += blockDim.x) {
     const int qi = i / d, j = i - qi * d;
-    qs[j * kRegQB + qi] = (q0 + qi < nq) ? q[(int64_t)(q0 + qi) * d + j] : 0.0f;
+    qs[j * kRegQB + qi] = (q0 + qi < nq) ? q[(int64_t)(rows ? rows[q0 + qi] : q0 + qi) * d + j] : 0.0f;
   }
   for (int qi = threadIdx.x; qi < kRegQB; qi += blockDim.x)
-    qn[qi] = (DIST == DIST_ANGULAR && q0 + qi < nq) ? qnorm[q0 + qi] : 1.0f;
+    qn[qi] = (DIST == DIST_ANGULAR && q0 + qi < nq) ? qnorm[rows ? rows[q0 + qi] : q0 + qi] : 1.0f;
   for (int i = threadIdx.x; i < kRegQB * C; i += blockDim.x) lists[i] = kEmptyKey;
   __syncthreads();  // lists are read by their owning warps (and written out even for an empty split)
   uint64_t thr[8];
@@ -460,6 +463,75 @@ __global__ void __launch_bounds__(256, 2) scan_float_reg_kernel(
 }
 
 template <int DIST, int EC>
+__global__ void __launch_bounds__(256, 2) scan_float_reg_kernel(
+    const float* __restrict__ xt, int64_t n, int d, const float* __restrict__ xnorm, const float* __restrict__ q,
+    int nq, const float* __restrict__ qnorm, int tiles_per_split, int splits, int nbuf, uint64_t* __restrict__ out) {
+  scan_reg_block<DIST, EC>(xt, n, d, xnorm, q, nq, qnorm, tiles_per_split, splits, nbuf, out, blockIdx.x * kRegQB,
+                           blockIdx.y, nullptr);
+}
+
+// The listed queries (list[0] of them): CTAs take (query block, split) items in turn, so that a
+// handful of queries still spreads over every SM and an empty list ends at once.
+template <int DIST, int EC>
+__global__ void __launch_bounds__(256, 2) scan_float_listed_kernel(
+    const float* __restrict__ xt, int64_t n, int d, const float* __restrict__ xnorm, const float* __restrict__ q,
+    const float* __restrict__ qnorm, const int* __restrict__ list, int tiles_per_split, int splits, int nbuf,
+    uint64_t* __restrict__ out) {
+  const int nq = list[0];
+  const int items = (nq + kRegQB - 1) / kRegQB * splits;
+  for (int it = blockIdx.x; it < items; it += gridDim.x) {
+    scan_reg_block<DIST, EC>(xt, n, d, xnorm, q, nq, qnorm, tiles_per_split, splits, nbuf, out,
+                             it / splits * kRegQB, it % splits, list + 1);
+    __syncthreads();  // the item's shared memory is done with
+  }
+}
+
+// The first k of each listed query's `splits` sorted lists of C keys, as points into its row of
+// `out` (one block a query).
+__global__ void listed_points_kernel(const uint64_t* __restrict__ part, const int* __restrict__ list, int splits, int C,
+                                     int k, lshg_point* __restrict__ out) {
+  extern __shared__ uint64_t ms[];
+  const int cnt = list[0];
+  for (int i = blockIdx.x; i < cnt; i += gridDim.x) {
+    const uint64_t* src = part + (int64_t)i * splits * C;
+    for (int j = threadIdx.x; j < C; j += blockDim.x) ms[j] = src[j];
+    __syncthreads();
+    for (int sp = 1; sp < splits; ++sp) {
+      for (int j = threadIdx.x; j < C; j += blockDim.x) {
+        const uint64_t b = src[(int64_t)sp * C + C - 1 - j];
+        if (b < ms[j]) ms[j] = b;
+      }
+      __syncthreads();
+      block_bitonic_merge(ms, C);
+    }
+    const int q = list[1 + i];
+    for (int j = threadIdx.x; j < k; j += blockDim.x) {
+      lshg_point pt;
+      if (ms[j] == kEmptyKey) { pt.ID = -1; pt.distance = kEmptyDistance; }
+      else { pt.ID = key_id(ms[j]); pt.distance = key_dist(ms[j]); }
+      out[(int64_t)q * k + j] = pt;
+    }
+    __syncthreads();
+  }
+}
+
+template <int EC>
+void launch_listed(const float* xt, int64_t n, int d, const float* xnorm, const float* q, const float* qnorm,
+                   const int* list, int splits, uint64_t* part, cudaStream_t s) {
+  const int nbuf = reg_scan_smem(d, 32 * EC, 1) <= kRegTwoCtaSmem ? 1 : 2;
+  size_t smem = reg_scan_smem(d, 32 * EC, nbuf);
+  const int nb = smem <= 220 * 1024 ? nbuf : 1;
+  smem = reg_scan_smem(d, 32 * EC, nb);
+  LSHG_REQUIRE(smem <= 220 * 1024, "listed scan: dimension too large");
+  auto kern = scan_float_listed_kernel<DIST_ANGULAR, EC>;
+  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int tps = ceil_div(ceil_div(n, kTile), splits);
+  kern<<<num_sms() * 2, 256, smem, s>>>(xt, n, d, xnorm, q, qnorm, list, tps, splits, nb, part);
+  count_launch();
+  LSHG_CHECK_LAUNCH();
+}
+
+template <int DIST, int EC>
 void launch_reg(const float* xt, int64_t n, int d, const float* xnorm, const float* q, int nq, const float* qnorm,
                 int splits, int nbuf, uint64_t* out, cudaStream_t s) {
   ProfScope _ps("scan_float", s);
@@ -556,6 +628,25 @@ int scan_float_splits(int64_t n, int nq, int C) {
     }
   }
   return best;
+}
+
+int scan_listed_splits(int64_t n, int nq, int C) {
+  // as many as spread one 64-query block over the SMs, while the lists stay below 256 MB
+  const int64_t fit = ((int64_t)256 << 20) / ((int64_t)nq * C * 8);
+  return (int)std::max<int64_t>(1, std::min<int64_t>({fit, 128, std::max(1, ceil_div(n, kTile) / 4)}));
+}
+
+void launch_scan_float_listed(const float* xt, int64_t n, int d, const float* xnorm, const float* q, int nq,
+                              const float* qnorm, const int* list, int C, int splits, uint64_t* part, int k,
+                              lshg_point* out, cudaStream_t s) {
+  ProfScope _ps("scan_float_listed", s);
+  if (C == 32) launch_listed<1>(xt, n, d, xnorm, q, qnorm, list, splits, part, s);
+  else if (C == 64) launch_listed<2>(xt, n, d, xnorm, q, qnorm, list, splits, part, s);
+  else if (C == 128) launch_listed<4>(xt, n, d, xnorm, q, qnorm, list, splits, part, s);
+  else throw Error(LSHG_ERR_INVALID_ARGUMENT, "listed scan: C must be 32, 64 or 128");
+  listed_points_kernel<<<std::min(nq, num_sms() * 4), 128, (size_t)C * 8, s>>>(part, list, splits, C, k, out);
+  count_launch();
+  LSHG_CHECK_LAUNCH();
 }
 
 int launch_scan_float(const float* xt, int64_t n, int d, const float* xnorm, const float* q, int nq,

@@ -423,11 +423,20 @@ __device__ __forceinline__ bool digit_of_rank(const unsigned* hist, int kk, int 
   return true;
 }
 
+// The threshold a query filters with: t - margin, lowered by 2 eps[q] where given (+inf, no
+// survivor, when that is not finite).
+__device__ __forceinline__ float lowered_tau(float t, float margin, const float* __restrict__ eps, int q) {
+  if (!eps) return t - margin;
+  const float e = eps[q];
+  return e < 1e30f ? t - margin - 2.0f * e : INFINITY;
+}
+
 // tau[q] = (CT-th largest of the row's M group maxima) - margin, or -inf when the row has
 // fewer than CT finite-or-infinite (non-NaN) maxima.  One warp per query: a 4-pass
 // 8-bit radix select on order-preserving keys, histogram in shared memory.
 __global__ void __launch_bounds__(256) tau_select_kernel(const float* __restrict__ gmax, int nq, int M, int CT,
-                                                          float margin, float* __restrict__ tau) {
+                                                          float margin, float* __restrict__ tau,
+                                                          const float* __restrict__ eps) {
   __shared__ unsigned hist[8][256];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q = blockIdx.x * 8 + w;
@@ -447,7 +456,7 @@ __global__ void __launch_bounds__(256) tau_select_kernel(const float* __restrict
     __syncwarp();
     int digit = 0, rem = 0;
     if (!digit_of_rank(hist[w], kk, lane, digit, rem)) {  // fewer than CT usable maxima (first pass only)
-      if (lane == 0) tau[q] = -INFINITY;
+      if (lane == 0) tau[q] = lowered_tau(-INFINITY, margin, eps, q);
       return;
     }
     prefix |= (uint32_t)digit << shift;
@@ -455,7 +464,7 @@ __global__ void __launch_bounds__(256) tau_select_kernel(const float* __restrict
     kk = rem;
     __syncwarp();
   }
-  if (lane == 0) tau[q] = ordered_to_float(prefix) - margin;
+  if (lane == 0) tau[q] = lowered_tau(ordered_to_float(prefix), margin, eps, q);
 }
 
 // tau_select_kernel for rows of at most 32 * R maxima (a multiple of 4), read once into
@@ -470,7 +479,8 @@ __global__ void __launch_bounds__(256) tau_select_kernel(const float* __restrict
 // largest is -inf, and so is tau, as in the exact select.
 template <int R>
 __global__ void __launch_bounds__(256) tau_select_reg_kernel(const float* __restrict__ gmax, int nq, int M, int CT,
-                                                              float margin, float* __restrict__ tau) {
+                                                              float margin, float* __restrict__ tau,
+                                                              const float* __restrict__ eps) {
   const int lane = threadIdx.x & 31;
   const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (q >= nq) return;  // warp-uniform
@@ -497,7 +507,7 @@ __global__ void __launch_bounds__(256) tau_select_reg_kernel(const float* __rest
     }
   }
   if (__reduce_add_sync(0xffffffffu, valid) < CT) {
-    if (lane == 0) tau[q] = -INFINITY;
+    if (lane == 0) tau[q] = lowered_tau(-INFINITY, margin, eps, q);
     return;
   }
   kmax = __reduce_max_sync(0xffffffffu, kmax);
@@ -512,7 +522,33 @@ __global__ void __launch_bounds__(256) tau_select_reg_kernel(const float* __rest
     if (__reduce_add_sync(0xffffffffu, c) >= CT) lo = mid;
     else hi = mid;
   }
-  if (lane == 0) tau[q] = ordered_to_float((uint32_t)lo) - margin;
+  if (lane == 0) tau[q] = lowered_tau(ordered_to_float((uint32_t)lo), margin, eps, q);
+}
+
+// The 32*E smallest of c keys, ascending (element e * 32 + lane), by one warp: sort each chunk
+// and merge it into the running result.
+template <int E>
+__device__ __forceinline__ void warp_top(const uint64_t* __restrict__ src, int c, int lane, uint64_t (&best)[E]) {
+  constexpr int CT = 32 * E;
+#pragma unroll
+  for (int e = 0; e < E; ++e) best[e] = kEmptyKey;
+  for (int base = 0; base < c; base += CT) {
+    uint64_t x[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int i = base + e * 32 + lane;
+      x[e] = i < c ? src[i] : kEmptyKey;
+    }
+    warp_bitonic<E>(x, lane, false);
+    // best ascending, x ascending: min(best[i], x[CT-1-i]) is bitonic and holds the CT
+    // smallest of the union
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const uint64_t r = __shfl_sync(0xffffffffu, x[E - 1 - e], 31 - lane);
+      best[e] = best[e] < r ? best[e] : r;
+    }
+    warp_bitonic<E>(best, lane, true);
+  }
 }
 
 // Per query (one warp): the CT = 32*E smallest keys of the survivors -- sort each chunk of
@@ -535,29 +571,49 @@ __global__ void __launch_bounds__(256) cand_select_kernel(const int* __restrict_
     if (lane == 0) ovf[1 + atomicAdd(ovf, 1)] = q;
     return;
   }
-  const uint64_t* src = cand + (int64_t)q * cap;
+  uint64_t best[E];
+  warp_top<E>(cand + (int64_t)q * cap, c, lane, best);
+#pragma unroll
+  for (int e = 0; e < E; ++e) dst[e * 32 + lane] = best[e];
+}
+
+// launch_exact_select: keys order by score, so the sorted top-CT gives the k-th best score and
+// the candidates are a prefix of it.
+template <int E>
+__global__ void __launch_bounds__(256) exact_select_kernel(const int* __restrict__ cnt,
+                                                            const uint64_t* __restrict__ cand, int cap, int k, int nq,
+                                                            const float* __restrict__ tau,
+                                                            const float* __restrict__ eps, uint64_t* __restrict__ out,
+                                                            int* __restrict__ ovf) {
+  constexpr int CT = 32 * E;
+  const int lane = threadIdx.x & 31;
+  const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (q >= nq) return;  // warp-uniform
+  const int c = cnt[q];
+  const float e2 = 2.0f * eps[q];
+  uint64_t* dst = out + (int64_t)q * CT;
+  bool listed = c > cap || c < k || !(e2 < 1e30f);
   uint64_t best[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) best[e] = kEmptyKey;
-  for (int base = 0; base < c; base += CT) {
-    uint64_t x[E];
+  float cut = 0.0f;
+  if (!listed) {
+    warp_top<E>(cand + (int64_t)q * cap, c, lane, best);
+    uint64_t kth = kEmptyKey, last = kEmptyKey;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-      const int i = base + e * 32 + lane;
-      x[e] = i < c ? src[i] : kEmptyKey;
+      const uint64_t v = __shfl_sync(0xffffffffu, best[e], (k - 1) & 31);
+      if (e == (k - 1) >> 5) kth = v;
+      last = best[e];
     }
-    warp_bitonic<E>(x, lane, false);
-    // best ascending, x ascending: min(best[i], x[CT-1-i]) is bitonic and holds the CT
-    // smallest of the union
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const uint64_t r = __shfl_sync(0xffffffffu, x[E - 1 - e], 31 - lane);
-      best[e] = best[e] < r ? best[e] : r;
-    }
-    warp_bitonic<E>(best, lane, true);
+    last = __shfl_sync(0xffffffffu, last, 31);
+    cut = -key_dist(kth) - e2;  // scores from here up
+    listed = (tau && tau[q] > cut) || (last != kEmptyKey && c > CT && -key_dist(last) >= cut);
   }
 #pragma unroll
-  for (int e = 0; e < E; ++e) dst[e * 32 + lane] = best[e];
+  for (int e = 0; e < E; ++e)
+    dst[e * 32 + lane] = !listed && best[e] != kEmptyKey && -key_dist(best[e]) >= cut ? best[e] : kEmptyKey;
+  if (listed && lane == 0) ovf[1 + atomicAdd(ovf, 1)] = q;
 }
 
 // Compact the bf16 rows of the listed queries into rows 0..count-1 of `dst` (the rest of
@@ -733,7 +789,7 @@ FilterMaps make_filter_maps(const void* q, int64_t qrows, const void* base, int6
 }
 
 void launch_filter_scan(const FilterMaps& m, const FilterPlan& plan, int nq, int64_t n, int d, int QT, float* tau,
-                        int* cnt, uint64_t* cand, int* err, cudaStream_t s) {
+                        int* cnt, uint64_t* cand, int* err, cudaStream_t s, const float* eps) {
   FilterArgs a{};
   a.hi_bytes = m.hi_cols * 2;
   a.nq = nq;
@@ -751,7 +807,7 @@ void launch_filter_scan(const FilterMaps& m, const FilterPlan& plan, int nq, int
     a.M = plan.M;
     if (plan.GW == 64) run_filter_fmt<MODE_GROUPMAX, 64>(m, a, "tc_prepass", s);
     else run_filter_fmt<MODE_GROUPMAX, 8>(m, a, "tc_prepass", s);
-    launch_tau_select(gmax.ptr, nq, plan.M, plan.rank, margin, tau, s);
+    launch_tau_select(gmax.ptr, nq, plan.M, plan.rank, margin, tau, s, eps);
   }
   a.gmax = nullptr;
   a.M = 0;
@@ -764,15 +820,16 @@ void launch_filter_scan(const FilterMaps& m, const FilterPlan& plan, int nq, int
   run_filter_fmt<MODE_FILTER, 64>(m, a, "tc_filter", s);
 }
 
-void launch_tau_select(const float* gmax, int nq, int M, int rank, float margin, float* tau, cudaStream_t s) {
+void launch_tau_select(const float* gmax, int nq, int M, int rank, float margin, float* tau, cudaStream_t s,
+                       const float* eps) {
   ProfScope _ps("tc_tau_select", s);
   // the register slots a lane walks in every bisection step: as few as cover M
   if (M <= 32 * kTauRegsFew && M % 4 == 0)
-    tau_select_reg_kernel<kTauRegsFew><<<ceil_div(nq, 8), 256, 0, s>>>(gmax, nq, M, rank, margin, tau);
+    tau_select_reg_kernel<kTauRegsFew><<<ceil_div(nq, 8), 256, 0, s>>>(gmax, nq, M, rank, margin, tau, eps);
   else if (M <= 32 * kTauRegs && M % 4 == 0)
-    tau_select_reg_kernel<kTauRegs><<<ceil_div(nq, 8), 256, 0, s>>>(gmax, nq, M, rank, margin, tau);
+    tau_select_reg_kernel<kTauRegs><<<ceil_div(nq, 8), 256, 0, s>>>(gmax, nq, M, rank, margin, tau, eps);
   else
-    tau_select_kernel<<<ceil_div(nq, 8), 256, 0, s>>>(gmax, nq, M, rank, margin, tau);
+    tau_select_kernel<<<ceil_div(nq, 8), 256, 0, s>>>(gmax, nq, M, rank, margin, tau, eps);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -784,6 +841,16 @@ void launch_cand_select(const int* cnt, const uint64_t* cand, int nq, int cap, i
   else if (CT == 64) cand_select_kernel<2><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf);
   else if (CT == 128) cand_select_kernel<4><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf);
   else throw Error(LSHG_ERR_INVALID_ARGUMENT, "tensor-core scan: candidate count must be 32, 64 or 128");
+  count_launch();
+  LSHG_CHECK_LAUNCH();
+}
+
+void launch_exact_select(const int* cnt, const uint64_t* cand, int nq, int cap, int k, int CT, const float* tau,
+                         const float* eps, uint64_t* out, int* ovf, cudaStream_t s) {
+  ProfScope _ps("exact_select", s);
+  if (CT == 128) exact_select_kernel<4><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, k, nq, tau, eps, out, ovf);
+  else if (CT == 256) exact_select_kernel<8><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, k, nq, tau, eps, out, ovf);
+  else throw Error(LSHG_ERR_INVALID_ARGUMENT, "exact scan: candidate count must be 128 or 256");
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

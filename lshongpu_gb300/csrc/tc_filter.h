@@ -42,17 +42,28 @@ struct FilterMaps {
 FilterMaps make_filter_maps(const void* q, int64_t qrows, const void* base, int64_t brows, int d, bool e4m3);
 
 // Prepass + threshold selection + filter pass: fills cnt[q] and cand[q][0..cap).
+// eps (optional, [nq]): thresholds are lowered by 2 eps[q]; a query whose eps is not finite keeps
+// no survivor.
 void launch_filter_scan(const FilterMaps& m, const FilterPlan& plan, int nq, int64_t n, int d, int QT, float* tau,
-                        int* cnt, uint64_t* cand, int* err, cudaStream_t s);
+                        int* cnt, uint64_t* cand, int* err, cudaStream_t s, const float* eps = nullptr);
 
 // tau[q] = a lower bound (within 1/65536 of the row's range) of the rank-th largest of the
 // row's M group maxima, minus margin; -inf when the row holds fewer than rank maxima.
-void launch_tau_select(const float* gmax, int nq, int M, int rank, float margin, float* tau, cudaStream_t s);
+void launch_tau_select(const float* gmax, int nq, int M, int rank, float margin, float* tau, cudaStream_t s,
+                       const float* eps = nullptr);
 
 // Top-CT keys a query from its survivors (CT = 32, 64 or 128); queries with more survivors
 // than cap or fewer than `need` are listed in ovf for the exact fallback.
 void launch_cand_select(const int* cnt, const uint64_t* cand, int nq, int cap, int need, int CT, uint64_t* out,
                         int* ovf, cudaStream_t s);
+
+// The candidates of an exact top-k among a query's survivors: every point whose score is
+// within 2 eps[q] of the k-th best one, out of the top-CT (CT = 128 or 256; the rest of the row
+// is empty keys).  Listed in ovf instead: queries with more survivors than cap or fewer than
+// k, with more than CT candidates, whose threshold tau[q] (nullptr: none) does not reach that
+// far down, or whose eps is not finite.
+void launch_exact_select(const int* cnt, const uint64_t* cand, int nq, int cap, int k, int CT, const float* tau,
+                         const float* eps, uint64_t* out, int* ovf, cudaStream_t s);
 
 // Tensor-core sketch scan (tc_hamming.cu): threshold plan for a base of n points and the
 // top-C of each query.  ok = false: no prepass shape bounds C well (use the popcount scan).

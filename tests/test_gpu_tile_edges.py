@@ -63,3 +63,79 @@ def test_filter_scan_edges_equal_list_kernel(engine, monkeypatch, n, nq, k, d, i
         assert len(set(a["ID"].tolist())) == k
         for i, dist in zip(a["ID"].tolist(), a["distance"].tolist()):
             assert exact.get(i, dist) == dist
+
+
+def scan_fp32(engine, idx, q, k):
+    """The FP32 scan of an exact index (the allocation-free entry point runs nothing else)."""
+    import torch
+
+    dq = torch.from_numpy(q).cuda()
+    out = torch.empty((q.shape[0], k, 2), dtype=torch.int32, device="cuda")
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    assert engine.lib().lshg_index_query_noalloc(idx.handle, dq.data_ptr(), q.shape[0], k, out.data_ptr(),
+                                                 st.cuda_stream) == 0
+    torch.cuda.synchronize()
+    return out.cpu().numpy().view(engine.POINT_DTYPE).reshape(q.shape[0], k)
+
+
+@pytest.mark.parametrize("n,nq,k,d", [
+    (4096, 1, 1, 16),        # the smallest filtered base; one K step; one neighbour
+    (4097, 129, 32, 64),     # one point in the last tile; a query tile of one row
+    (20011, 257, 33, 65),    # 256 candidates; a second K chunk of one step
+    (70000, 300, 128, 100),  # the largest filtered k
+    (70000, 300, 10, 127),   # rows that are not 16-byte multiples
+    (300000, 700, 32, 100),  # a sampled prepass
+    (5000, 40, 200, 100),    # k beyond the filter: the FP32 scan
+    (5000, 40, 32, 129),     # d beyond it
+])
+def test_exact_filter_equals_fp32_scan(engine, monkeypatch, n, nq, k, d):
+    """Ids and distances of the filtered exact scan, and of its listed form, are the FP32
+    scan's bit for bit; queries with no direction, no finite norm or a norm out of range
+    included, and scaled queries (angular distance does not see the scale, FP32 rounding does)."""
+    x, q = data(n, nq, d)
+    q[::7] *= np.float32(1000.3)
+    q[1::11] *= np.float32(1e-9)
+    if nq > 20:
+        q[3] = 0
+        q[5, 0] = np.nan
+        q[7, d - 1] = np.inf
+        q[9] *= np.float32(1e18)
+        q[11] *= np.float32(1e-25)
+        q[13] = x[n - 1]
+    idx = engine.Index(x, implementation=2, distanceFunc=1)
+    want = scan_fp32(engine, idx, q, k)
+    assert idx.query(q, k).tobytes() == want.tobytes()
+    monkeypatch.setenv("LSHG_TC_FORCE_FALLBACK", "1")
+    assert idx.query(q, k).tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("case", ["duplicates", "near ties", "zero row", "nan row", "huge row", "isotropic"])
+def test_exact_filter_hard_bases(engine, case):
+    """Bases that leave the filter too many candidates, or none of its bounds, give the FP32
+    scan's results too."""
+    n, d, nq, k = 30000, 100, 150, 32
+    x, q = data(n, nq, d)
+    if case == "duplicates":
+        x[::2] = x[0]
+        q[:50] = x[0]
+    elif case == "near ties":  # every point within the scores' error of every other
+        rng = np.random.default_rng(3)
+        x = (x[:1] + 1e-4 * rng.standard_normal((n, d))).astype(np.float32)
+    elif case == "isotropic":
+        rng = np.random.default_rng(4)
+        x, q = rng.standard_normal((n, d)).astype(np.float32), rng.standard_normal((nq, d)).astype(np.float32)
+    else:
+        x[12345] = {"zero row": 0.0, "nan row": np.nan, "huge row": 1e17}[case]
+    idx = engine.Index(x, implementation=2, distanceFunc=1)
+    assert idx.query(q, k).tobytes() == scan_fp32(engine, idx, q, k).tobytes()
+
+
+def test_exact_filter_saved_index(engine, tmp_path):
+    """A loaded exact index derives the filter's rows again; its file does not hold them."""
+    x, q = data(9000, 200)
+    idx = engine.Index(x, implementation=2, distanceFunc=1)
+    path = str(tmp_path / "exact.lshg")
+    idx.save(path)
+    assert (tmp_path / "exact.lshg").stat().st_size < 9000 * 100 * 4 * 2.2
+    assert engine.Index.load(path).query(q, 32).tobytes() == idx.query(q, 32).tobytes()
