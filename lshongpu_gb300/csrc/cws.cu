@@ -25,8 +25,8 @@
 // code is replaced by its rank in its position's dictionary (a byte; 255 for a code the
 // base does not have there), so the scan compares bytes like the byte weighted MinHash;
 // otherwise the 16-bit codes are kept.  The codes are bit-sliced into 8 or 16 planes and
-// go through the byte scan's threshold filter (slice_filter.cuh).  Batches below 64 queries, queries whose
-// survivors the filter cannot select exactly, and bases whose codes would need more than
+// go through the byte scan's threshold filter (slice_filter.cuh).  Queries whose survivors
+// the filter cannot select exactly, candidate lists too long for the base, and bases whose codes would need more than
 // 16 bits are scanned directly over the (index, t) pairs.  Either way the candidates are
 // the exact top-C by (1 - matches / S, id).
 #include <cmath>
@@ -497,7 +497,7 @@ void launch_cws_scan(const uint32_t* xsl_t, const uint32_t* xst, int64_t n, int 
   ProfScope _ps("scan_cws", s);
   const int ng = (S + 31) / 32;
   int fs = 0, fr = 0, fc = 0;
-  if (c.pl && xsl_t && nq >= 64 && byte_filter_plan(n, C, &fs, &fr, &fc)) {
+  if (c.pl && xsl_t && byte_filter_plan(n, C, &fs, &fr, &fc)) {
     DevBuf<uint32_t> qsl((size_t)nq * ng * c.pl, s);
     launch_cws_slice(qs, nq, S, d, c, true, qsl.ptr, s);
     DevBuf<int> list((size_t)nq + 1, s);

@@ -19,9 +19,22 @@
 
 namespace lshg {
 
-// Batches from this many queries up take the tensor-core sketch scan by default (a
-// 128-query tile is the MMA's M; below this most of it would be padding).
-constexpr int kTcSketchMinQueries = 64;
+// The tensor-core sketch scan takes every batch but the smallest on short candidate lists: a
+// 128-query tile is mostly padding for a few queries, but the scan then costs little more than
+// reading the base once, where the popcount scan folds each query's candidates by itself.
+// Measured, popcount against tensor cores: 1.2M x 1,024 bits, C = 128: one query 325 / 199 us, 16
+// 1,141 / 214; C = 1,024: one 827 / 203, 63 3,061 / 231; 10k points, C = 128: one 95 / 100, four
+// 106 / 107, 16 155 / 114; C = 1,024: one 180 / 94.
+constexpr int kTcSketchLongList = 128;       // candidates above which every batch takes it
+constexpr int64_t kTcSketchMinPairs = 65536; // (query, point) pairs from which every list does
+// Byte samples: a CTA of the filter serves 64 queries, and even one query's pass beats the scan
+// that keeps its top-C as it goes, down to 32 candidates of 10,000 points.  Popcount against
+// filter, 256 samples: 500k points, C = 4,096: one query 1,339 / 341 us, 64 2,301 / 450; C = 128:
+// one 334 / 313, 64 1,374 / 388; 10k points: C = 128 one 114 / 114, C = 32 one 102 / 114, 16 215 / 175.
+constexpr int64_t kByteFilterMinPairs = 16384;
+bool tensor_sketch_batch(int64_t n, int nq, int C) {
+  return C > kTcSketchLongList || (int64_t)nq * n >= kTcSketchMinPairs;
+}
 
 int next_pow2(int v) {
   int p = 1;
@@ -666,7 +679,7 @@ void query_index(Index& I, float* q, int nq, int k, lshg_point* out, cudaStream_
   } else {
     const int op = impl == 3 ? OP_HAMMING : (impl == 4 ? OP_BYTE_JACCARD : OP_ONEBIT_JACCARD);
     const int mode = I.p.opt.sketch_scan;
-    if (I.xse.ptr && (mode == 2 || (mode == 0 && nq >= kTcSketchMinQueries)) && tc::plan_hamming(I.n, C).ok) {
+    if (I.xse.ptr && (mode == 2 || (mode == 0 && tensor_sketch_batch(I.n, nq, C))) && tc::plan_hamming(I.n, C).ok) {
       // tensor cores: the exact top-C by (sketch distance, id), then the same re-rank
       part.alloc((size_t)nq * C, s);
       tc::launch_tc_hamming(I.xse.ptr, I.n, I.xst.ptr, I.wp, I.words, qs.ptr, nq, op, C, part.ptr, I.error_word(s), s);
@@ -675,7 +688,7 @@ void query_index(Index& I, float* q, int nq, int k, lshg_point* out, cudaStream_
       return;
     }
     int fs = 0, fr = 0, fc = 0;
-    if (I.xsl.ptr && C > 128 && (mode == 2 || (mode == 0 && nq >= kTcSketchMinQueries)) &&
+    if (I.xsl.ptr && (mode == 2 || C > 32 || (int64_t)nq * I.n >= kByteFilterMinPairs) &&
         byte_filter_plan(I.n, C, &fs, &fr, &fc)) {
       // byte samples: bit-sliced threshold filter, the exact top-C, then the same re-rank
       part.alloc((size_t)nq * C, s);

@@ -1,7 +1,7 @@
 // Threshold-filter scan of byte weighted-MinHash samples (implementation 4) for long
 // candidate lists: the reference's scanJaccardDistance (sketchedDistanceScanners.cuh:
 // 194-274) with the byte distance 1 - (#equal samples) / sketchDim (distanceFunctions.cuh:
-// 102-116), for C > 128 candidates and batches of 64 queries or more.
+// 102-116).
 //
 // Two changes from the per-query top-C scan of scan_bits.cu:
 //  * bit-sliced samples: a row holds, for every group of 32 samples, 8 words -- word i
@@ -113,7 +113,9 @@ bool byte_filter_plan(int64_t n, int C, int* stride, int* rank, int* cap) {
   for (int S : {16, 8, 4, 2}) {
     const double m = (double)C / S;
     const int r = (int)std::ceil(m + 4.0 * std::sqrt(m) + 8.0);
-    if ((int64_t)ceil_div(NT, S) * kTile >= 4 * (int64_t)r && r < C) {
+    // the sample holds the r-th place with room to spare (the histogram of its match counts
+    // bounds tau as tightly from a small sample as from a large one)
+    if (8 * (int64_t)ceil_div(NT, S) * kTile >= 9 * (int64_t)r && r < C) {
       *stride = S;
       *rank = r;
       int64_t c = 1024;

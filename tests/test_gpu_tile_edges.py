@@ -139,3 +139,36 @@ def test_exact_filter_saved_index(engine, tmp_path):
     idx.save(path)
     assert (tmp_path / "exact.lshg").stat().st_size < 9000 * 100 * 4 * 2.2
     assert engine.Index.load(path).query(q, 32).tobytes() == idx.query(q, 32).tobytes()
+
+
+@pytest.mark.parametrize("impl", [4, 10])
+@pytest.mark.parametrize("n,nq,S,C", [
+    (10000, 1, 256, 128),    # one query; candidates by the warp select
+    (4700, 3, 64, 1024),     # the sample barely holds the rank
+    (17000, 65, 96, 4096),   # a second block of queries; candidates a quarter of the base
+    (129, 2, 32, 32),        # one point in the second tile
+])
+def test_sample_filter_edges_equal_direct(engine, impl, n, nq, S, C):
+    """Small batches, short lists and small bases of byte MinHash (4) and consistent weighted
+    samples (10): the threshold filter's results are the direct scan's."""
+    x, q = datasets.sparse_gamma(n, D, 71), datasets.sparse_gamma(nq, D, 72)
+    res = [engine.Index(x, implementation=impl, distanceFunc=2, sketchDim=S,
+                        options=engine.make_options(candidates=C, sketch_scan=mode)).query(q, 32)
+           for mode in (0, TENSOR, POPCOUNT)]
+    assert np.array_equal(res[0], res[2])
+    assert np.array_equal(res[1], res[2])
+
+
+@pytest.mark.parametrize("n,nq,words,C", [
+    (10000, 1, 4, 128),      # below the pairs that take the tensor cores
+    (36800, 2, 8, 4096),     # the largest base that keeps every point at C = 4,096
+    (37000, 3, 8, 4096),     # 8-point maxima of every tile, rank near their number
+    (20000, 5, 32, 2048),
+])
+def test_sketch_scan_small_batches_equal_popcount(engine, n, nq, words, C):
+    x, q = data(n, nq)
+    res = [engine.Index(x, implementation=3, sketchDim=words,
+                        options=engine.make_options(candidates=C, sketch_scan=mode)).query(q, 32)
+           for mode in (0, TENSOR, POPCOUNT)]
+    assert np.array_equal(res[0], res[2])
+    assert np.array_equal(res[1], res[2])
