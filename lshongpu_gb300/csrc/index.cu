@@ -595,6 +595,11 @@ void query_index(Index& I, float* q, int nq, int k, lshg_point* out, cudaStream_
   DevBuf<float> qsf;
   DevBuf<uint16_t> qkeys;
   sketch_queries(I, q, nq, &qs, &qsf, &qkeys, s);
+  if (I.p.framework == 0 && (impl == 8 || impl == 9)) {
+    launch_tc_scan(I, q, nq, k, out, s, extra);
+    return;
+  }
+  if (I.p.framework == 0 && impl == 2 && query_exact_filtered(I, q, nq, k, out, s)) return;
   DevBuf<float> qnorm;
   if (I.dist == DIST_ANGULAR) {
     qnorm.alloc(nq, s);
@@ -641,18 +646,14 @@ void query_index(Index& I, float* q, int nq, int k, lshg_point* out, cudaStream_
     launch_lsh_query(a, out, s);
     return;
   }
-  if (impl == 8 || impl == 9) {
-    launch_tc_scan(I, q, nq, k, out, s, extra);
-    return;
-  }
   if (impl == 2) {
-    if (query_exact_filtered(I, q, nq, qnorm.ptr, k, out, s)) return;
     const int C = kp;
     int splits = scan_float_splits(I.n, nq, C);
     DevBuf<uint64_t> part((size_t)nq * splits * C, s);
     launch_scan_float(I.xt.ptr, I.n, I.d, I.xnorm.ptr, q, nq, qnorm.ptr, I.dist, C, splits, part.ptr, s);
     const uint64_t* keys = part.ptr;
     DevBuf<uint64_t> merged;
+    if (launch_merge_points(part.ptr, nq, splits, C, k, out, s)) return;
     if (splits > 1) {
       merged.alloc((size_t)nq * C, s);
       launch_merge_splits(part.ptr, nq, splits, C, merged.ptr, s);

@@ -154,8 +154,7 @@ void derive_exact(Index& idx, cudaStream_t stream);
 // Exact angular top-k through the tensor-core filter (scan_exact.cu): the ids and distances of
 // the FP32 scan.  False when the index, k or the batch is not one it serves, or its
 // temporaries do not fit: nothing has been written to `out` then.
-bool query_exact_filtered(Index& idx, const float* q, int nq, const float* qnorm, int k, lshg_point* out,
-                          cudaStream_t stream);
+bool query_exact_filtered(Index& idx, const float* q, int nq, int k, lshg_point* out, cudaStream_t stream);
 
 // Persistence (persist.cpp): checksummed binary image of a built index.
 void save_index(const Index& idx, const char* path);

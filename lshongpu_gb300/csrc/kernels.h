@@ -144,6 +144,9 @@ void launch_scan_float_listed(const float* xt, int64_t n, int d, const float* xn
                               const float* qnorm, const int* list, int C, int splits, uint64_t* part, int k,
                               struct ::lshg_point_s* out, cudaStream_t s);
 void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t* out, cudaStream_t s);
+// The same with the first k keys written as points; false when C or k is not one it serves.
+bool launch_merge_points(const uint64_t* in, int nq, int splits, int C, int k, struct ::lshg_point_s* out,
+                         cudaStream_t s);
 // Places of the FP64 re-check besides k (requests of smaller k answered from the same
 // launch); n <= 4.  Passed in device memory, so that a recorded launch can be replayed with
 // other places.
@@ -156,10 +159,12 @@ struct RerankBounds {
 // fp64_recheck: re-score, in double precision, the run of candidates around the k-th
 // place whose FP32 distances lie within the FP32 error bound of one another (among the
 // first 128) and order that run by the FP64 distance.
+// qnorm == nullptr (angular, C < 1024): the kernel computes the query norms itself, and writes
+// them to qnorm_out where given.
 void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t n, int d,
                    const float* xnorm, const float* q, const float* qnorm, int dist, int k,
                    struct ::lshg_point_s* out, cudaStream_t s, int* err = nullptr, bool fp64_recheck = false,
-                   const double* xn64 = nullptr, const RerankBounds* extra_dev = nullptr);
+                   const double* xn64 = nullptr, const RerankBounds* extra_dev = nullptr, float* qnorm_out = nullptr);
 // Row norms in double precision (sum of squares in dimension order, then sqrt): the FP64
 // re-check's base magnitudes.
 void launch_row_norms_fp64(const float* x, int64_t n, int d, double* out, cudaStream_t s);

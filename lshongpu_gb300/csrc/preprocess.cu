@@ -17,42 +17,55 @@ namespace lshg {
 namespace {
 
 constexpr int kRowsPerBlock = 32;  // small blocks: a 10k-row query batch spreads over every SM
+constexpr int kNormThreads = 128;
+constexpr int kNormRows = kRowsPerBlock / (kNormThreads / 32);  // rows a warp stages
 
-// Stage kRowsPerBlock rows into shared memory with an odd row pitch (conflict-free
-// column walks), then let thread t own row t.
+// Stage kRowsPerBlock rows into shared memory with an odd row pitch (conflict-free column
+// walks), then let thread t own row t.  A small batch is bounded by the latency of its loads: a
+// warp takes kNormRows rows and issues the loads of 64 of their columns before it uses one
+// (each thread had walked the block's elements, an index division and a load's latency apart:
+// 1M x 128 norms 245 -> 80 us, normalisation 476 -> 172 us).
 template <bool kNormalize>
-__global__ void row_norm_kernel(float* __restrict__ x, int64_t n, int d, float* __restrict__ norms) {
+__global__ void __launch_bounds__(kNormThreads) row_norm_kernel(float* __restrict__ x, int64_t n, int d,
+                                                                float* __restrict__ norms) {
   extern __shared__ float sm[];
   const int pitch = d | 1;
   const int64_t row0 = (int64_t)blockIdx.x * kRowsPerBlock;
   const int rows = (int)imin<int64_t>(kRowsPerBlock, n - row0);
+  const int lane = threadIdx.x & 31, r0 = (threadIdx.x >> 5) * kNormRows;
   const float* src = x + row0 * d;
-  for (int i = threadIdx.x; i < rows * d; i += blockDim.x) {
-    int r = i / d, c = i - r * d;
-    sm[r * pitch + c] = src[i];
+  for (int c0 = lane; c0 < d; c0 += 64) {
+    float v[2][kNormRows];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < kNormRows; ++i)
+        v[h][i] = (r0 + i < rows && c0 + 32 * h < d) ? src[(int64_t)(r0 + i) * d + c0 + 32 * h] : 0.0f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < kNormRows; ++i)
+        if (c0 + 32 * h < d) sm[(r0 + i) * pitch + c0 + 32 * h] = v[h][i];
   }
   __syncthreads();
   __shared__ float mags[kRowsPerBlock];
   if (threadIdx.x < rows) {
     const float* row = sm + threadIdx.x * pitch;
     float m = 0.0f;
+#pragma unroll 8
     for (int j = 0; j < d; ++j) m = __fmaf_rn(row[j], row[j], m);
     m = __fsqrt_rn(m);
     if (kNormalize) mags[threadIdx.x] = m;
     else norms[row0 + threadIdx.x] = m;
   }
-  if (kNormalize) {  // the divides are independent: every thread takes a share
-    __syncthreads();
-    for (int i = threadIdx.x; i < rows * d; i += blockDim.x) {
-      const int r = i / d, c = i - r * d;
-      sm[r * pitch + c] = __fdiv_rn(sm[r * pitch + c], mags[r]);
-    }
+  if (kNormalize) {  // the divides are independent: every warp takes its rows
     __syncthreads();
     float* dst = x + row0 * d;
-    for (int i = threadIdx.x; i < rows * d; i += blockDim.x) {
-      int r = i / d, c = i - r * d;
-      dst[i] = sm[r * pitch + c];
-    }
+    for (int c = lane; c < d; c += 32)
+#pragma unroll
+      for (int i = 0; i < kNormRows; ++i)
+        if (r0 + i < rows)
+          dst[(int64_t)(r0 + i) * d + c] = __fdiv_rn(sm[(r0 + i) * pitch + c], mags[r0 + i]);
   }
 }
 
@@ -188,7 +201,7 @@ void launch_row_norms(const float* x, int64_t n, int d, float* norms, cudaStream
   size_t smem = staged_smem(kRowsPerBlock, d);
   LSHG_REQUIRE(smem <= 200 * 1024, "dimension too large for row_norms");
   LSHG_CUDA(cudaFuncSetAttribute(row_norm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  row_norm_kernel<false><<<ceil_div(n, kRowsPerBlock), 128, smem, s>>>(const_cast<float*>(x), n, d, norms);
+  row_norm_kernel<false><<<ceil_div(n, kRowsPerBlock), kNormThreads, smem, s>>>(const_cast<float*>(x), n, d, norms);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -198,7 +211,7 @@ void launch_normalize(float* x, int64_t n, int d, cudaStream_t s) {
   size_t smem = staged_smem(kRowsPerBlock, d);
   LSHG_REQUIRE(smem <= 200 * 1024, "dimension too large for normalize");
   LSHG_CUDA(cudaFuncSetAttribute(row_norm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  row_norm_kernel<true><<<ceil_div(n, kRowsPerBlock), 128, smem, s>>>(x, n, d, nullptr);
+  row_norm_kernel<true><<<ceil_div(n, kRowsPerBlock), kNormThreads, smem, s>>>(x, n, d, nullptr);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

@@ -136,6 +136,14 @@ __device__ void fp64_boundary(uint64_t* keys, int C, int k, const float* __restr
   __syncthreads();
 }
 
+// A row's magnitude by the reference's arithmetic (row_norm_kernel's chain).
+__device__ __forceinline__ float query_norm(const float* row, int d) {
+  float m = 0.0f;
+#pragma unroll 8
+  for (int j = 0; j < d; ++j) m = __fmaf_rn(row[j], row[j], m);
+  return __fsqrt_rn(m);
+}
+
 // One block per query: fold S sorted lists of C keys into one.
 __global__ void merge_splits_kernel(const uint64_t* __restrict__ in, int nq, int splits, int C,
                                     uint64_t* __restrict__ out) {
@@ -156,18 +164,85 @@ __global__ void merge_splits_kernel(const uint64_t* __restrict__ in, int nq, int
   for (int i = threadIdx.x; i < C; i += blockDim.x) out[(int64_t)q * C + i] = ms[i];
 }
 
+// The same fold for lists of C = 32 * E <= 128 keys: warp w folds lists w, w + W, ... in
+// registers (the next list's load in flight), then the W results are folded pairwise.  One
+// list after the other with the whole block cost a load's latency and log2 C barriers each
+// (64 lists of 32 keys, 129 queries: 52 us; this way 8.5).  pts (optional): the first k as points
+// in place of the keys.
+template <int E>
+__global__ void __launch_bounds__(256) merge_short_kernel(const uint64_t* __restrict__ in, int splits, int k,
+                                                           uint64_t* __restrict__ out, lshg_point* __restrict__ pts) {
+  constexpr int C = 32 * E;
+  __shared__ uint64_t lists[8][C];
+  const int q = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const uint64_t* src = in + (int64_t)q * splits * C;
+  uint64_t best[E], x[E];
+  auto load = [&](int s) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) x[e] = s < splits ? src[(int64_t)s * C + e * 32 + lane] : kEmptyKey;
+  };
+  load(warp);
+#pragma unroll
+  for (int e = 0; e < E; ++e) best[e] = x[e];
+  load(warp + W);
+  for (int s = warp + W; s < splits; s += W) {
+    // both ascending: min(best[i], x[C - 1 - i]) is bitonic and holds the C smallest
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const uint64_t r = __shfl_sync(0xffffffffu, x[E - 1 - e], 31 - lane);
+      best[e] = best[e] < r ? best[e] : r;
+    }
+    load(s + W);
+    warp_bitonic<E>(best, lane, true);
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e) lists[warp][e * 32 + lane] = best[e];
+  __syncthreads();
+  for (int half = W >> 1; half >= 1; half >>= 1) {
+    if (warp < half) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const uint64_t r = lists[warp + half][(E - 1 - e) * 32 + (31 - lane)];
+        best[e] = best[e] < r ? best[e] : r;
+      }
+      warp_bitonic<E>(best, lane, true);
+#pragma unroll
+      for (int e = 0; e < E; ++e) lists[warp][e * 32 + lane] = best[e];
+    }
+    __syncthreads();
+  }
+  if (warp != 0) return;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = e * 32 + lane;
+    if (!pts) {
+      out[(int64_t)q * C + i] = best[e];
+    } else if (i < k) {
+      lshg_point pt;
+      if (best[e] == kEmptyKey) { pt.ID = -1; pt.distance = kEmptyDistance; }
+      else { pt.ID = key_id(best[e]); pt.distance = key_dist(best[e]); }
+      pts[(int64_t)q * k + i] = pt;
+    }
+  }
+}
+
 template <int DIST>
 __global__ void rerank_kernel(const uint64_t* __restrict__ cand, int nq, int C, const float* __restrict__ x,
                               int64_t n, int d, const float* __restrict__ xnorm, const float* __restrict__ q,
-                              const float* __restrict__ qnorm, int k, lshg_point* __restrict__ out, float band_abs,
-                              float band_rel, const double* __restrict__ xn64, const RerankBounds* __restrict__ kx) {
+                              const float* qnorm, float* qnorm_out, int k, lshg_point* __restrict__ out,
+                              float band_abs, float band_rel, const double* __restrict__ xn64,
+                              const RerankBounds* __restrict__ kx) {
   extern __shared__ __align__(16) unsigned char rsm[];
   uint64_t* keys = reinterpret_cast<uint64_t*>(rsm);
   float* qr = reinterpret_cast<float*>(rsm + (size_t)C * 8);
   const int qi = blockIdx.x;
   for (int j = threadIdx.x; j < d; j += blockDim.x) qr[j] = q[(int64_t)qi * d + j];
   __syncthreads();
-  const float qn = (DIST == DIST_ANGULAR) ? qnorm[qi] : 1.0f;
+  float qn = 1.0f;
+  if (DIST == DIST_ANGULAR) {
+    qn = qnorm ? qnorm[qi] : query_norm(qr, d);
+    if (qnorm_out && threadIdx.x == 0) qnorm_out[qi] = qn;
+  }
   for (int i = threadIdx.x; i < C; i += blockDim.x) {
     uint64_t kin = cand[(int64_t)qi * C + i];
     uint64_t ko = kEmptyKey;
@@ -207,8 +282,8 @@ __global__ void rerank_kernel(const uint64_t* __restrict__ cand, int nq, int C, 
 template <int DIST>
 __global__ void rerank_staged_kernel(const uint64_t* __restrict__ cand, int nq, int C, const float* __restrict__ x,
                                      int64_t n, int d, const float* __restrict__ xnorm, const float* __restrict__ q,
-                                     const float* __restrict__ qnorm, int k, lshg_point* __restrict__ out, int* err,
-                                     float band_abs, float band_rel, const double* __restrict__ xn64, int test_stall,
+                                     const float* qnorm, float* qnorm_out, int k, lshg_point* __restrict__ out,
+                                     int* err, float band_abs, float band_rel, const double* __restrict__ xn64, int test_stall,
                                      const RerankBounds* __restrict__ kx) {
   extern __shared__ __align__(128) unsigned char rsm[];
   const int CH = blockDim.x;
@@ -217,6 +292,7 @@ __global__ void rerank_staged_kernel(const uint64_t* __restrict__ cand, int nq, 
   uint64_t* keys = reinterpret_cast<uint64_t*>(rsm + (size_t)CH * slot);
   float* qr = reinterpret_cast<float*>(keys + C);
   __shared__ __align__(8) uint64_t bar, never;
+  __shared__ float s_qn;
   const int qi = blockIdx.x, tid = threadIdx.x;
   const uint32_t bar_a = tc::smem_u32(&bar);
   // test_stall: the first wait is made on `never`, a barrier nothing arrives on, with a
@@ -228,7 +304,7 @@ __global__ void rerank_staged_kernel(const uint64_t* __restrict__ cand, int nq, 
     tc::mbar_init(never_a, 1);
   }
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  const float qn = (DIST == DIST_ANGULAR) ? qnorm[qi] : 1.0f;
+  float qn = (DIST == DIST_ANGULAR && qnorm) ? qnorm[qi] : 1.0f;
   unsigned char* dst = stage + (size_t)tid * slot;
   uint32_t phase = 0, pending = 0;
   bool ok = true;  // block-uniform
@@ -252,8 +328,18 @@ __global__ void rerank_staged_kernel(const uint64_t* __restrict__ cand, int nq, 
     }
     // the query row while the first chunk's rows are in flight; published by the barrier
     // that ends this chunk's wait (or the next chunk's count when this one has no rows)
-    if (c0 == 0)
+    if (c0 == 0) {
       for (int j = tid; j < d; j += CH) qr[j] = q[(int64_t)qi * d + j];
+      // the query's norm by warp 0 (every lane the same chain; published by the barrier that ends this chunk)
+      if (DIST == DIST_ANGULAR && !qnorm && tid < 32) {
+        const float m = query_norm(q + (int64_t)qi * d, d);
+        if (tid == 0) {
+          s_qn = m;
+          if (qnorm_out) qnorm_out[qi] = m;
+        }
+      }
+      if (!(ok && nv > 0)) __syncthreads();
+    }
     if (ok && nv > 0) {
       const bool stall = test_stall && c0 == 0;
       const uint32_t wbar = stall ? never_a : bar_a;
@@ -271,6 +357,7 @@ __global__ void rerank_staged_kernel(const uint64_t* __restrict__ cand, int nq, 
       }
       phase ^= 1u;
     }
+    if (c0 == 0 && DIST == DIST_ANGULAR && !qnorm) qn = s_qn;
     if (i < C) {
       uint64_t ko = kEmptyKey;
       if (id >= 0) {
@@ -523,14 +610,38 @@ __global__ void keys_to_points_kernel(const uint64_t* __restrict__ keys, int nq,
 
 }  // namespace
 
+namespace {
+void merge_short(const uint64_t* in, int nq, int splits, int C, int k, uint64_t* out, lshg_point* pts, cudaStream_t s) {
+  int W = 1;  // warps: a power of two, no more than lists
+  while (W < 8 && 2 * W <= splits) W <<= 1;
+  if (C == 32) merge_short_kernel<1><<<nq, 32 * W, 0, s>>>(in, splits, k, out, pts);
+  else if (C == 64) merge_short_kernel<2><<<nq, 32 * W, 0, s>>>(in, splits, k, out, pts);
+  else merge_short_kernel<4><<<nq, 32 * W, 0, s>>>(in, splits, k, out, pts);
+  count_launch();
+  LSHG_CHECK_LAUNCH();
+}
+}  // namespace
+
 void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t* out, cudaStream_t s) {
   if (nq <= 0) return;
   ProfScope _ps("merge_splits", s);
+  if (C == 32 || C == 64 || C == 128) {
+    merge_short(in, nq, splits, C, 0, out, nullptr, s);
+    return;
+  }
   size_t smem = (size_t)C * 8;
   LSHG_CUDA(cudaFuncSetAttribute(merge_splits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   merge_splits_kernel<<<nq, 128, smem, s>>>(in, nq, splits, C, out);
   count_launch();
   LSHG_CHECK_LAUNCH();
+}
+
+bool launch_merge_points(const uint64_t* in, int nq, int splits, int C, int k, lshg_point* out, cudaStream_t s) {
+  if ((C != 32 && C != 64 && C != 128) || k > C) return false;
+  if (nq <= 0) return true;
+  ProfScope _ps("merge_splits", s);
+  merge_short(in, nq, splits, C, k, nullptr, out, s);
+  return true;
 }
 
 void fp64_band(int dist, int d, float* band_abs, float* band_rel) {
@@ -550,7 +661,7 @@ void fp64_band(int dist, int d, float* band_abs, float* band_rel) {
 
 void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t n, int d, const float* xnorm,
                    const float* q, const float* qnorm, int dist, int k, lshg_point* out, cudaStream_t s, int* err,
-                   bool fp64_recheck, const double* xn64, const RerankBounds* extra_dev) {
+                   bool fp64_recheck, const double* xn64, const RerankBounds* extra_dev, float* qnorm_out) {
   if (nq <= 0) return;
   float band_abs = -1.0f, band_rel = 0.0f;
   if (fp64_recheck) fp64_band(dist, d, &band_abs, &band_rel);
@@ -567,6 +678,7 @@ void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t 
   const bool stageable = d % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
   const size_t gather_smem = (size_t)128 * stage_slot_bytes(d) + (size_t)d * 4 + 16;
   const size_t select_smem = (size_t)C * 8 + (size_t)d * 4 + 16;
+  LSHG_REQUIRE(dist != DIST_ANGULAR || qnorm || C < 1024, "re-rank: long lists need the query norms");
   if (stageable && C >= 1024 && !test_stall && gather_smem <= 96 * 1024 && select_smem <= 200 * 1024) {
     DevBuf<uint64_t> gk((size_t)nq * C, s);
     // lists in base order when the rows do not fit in a quarter of L2 (the gather then
@@ -619,8 +731,8 @@ void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t 
   do {                                                                                                         \
     LSHG_CUDA(cudaFuncSetAttribute(rerank_staged_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
                                    (int)staged_smem));                                                         \
-    rerank_staged_kernel<DV><<<nq, CH, staged_smem, s>>>(cand, nq, C, x, n, d, xnorm, q, qnorm, k, out, err, \
-                                                         band_abs, band_rel, xn64, test_stall, kb);          \
+    rerank_staged_kernel<DV><<<nq, CH, staged_smem, s>>>(cand, nq, C, x, n, d, xnorm, q, qnorm, qnorm_out, k,  \
+                                                         out, err, band_abs, band_rel, xn64, test_stall, kb); \
   } while (0)
     switch (dist) {
       case DIST_ANGULAR: LSHG_RRS(DIST_ANGULAR); break;
@@ -640,8 +752,8 @@ void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t 
 #define LSHG_RR(DV)                                                                                       \
   do {                                                                                                    \
     LSHG_CUDA(cudaFuncSetAttribute(rerank_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    rerank_kernel<DV><<<nq, threads, smem, s>>>(cand, nq, C, x, n, d, xnorm, q, qnorm, k, out, band_abs,   \
-                                                band_rel, xn64, kb);                                      \
+    rerank_kernel<DV><<<nq, threads, smem, s>>>(cand, nq, C, x, n, d, xnorm, q, qnorm, qnorm_out, k, out,      \
+                                                band_abs, band_rel, xn64, kb);                            \
   } while (0)
   switch (dist) {
     case DIST_ANGULAR: LSHG_RR(DIST_ANGULAR); break;

@@ -134,8 +134,7 @@ void derive_exact(Index& I, cudaStream_t s) {
   if (bad) I.ebf.release();
 }
 
-bool query_exact_filtered(Index& I, const float* q, int nq, const float* qnorm, int k, lshg_point* out,
-                          cudaStream_t s) {
+bool query_exact_filtered(Index& I, const float* q, int nq, int k, lshg_point* out, cudaStream_t s) {
   using namespace tc;
   if (!I.ebf.ptr || k > 128 || (int64_t)nq * I.n < kExactFilterMinPairs) return false;
   const int CT = k <= 32 && I.n < kExactFewCandidatesBase ? 128 : 256;
@@ -148,7 +147,7 @@ bool query_exact_filtered(Index& I, const float* q, int nq, const float* qnorm, 
   const int splits = scan_listed_splits(I.n, nq, C);
   try {
     DevBuf<uint16_t> qbf((size_t)qpad * KD, s);
-    DevBuf<float> eps((size_t)nq, s), tau((size_t)nq, s);
+    DevBuf<float> eps((size_t)nq, s), tau((size_t)nq, s), qnorm((size_t)nq, s);
     DevBuf<int> cnt((size_t)nq + 1 + nq, s);  // [0, nq): survivors; [nq]: listed; then the list
     DevBuf<uint64_t> cand((size_t)nq * std::max(plan.cap, 1), s), best((size_t)nq * CT, s);
     DevBuf<uint64_t> part((size_t)nq * splits * C, s);
@@ -160,9 +159,9 @@ bool query_exact_filtered(Index& I, const float* q, int nq, const float* qnorm, 
                        eps.ptr);
     launch_exact_select(cnt.ptr, cand.ptr, nq, plan.cap, (int)std::min<int64_t>(k, I.n), CT,
                         plan.M > 0 ? tau.ptr : nullptr, eps.ptr, best.ptr, ovf, s);
-    launch_rerank(best.ptr, nq, CT, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, qnorm, DIST_ANGULAR, k, out, s,
-                  I.error_word(s));
-    launch_scan_float_listed(I.xt.ptr, I.n, I.d, I.xnorm.ptr, q, nq, qnorm, ovf, C, splits, part.ptr, k, out, s);
+    launch_rerank(best.ptr, nq, CT, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, nullptr, DIST_ANGULAR, k, out, s,
+                  I.error_word(s), false, nullptr, nullptr, qnorm.ptr);
+    launch_scan_float_listed(I.xt.ptr, I.n, I.d, I.xnorm.ptr, q, nq, qnorm.ptr, ovf, C, splits, part.ptr, k, out, s);
   } catch (const Error& e) {
     if (e.status != LSHG_ERR_OUT_OF_MEMORY) throw;
     cudaGetLastError();  // temporaries that do not fit: the FP32 scan needs fewer

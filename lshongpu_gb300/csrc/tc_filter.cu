@@ -558,7 +558,8 @@ template <int E>
 __global__ void __launch_bounds__(256) cand_select_kernel(const int* __restrict__ cnt,
                                                            const uint64_t* __restrict__ cand, int cap, int need,
                                                            int nq, uint64_t* __restrict__ out,
-                                                           int* __restrict__ ovf) {
+                                                           int* __restrict__ ovf, const uint16_t* __restrict__ rows,
+                                                           uint16_t* __restrict__ gathered) {
   constexpr int CT = 32 * E;
   const int lane = threadIdx.x & 31;
   const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -568,7 +569,16 @@ __global__ void __launch_bounds__(256) cand_select_kernel(const int* __restrict_
   if (c > cap || c < need) {
 #pragma unroll
     for (int e = 0; e < E; ++e) dst[e * 32 + lane] = kEmptyKey;
-    if (lane == 0) ovf[1 + atomicAdd(ovf, 1)] = q;
+    int at = 0;
+    if (lane == 0) {
+      at = atomicAdd(ovf, 1);
+      ovf[1 + at] = q;
+    }
+    at = __shfl_sync(0xffffffffu, at, 0);
+    // its row for the list kernel (rows past the count are never read out)
+    if (gathered)
+      reinterpret_cast<uint2*>(gathered + (int64_t)at * KD)[lane] =
+          reinterpret_cast<const uint2*>(rows + (int64_t)q * KD)[lane];
     return;
   }
   uint64_t best[E];
@@ -614,22 +624,6 @@ __global__ void __launch_bounds__(256) exact_select_kernel(const int* __restrict
   for (int e = 0; e < E; ++e)
     dst[e * 32 + lane] = !listed && best[e] != kEmptyKey && -key_dist(best[e]) >= cut ? best[e] : kEmptyKey;
   if (listed && lane == 0) ovf[1 + atomicAdd(ovf, 1)] = q;
-}
-
-// Compact the bf16 rows of the listed queries into rows 0..count-1 of `dst` (the rest of
-// the last 128-row tile is zeroed).
-__global__ void gather_rows_kernel(const uint16_t* __restrict__ src, const int* __restrict__ ovf,
-                                   uint16_t* __restrict__ dst) {
-  const int cntq = ovf[0];
-  const int64_t rows = (int64_t)((cntq + BM - 1) / BM) * BM;
-  const int64_t chunks = rows * (KD / 8);
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < chunks; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t / (KD / 8);
-    const int c = (int)(t % (KD / 8));
-    uint4 val = make_uint4(0, 0, 0, 0);
-    if (i < cntq) val = reinterpret_cast<const uint4*>(src + (int64_t)ovf[1 + i] * KD)[c];
-    reinterpret_cast<uint4*>(dst + i * KD)[c] = val;
-  }
 }
 
 // Merge the list kernel's per-CTA partial lists of every listed query and write the
@@ -835,11 +829,11 @@ void launch_tau_select(const float* gmax, int nq, int M, int rank, float margin,
 }
 
 void launch_cand_select(const int* cnt, const uint64_t* cand, int nq, int cap, int need, int CT, uint64_t* out,
-                        int* ovf, cudaStream_t s) {
+                        int* ovf, const uint16_t* rows, uint16_t* gathered, cudaStream_t s) {
   ProfScope _ps("tc_cand_select", s);
-  if (CT == 32) cand_select_kernel<1><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf);
-  else if (CT == 64) cand_select_kernel<2><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf);
-  else if (CT == 128) cand_select_kernel<4><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf);
+  if (CT == 32) cand_select_kernel<1><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf, rows, gathered);
+  else if (CT == 64) cand_select_kernel<2><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf, rows, gathered);
+  else if (CT == 128) cand_select_kernel<4><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf, rows, gathered);
   else throw Error(LSHG_ERR_INVALID_ARGUMENT, "tensor-core scan: candidate count must be 32, 64 or 128");
   count_launch();
   LSHG_CHECK_LAUNCH();
@@ -851,14 +845,6 @@ void launch_exact_select(const int* cnt, const uint64_t* cand, int nq, int cap, 
   if (CT == 128) exact_select_kernel<4><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, k, nq, tau, eps, out, ovf);
   else if (CT == 256) exact_select_kernel<8><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, k, nq, tau, eps, out, ovf);
   else throw Error(LSHG_ERR_INVALID_ARGUMENT, "exact scan: candidate count must be 128 or 256");
-  count_launch();
-  LSHG_CHECK_LAUNCH();
-}
-
-void launch_gather_rows(const uint16_t* src, const int* ovf, int nq, uint16_t* dst, cudaStream_t s) {
-  const int64_t chunks = (int64_t)ceil_div(nq, BM) * BM * (KD / 8);
-  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((chunks + 255) / 256, (int64_t)num_sms() * 4));
-  gather_rows_kernel<<<blocks, 256, 0, s>>>(src, ovf, dst);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

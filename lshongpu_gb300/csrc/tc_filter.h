@@ -54,8 +54,10 @@ void launch_tau_select(const float* gmax, int nq, int M, int rank, float margin,
 
 // Top-CT keys a query from its survivors (CT = 32, 64 or 128); queries with more survivors
 // than cap or fewer than `need` are listed in ovf for the exact fallback.
+// rows / gathered: BF16 query rows of 128 columns; the row of the i-th listed query is copied to
+// row i of `gathered` (may be nullptr when no query can be listed).
 void launch_cand_select(const int* cnt, const uint64_t* cand, int nq, int cap, int need, int CT, uint64_t* out,
-                        int* ovf, cudaStream_t s);
+                        int* ovf, const uint16_t* rows, uint16_t* gathered, cudaStream_t s);
 
 // The candidates of an exact top-k among a query's survivors: every point whose score is
 // within 2 eps[q] of the k-th best one, out of the top-CT (CT = 128 or 256; the rest of the row
@@ -109,8 +111,6 @@ void launch_split_bf16(const float* x, int64_t n, int d, int64_t rows_pad, int o
                        cudaStream_t s);
 void launch_tc_signs(const float* x, int64_t n, int d, const uint16_t* planes_split, const float* pnorm,
                      const float* planes, int P, int words, uint32_t* out32, int* err, cudaStream_t s);
-
-void launch_gather_rows(const uint16_t* src, const int* ovf, int nq, uint16_t* dst, cudaStream_t s);
 
 void launch_merge_fallback(const uint64_t* part, const int* ovf, int nq, int NT, int grid, int CT, uint64_t* out,
                            cudaStream_t s);

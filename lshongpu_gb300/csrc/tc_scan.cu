@@ -16,7 +16,7 @@
 //
 // tc_list_kernel is persistent (one CTA per SM) with a stream-K split of the (query tile,
 // base tile) space; its CTA count and split are derived on the device from the gathered
-// row count, so the fallback costs three near-empty launches when nothing overflowed.
+// row count, so the fallback costs two near-empty launches when nothing overflowed.
 // Warp roles:
 //   warp 0  TMA producer (cp.async.bulk.tensor, 128B swizzle, mbarrier complete_tx)
 //   warp 1  MMA issuer (one thread: tcgen05.mma kind::f16, M=128 N=128 K=16 x 8)
@@ -570,15 +570,17 @@ void launch_tc_scan(Index& I, const float* q, int nq, int k, lshg_point* out, cu
   // 3. top-CT of the survivors
   DevBuf<uint64_t> best((size_t)nq * CT, s);
   // a query needs min(CT, n) survivors: fewer means its sampled threshold was too high
-  launch_cand_select(cnt.ptr, cand.ptr, nq, plan.cap, (int)std::min<int64_t>(CT, I.n), CT, best.ptr, ovf, s);
+  // (listed queries' BF16 rows are gathered for the list kernel by the same launch)
+  const bool fallback = (int64_t)plan.cap < I.n || plan.rank < CT;
+  DevBuf<uint16_t> qg(fallback ? (size_t)qpad * KD : 0, s);
+  launch_cand_select(cnt.ptr, cand.ptr, nq, plan.cap, (int)std::min<int64_t>(CT, I.n), CT, best.ptr, ovf, qbf.ptr,
+                     qg.ptr, s);
 
   // 4. fallback for queries with more survivors than slots (massive ties) or fewer than CT
   //    (a sampled threshold above the query's CT-th best score)
-  if ((int64_t)plan.cap < I.n || plan.rank < CT) {
+  if (fallback) {
     ProfScope _ps("tc_fallback", s);
     const int G = num_sms();
-    DevBuf<uint16_t> qg((size_t)qpad * KD, s);
-    launch_gather_rows(qbf.ptr, ovf, nq, qg.ptr, s);
     const CUtensorMap mg = make_map(qg.ptr, qpad);
     DevBuf<uint64_t> part((size_t)BM * (G + 2 * QT) * CT, s);
     if (CT == 64) run_list_kernel<3, 64>(mg, mb, ovf, I.n, NT, I.d, G, part.ptr, err, s);
@@ -587,9 +589,7 @@ void launch_tc_scan(Index& I, const float* q, int nq, int k, lshg_point* out, cu
   }
 
   // 5. exact FP32 re-rank with the reference's angular formula
-  DevBuf<float> qn((size_t)nq, s);
-  launch_row_norms(q, nq, I.d, qn.ptr, s);
-  launch_rerank(best.ptr, nq, CT, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, qn.ptr, DIST_ANGULAR, k, out, s, err,
+  launch_rerank(best.ptr, nq, CT, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, nullptr, DIST_ANGULAR, k, out, s, err,
                 I.p.opt.fp64_recheck != 0, I.xnorm64.ptr, extra);
 }
 

@@ -172,3 +172,30 @@ def test_sketch_scan_small_batches_equal_popcount(engine, n, nq, words, C):
            for mode in (0, TENSOR, POPCOUNT)]
     assert np.array_equal(res[0], res[2])
     assert np.array_equal(res[1], res[2])
+
+
+@pytest.mark.parametrize("n,nq,k,d,dist", [
+    (500, 3, 32, 100, 2),     # one split
+    (5000, 70, 64, 37, 2),    # lists of 64, rows with an odd pitch
+    (60013, 129, 100, 64, 3),  # many splits, lists of 128
+    (3000, 5, 300, 65, 2),    # lists beyond the short merge
+    (70000, 2, 10, 130, 1),   # an FP32 angular scan of many splits
+])
+def test_exact_scan_split_merges(engine, orc, n, nq, k, d, dist):
+    """The FP32 scan's split lists merge to the oracle's top-k: ids and distances of the Jaccard
+    and angular scans bit for bit; Euclidean distances within the two square's rounding of
+    the oracle's (d terms, 2^-24 each), in order."""
+    if dist == 2:
+        x, q = datasets.sparse_gamma(n, d, 91), datasets.sparse_gamma(nq, d, 92)
+        xo, qo = orc.normalize(x), orc.normalize(q)
+    else:
+        x, q = data(n, nq, d)
+        xo, qo = x, q
+    res = engine.Index(x, implementation=2, distanceFunc=dist).query(q, k)
+    ids, ds = orc.exact_topk(xo, qo, k, dist=dist)
+    if dist == 3:
+        assert np.max(np.abs(res["distance"] - ds)) <= 2 * (d + 3) * 2.0**-24 * np.max(ds)
+        assert np.all(np.diff(res["distance"], axis=1) >= 0)
+    else:
+        assert np.array_equal(res["ID"], ids)
+        assert np.array_equal(res["distance"], ds)
