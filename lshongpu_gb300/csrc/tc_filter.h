@@ -93,8 +93,8 @@ void launch_expand_bits(const uint32_t* xs, int64_t n, int wp, int words, int64_
 void launch_tc_hamming(const uint8_t* xse, int64_t n, const uint32_t* xst, int wp, int words, const uint32_t* qs,
                        int nq, int op, int C, uint64_t* out, int* err, cudaStream_t s);
 // Top-C keys [nq][C] of each query's survivors (keys make_key(-score, id), integer scores in
-// [-bits, bits]): a warp sort for C <= 128, a histogram of the scores and a sort of the
-// ties at the C-th score beyond; queries with fewer than `need` or more than `cap`
+// [-bits, bits]): a warp sort for C <= 128, bisection over the scores and the ids at the C-th
+// score beyond; queries with fewer than `need` or more than `cap`
 // survivors (or too many ties) are listed in ovf and their rows left for a rescan.
 void launch_int_select(const int* cnt, const uint64_t* cand, int cap, int need, int C, int bits, int nq, uint64_t* out,
                        int* ovf, cudaStream_t s);

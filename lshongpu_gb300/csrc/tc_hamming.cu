@@ -25,8 +25,8 @@
 //            in shared memory and moved to the query's candidate array with one atomicAdd
 //            a batch;
 //   select   keeps each query's first C survivors by (score desc, id asc): a warp sort for
-//            C <= 128, a histogram of the integer scores and a sort of the ties at the
-//            C-th score beyond.
+//            C <= 128, bisection over the integer scores and over the ids at the C-th score
+//            beyond.
 //            A query with fewer than C survivors (tau above its C-th best score: the
 //            sample was unrepresentative) or more than its array holds (massive ties) is
 //            listed and rescanned exactly by the popcount scan on the device, so the result
@@ -710,20 +710,49 @@ __global__ void __launch_bounds__(256) hsel_warp_kernel(const int* __restrict__ 
 }
 
 // Top-C (C > 128) of each query's survivors as a set, one block a query, using the integer
-// scores: a histogram of the scores (2 * bits + 1 bins) gives the score t of the C-th best
-// survivor; every survivor above t is in, and of those at t the ones with the lowest ids
-// (the survivors' keys sorted in shared memory: they order by id within one score).  The
-// set goes out unordered -- the re-rank sorts it.  A query whose survivors at t exceed
-// H_TIE_MAX is listed for the exact rescan, as are those with fewer than `need` or more
-// than `cap` survivors.
+// scores: t is the score of the C-th best survivor; every survivor above t is in, and of those
+// at t the ones with the lowest ids.  The set goes out unordered -- the re-rank sorts it.  Up to
+// kSelRegs keys a thread, t is found by bisection over the scores held in registers, and the
+// id that ends the tied ones by bisection over their ids; longer lists (bases that keep every
+// point) take t from a histogram of the scores (2 * bits + 1 bins).  A query whose survivors at
+// t exceed H_TIE_MAX is listed for the exact rescan, as are those with fewer than `need` or
+// more than `cap` survivors.
+//
+// Bisection costs a compare a key and a block sum a step, about 25 steps; the histogram's
+// shared-memory atomics pile up on the few scores next to the threshold (10,000 queries, C =
+// 4,096, 6,500 survivors of 256-bit sketches: 825 us, by bisection 371).
 constexpr int H_TIE_MAX = 4096;
 constexpr int H_BINS_MAX = 2049;
+constexpr int kSelRegs = 16;
 
-__global__ void __launch_bounds__(512) hsel_hist_kernel(const int* __restrict__ cnt, const uint64_t* __restrict__ cand,
-                                                        int cap, int need, int C, int bits,
-                                                        uint64_t* __restrict__ out, int* __restrict__ ovf) {
-  __shared__ uint64_t tie[H_TIE_MAX];
+// Sum over the block of each thread's c (every thread; buf alternates between calls).
+template <int T>
+__device__ __forceinline__ int block_sum(int c, int (&part)[2][T / 32], int buf) {
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0) part[buf][threadIdx.x >> 5] = c;
+  __syncthreads();
+  // every warp adds the warps' sums
+  const int l = threadIdx.x & 31;
+  return __reduce_add_sync(0xffffffffu, l < T / 32 ? part[buf][l] : 0);
+}
+
+// One slot a lane with `in` set, from a shared counter: one atomic a warp.
+__device__ __forceinline__ int warp_slot(bool in, int* counter) {
+  const unsigned mk = __ballot_sync(0xffffffffu, in);
+  const int lane = threadIdx.x & 31;
+  int base = 0;
+  if (lane == 0 && mk) base = atomicAdd(counter, __popc(mk));
+  return __shfl_sync(0xffffffffu, base, 0) + __popc(mk & ((1u << lane) - 1u));
+}
+
+// T threads: 256 for C <= 1024, whose survivors they hold, else 512.
+template <int T>
+__global__ void __launch_bounds__(T, 1536 / T)
+    hsel_kernel(const int* __restrict__ cnt, const uint64_t* __restrict__ cand, int cap, int need, int C, int bits,
+                uint64_t* __restrict__ out, int* __restrict__ ovf) {
+  __shared__ int tie[H_TIE_MAX];  // ids at the C-th score
   __shared__ int hist[H_BINS_MAX];
+  __shared__ int part[2][T / 32];
   __shared__ int s_t, s_below, s_nout, s_ntie;
   const int q = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
   const int c = cnt[q];
@@ -734,63 +763,137 @@ __global__ void __launch_bounds__(512) hsel_hist_kernel(const int* __restrict__ 
   const uint64_t* src = cand + (int64_t)q * cap;
   uint64_t* dst = out + (int64_t)q * C;
   if (c <= C) {  // a base of fewer than C points: all of them, then empty keys
-    for (int i = tid; i < C; i += blockDim.x) dst[i] = i < c ? src[i] : kEmptyKey;
+    for (int i = tid; i < C; i += T) dst[i] = i < c ? src[i] : kEmptyKey;
     return;
   }
-  const int nb = 2 * bits + 1;
-  for (int i = tid; i < nb; i += blockDim.x) hist[i] = 0;
   if (tid == 0) {
     s_nout = 0;
     s_ntie = 0;
   }
-  __syncthreads();
-  // a key holds -score; bin = bits - score: 0 is the best score
-  for (int i = tid; i < c; i += blockDim.x) atomicAdd(&hist[(int)key_dist(src[i]) + bits], 1);
-  __syncthreads();
-  if (tid < 32) {  // the bin where the running count reaches C
-    const int per = (nb + 31) / 32, b0 = lane * per, b1 = min(nb, b0 + per);
-    int own = 0;
-    for (int b = b0; b < b1; ++b) own += hist[b];
-    int incl = own;
+  // a key holds -score: the smallest are the best
+  int thr, below;  // -(C-th score); survivors above it
+  if (c <= kSelRegs * T) {
+    int v[kSelRegs];
+    int mn = INT_MAX, mx = INT_MIN;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    const unsigned hit = __ballot_sync(0xffffffffu, incl >= C);
-    const int L = __ffs(hit) - 1;  // hit != 0: the bins hold c > C keys
-    if (lane == L) {
-      int acc = incl - own;
-      for (int b = b0; b < b1; ++b) {
-        if (acc + hist[b] >= C) {
-          s_t = b;
-          s_below = acc;
-          break;
-        }
-        acc += hist[b];
+    for (int e = 0; e < kSelRegs; ++e) {
+      const int i = e * T + tid;
+      v[e] = INT_MAX;
+      if (i < c) {
+        v[e] = (int)key_dist(src[i]);
+        mn = min(mn, v[e]);
+        mx = max(mx, v[e]);
       }
     }
+    mn = __reduce_min_sync(0xffffffffu, mn);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) {
+      part[0][tid >> 5] = mn;
+      part[1][tid >> 5] = mx;
+    }
+    __syncthreads();
+    int lo = __reduce_min_sync(0xffffffffu, lane < T / 32 ? part[0][lane] : INT_MAX) - 1;
+    int hi = __reduce_max_sync(0xffffffffu, lane < T / 32 ? part[1][lane] : INT_MIN);
+    __syncthreads();
+    below = 0;  // count(<= lo) = below < C <= count(<= hi)
+    for (int it = 0; hi - lo > 1; ++it) {  // block-uniform
+      const int mid = lo + ((hi - lo) >> 1);
+      int n = 0;
+#pragma unroll
+      for (int e = 0; e < kSelRegs; ++e) n += v[e] <= mid ? 1 : 0;
+      n = block_sum<T>(n, part, it & 1);
+      if (n >= C) {
+        hi = mid;
+      } else {
+        lo = mid;
+        below = n;
+      }
+    }
+    thr = hi;
+  } else {
+    const int nb = 2 * bits + 1;
+    for (int i = tid; i < nb; i += T) hist[i] = 0;
+    __syncthreads();
+    for (int i = tid; i < c; i += T) atomicAdd(&hist[(int)key_dist(src[i]) + bits], 1);
+    __syncthreads();
+    if (tid < 32) {  // the bin where the running count reaches C
+      const int per = (nb + 31) / 32, b0 = lane * per, b1 = min(nb, b0 + per);
+      int own = 0;
+      for (int b = b0; b < b1; ++b) own += hist[b];
+      int incl = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+      }
+      const unsigned hit = __ballot_sync(0xffffffffu, incl >= C);
+      const int L = __ffs(hit) - 1;  // hit != 0: the bins hold c > C keys
+      if (lane == L) {
+        int acc = incl - own;
+        for (int b = b0; b < b1; ++b) {
+          if (acc + hist[b] >= C) {
+            s_t = b - bits;
+            s_below = acc;
+            break;
+          }
+          acc += hist[b];
+        }
+      }
+    }
+    __syncthreads();
+    thr = s_t;
+    below = s_below;
   }
   __syncthreads();
-  const int t = s_t, below = s_below;
-  const int nt = hist[t];
+  for (int i0 = 0; i0 < c; i0 += T) {  // whole warps: their slots are taken together
+    const int i = i0 + tid;
+    const uint64_t key = i < c ? src[i] : kEmptyKey;
+    const int d = i < c ? (int)key_dist(key) : INT_MAX;
+    const int at = warp_slot(d < thr, &s_nout);
+    if (d < thr) dst[at] = key;
+    const int tt = warp_slot(d == thr, &s_ntie);
+    if (d == thr && tt < H_TIE_MAX) tie[tt] = key_id(key);
+  }
+  __syncthreads();
+  const int nt = s_ntie, want = C - below;  // 1 <= want <= nt
   if (nt > H_TIE_MAX) {  // block-uniform
     if (tid == 0) ovf[1 + atomicAdd(ovf, 1)] = q;
     return;
   }
-  for (int i = tid; i < c; i += blockDim.x) {
-    const uint64_t key = src[i];
-    const int b = (int)key_dist(key) + bits;
-    if (b < t) dst[atomicAdd(&s_nout, 1)] = key;
-    else if (b == t) tie[atomicAdd(&s_ntie, 1)] = key;
+  // the want-th lowest id of the tied ones (ids are distinct)
+  int lo = -1, hi = INT_MAX - 1;  // count(id <= lo) < want <= count(id <= hi)
+  if (nt > want) {
+    constexpr int R = H_TIE_MAX / T;
+    int v[R];
+    int mx = 0;
+#pragma unroll
+    for (int e = 0; e < R; ++e) {
+      v[e] = e * T + tid < nt ? tie[e * T + tid] : INT_MAX;
+      if (v[e] != INT_MAX) mx = max(mx, v[e]);
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) part[0][tid >> 5] = mx;
+    __syncthreads();
+    hi = __reduce_max_sync(0xffffffffu, lane < T / 32 ? part[0][lane] : 0);
+    __syncthreads();
+    for (int it = 0; hi - lo > 1; ++it) {
+      const int mid = lo + ((hi - lo) >> 1);
+      int n = 0;
+#pragma unroll
+      for (int e = 0; e < R; ++e) n += v[e] <= mid ? 1 : 0;
+      n = block_sum<T>(n, part, it & 1);
+      if (n >= want) hi = mid;
+      else lo = mid;
+      if (n == want) break;  // exactly the ids up to mid
+    }
   }
-  __syncthreads();
-  int P = 64;
-  while (P < nt) P <<= 1;
-  for (int i = nt + tid; i < P; i += blockDim.x) tie[i] = kEmptyKey;
-  __syncthreads();
-  block_bitonic_sort(tie, P);
-  for (int i = tid; i < C - below; i += blockDim.x) dst[below + i] = tie[i];
+  const float dist = (float)thr;
+  for (int i0 = 0; i0 < nt; i0 += T) {
+    const int i = i0 + tid;
+    const bool in = i < nt && tie[i] <= hi;
+    const int at = warp_slot(in, &s_nout);  // s_nout == below
+    if (in) dst[at] = make_key(dist, tie[i]);
+  }
 }
 
 // Rows of kp bytes (a multiple of 128); boxes of 128 bytes x box_rows rows, 128-byte swizzle.
@@ -1058,7 +1161,8 @@ void launch_int_select(const int* cnt, const uint64_t* cand, int cap, int need, 
     else if (C == 64) hsel_warp_kernel<2><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf);
     else hsel_warp_kernel<4><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf);
   } else {
-    hsel_hist_kernel<<<nq, 512, 0, s>>>(cnt, cand, cap, need, C, bits, out, ovf);
+    if (C <= 1024) hsel_kernel<256><<<nq, 256, 0, s>>>(cnt, cand, cap, need, C, bits, out, ovf);
+    else hsel_kernel<512><<<nq, 512, 0, s>>>(cnt, cand, cap, need, C, bits, out, ovf);
   }
   count_launch();
   LSHG_CHECK_LAUNCH();
