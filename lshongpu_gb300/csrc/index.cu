@@ -336,7 +336,8 @@ Index::~Index() {
   x.release(); xnorm.release(); xt.release(); xs.release(); xse.release(); xsl.release(); xsf.release(); xsft.release();
   sk_planes.release(); sk_split.release(); sk_pnorm.release();
   keys.release(); offsets.release(); buckets.release(); key_planes.release(); cp_diag.release(); bitmaps.release();
-  xbf.release(); xbf_scale.release(); xf8.release(); ebf.release(); ebf_res.release(); xnorm64.release(); xst.release(); qstats.release();
+  xbf.release(); xbf_scale.release(); xf8.release(); ebf.release(); ebf_res.release();
+  xq8.release(); xnorm64.release(); xst.release(); qstats.release();
   cws_tab.release(); cws_rank.release(); cws_key_tab.release();
   for (auto* ops : {&ops_keys, &ops_sketch})
     for (auto& op : *ops)
@@ -536,6 +537,7 @@ std::unique_ptr<Index> build_index(const lshg_index_params& p, DevBuf<float>&& b
       I.xs = std::move(packed);
       if (p.framework == 0) tile_sketches(I, s);
     }
+    derive_rerank_bounds(I, s);
   }
 
   // exact-distance arrays
@@ -663,14 +665,18 @@ void query_index(Index& I, float* q, int nq, int k, lshg_point* out, cudaStream_
     return;
   }
   const int C = std::max(I.C, kp);
+  auto rerank = [&](const uint64_t* cands, int count) {
+    if (rerank_by_bounds(I, cands, nq, count, q, k, out, s)) return;
+    launch_rerank(cands, nq, count, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, qnorm.ptr, I.dist, k, out, s, I.error_word(s),
+                  I.p.opt.fp64_recheck > 0, nullptr, extra);
+  };
   DevBuf<uint64_t> part;
   int splits;
   if (impl == 10) {  // CWS: the exact top-C by (1 - matches / S, id), then the generalized-Jaccard re-rank
     part.alloc((size_t)nq * C, s);
     launch_cws_scan(I.cws.pl ? I.xsl.ptr : nullptr, I.xst.ptr, I.n, I.cws_S, I.d, I.cws, qs.ptr, nq, C, part.ptr,
                     I.error_word(s), s);
-    launch_rerank(part.ptr, nq, C, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, qnorm.ptr, I.dist, k, out, s, I.error_word(s),
-                  I.p.opt.fp64_recheck > 0, nullptr, extra);
+    rerank(part.ptr, C);
     return;
   }
   if (impl == 6) {
@@ -684,8 +690,7 @@ void query_index(Index& I, float* q, int nq, int k, lshg_point* out, cudaStream_
       // tensor cores: the exact top-C by (sketch distance, id), then the same re-rank
       part.alloc((size_t)nq * C, s);
       tc::launch_tc_hamming(I.xse.ptr, I.n, I.xst.ptr, I.wp, I.words, qs.ptr, nq, op, C, part.ptr, I.error_word(s), s);
-      launch_rerank(part.ptr, nq, C, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, qnorm.ptr, I.dist, k, out, s, I.error_word(s),
-                    I.p.opt.fp64_recheck > 0, nullptr, extra);
+      rerank(part.ptr, C);
       return;
     }
     int fs = 0, fr = 0, fc = 0;
@@ -694,8 +699,7 @@ void query_index(Index& I, float* q, int nq, int k, lshg_point* out, cudaStream_
       // byte samples: bit-sliced threshold filter, the exact top-C, then the same re-rank
       part.alloc((size_t)nq * C, s);
       launch_byte_filter_scan(I.xsl.ptr, I.xst.ptr, I.n, I.wp, I.sbytes, qs.ptr, nq, C, part.ptr, I.error_word(s), s);
-      launch_rerank(part.ptr, nq, C, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, qnorm.ptr, I.dist, k, out, s, I.error_word(s),
-                    I.p.opt.fp64_recheck > 0, nullptr, extra);
+      rerank(part.ptr, C);
       return;
     }
     splits = scan_bits_splits(I.n, nq, C);
@@ -709,8 +713,7 @@ void query_index(Index& I, float* q, int nq, int k, lshg_point* out, cudaStream_
     launch_merge_splits(part.ptr, nq, splits, C, merged.ptr, s);
     cand = merged.ptr;
   }
-  launch_rerank(cand, nq, C, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, qnorm.ptr, I.dist, k, out, s, I.error_word(s),
-                I.p.opt.fp64_recheck > 0, nullptr, extra);
+  rerank(cand, C);
 }
 
 }  // namespace lshg

@@ -159,6 +159,10 @@ struct RerankBounds {
 // fp64_recheck: re-score, in double precision, the run of candidates around the k-th
 // place whose FP32 distances lie within the FP32 error bound of one another (among the
 // first 128) and order that run by the FP64 distance.
+// The Jaccard re-rank (k <= 128, C = 1024, 2048 or 4096) of the listed queries alone (listed[0] of
+// them, then their rows), into their rows of `out`.
+void launch_rerank_listed(const uint64_t* cand, int C, const float* x, int64_t n, int d, const float* q,
+                          const int* listed, int nq, int k, struct ::lshg_point_s* out, cudaStream_t s);
 // qnorm == nullptr (angular, C < 1024): the kernel computes the query norms itself, and writes
 // them to qnorm_out where given.
 void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t n, int d,

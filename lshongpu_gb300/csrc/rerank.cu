@@ -594,6 +594,42 @@ __global__ void __launch_bounds__(512) rerank_top_kernel(const uint64_t* __restr
   }
 }
 
+// Every candidate of the listed queries, a thread a candidate, then the block-wide sort: the rare
+// queries whose bounds leave too many candidates (rerank_bounds.cu).
+__global__ void __launch_bounds__(512) rerank_listed_kernel(const uint64_t* __restrict__ cand, int C,
+                                                            const float* __restrict__ x, int64_t n, int d,
+                                                            const float* __restrict__ q,
+                                                            const int* __restrict__ listed, int k,
+                                                            lshg_point* __restrict__ out) {
+  extern __shared__ __align__(16) unsigned char rsm[];
+  uint64_t* keys = reinterpret_cast<uint64_t*>(rsm);
+  float* qr = reinterpret_cast<float*>(rsm + (size_t)C * 8);
+  const int cnt = listed[0];
+  for (int t = blockIdx.x; t < cnt; t += gridDim.x) {
+    const int qi = listed[1 + t];
+    for (int j = threadIdx.x; j < d; j += blockDim.x) qr[j] = q[(int64_t)qi * d + j];
+    __syncthreads();
+    for (int i = threadIdx.x; i < C; i += blockDim.x) {
+      const uint64_t kin = cand[(int64_t)qi * C + i];
+      const int id = key_id(kin);
+      uint64_t ko = kEmptyKey;
+      if (kin != kEmptyKey && id >= 0 && id < n)
+        ko = make_key(exact_distance<DIST_JACCARD>(x + (int64_t)id * d, qr, d, 1.0f, 1.0f), id);
+      keys[i] = ko;
+    }
+    __syncthreads();
+    block_bitonic_sort(keys, C);
+    for (int i = threadIdx.x; i < k; i += blockDim.x) {
+      const uint64_t kk = keys[i];
+      lshg_point pt;
+      if (kk == kEmptyKey) { pt.ID = -1; pt.distance = kEmptyDistance; }
+      else { pt.ID = key_id(kk); pt.distance = key_dist(kk); }
+      out[(int64_t)qi * k + i] = pt;
+    }
+    __syncthreads();
+  }
+}
+
 __global__ void keys_to_points_kernel(const uint64_t* __restrict__ keys, int nq, int C, int k,
                                       lshg_point* __restrict__ out) {
   int64_t total = (int64_t)nq * k;
@@ -763,6 +799,18 @@ void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t 
     default: throw Error(LSHG_ERR_INVALID_ARGUMENT, "re-rank: invalid distance function");
   }
 #undef LSHG_RR
+  count_launch();
+  LSHG_CHECK_LAUNCH();
+}
+
+void launch_rerank_listed(const uint64_t* cand, int C, const float* x, int64_t n, int d, const float* q,
+                          const int* listed, int nq, int k, lshg_point* out, cudaStream_t s) {
+  if (nq <= 0) return;
+  LSHG_REQUIRE(k <= C && C <= 4096 && (C & (C - 1)) == 0, "listed re-rank: C must be a power of two up to 4096");
+  ProfScope _ps("rerank_listed", s);
+  const size_t smem = (size_t)C * 8 + (size_t)d * 4 + 16;
+  LSHG_CUDA(cudaFuncSetAttribute(rerank_listed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  rerank_listed_kernel<<<std::min(nq, num_sms() * 4), 512, smem, s>>>(cand, C, x, n, d, q, listed, k, out);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

@@ -199,3 +199,27 @@ def test_exact_scan_split_merges(engine, orc, n, nq, k, d, dist):
     else:
         assert np.array_equal(res["ID"], ids)
         assert np.array_equal(res["distance"], ds)
+
+
+@pytest.mark.parametrize("n,nq,k,d,C", [
+    (4000, 40, 32, 100, 4096),   # 128-byte quantised rows
+    (2000, 33, 128, 120, 2048),  # the widest; the longest k
+    (1000, 20, 1, 16, 1024),     # 32-byte rows
+    (1000, 20, 10, 121, 1024),   # beyond them: every candidate is scored
+    (3000, 20, 200, 50, 4096),   # k beyond them
+])
+@pytest.mark.parametrize("hard", [False, True])
+def test_jaccard_bounds_rerank_equals_exact_scan(engine, n, nq, k, d, C, hard):
+    """A list that holds the whole base re-ranks to the exact generalized-Jaccard scan, bit for
+    bit: through the bounds, and where they leave too many candidates (copies of one row) or
+    do not apply (a query with negative values)."""
+    x, q = datasets.sparse_gamma(n, d, 101), datasets.sparse_gamma(nq, d, 102)
+    if hard:
+        x[::2] = x[0]
+        q[::5] = x[0]
+        q[3, : d // 2] = -2.5
+        q[4] = 0
+        q[4, 0] = 1e-6
+    idx = engine.Index(x, implementation=10, distanceFunc=2, sketchDim=64, options=engine.make_options(candidates=C))
+    ex = engine.Index(x, implementation=2, distanceFunc=2)
+    assert idx.query(q, k).tobytes() == ex.query(q, k).tobytes()
