@@ -337,7 +337,7 @@ Index::~Index() {
   sk_planes.release(); sk_split.release(); sk_pnorm.release();
   keys.release(); offsets.release(); buckets.release(); key_planes.release(); cp_diag.release(); bitmaps.release();
   xbf.release(); xbf_scale.release(); xf8.release(); ebf.release(); ebf_res.release();
-  xq8.release(); xnorm64.release(); xst.release(); qstats.release();
+  xq8.release(); xq8_tail.release(); xnorm64.release(); xst.release(); qstats.release();
   cws_tab.release(); cws_rank.release(); cws_key_tab.release();
   for (auto* ops : {&ops_keys, &ops_sketch})
     for (auto& op : *ops)
@@ -537,8 +537,8 @@ std::unique_ptr<Index> build_index(const lshg_index_params& p, DevBuf<float>&& b
       I.xs = std::move(packed);
       if (p.framework == 0) tile_sketches(I, s);
     }
-    derive_rerank_bounds(I, s);
   }
+  derive_rerank_bounds(I, s);
 
   // exact-distance arrays
   if (I.dist == DIST_ANGULAR) {
@@ -644,6 +644,8 @@ void query_index(Index& I, float* q, int nq, int k, lshg_point* out, cudaStream_
     if (a.split_cap == 0) LSHG_CUDA(cudaMemsetAsync(bm.ptr, 0, bm.bytes(), s));
     a.bitmaps = bm.ptr;
     a.stats = I.qstats.ptr;
+    a.xq8 = I.xq8.ptr;
+    a.xq8_tail = I.xq8_tail.ptr;
     a.err = I.error_word(s);
     launch_lsh_query(a, out, s);
     return;
@@ -666,7 +668,7 @@ void query_index(Index& I, float* q, int nq, int k, lshg_point* out, cudaStream_
   }
   const int C = std::max(I.C, kp);
   auto rerank = [&](const uint64_t* cands, int count) {
-    if (rerank_by_bounds(I, cands, nq, count, q, k, out, s)) return;
+    if (rerank_by_bounds(I, cands, nq, count, q, qnorm.ptr, k, out, s)) return;
     launch_rerank(cands, nq, count, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, qnorm.ptr, I.dist, k, out, s, I.error_word(s),
                   I.p.opt.fp64_recheck > 0, nullptr, extra);
   };

@@ -71,9 +71,11 @@ struct Index {
   CwsCodes cws;              // CWS code plan (derived from xs at build and at load)
   DevBuf<uint8_t> cws_rank;  // CWS per-position code dictionaries (derived, not stored)
 
-  // Jaccard re-rank of long lists: rows quantised to 8 bits at scale xq8_scale, with their sums and
-  // residuals (rerank_bounds.cu; derived, not stored; empty when the data have no such bounds)
+  // Re-rank of long lists and scoring of LSH candidates: rows quantised to 8 bits, with the sums,
+  // scales and residuals that bound distances from them (rerank_bounds.cu; derived, not stored;
+  // empty when the data have no such bounds)
   DevBuf<uint8_t> xq8;
+  DevBuf<float2> xq8_tail;
   float xq8_scale = 0.0f;
 
   // LSH
@@ -154,12 +156,12 @@ void tile_sketches(Index& idx, cudaStream_t stream);
 // and the split SimHash planes of the tensor-core projection.
 void derive_tc(Index& idx, cudaStream_t stream);
 void derive_simhash(Index& idx, cudaStream_t stream);
-// The Jaccard re-rank's quantised rows (Index::xq8), and the re-rank through them: the results of
+// The re-rank's quantised rows (Index::xq8), and the re-rank through them: the results of
 // launch_rerank over the candidates.  False when the index, C or k is not one it serves or its
 // temporaries do not fit: nothing has been written to `out` then.
 void derive_rerank_bounds(Index& idx, cudaStream_t stream);
-bool rerank_by_bounds(Index& idx, const uint64_t* cand, int nq, int C, const float* q, int k, lshg_point* out,
-                      cudaStream_t stream);
+bool rerank_by_bounds(Index& idx, const uint64_t* cand, int nq, int C, const float* q, const float* qnorm, int k,
+                      lshg_point* out, cudaStream_t stream);
 // The exact angular scan's BF16 rows (Index::ebf); waits for the stream.
 void derive_exact(Index& idx, cudaStream_t stream);
 // Exact angular top-k through the tensor-core filter (scan_exact.cu): the ids and distances of

@@ -159,10 +159,18 @@ struct RerankBounds {
 // fp64_recheck: re-score, in double precision, the run of candidates around the k-th
 // place whose FP32 distances lie within the FP32 error bound of one another (among the
 // first 128) and order that run by the FP64 distance.
-// The Jaccard re-rank (k <= 128, C = 1024, 2048 or 4096) of the listed queries alone (listed[0] of
-// them, then their rows), into their rows of `out`.
-void launch_rerank_listed(const uint64_t* cand, int C, const float* x, int64_t n, int d, const float* q,
-                          const int* listed, int nq, int k, struct ::lshg_point_s* out, cudaStream_t s);
+// The re-rank (k <= 128, C = 1024, 2048 or 4096; Jaccard or angular) of the listed queries alone
+// (listed[0] of them, then their rows), into their rows of `out`.
+void launch_rerank_listed(const uint64_t* cand, int C, const float* x, int64_t n, int d, const float* xnorm,
+                          const float* q, const float* qnorm, int dist, const int* listed, int nq, int k,
+                          struct ::lshg_point_s* out, cudaStream_t s);
+// Angular candidates (lists of at most cap <= kListBounds ids, ccnt[q] of them) reduced by bounds to
+// those that can be in the top-k: kept[nq][kBoundsKeep] keys; listed: count, then the queries to score
+// in full (rerank_bounds.cu).  Queries with more than cap ids are left out (their kept is empty).
+constexpr int kBoundsKeep = 256;
+constexpr int kListBounds = 6144;
+void launch_list_bounds(const int* list, int cap, const int* ccnt, const uint8_t* rows, const float2* tails, int64_t n,
+                        int d, const float* q, int nq, int k, uint64_t* kept, int* listed, cudaStream_t s);
 // qnorm == nullptr (angular, C < 1024): the kernel computes the query norms itself, and writes
 // them to qnorm_out where given.
 void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t n, int d,
@@ -222,6 +230,8 @@ struct LshQueryArgs {
   int* qctr;                  // internal: the fused kernel's query counter (zero at launch)
   const int* qlist;           // internal: queries to answer ([0] = count, then indices); nullptr = all
   int* lists;                 // internal: the fused kernel's distinct-id lists, [grid][list capacity]
+  const uint8_t* xq8;         // angular: 8-bit rows and their tails for the bounds (nullptr: none)
+  const float2* xq8_tail;
 };
 void launch_lsh_query(const LshQueryArgs& a, struct ::lshg_point_s* out, cudaStream_t s);
 

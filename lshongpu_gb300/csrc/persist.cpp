@@ -428,7 +428,7 @@ std::unique_ptr<Index> load_index(const char* path) {
   if (I.p.framework == 0 && (I.p.implementation == 8 || I.p.implementation == 9)) derive_tc(I, s);
   if (I.p.framework == 0 && (I.p.implementation == 1 || I.p.implementation == 2)) derive_exact(I, s);
   derive_simhash(I, s);
-  if (I.sk_kind) derive_rerank_bounds(I, s);
+  derive_rerank_bounds(I, s);
   I.qstats.alloc(2, s);
   LSHG_CUDA(cudaMemsetAsync(I.qstats.ptr, 0, I.qstats.bytes(), s));
   LSHG_CUDA(cudaStreamSynchronize(s));

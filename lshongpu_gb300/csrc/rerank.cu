@@ -596,9 +596,12 @@ __global__ void __launch_bounds__(512) rerank_top_kernel(const uint64_t* __restr
 
 // Every candidate of the listed queries, a thread a candidate, then the block-wide sort: the rare
 // queries whose bounds leave too many candidates (rerank_bounds.cu).
+template <int DIST>
 __global__ void __launch_bounds__(512) rerank_listed_kernel(const uint64_t* __restrict__ cand, int C,
                                                             const float* __restrict__ x, int64_t n, int d,
+                                                            const float* __restrict__ xnorm,
                                                             const float* __restrict__ q,
+                                                            const float* __restrict__ qnorm,
                                                             const int* __restrict__ listed, int k,
                                                             lshg_point* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char rsm[];
@@ -614,7 +617,9 @@ __global__ void __launch_bounds__(512) rerank_listed_kernel(const uint64_t* __re
       const int id = key_id(kin);
       uint64_t ko = kEmptyKey;
       if (kin != kEmptyKey && id >= 0 && id < n)
-        ko = make_key(exact_distance<DIST_JACCARD>(x + (int64_t)id * d, qr, d, 1.0f, 1.0f), id);
+        ko = make_key(exact_distance<DIST>(x + (int64_t)id * d, qr, d, DIST == DIST_ANGULAR ? qnorm[qi] : 1.0f,
+                                           DIST == DIST_ANGULAR ? xnorm[id] : 1.0f),
+                      id);
       keys[i] = ko;
     }
     __syncthreads();
@@ -803,14 +808,16 @@ void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t 
   LSHG_CHECK_LAUNCH();
 }
 
-void launch_rerank_listed(const uint64_t* cand, int C, const float* x, int64_t n, int d, const float* q,
-                          const int* listed, int nq, int k, lshg_point* out, cudaStream_t s) {
+void launch_rerank_listed(const uint64_t* cand, int C, const float* x, int64_t n, int d, const float* xnorm,
+                          const float* q, const float* qnorm, int dist, const int* listed, int nq, int k,
+                          lshg_point* out, cudaStream_t s) {
   if (nq <= 0) return;
   LSHG_REQUIRE(k <= C && C <= 4096 && (C & (C - 1)) == 0, "listed re-rank: C must be a power of two up to 4096");
   ProfScope _ps("rerank_listed", s);
   const size_t smem = (size_t)C * 8 + (size_t)d * 4 + 16;
-  LSHG_CUDA(cudaFuncSetAttribute(rerank_listed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  rerank_listed_kernel<<<std::min(nq, num_sms() * 4), 512, smem, s>>>(cand, C, x, n, d, q, listed, k, out);
+  auto kern = dist == DIST_JACCARD ? rerank_listed_kernel<DIST_JACCARD> : rerank_listed_kernel<DIST_ANGULAR>;
+  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<std::min(nq, num_sms() * 4), 512, smem, s>>>(cand, C, x, n, d, xnorm, q, qnorm, listed, k, out);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

@@ -223,3 +223,32 @@ def test_jaccard_bounds_rerank_equals_exact_scan(engine, n, nq, k, d, C, hard):
     idx = engine.Index(x, implementation=10, distanceFunc=2, sketchDim=64, options=engine.make_options(candidates=C))
     ex = engine.Index(x, implementation=2, distanceFunc=2)
     assert idx.query(q, k).tobytes() == ex.query(q, k).tobytes()
+
+
+@pytest.mark.parametrize("n,nq,k,d,hashes,tables", [
+    (30000, 40, 32, 100, 2, 24),   # lists through the bounds
+    (30000, 40, 128, 128, 2, 32),  # the longest k and widest rows
+    (30000, 40, 10, 16, 2, 24),    # many candidates within the bounds: scored in full
+    (30000, 30, 32, 37, 2, 24),    # rows without 16-byte loads: the fused kernel
+])
+@pytest.mark.parametrize("hard", [False, True])
+def test_lsh_bounds_scoring_equals_oracle(engine, orc, n, nq, k, d, hashes, tables, hard):
+    """LSH queries whose candidates are reduced by bounds return the oracle's walk and scoring of
+    the same tables, bit for bit; copies of one row, which the bounds cannot separate, too."""
+    x, q = data(n, nq, d, count=60)
+    if hard:
+        x[::3] = x[0]
+        q[:10] = x[0]
+    P = 1 << (d - 1).bit_length()
+    bits = hashes * P.bit_length()
+    idx = engine.Index(x, implementation=2, distanceFunc=1, framework=1, keysImplementation=7, bucketKeyBits=bits,
+                       tables=tables, options=engine.make_options(cp_hashes=hashes))
+    xn, qn = orc.normalize(x), orc.normalize(q)
+    diag = engine.random_plus_minus(P * tables * 3 * hashes)
+    okeys, oqk = (orc.crosspoly(v, P, tables, hashes, 3, diag) for v in (xn, qn))
+    ooff, obk = orc.lsh_build(okeys, tables, 1 << bits)
+    ids, ds = orc.lsh_query(xn, qn, oqk, tables, 1 << bits, ooff, obk, 0, 0, None, None, 0,
+                            max(32, 1 << (k - 1).bit_length()), 1, k)
+    res = idx.query(q, k)
+    assert np.array_equal(res["ID"], ids)
+    assert np.array_equal(res["distance"], ds)
