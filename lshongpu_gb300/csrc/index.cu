@@ -337,7 +337,7 @@ Index::~Index() {
   sk_planes.release(); sk_split.release(); sk_pnorm.release();
   keys.release(); offsets.release(); buckets.release(); key_planes.release(); cp_diag.release(); bitmaps.release();
   xbf.release(); xbf_scale.release(); xf8.release(); ebf.release(); ebf_res.release();
-  xq8.release(); xq8_tail.release(); xnorm64.release(); xst.release(); qstats.release();
+  xq8.release(); xq8_tail.release(); jq.release(); jq_tail.release(); xnorm64.release(); xst.release(); qstats.release();
   cws_tab.release(); cws_rank.release(); cws_key_tab.release();
   for (auto* ops : {&ops_keys, &ops_sketch})
     for (auto& op : *ops)
@@ -549,6 +549,7 @@ std::unique_ptr<Index> build_index(const lshg_index_params& p, DevBuf<float>&& b
     I.xt.alloc((size_t)ceil_div(n, 128) * 128 * d, s);
     launch_tile_transpose(X, n, d, I.xt.ptr, s);
     derive_exact(I, s);
+    derive_jaccard_scan(I, s);
   }
   if (p.framework == 0 && (impl == 8 || impl == 9)) tc_prepare(I, s);
   if (p.framework == 1) I.lsh_grid = lsh_query_grid(1 << 30);
@@ -601,7 +602,9 @@ void query_index(Index& I, float* q, int nq, int k, lshg_point* out, cudaStream_
     launch_tc_scan(I, q, nq, k, out, s, extra);
     return;
   }
-  if (I.p.framework == 0 && impl == 2 && query_exact_filtered(I, q, nq, k, out, s)) return;
+  if (I.p.framework == 0 && impl == 2 &&
+      (query_exact_filtered(I, q, nq, k, out, s) || query_jaccard_filtered(I, q, nq, k, out, s)))
+    return;
   DevBuf<float> qnorm;
   if (I.dist == DIST_ANGULAR) {
     qnorm.alloc(nq, s);

@@ -77,6 +77,11 @@ struct Index {
   DevBuf<uint8_t> xq8;
   DevBuf<float2> xq8_tail;
   float xq8_scale = 0.0f;
+  // Exact Jaccard scan: 8-bit codes in 128-point tiles and the rows' sums and residuals
+  // (scan_jaccard.cu; derived, not stored)
+  DevBuf<uint32_t> jq;
+  DevBuf<float4> jq_tail;
+  float jq_scale = 0.0f, jq_lo = 0.0f;
 
   // LSH
   int key_kind = 0;
@@ -162,6 +167,13 @@ void derive_simhash(Index& idx, cudaStream_t stream);
 void derive_rerank_bounds(Index& idx, cudaStream_t stream);
 bool rerank_by_bounds(Index& idx, const uint64_t* cand, int nq, int C, const float* q, const float* qnorm, int k,
                       lshg_point* out, cudaStream_t stream);
+// The smallest and largest of `total` values (device); false when one is negative, not finite or
+// beyond 1e18, or all are below 1e-18.  Waits for the stream.
+bool base_range(const float* x, int64_t total, float* lo, float* hi, cudaStream_t stream);
+// The exact Jaccard scan's codes (Index::jq), and the scan through them: as the exact angular
+// scan's below.
+void derive_jaccard_scan(Index& idx, cudaStream_t stream);
+bool query_jaccard_filtered(Index& idx, const float* q, int nq, int k, lshg_point* out, cudaStream_t stream);
 // The exact angular scan's BF16 rows (Index::ebf); waits for the stream.
 void derive_exact(Index& idx, cudaStream_t stream);
 // Exact angular top-k through the tensor-core filter (scan_exact.cu): the ids and distances of

@@ -136,13 +136,13 @@ void launch_cws_scan(const uint32_t* xsl_t, const uint32_t* xst, int64_t n, int 
 
 // ---- rerank.cu -------------------------------------------------------------------
 // Merge per-split sorted lists into one sorted list of C keys per query.
-// The exact angular top-k of the queries listed on the device (list[0] = count, list[1..] =
+// The exact top-k (angular or Jaccard) of the queries listed on the device (list[0] = count, list[1..] =
 // rows of q), written to their rows of `out`; k <= 128.  part: nq * listed_splits(n, nq, C) * C
 // keys, C = the power of two >= max(32, k).
 int scan_listed_splits(int64_t n, int nq, int C);
 void launch_scan_float_listed(const float* xt, int64_t n, int d, const float* xnorm, const float* q, int nq,
-                              const float* qnorm, const int* list, int C, int splits, uint64_t* part, int k,
-                              struct ::lshg_point_s* out, cudaStream_t s);
+                              const float* qnorm, int dist, const int* list, int C, int splits, uint64_t* part,
+                              int k, struct ::lshg_point_s* out, cudaStream_t s);
 void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t* out, cudaStream_t s);
 // The same with the first k keys written as points; false when C or k is not one it serves.
 bool launch_merge_points(const uint64_t* in, int nq, int splits, int C, int k, struct ::lshg_point_s* out,

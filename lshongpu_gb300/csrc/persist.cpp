@@ -426,7 +426,10 @@ std::unique_ptr<Index> load_index(const char* path) {
   for (auto& kv : r.staged) kv.second.upload(s);
   if (I.p.framework == 0 && I.xs.n) tile_sketches(I, s);  // derived layouts, not stored
   if (I.p.framework == 0 && (I.p.implementation == 8 || I.p.implementation == 9)) derive_tc(I, s);
-  if (I.p.framework == 0 && (I.p.implementation == 1 || I.p.implementation == 2)) derive_exact(I, s);
+  if (I.p.framework == 0 && (I.p.implementation == 1 || I.p.implementation == 2)) {
+    derive_exact(I, s);
+    derive_jaccard_scan(I, s);
+  }
   derive_simhash(I, s);
   derive_rerank_bounds(I, s);
   I.qstats.alloc(2, s);

@@ -57,19 +57,22 @@ constexpr int64_t kBoundsMinCandidates = 16384;
 int jaccard_pitch(int d) { return (d + 8 + 31) / 32 * 32; }
 int angular_pitch(int d) { return (d + 15) / 16 * 16; }
 
-// stat[0]: bits of the largest value; stat[1]: 1 when a value is negative or not finite.
-__global__ void base_max_kernel(const float* __restrict__ x, int64_t total, unsigned* stat) {
-  float m = 0.0f;
+// stat[0]: bits of the largest value; stat[1]: 1 when a value is negative or not finite; stat[2]:
+// complement of the bits of the smallest value.
+__global__ void base_range_kernel(const float* __restrict__ x, int64_t total, unsigned* stat) {
+  float m = 0.0f, lo = INFINITY;
   bool bad = false;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const float v = x[i];
-    if (v >= 0.0f && v <= 1e18f) m = fmaxf(m, v);
+    const float v = fabsf(x[i]) == 0.0f ? 0.0f : x[i];  // -0: its bits are not ordered
+    if (v >= 0.0f && v <= 1e18f) m = fmaxf(m, v), lo = fminf(lo, v);
     else bad = true;
   }
   const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+  const unsigned wl = __reduce_max_sync(0xffffffffu, ~__float_as_uint(lo));
   const bool wb = __any_sync(0xffffffffu, bad);
   if ((threadIdx.x & 31) == 0) {
     atomicMax(stat, w);
+    atomicMax(stat + 2, wl);
     if (wb) atomicExch(stat + 1, 1u);
   }
 }
@@ -425,21 +428,10 @@ void launch_bounds(const uint64_t* cand, const int* list, int list_cap, const in
 }
 
 void derive_jaccard(Index& I, cudaStream_t s) {
-  DevBuf<unsigned> stat(2, s);
-  LSHG_CUDA(cudaMemsetAsync(stat.ptr, 0, stat.bytes(), s));
-  const int64_t total = I.n * I.d;
-  base_max_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, (int64_t)num_sms() * 8)), 256, 0,
-                    s>>>(I.x.ptr, total, stat.ptr);
-  count_launch();
-  LSHG_CHECK_LAUNCH();
-  unsigned h[2];
-  LSHG_CUDA(cudaMemcpyAsync(h, stat.ptr, sizeof(h), cudaMemcpyDeviceToHost, s));
-  LSHG_CUDA(cudaStreamSynchronize(s));
-  float mx;
-  memcpy(&mx, &h[0], 4);
-  if (h[1] || !(mx > 1e-18f)) return;  // no such bounds: every candidate is scored
+  float lo, hi;
+  if (!base_range(I.x.ptr, I.n * I.d, &lo, &hi, s)) return;  // no such bounds: every candidate is scored
   I.xq8.alloc((size_t)I.n * jaccard_pitch(I.d), s);
-  I.xq8_scale = 255.0f / mx;
+  I.xq8_scale = 255.0f / hi;
   quantise_rows_kernel<<<(int)std::min<int64_t>((I.n * 32 + 255) / 256, (int64_t)num_sms() * 16), 256, 0, s>>>(
       I.x.ptr, I.n, I.d, jaccard_pitch(I.d), I.xq8_scale, I.xq8.ptr);
   count_launch();
@@ -463,6 +455,22 @@ void derive_angular(Index& I, cudaStream_t s) {
 }
 
 }  // namespace
+
+bool base_range(const float* x, int64_t total, float* lo, float* hi, cudaStream_t s) {
+  DevBuf<unsigned> stat(3, s);
+  LSHG_CUDA(cudaMemsetAsync(stat.ptr, 0, stat.bytes(), s));
+  base_range_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, (int64_t)num_sms() * 8)), 256, 0,
+                      s>>>(x, total, stat.ptr);
+  count_launch();
+  LSHG_CHECK_LAUNCH();
+  unsigned h[3];
+  LSHG_CUDA(cudaMemcpyAsync(h, stat.ptr, sizeof(h), cudaMemcpyDeviceToHost, s));
+  LSHG_CUDA(cudaStreamSynchronize(s));
+  h[2] = ~h[2];
+  memcpy(hi, &h[0], 4);
+  memcpy(lo, &h[2], 4);
+  return !h[1] && *hi > 1e-18f;
+}
 
 void derive_rerank_bounds(Index& I, cudaStream_t s) {
   const bool linear = I.p.framework == 0 && I.C >= 1024;

@@ -161,7 +161,7 @@ bool query_exact_filtered(Index& I, const float* q, int nq, int k, lshg_point* o
                         plan.M > 0 ? tau.ptr : nullptr, eps.ptr, best.ptr, ovf, s);
     launch_rerank(best.ptr, nq, CT, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, nullptr, DIST_ANGULAR, k, out, s,
                   I.error_word(s), false, nullptr, nullptr, qnorm.ptr);
-    launch_scan_float_listed(I.xt.ptr, I.n, I.d, I.xnorm.ptr, q, nq, qnorm.ptr, ovf, C, splits, part.ptr, k, out, s);
+    launch_scan_float_listed(I.xt.ptr, I.n, I.d, I.xnorm.ptr, q, nq, qnorm.ptr, DIST_ANGULAR, ovf, C, splits, part.ptr, k, out, s);
   } catch (const Error& e) {
     if (e.status != LSHG_ERR_OUT_OF_MEMORY) throw;
     cudaGetLastError();  // temporaries that do not fit: the FP32 scan needs fewer

@@ -515,7 +515,7 @@ __global__ void listed_points_kernel(const uint64_t* __restrict__ part, const in
   }
 }
 
-template <int EC>
+template <int DIST, int EC>
 void launch_listed(const float* xt, int64_t n, int d, const float* xnorm, const float* q, const float* qnorm,
                    const int* list, int splits, uint64_t* part, cudaStream_t s) {
   const int nbuf = reg_scan_smem(d, 32 * EC, 1) <= kRegTwoCtaSmem ? 1 : 2;
@@ -523,7 +523,7 @@ void launch_listed(const float* xt, int64_t n, int d, const float* xnorm, const 
   const int nb = smem <= 220 * 1024 ? nbuf : 1;
   smem = reg_scan_smem(d, 32 * EC, nb);
   LSHG_REQUIRE(smem <= 220 * 1024, "listed scan: dimension too large");
-  auto kern = scan_float_listed_kernel<DIST_ANGULAR, EC>;
+  auto kern = scan_float_listed_kernel<DIST, EC>;
   LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int tps = ceil_div(ceil_div(n, kTile), splits);
   kern<<<num_sms() * 2, 256, smem, s>>>(xt, n, d, xnorm, q, qnorm, list, tps, splits, nb, part);
@@ -637,13 +637,20 @@ int scan_listed_splits(int64_t n, int nq, int C) {
 }
 
 void launch_scan_float_listed(const float* xt, int64_t n, int d, const float* xnorm, const float* q, int nq,
-                              const float* qnorm, const int* list, int C, int splits, uint64_t* part, int k,
-                              lshg_point* out, cudaStream_t s) {
+                              const float* qnorm, int dist, const int* list, int C, int splits, uint64_t* part,
+                              int k, lshg_point* out, cudaStream_t s) {
   ProfScope _ps("scan_float_listed", s);
-  if (C == 32) launch_listed<1>(xt, n, d, xnorm, q, qnorm, list, splits, part, s);
-  else if (C == 64) launch_listed<2>(xt, n, d, xnorm, q, qnorm, list, splits, part, s);
-  else if (C == 128) launch_listed<4>(xt, n, d, xnorm, q, qnorm, list, splits, part, s);
+  const bool jac = dist == DIST_JACCARD;
+#define LSHG_LS(EC)                                                                                          \
+  do {                                                                                                       \
+    if (jac) launch_listed<DIST_JACCARD, EC>(xt, n, d, xnorm, q, qnorm, list, splits, part, s);              \
+    else launch_listed<DIST_ANGULAR, EC>(xt, n, d, xnorm, q, qnorm, list, splits, part, s);                  \
+  } while (0)
+  if (C == 32) LSHG_LS(1);
+  else if (C == 64) LSHG_LS(2);
+  else if (C == 128) LSHG_LS(4);
   else throw Error(LSHG_ERR_INVALID_ARGUMENT, "listed scan: C must be 32, 64 or 128");
+#undef LSHG_LS
   listed_points_kernel<<<std::min(nq, num_sms() * 4), 128, (size_t)C * 8, s>>>(part, list, splits, C, k, out);
   count_launch();
   LSHG_CHECK_LAUNCH();

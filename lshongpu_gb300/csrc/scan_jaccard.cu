@@ -1,0 +1,313 @@
+// Exact generalized-Jaccard top-k through 8-bit rows (implementation 2; the reference's plain exact
+// scan, memOptimizedLinearScan.cu:20-106, with generalizedJaccard, distanceFunctions.cuh:10-21):
+// ids and distances are those of the FP32 scan of scan_float.cu, bit for bit.
+//
+// The FP32 scan pays two minima or maxima (half rate) and two additions a dimension of every
+// pair.  Here every pair is first bounded from 8-bit codes, four dimensions an instruction: with
+// the codes u = rint(s (x - lo)) of [lo, lo + 255 / s], the base's range,
+// sum min(u_q, u_x) = (sum u_q + sum u_x - sum |u_q - u_x|) / 2, and the distance lies between the
+// bounds of rerank_bounds.cu (the same residuals and allowance for FP32 arithmetic).  Two passes:
+//   thresholds  the smallest upper bound of every 32 points of every S-th tile; T[q] = the k-th
+//               smallest of these (k different points have at most it), so the k-th smallest
+//               distance is at most T;
+//   candidates  points whose lower bound is at most T -- every point of the top-k -- are listed
+//               (at most 512 or 1,024 a query) and scored with the reference's formula (launch_rerank).
+// Queries with more candidates, or with a negative or non-finite value, are scanned by the FP32
+// scan from a list on the device.  A base with such a value always takes it.
+//
+// scan kernel: a CTA takes 64 queries and a run of 128-point tiles, warp w queries 8w .. 8w + 7,
+// lane l points 4l .. 4l + 3: 32 sums a thread, three shared 16-byte loads a four-dimension step.
+// Measured (60,013 x 100, 129 queries, k = 10): the FP32 scan 413 us, this 120 (the two
+// passes 19 + 31; the rest is launches and latency); 1M x 100, one query 2,140 -> 246, 100 queries,
+// k = 32, 2,640 -> 1,000.  The divisions of every bound instead of the linear form below: 49 us for
+// the second pass.
+#include <algorithm>
+
+#include "index.h"
+#include "launch_count.h"
+#include "profile.h"
+#include "tc_filter.h"
+
+namespace lshg {
+
+namespace {
+
+constexpr int kTile = 128;
+constexpr int kQB = 64;
+constexpr int kMinDim = 16;   // 8-bit codes of fewer dimensions leave too many candidates
+constexpr int kMaxDim = 128;  // the listed FP32 scan's shared memory
+constexpr int kMinBase = 4096;
+constexpr int64_t kMinPairs = 16384;
+
+__device__ __forceinline__ unsigned code(float v, float s) {
+  return (unsigned)__float2int_rn(fminf(fmaxf(v * s, 0.0f), 255.0f));
+}
+
+__device__ __forceinline__ unsigned sad4(unsigned a, unsigned b, unsigned c) {  // c + sum |a_i - b_i|
+  unsigned r;
+  asm("vabsdiff4.u32.u32.u32.add %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+  return r;
+}
+
+__device__ __forceinline__ float delta(int d) { return (2.0f * d + 7.0f) * 1.2e-7f + 2e-6f; }
+
+// ROWS rows a block: their codes as [wd][ROWS] words (byte j of word w = dimension 4w + j), and for
+// each row (2 s S, U - 2 s E, U + 2 s E, 0): S its sum, U its codes' sum + s lo d, E its share of what the
+// codes and the FP32 sums hide.  With these of a query and a point added and A = sum |u_q - u_x|,
+// A_lo = (P - A) / 2 s and A_hi = (Q - A) / 2 s bound the sum of minima.  bad[i] = 1 for a row without
+// bounds.
+template <int ROWS>
+__global__ void __launch_bounds__(256) code_tiles_kernel(const float* __restrict__ x, int64_t n, int d, int wd, float lo,
+                                                         float s, uint32_t* __restrict__ out, float4* __restrict__ tails,
+                                                         int* __restrict__ bad) {
+  extern __shared__ uint32_t rows[];  // [ROWS][wd | 1]
+  const int pitch = wd | 1, lane = threadIdx.x & 31;
+  const int64_t row0 = (int64_t)blockIdx.x * ROWS;
+  const float inv = 1.0f / s;
+  for (int r = threadIdx.x >> 5; r < ROWS; r += 8) {
+    const int64_t i = row0 + r;
+    uint8_t* codes = reinterpret_cast<uint8_t*>(rows + r * pitch);
+    float sum = 0.0f, err = 0.0f;
+    unsigned total = 0;
+    bool wrong = false;
+    for (int c = lane; c < 4 * wd; c += 32) {
+      const float v = i < n && c < d ? x[i * d + c] : 0.0f;
+      if (c >= d) {
+        codes[c] = 0;
+        continue;
+      }
+      wrong |= !(v >= 0.0f && v <= 1e18f);
+      const unsigned u = code(v - lo, s);
+      codes[c] = (uint8_t)u;
+      total += u;
+      sum += v;
+      err += fabsf(v - (lo + (float)u * inv));
+    }
+    total = __reduce_add_sync(0xffffffffu, total);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      err += __shfl_xor_sync(0xffffffffu, err, o);
+    }
+    wrong = __any_sync(0xffffffffu, wrong) || !(sum > 1e-6f && 2.0f * s * sum < 1e30f);
+    if (lane == 0) {
+      const float e = 2.0f * s * (err * 1.0001f + sum * 2e-5f);
+      const float u = (float)total + s * lo * (float)d;
+      tails[row0 + r] = make_float4(2.0f * s * sum, u - e, u + e, 0.0f);
+      if (bad && i < n) bad[i] = wrong ? 1 : 0;
+    }
+  }
+  __syncthreads();
+  uint32_t* dst = out + (int64_t)blockIdx.x * wd * ROWS;
+  for (int i = threadIdx.x; i < wd * ROWS; i += 256) dst[i] = rows[(i % ROWS) * pitch + i / ROWS];
+}
+
+// Tiles 0, stride, 2 stride, ... (ntiles of them; tile i below is the i-th).
+// MODE 0: gmax[q][4 i + g] = -(smallest upper bound of tile i's 32 points of group g).
+// MODE 1: points with a lower bound <= T = -tau[q] appended to cand[q][0..cap) (cnt[q] counts
+// all).  The sums start at 2^23 as a float's bits, so they are read as floats without conversions.
+template <int MODE>
+__global__ void __launch_bounds__(256, 4)
+    jaccard_scan_kernel(const uint32_t* __restrict__ xt, const float4* __restrict__ xtail, int64_t n, int wd, int d,
+                        const uint32_t* __restrict__ qt, const float4* __restrict__ qtail,
+                        const int* __restrict__ qbad, int nq, int ntiles, int tiles_per_split, int stride,
+                        float* __restrict__ gmax, const float* __restrict__ tau, int* __restrict__ cnt,
+                        uint64_t* __restrict__ cand, int cap) {
+  constexpr unsigned kOne = 0x4b000000u;  // 2^23
+  extern __shared__ __align__(16) uint32_t sm[];
+  uint32_t* xs = sm;               // [wd][128]
+  uint32_t* qs = sm + wd * kTile;  // [wd][64]
+  __shared__ float2 xl[kTile], ql[kQB];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int q0 = blockIdx.x * kQB;
+  const int t0 = blockIdx.y * tiles_per_split, t1 = min(ntiles, t0 + tiles_per_split);
+  for (int i = tid; i < wd * kQB / 4; i += 256)
+    reinterpret_cast<uint4*>(qs)[i] = reinterpret_cast<const uint4*>(qt + (int64_t)blockIdx.x * wd * kQB)[i];
+  if (tid < kQB) {
+    const int q = q0 + tid;
+    const float4 v = qtail[q];
+    if (MODE == 0) {
+      ql[tid] = make_float2(v.x, v.y);
+    } else {
+      // 1 - A_hi / (S - A_hi) - delta <= T  <=>  A_hi >= S c / (1 + c), c = 1 - delta - T
+      //                                    <=>  A <= Q - (2 s S) c / (1 + c);
+      // two units for the roundings at 2^23
+      float r = 0.0f, lim = -INFINITY;
+      if (q < nq && !qbad[q]) {
+        const float c = 1.0f - delta(d) + tau[q];
+        r = -c / (1.0f + c);
+        lim = v.z + r * v.x + (8388608.0f + 2.0f);
+        if (!(tau[q] > -2.0f)) { r = 0.0f; lim = INFINITY; }  // no threshold
+      }
+      ql[tid] = make_float2(r, lim);
+    }
+  }
+  for (int t = t0; t < t1; ++t) {
+    __syncthreads();  // the previous tile has been read
+    const int64_t row0 = (int64_t)t * stride * kTile;
+    for (int i = tid; i < wd * kTile / 4; i += 256)
+      reinterpret_cast<uint4*>(xs)[i] = __ldg(reinterpret_cast<const uint4*>(xt + row0 * wd) + i);
+    if (tid < kTile) {
+      const float4 v = __ldg(xtail + row0 + tid);
+      xl[tid] = make_float2(v.x, MODE == 0 ? v.y : v.z);
+    }
+    __syncthreads();
+    if (q0 + 8 * w >= nq) continue;  // no query of this warp: it only copies
+    unsigned acc[8][4];
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) acc[a][b] = kOne;
+#pragma unroll 2
+    for (int j = 0; j < wd; ++j) {
+      const uint4 xv = *reinterpret_cast<const uint4*>(xs + j * kTile + 4 * lane);
+      const uint4 qa = *reinterpret_cast<const uint4*>(qs + j * kQB + 8 * w);
+      const uint4 qb = *reinterpret_cast<const uint4*>(qs + j * kQB + 8 * w + 4);
+      const unsigned xb[4] = {xv.x, xv.y, xv.z, xv.w};
+      const unsigned qv[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+      for (int a = 0; a < 8; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] = sad4(xb[b], qv[a], acc[a][b]);
+    }
+    const int64_t left = n - row0 - 4 * lane;  // points of this thread that exist
+    float2 xv[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) xv[b] = xl[4 * lane + b];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      const float2 qv = ql[8 * w + a];
+      const int q = q0 + 8 * w + a;
+      if (MODE == 0) {
+        float best = 0.0f;  // the largest A_lo / S
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const float A = __uint_as_float(acc[a][b]) - 8388608.0f;
+          const float R = __fdividef(qv.y + xv[b].y - A, qv.x + xv[b].x);
+          if (b < left) best = fmaxf(best, R);
+        }
+        best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, 1));
+        best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, 2));
+        best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, 4));
+        // a group without points bounds nothing
+        if ((lane & 7) == 0 && q < nq)
+          gmax[(int64_t)q * 4 * ntiles + 4 * t + (lane >> 3)] =
+              left > 0 ? __fdividef(best, 1.0f - best) - 1.0f - delta(d) : -INFINITY;
+      } else {
+        unsigned hits = 0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+          if (__uint_as_float(acc[a][b]) <= fmaf(qv.x, xv[b].x, xv[b].y) + qv.y && b < left) hits |= 1u << b;
+        if (hits) {  // q < nq: the limit is -inf beyond
+          int pos = atomicAdd(cnt + q, __popc(hits));
+          // a query past its places is scanned in full: its other points need not be looked for
+          if (pos >= cap) ql[8 * w + a] = make_float2(0.0f, -INFINITY);
+          for (unsigned h = hits; h; h &= h - 1, ++pos)
+            if (pos < cap) cand[(int64_t)q * cap + pos] = make_key(0.0f, (int)(row0 + 4 * lane + __ffs(h) - 1));
+        }
+      }
+    }
+  }
+}
+
+// Queries to scan in full: more candidates than places, fewer than k, or no bounds.  The re-rank has
+// nothing of them to do: their candidates are emptied.
+__global__ void list_hard_kernel(const int* __restrict__ cnt, const int* __restrict__ bad, int nq, int k,
+                                 int cap, uint64_t* __restrict__ cand, int* __restrict__ list) {
+  const int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (q >= nq) return;
+  const int c = cnt[q];
+  const bool hard = bad[q] || c > cap || c < k;
+  for (int i = lane + (hard ? 0 : c); i < cap; i += 32) cand[(int64_t)q * cap + i] = kEmptyKey;
+  if (hard && lane == 0) list[1 + atomicAdd(list, 1)] = q;
+}
+
+size_t tile_smem(int wd, int rows) { return (size_t)rows * (wd | 1) * 4; }
+
+}  // namespace
+
+void derive_jaccard_scan(Index& I, cudaStream_t s) {
+  if (I.p.framework != 0 || I.dist != DIST_JACCARD || I.d < kMinDim || I.d > kMaxDim || I.n < kMinBase) return;
+  float lo, hi;
+  if (!base_range(I.x.ptr, I.n * I.d, &lo, &hi, s)) return;
+  const int wd = ceil_div(I.d, 4), tiles = ceil_div(I.n, kTile);
+  try {
+    I.jq.alloc((size_t)tiles * wd * kTile, s);
+    I.jq_tail.alloc((size_t)tiles * kTile, s);
+  } catch (const Error& e) {  // no room for the codes: the FP32 scan needs none
+    if (e.status != LSHG_ERR_OUT_OF_MEMORY) throw;
+    cudaGetLastError();
+    I.jq.release();
+    return;
+  }
+  I.jq_lo = lo;
+  I.jq_scale = 255.0f / std::max(hi - lo, 1e-6f * hi);
+  const size_t smem = tile_smem(wd, kTile);
+  LSHG_CUDA(cudaFuncSetAttribute(code_tiles_kernel<kTile>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  code_tiles_kernel<kTile><<<tiles, 256, smem, s>>>(I.x.ptr, I.n, I.d, wd, I.jq_lo, I.jq_scale, I.jq.ptr, I.jq_tail.ptr, nullptr);
+  count_launch();
+  LSHG_CHECK_LAUNCH();
+}
+
+bool query_jaccard_filtered(Index& I, const float* q, int nq, int k, lshg_point* out, cudaStream_t s) {
+  const int wd = ceil_div(I.d, 4), tiles = ceil_div(I.n, kTile), qblocks = ceil_div(nq, kQB);
+  if (!I.jq.ptr || k > std::min(128, tiles) || (int64_t)nq * I.n < kMinPairs) return false;
+  const int cap = k <= 64 ? 512 : 1024;  // candidates a query, re-scored
+  // Every S-th tile for the thresholds: the bounds pass about 5 S k candidates (60,013 sparse rows of
+  // 100: 150 at S k = 32, at most 255), within the places, and never fewer than 4 k groups.
+  const int S = std::max(1, std::min({8, cap / 16 / k, tiles / k})), stiles = ceil_div(tiles, S);
+  int C = 32;
+  while (C < k) C <<= 1;
+  const int lsplits = scan_listed_splits(I.n, nq, C);
+  try {
+    DevBuf<uint32_t> qt((size_t)qblocks * wd * kQB, s);
+    DevBuf<float4> qtail((size_t)qblocks * kQB, s);
+    DevBuf<int> ctl((size_t)3 * nq + 1, s);  // [0, nq): candidates; [nq, 2 nq): no bounds; then count and list
+    DevBuf<float> gmax((size_t)nq * 4 * stiles, s), tau((size_t)nq, s);
+    DevBuf<uint64_t> cand((size_t)nq * cap, s), part((size_t)nq * lsplits * C, s);
+    int *cnt = ctl.ptr, *bad = ctl.ptr + nq, *list = ctl.ptr + 2 * nq;
+    LSHG_CUDA(cudaMemsetAsync(ctl.ptr, 0, ctl.bytes(), s));
+    const size_t qsm = tile_smem(wd, kQB);
+    LSHG_CUDA(cudaFuncSetAttribute(code_tiles_kernel<kQB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qsm));
+    code_tiles_kernel<kQB><<<qblocks, 256, qsm, s>>>(q, nq, I.d, wd, I.jq_lo, I.jq_scale, qt.ptr, qtail.ptr, bad);
+    count_launch();
+    LSHG_CHECK_LAUNCH();
+    // two rounds of four CTAs an SM where there are tiles enough, at least two tiles each
+    auto split = [&](int nt) {
+      return ceil_div(nt, std::max(1, std::min(ceil_div(nt, 2), ceil_div(num_sms() * 8, qblocks))));
+    };
+    const int tps0 = split(stiles), tps = split(tiles);
+    const dim3 grid0(qblocks, ceil_div(stiles, tps0)), grid(qblocks, ceil_div(tiles, tps));
+    const size_t smem = (size_t)wd * (kTile + kQB) * 4;
+    LSHG_CUDA(cudaFuncSetAttribute(jaccard_scan_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    LSHG_CUDA(cudaFuncSetAttribute(jaccard_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    {
+      ProfScope _ps("jaccard_bounds", s);
+      jaccard_scan_kernel<0><<<grid0, 256, smem, s>>>(I.jq.ptr, I.jq_tail.ptr, I.n, wd, I.d, qt.ptr, qtail.ptr, bad, nq,
+                                                      stiles, tps0, S, gmax.ptr, nullptr, nullptr, nullptr, 0);
+      count_launch();
+      LSHG_CHECK_LAUNCH();
+    }
+    tc::launch_tau_select(gmax.ptr, nq, 4 * stiles, k, 0.0f, tau.ptr, s);
+    {
+      ProfScope _ps("jaccard_filter", s);
+      jaccard_scan_kernel<1><<<grid, 256, smem, s>>>(I.jq.ptr, I.jq_tail.ptr, I.n, wd, I.d, qt.ptr, qtail.ptr, bad, nq,
+                                                     tiles, tps, 1, nullptr, tau.ptr, cnt, cand.ptr, cap);
+      count_launch();
+      LSHG_CHECK_LAUNCH();
+    }
+    list_hard_kernel<<<ceil_div(nq, 8), 256, 0, s>>>(cnt, bad, nq, (int)std::min<int64_t>(k, I.n), cap, cand.ptr, list);
+    count_launch();
+    LSHG_CHECK_LAUNCH();
+    launch_rerank(cand.ptr, nq, cap, I.x.ptr, I.n, I.d, nullptr, q, nullptr, DIST_JACCARD, k, out, s, I.error_word(s));
+    launch_scan_float_listed(I.xt.ptr, I.n, I.d, nullptr, q, nq, nullptr, DIST_JACCARD, list, C, lsplits, part.ptr, k,
+                             out, s);
+  } catch (const Error& e) {
+    if (e.status != LSHG_ERR_OUT_OF_MEMORY) throw;
+    cudaGetLastError();  // temporaries that do not fit: the FP32 scan needs fewer
+    return false;
+  }
+  return true;
+}
+
+}  // namespace lshg

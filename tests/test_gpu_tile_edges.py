@@ -252,3 +252,48 @@ def test_lsh_bounds_scoring_equals_oracle(engine, orc, n, nq, k, d, hashes, tabl
     res = idx.query(q, k)
     assert np.array_equal(res["ID"], ids)
     assert np.array_equal(res["distance"], ds)
+
+
+@pytest.mark.parametrize("n,nq,k,d", [
+    (4096, 4, 32, 100),     # the smallest base and batch that are filtered, the longest k of it
+    (4097, 65, 1, 16),      # one point in the last tile, one query in the second block; the narrowest rows
+    (8193, 9, 64, 101),     # the longest k of 512 candidates, of as many tiles as k; a padded word
+    (30000, 33, 128, 99),   # the longest k
+    (20001, 129, 10, 128),  # the widest rows
+    (60000, 200, 16, 3),    # d below the filter: the FP32 scan
+    (5000, 40, 40, 100),    # k beyond it at this size
+    (5000, 40, 10, 129),    # d beyond it
+])
+@pytest.mark.parametrize("case", ["plain", "copies", "dense", "offset", "queries", "base"])
+def test_jaccard_filter_equals_fp32_scan(engine, n, nq, k, d, case):
+    """Ids and distances of the filtered exact Jaccard scan are the FP32 scan's bit for bit, also
+    where the bounds leave too many candidates or none apply."""
+    x, q = datasets.sparse_gamma(n, d, 111), datasets.sparse_gamma(nq, d, 112)
+    if case == "copies":
+        x[::2] = x[0]
+        q[::3] = x[0]
+    elif case == "dense":  # every distance near every other
+        rng = np.random.default_rng(7)
+        x, q = rng.random((n, d), dtype=np.float32), rng.random((nq, d), dtype=np.float32)
+    elif case == "offset":  # a narrow range far from zero, queries beyond it on both sides
+        rng = np.random.default_rng(8)
+        x = 7 + 1e-3 * rng.random((n, d), dtype=np.float32)
+        q = 7 + 2e-3 * rng.random((nq, d), dtype=np.float32) - np.float32(5e-4)
+    elif case == "queries":
+        q[0] = 0
+        q[1, 0] = -0.5
+        q[2, d - 1] = np.nan
+        q[3] *= np.float32(1e6)
+    elif case == "base":
+        x[n - 1, 0] = -1.0
+    idx = engine.Index(x, implementation=2, distanceFunc=2)
+    want = idx.query(q, 129)[:, :k]  # k beyond the filter: the FP32 scan
+    assert idx.query(q, k).tobytes() == want.tobytes()
+
+
+def test_jaccard_filter_saved_index(engine, tmp_path):
+    x, q = datasets.sparse_gamma(9000, D, 113), datasets.sparse_gamma(70, D, 114)
+    idx = engine.Index(x, implementation=2, distanceFunc=2)
+    path = str(tmp_path / "jaccard.lshg")
+    idx.save(path)
+    assert engine.Index.load(path).query(q, 32).tobytes() == idx.query(q, 32).tobytes()
