@@ -109,7 +109,8 @@ void run_reference_call(const lshg_index_params& p, int k, int N_query, int N_da
   auto t0 = std::chrono::steady_clock::now();
   DevBuf<float> base = upload_floats(data, (size_t)N_data * p.d, s);
   DevBuf<float> comp = upload_floats(queries, (size_t)N_query * p.d, s);
-  DevBuf<float> q = upload_floats(queries, (size_t)N_query * p.d, s);
+  DevBuf<float> q((size_t)N_query * p.d, s);  // the build transforms comp in place
+  LSHG_CUDA(cudaMemcpyAsync(q.ptr, comp.ptr, q.bytes(), cudaMemcpyDeviceToDevice, s));
   double prep = 0, build = 0;
   auto idx = build_index(p, std::move(base), N_data, comp.ptr, N_query, s, &prep, &build);
   comp.release();

@@ -311,10 +311,14 @@ int* Index::error_word(cudaStream_t s) {
   if (cs != cudaStreamCaptureStatusNone)
     throw Error(LSHG_ERR_INVALID_ARGUMENT,
                 "first query of an index on this stream during a stream capture: run one query on the stream first");
+  // The index's own stream outlives its words: from the stream's pool (a one-shot call spent 150
+  // of its 520 us in cudaMalloc and cudaFree of these four bytes).  Other streams may be gone
+  // when the index is destroyed.
+  const bool own = stream && s == stream;
   int* w = nullptr;
-  LSHG_CUDA(cudaMalloc(&w, sizeof(int)));
+  LSHG_CUDA(own ? cudaMallocAsync(&w, sizeof(int), s) : cudaMalloc(&w, sizeof(int)));
   if (cudaMemsetAsync(w, 0, sizeof(int), s) != cudaSuccess) {
-    cudaFree(w);
+    own ? cudaFreeAsync(w, s) : cudaFree(w);
     LSHG_CUDA(cudaGetLastError());
   }
   err_words.emplace(s, w);
@@ -332,7 +336,9 @@ void derive_simhash(Index& I, cudaStream_t s) {
 
 Index::~Index() {
   if (stream) cudaStreamSynchronize(stream);
-  for (auto& kv : err_words) cudaFree(kv.second);  // cudaFree waits for work that may still write it
+  for (auto& kv : err_words)
+    if (stream && kv.first == stream) cudaFreeAsync(kv.second, stream);
+    else cudaFree(kv.second);  // waits for work that may still write it
   x.release(); xnorm.release(); xt.release(); xs.release(); xse.release(); xsl.release(); xsf.release(); xsft.release();
   sk_planes.release(); sk_split.release(); sk_pnorm.release();
   keys.release(); offsets.release(); buckets.release(); key_planes.release(); cp_diag.release(); bitmaps.release();
