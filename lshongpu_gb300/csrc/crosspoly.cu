@@ -17,6 +17,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 
 namespace lshg {
 
@@ -42,6 +43,7 @@ __global__ void __launch_bounds__(256, W == 32 ? 3 : 1) crosspoly_kernel(const f
                                                         int tables, int hashes, int rounds,
                                                         const int* __restrict__ diag, uint16_t* __restrict__ keys,
                                                         bool vec) {
+  grid_ready();
   constexpr int R = W < 4 ? W : 4;  // values a chunk
   constexpr int NC = W / R;         // chunks a lane
   const int lane = threadIdx.x & 31;
@@ -165,7 +167,7 @@ void launch_crosspoly(const float* x, int64_t n, int d, int P, int tables, int h
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((warps * 32 + 255) / 256, (int64_t)num_sms() * 16));
   switch (W) {
 #define LSHG_CP(WV) \
-  case WV: crosspoly_kernel<WV><<<blocks, 256, 0, s>>>(x, n, d, P, tables, hashes, rounds, diag, keys, vec); break;
+  case WV: launch_next(crosspoly_kernel<WV>, blocks, 256, 0, s, x, n, d, P, tables, hashes, rounds, diag, keys, vec); break;
     LSHG_CP(1) LSHG_CP(2) LSHG_CP(4) LSHG_CP(8) LSHG_CP(16) LSHG_CP(32)
 #undef LSHG_CP
     default: throw Error(LSHG_ERR_INVALID_ARGUMENT, "cross-polytope: unsupported P");

@@ -37,6 +37,7 @@
 #include "profile.h"
 #include "select.cuh"
 #include "slice_filter.cuh"
+#include "launch_next.cuh"
 
 namespace lshg {
 
@@ -80,6 +81,7 @@ __device__ __forceinline__ float cws_logf(float x) {
 // dimension's draws for 32 consecutive samples one contiguous 512-byte read.
 __global__ void __launch_bounds__(256) cws_sketch_kernel(const float* __restrict__ x, int64_t rows, int d, int S,
                                                          const float4* __restrict__ tab, int2* __restrict__ out) {
+  grid_ready();
   extern __shared__ float lns[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* L = lns + (size_t)warp * d;
@@ -185,6 +187,7 @@ __global__ void __launch_bounds__(256) cws_dict_rank_kernel(const uint32_t* __re
 template <int PL>
 __global__ void cws_slice_kernel(const int2* __restrict__ smp, int64_t rows, int S, int ng, int d, int tmin, int tb,
                                  const uint8_t* __restrict__ rank, int rlog, uint32_t pad, uint32_t* __restrict__ out) {
+  grid_ready();
   const int64_t total = rows * ng;
   const uint32_t tspan = 1u << tb, sentinel = (uint32_t)(d + 1) << tb;
   for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (int64_t)gridDim.x * blockDim.x) {
@@ -226,6 +229,7 @@ __device__ __forceinline__ uint64_t key_mix(uint64_t z) {
 }
 __global__ void cws_keys_kernel(const int2* __restrict__ smp, int64_t rows, int L, int K, int bits,
                                 uint16_t* __restrict__ keys) {
+  grid_ready();
   const int64_t total = rows * L;
   for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = w / L;
@@ -272,6 +276,7 @@ template <int KBUF, int T>
 __global__ void __launch_bounds__(256, 2)
     cws_direct_kernel(const uint4* __restrict__ xst, int64_t n, int S, const int2* __restrict__ qs, int nq, int C,
                       int tiles_per_split, int splits, uint64_t* __restrict__ out, const int* __restrict__ list) {
+  grid_ready();
   constexpr int QB = 2;
   static_assert(KBUF >= T * kTile, "append buffer must absorb T tiles");
   constexpr int kLimit = KBUF - T * kTile;
@@ -345,7 +350,7 @@ void launch_direct_cfg(const uint32_t* xst, int64_t n, int S, const uint32_t* qs
   const int ntiles = ceil_div(n, kTile);
   const int tps = ceil_div(ntiles, splits);
   dim3 grid(ceil_div(nq, 2), splits);
-  kern<<<grid, 256, smem, s>>>(reinterpret_cast<const uint4*>(xst), n, S, reinterpret_cast<const int2*>(qs), nq, C,
+  launch_next(kern, grid, 256, smem, s, reinterpret_cast<const uint4*>(xst), n, S, reinterpret_cast<const int2*>(qs), nq, C,
                                tps, splits, out, list);
   count_launch();
   LSHG_CHECK_LAUNCH();
@@ -396,7 +401,7 @@ void launch_cws_keys(const uint32_t* smp, int64_t rows, int L, int K, int bits, 
   if (total <= 0) return;
   LSHG_REQUIRE(bits >= 1 && bits <= 16 && K >= 1, "CWS keys: bucketKeyBits in [1, 16], K >= 1");
   const int blocks = (int)std::min<int64_t>((total + 255) / 256, (int64_t)num_sms() * 16);
-  cws_keys_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<const int2*>(smp), rows, L, K, bits, keys);
+  launch_next(cws_keys_kernel, blocks, 256, 0, s, reinterpret_cast<const int2*>(smp), rows, L, K, bits, keys);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -407,7 +412,7 @@ void launch_cws_sketch(const float* x, int64_t rows, int d, int S, const float* 
   const size_t smem = (size_t)8 * d * sizeof(float);
   LSHG_CUDA(cudaFuncSetAttribute(cws_sketch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int blocks = (int)std::min<int64_t>((rows + 7) / 8, (int64_t)num_sms() * 8);
-  cws_sketch_kernel<<<blocks, 256, smem, s>>>(x, rows, d, S, reinterpret_cast<const float4*>(tab),
+  launch_next(cws_sketch_kernel, blocks, 256, smem, s, x, rows, d, S, reinterpret_cast<const float4*>(tab),
                                               reinterpret_cast<int2*>(out));
   count_launch();
   LSHG_CHECK_LAUNCH();
@@ -481,10 +486,10 @@ void launch_cws_slice(const uint32_t* smp, int64_t rows, int S, int d, const Cws
   const int blocks = (int)std::min<int64_t>((total + 255) / 256, (int64_t)num_sms() * 16);
   const int2* v = reinterpret_cast<const int2*>(smp);
   if (c.pl == 8)
-    cws_slice_kernel<8><<<blocks, 256, 0, s>>>(v, rows, S, ng, d, c.tmin, c.tb, c.rank, c.rlog, query ? 0xFFu : 0u,
+    launch_next(cws_slice_kernel<8>, blocks, 256, 0, s, v, rows, S, ng, d, c.tmin, c.tb, c.rank, c.rlog, query ? 0xFFu : 0u,
                                                out);
   else
-    cws_slice_kernel<16><<<blocks, 256, 0, s>>>(v, rows, S, ng, d, c.tmin, c.tb, nullptr, 0, query ? 0xFFFFu : 0u,
+    launch_next(cws_slice_kernel<16>, blocks, 256, 0, s, v, rows, S, ng, d, c.tmin, c.tb, nullptr, 0, query ? 0xFFFFu : 0u,
                                                 out);
   count_launch();
   LSHG_CHECK_LAUNCH();

@@ -21,6 +21,7 @@
 #include "distance.cuh"
 #include "kernels.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 #include "profile.h"
 #include "select.cuh"
 #include "tc_ptx.cuh"
@@ -191,6 +192,7 @@ __device__ __forceinline__ int entry_table(const int* pref, int tables, int idx)
 // order does not matter: keys (distance, id) are unique, so the kept set is the same.
 template <int DIST>
 __global__ void __launch_bounds__(kQThreads, kQueryCtasPerSm) lsh_query_kernel(LshQueryArgs a, lshg_point* __restrict__ out) {
+  grid_ready();
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int NW = kQThreads / 32;
   const uint32_t stage_slot = stage_slot_bytes(a.d);
@@ -436,6 +438,7 @@ __device__ __forceinline__ void seen_clear(int* seen, int tid) {
 __global__ void __launch_bounds__(kQThreads, kWalkCtasPerSm)
     lsh_walk_kernel(LshQueryArgs a, int* __restrict__ cand, int cap, int* __restrict__ ccnt, int* __restrict__ ovf,
                     int* __restrict__ qctr) {
+  grid_ready();
   extern __shared__ __align__(16) int seen[];  // kWalkSlots ids
   __shared__ int bstart[kMaxTables], pref[kMaxTables + 1];
   __shared__ int wcnt, qcur;
@@ -520,6 +523,7 @@ template <int DIST>
 __global__ void __launch_bounds__(kQThreads, kScoreCtasPerSm)
     lsh_score_kernel(LshQueryArgs a, const int* __restrict__ cand, int cap, const int* __restrict__ ccnt,
                      lshg_point* __restrict__ out, int* __restrict__ qctr, const int* __restrict__ only) {
+  grid_ready();
   extern __shared__ __align__(128) unsigned char smem[];
   const int todo = only ? only[0] : a.nq;
   if (todo == 0) return;
@@ -662,7 +666,7 @@ static void launch_split(const LshQueryArgs& a, int cap, size_t fused_smem, lshg
   DevBuf<int> cand((size_t)a.nq * cap, s), ccnt((size_t)a.nq, s), ctl((size_t)a.nq + 4, s);
   LSHG_CUDA(cudaMemsetAsync(ctl.ptr, 0, 4 * sizeof(int), s));
   int* ovf = ctl.ptr + 3;
-  lsh_walk_kernel<<<a.walk_grid, kQThreads, kWalkSlots * 4, s>>>(a, cand.ptr, cap, ccnt.ptr, ovf, ctl.ptr);
+  launch_next(lsh_walk_kernel, a.walk_grid, kQThreads, kWalkSlots * 4, s, a, cand.ptr, cap, ccnt.ptr, ovf, ctl.ptr);
   count_launch();
   LSHG_CHECK_LAUNCH();
   const size_t ssmem = lsh_stage_bytes(a.d) + (size_t)(a.C + kQBuf) * 8 + (size_t)((a.d + 3) & ~3) * 4 + 16;
@@ -688,7 +692,7 @@ static void launch_split(const LshQueryArgs& a, int cap, size_t fused_smem, lshg
     launch_rerank(kept.ptr, a.nq, kBoundsKeep, a.x, a.n, a.d, a.xnorm, a.q, a.qnorm, DIST_ANGULAR, a.k, out, s, a.err);
     only = hard.ptr;
   }
-  lsh_score_kernel<DV><<<sgrid, kQThreads, ssmem, s>>>(a, cand.ptr, cap, ccnt.ptr, out, ctl.ptr + 1, only);
+  launch_next(lsh_score_kernel<DV>, sgrid, kQThreads, ssmem, s, a, cand.ptr, cap, ccnt.ptr, out, ctl.ptr + 1, only);
   count_launch();
   LSHG_CHECK_LAUNCH();
   LshQueryArgs f = a;  // queries with more than cap distinct candidates: the fused kernel
@@ -698,7 +702,7 @@ static void launch_split(const LshQueryArgs& a, int cap, size_t fused_smem, lshg
   DevBuf<int> lists((size_t)a.grid * kListCap, s);
   f.lists = lists.ptr;
   LSHG_CUDA(cudaFuncSetAttribute(lsh_query_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem));
-  lsh_query_kernel<DV><<<a.grid, kQThreads, fused_smem, s>>>(f, out);
+  launch_next(lsh_query_kernel<DV>, a.grid, kQThreads, fused_smem, s, f, out);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -730,7 +734,7 @@ void launch_lsh_query(const LshQueryArgs& a, lshg_point* out, cudaStream_t s) {
 #define LSHG_LQ(DV)                                                                                        \
   do {                                                                                                     \
     LSHG_CUDA(cudaFuncSetAttribute(lsh_query_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    lsh_query_kernel<DV><<<a.grid, kQThreads, smem, s>>>(f, out);                                          \
+    launch_next(lsh_query_kernel<DV>, a.grid, kQThreads, smem, s, f, out);                                          \
   } while (0)
   switch (a.dist) {
     case DIST_ANGULAR: LSHG_LQ(DIST_ANGULAR); break;

@@ -11,6 +11,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 
 namespace lshg {
 
@@ -28,6 +29,7 @@ constexpr int kNormRows = kRowsPerBlock / (kNormThreads / 32);  // rows a warp s
 template <bool kNormalize>
 __global__ void __launch_bounds__(kNormThreads) row_norm_kernel(float* __restrict__ x, int64_t n, int d,
                                                                 float* __restrict__ norms) {
+  grid_ready();
   extern __shared__ float sm[];
   const int pitch = d | 1;
   const int64_t row0 = (int64_t)blockIdx.x * kRowsPerBlock;
@@ -99,6 +101,7 @@ __global__ void min_floor_kernel(const float* __restrict__ x, int64_t n, int d, 
 
 // x += abs(minv[dim]) (processingUtils.cuh:33-45): float + (float)int.
 __global__ void shift_abs_kernel(float* __restrict__ x, int64_t n, int d, const int* __restrict__ minv) {
+  grid_ready();
   int64_t total = n * d;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     int j = (int)(i % d);
@@ -130,6 +133,7 @@ __global__ void u32_to_u8_kernel(const uint32_t* in, int64_t n, uint8_t* out) {
 }
 
 __global__ void pad_words_kernel(const uint32_t* in, int64_t n, int words, uint32_t* out, int wp, uint32_t pad) {
+  grid_ready();
   int64_t total = n * wp;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     int64_t r = i / wp;
@@ -201,7 +205,7 @@ void launch_row_norms(const float* x, int64_t n, int d, float* norms, cudaStream
   size_t smem = staged_smem(kRowsPerBlock, d);
   LSHG_REQUIRE(smem <= 200 * 1024, "dimension too large for row_norms");
   LSHG_CUDA(cudaFuncSetAttribute(row_norm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  row_norm_kernel<false><<<ceil_div(n, kRowsPerBlock), kNormThreads, smem, s>>>(const_cast<float*>(x), n, d, norms);
+  launch_next(row_norm_kernel<false>, ceil_div(n, kRowsPerBlock), kNormThreads, smem, s, const_cast<float*>(x), n, d, norms);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -211,7 +215,7 @@ void launch_normalize(float* x, int64_t n, int d, cudaStream_t s) {
   size_t smem = staged_smem(kRowsPerBlock, d);
   LSHG_REQUIRE(smem <= 200 * 1024, "dimension too large for normalize");
   LSHG_CUDA(cudaFuncSetAttribute(row_norm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  row_norm_kernel<true><<<ceil_div(n, kRowsPerBlock), kNormThreads, smem, s>>>(x, n, d, nullptr);
+  launch_next(row_norm_kernel<true>, ceil_div(n, kRowsPerBlock), kNormThreads, smem, s, x, n, d, nullptr);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -236,7 +240,7 @@ void launch_min_floor(const float* x, int64_t n, int d, int* minv, cudaStream_t 
 
 void launch_shift_abs(float* x, int64_t n, int d, const int* minv, cudaStream_t s) {
   if (n <= 0) return;
-  shift_abs_kernel<<<grid_for(n * d, 256), 256, 0, s>>>(x, n, d, minv);
+  launch_next(shift_abs_kernel, grid_for(n * d, 256), 256, 0, s, x, n, d, minv);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -273,7 +277,7 @@ void launch_u32_to_u8(const uint32_t* in, int64_t n, uint8_t* out, cudaStream_t 
 void launch_pad_words(const uint32_t* in, int64_t n, int words, uint32_t* out, int wp, uint32_t pad,
                       cudaStream_t s) {
   if (n <= 0) return;
-  pad_words_kernel<<<grid_for(n * wp, 256), 256, 0, s>>>(in, n, words, out, wp, pad);
+  launch_next(pad_words_kernel, grid_for(n * wp, 256), 256, 0, s, in, n, words, out, wp, pad);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 #include "profile.h"
 
 namespace lshg {
@@ -24,6 +25,7 @@ __global__ void __launch_bounds__(256) project_kernel(const float* __restrict__ 
                                                       int mode, int bits, int words,
                                                       uint32_t* __restrict__ out32, float* __restrict__ outf,
                                                       const int* __restrict__ gate) {
+  grid_ready();
   if (gate && *gate == 0) return;  // block-uniform
   extern __shared__ __align__(16) float sm[];
   float* xs = sm;                 // [d][kPitch]
@@ -118,7 +120,7 @@ void launch_project(const float* x, int64_t n, int d, const float* planes, int n
   ProfScope _ps(mode == 1 ? "project_jl" : "project_simhash", s);
   LSHG_CUDA(cudaFuncSetAttribute(project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid(ceil_div(n, kTP), ceil_div(nplanes, kTL));
-  project_kernel<<<grid, 256, smem, s>>>(x, n, d, planes, nplanes, mode, bits, words, out32, out_f, nullptr);
+  launch_next(project_kernel, grid, 256, smem, s, x, n, d, planes, nplanes, mode, bits, words, out32, out_f, nullptr);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -130,7 +132,7 @@ void launch_project_gated(const float* x, int64_t n, int d, const float* planes,
   LSHG_REQUIRE(smem <= 220 * 1024 && nplanes == 32 * words, "bad projection shape");
   LSHG_CUDA(cudaFuncSetAttribute(project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid(ceil_div(n, kTP), ceil_div(nplanes, kTL));
-  project_kernel<<<grid, 256, smem, s>>>(x, n, d, planes, nplanes, 0, 32, words, out32, nullptr, gate);
+  launch_next(project_kernel, grid, 256, smem, s, x, n, d, planes, nplanes, 0, 32, words, out32, nullptr, gate);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 #include "select.cuh"
 #include "distance.cuh"
 #include "profile.h"
@@ -147,6 +148,7 @@ __device__ __forceinline__ float query_norm(const float* row, int d) {
 // One block per query: fold S sorted lists of C keys into one.
 __global__ void merge_splits_kernel(const uint64_t* __restrict__ in, int nq, int splits, int C,
                                     uint64_t* __restrict__ out) {
+  grid_ready();
   extern __shared__ uint64_t ms[];
   const int q = blockIdx.x;
   const uint64_t* src = in + (int64_t)q * splits * C;
@@ -172,6 +174,7 @@ __global__ void merge_splits_kernel(const uint64_t* __restrict__ in, int nq, int
 template <int E>
 __global__ void __launch_bounds__(256) merge_short_kernel(const uint64_t* __restrict__ in, int splits, int k,
                                                            uint64_t* __restrict__ out, lshg_point* __restrict__ pts) {
+  grid_ready();
   constexpr int C = 32 * E;
   __shared__ uint64_t lists[8][C];
   const int q = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
@@ -232,6 +235,7 @@ __global__ void rerank_kernel(const uint64_t* __restrict__ cand, int nq, int C, 
                               const float* qnorm, float* qnorm_out, int k, lshg_point* __restrict__ out,
                               float band_abs, float band_rel, const double* __restrict__ xn64,
                               const RerankBounds* __restrict__ kx) {
+  grid_ready();
   extern __shared__ __align__(16) unsigned char rsm[];
   uint64_t* keys = reinterpret_cast<uint64_t*>(rsm);
   float* qr = reinterpret_cast<float*>(rsm + (size_t)C * 8);
@@ -285,6 +289,7 @@ __global__ void rerank_staged_kernel(const uint64_t* __restrict__ cand, int nq, 
                                      const float* qnorm, float* qnorm_out, int k, lshg_point* __restrict__ out,
                                      int* err, float band_abs, float band_rel, const double* __restrict__ xn64, int test_stall,
                                      const RerankBounds* __restrict__ kx) {
+  grid_ready();
   extern __shared__ __align__(128) unsigned char rsm[];
   const int CH = blockDim.x;
   const uint32_t slot = stage_slot_bytes(d), rowb = (uint32_t)d * 4u;
@@ -405,6 +410,7 @@ __global__ void rerank_staged_kernel(const uint64_t* __restrict__ cand, int nq, 
 constexpr int kPartPer = 8;  // keys a thread; C <= 512 * kPartPer
 __global__ void __launch_bounds__(512) cand_partition_kernel(const uint64_t* __restrict__ cand, int C, int64_t n,
                                                              uint64_t* __restrict__ out) {
+  grid_ready();
   __shared__ int cnt[4096 / 128 + 1];
   const int B = C / 128, qi = blockIdx.x;
   for (int b = threadIdx.x; b <= B; b += blockDim.x) cnt[b] = 0;
@@ -449,6 +455,7 @@ template <int DIST>
 __global__ void rerank_gather_kernel(const uint64_t* cand, int C, const float* __restrict__ x, int64_t n,
                                      int d, const float* __restrict__ xnorm, const float* __restrict__ q,
                                      const float* __restrict__ qnorm, uint64_t* keys_out, int* err) {
+  grid_ready();
   extern __shared__ __align__(128) unsigned char rsm[];
   const int CH = blockDim.x;
   const uint32_t slot = stage_slot_bytes(d), rowb = (uint32_t)d * 4u;
@@ -508,6 +515,7 @@ template <int DIST>
 __global__ void rerank_select_kernel(const uint64_t* __restrict__ keys_in, int C, const float* __restrict__ x, int d,
                                      const float* __restrict__ q, int k, lshg_point* __restrict__ out, float band_abs,
                                      float band_rel, const double* __restrict__ xn64, const RerankBounds* __restrict__ kx) {
+  grid_ready();
   extern __shared__ __align__(16) unsigned char rsm[];
   uint64_t* keys = reinterpret_cast<uint64_t*>(rsm);
   float* qr = reinterpret_cast<float*>(rsm + (size_t)C * 8);
@@ -545,6 +553,7 @@ __global__ void __launch_bounds__(512) rerank_top_kernel(const uint64_t* __restr
                                                          lshg_point* __restrict__ out, float band_abs, float band_rel,
                                                          const double* __restrict__ xn64,
                                                          const RerankBounds* __restrict__ kx) {
+  grid_ready();
   constexpr int P = 128, EP = P / 32;
   __shared__ uint64_t lists[16][P];
   extern __shared__ __align__(16) unsigned char rsm[];
@@ -604,6 +613,7 @@ __global__ void __launch_bounds__(512) rerank_listed_kernel(const uint64_t* __re
                                                             const float* __restrict__ qnorm,
                                                             const int* __restrict__ listed, int k,
                                                             lshg_point* __restrict__ out) {
+  grid_ready();
   extern __shared__ __align__(16) unsigned char rsm[];
   uint64_t* keys = reinterpret_cast<uint64_t*>(rsm);
   float* qr = reinterpret_cast<float*>(rsm + (size_t)C * 8);
@@ -637,6 +647,7 @@ __global__ void __launch_bounds__(512) rerank_listed_kernel(const uint64_t* __re
 
 __global__ void keys_to_points_kernel(const uint64_t* __restrict__ keys, int nq, int C, int k,
                                       lshg_point* __restrict__ out) {
+  grid_ready();
   int64_t total = (int64_t)nq * k;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     int64_t qi = t / k;
@@ -655,9 +666,9 @@ namespace {
 void merge_short(const uint64_t* in, int nq, int splits, int C, int k, uint64_t* out, lshg_point* pts, cudaStream_t s) {
   int W = 1;  // warps: a power of two, no more than lists
   while (W < 8 && 2 * W <= splits) W <<= 1;
-  if (C == 32) merge_short_kernel<1><<<nq, 32 * W, 0, s>>>(in, splits, k, out, pts);
-  else if (C == 64) merge_short_kernel<2><<<nq, 32 * W, 0, s>>>(in, splits, k, out, pts);
-  else merge_short_kernel<4><<<nq, 32 * W, 0, s>>>(in, splits, k, out, pts);
+  if (C == 32) launch_next(merge_short_kernel<1>, nq, 32 * W, 0, s, in, splits, k, out, pts);
+  else if (C == 64) launch_next(merge_short_kernel<2>, nq, 32 * W, 0, s, in, splits, k, out, pts);
+  else launch_next(merge_short_kernel<4>, nq, 32 * W, 0, s, in, splits, k, out, pts);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -672,7 +683,7 @@ void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t
   }
   size_t smem = (size_t)C * 8;
   LSHG_CUDA(cudaFuncSetAttribute(merge_splits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  merge_splits_kernel<<<nq, 128, smem, s>>>(in, nq, splits, C, out);
+  launch_next(merge_splits_kernel, nq, 128, smem, s, in, nq, splits, C, out);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -726,7 +737,7 @@ void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t 
     // reads them in place)
     const uint64_t* gin = cand;
     if (C <= 512 * kPartPer && (uint64_t)n * (uint64_t)d * 4u > kPartitionBytes) {
-      cand_partition_kernel<<<nq, 512, 0, s>>>(cand, C, n, gk.ptr);
+      launch_next(cand_partition_kernel, nq, 512, 0, s, cand, C, n, gk.ptr);
       count_launch();
       LSHG_CHECK_LAUNCH();
       gin = gk.ptr;
@@ -735,23 +746,23 @@ void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t 
   do {                                                                                                          \
     LSHG_CUDA(cudaFuncSetAttribute(rerank_gather_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
                                    (int)gather_smem));                                                          \
-    rerank_gather_kernel<DV><<<dim3(nq, C / 128), 128, gather_smem, s>>>(gin, C, x, n, d, xnorm, q, qnorm,      \
+    launch_next(rerank_gather_kernel<DV>, dim3(nq, C / 128), 128, gather_smem, s, gin, C, x, n, d, xnorm, q, qnorm,      \
                                                                          gk.ptr, err);                          \
     count_launch();                                                                                             \
     LSHG_CHECK_LAUNCH();                                                                                        \
     if (k <= 128 && C == 4096)                                                                                  \
-      rerank_top_kernel<DV, 8><<<nq, 512, (size_t)d * 4, s>>>(gk.ptr, C, x, d, q, k, out, band_abs, band_rel,   \
+      launch_next(rerank_top_kernel<DV, 8>, nq, 512, (size_t)d * 4, s, gk.ptr, C, x, d, q, k, out, band_abs, band_rel,   \
                                                               xn64, kb);                                        \
     else if (k <= 128 && C == 2048)                                                                             \
-      rerank_top_kernel<DV, 4><<<nq, 512, (size_t)d * 4, s>>>(gk.ptr, C, x, d, q, k, out, band_abs, band_rel,   \
+      launch_next(rerank_top_kernel<DV, 4>, nq, 512, (size_t)d * 4, s, gk.ptr, C, x, d, q, k, out, band_abs, band_rel,   \
                                                               xn64, kb);                                        \
     else if (k <= 128 && C == 1024)                                                                             \
-      rerank_top_kernel<DV, 2><<<nq, 512, (size_t)d * 4, s>>>(gk.ptr, C, x, d, q, k, out, band_abs, band_rel,   \
+      launch_next(rerank_top_kernel<DV, 2>, nq, 512, (size_t)d * 4, s, gk.ptr, C, x, d, q, k, out, band_abs, band_rel,   \
                                                               xn64, kb);                                        \
     else {                                                                                                      \
       LSHG_CUDA(cudaFuncSetAttribute(rerank_select_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
                                      (int)select_smem));                                                        \
-      rerank_select_kernel<DV><<<nq, 512, select_smem, s>>>(gk.ptr, C, x, d, q, k, out, band_abs, band_rel,     \
+      launch_next(rerank_select_kernel<DV>, nq, 512, select_smem, s, gk.ptr, C, x, d, q, k, out, band_abs, band_rel,     \
                                                             xn64, kb);                                          \
     }                                                                                                           \
   } while (0)
@@ -772,7 +783,7 @@ void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t 
   do {                                                                                                         \
     LSHG_CUDA(cudaFuncSetAttribute(rerank_staged_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
                                    (int)staged_smem));                                                         \
-    rerank_staged_kernel<DV><<<nq, CH, staged_smem, s>>>(cand, nq, C, x, n, d, xnorm, q, qnorm, qnorm_out, k,  \
+    launch_next(rerank_staged_kernel<DV>, nq, CH, staged_smem, s, cand, nq, C, x, n, d, xnorm, q, qnorm, qnorm_out, k,  \
                                                          out, err, band_abs, band_rel, xn64, test_stall, kb); \
   } while (0)
     switch (dist) {
@@ -793,7 +804,7 @@ void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t 
 #define LSHG_RR(DV)                                                                                       \
   do {                                                                                                    \
     LSHG_CUDA(cudaFuncSetAttribute(rerank_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    rerank_kernel<DV><<<nq, threads, smem, s>>>(cand, nq, C, x, n, d, xnorm, q, qnorm, qnorm_out, k, out,      \
+    launch_next(rerank_kernel<DV>, nq, threads, smem, s, cand, nq, C, x, n, d, xnorm, q, qnorm, qnorm_out, k, out,      \
                                                 band_abs, band_rel, xn64, kb);                            \
   } while (0)
   switch (dist) {
@@ -846,7 +857,7 @@ void launch_keys_to_points(const uint64_t* keys, int nq, int C, int k, lshg_poin
   ProfScope _ps("keys_to_points", s);
   int64_t total = (int64_t)nq * k;
   int blocks = (int)std::min<int64_t>((total + 255) / 256, (int64_t)num_sms() * 8);
-  keys_to_points_kernel<<<blocks, 256, 0, s>>>(keys, nq, C, k, out);
+  launch_next(keys_to_points_kernel, blocks, 256, 0, s, keys, nq, C, k, out);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

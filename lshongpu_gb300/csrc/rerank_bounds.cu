@@ -38,6 +38,7 @@
 #include "index.h"
 #include "kernels.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 #include "profile.h"
 
 namespace lshg {
@@ -193,6 +194,7 @@ __global__ void __launch_bounds__(kBoundThreads, 5) bounds_kernel(
     const uint64_t* __restrict__ cand, const int* __restrict__ list, int list_cap, const int* __restrict__ ccnt,
     const uint8_t* __restrict__ rows, const float2* __restrict__ tails, int pitch, float s, int64_t n, int d,
     const float* __restrict__ q, int k, uint64_t* __restrict__ kept, int* __restrict__ listed) {
+  grid_ready();
   constexpr bool JAC = DIST == DIST_JACCARD;
   constexpr int W = kBoundThreads / 32, PER = C / kBoundThreads;
   extern __shared__ uint32_t bnd[];  // [C] lower bound << 16 | upper bound, in steps of kStep from kBase
@@ -422,7 +424,7 @@ void launch_bounds(const uint64_t* cand, const int* list, int list_cap, const in
   constexpr int smem = C * (int)sizeof(uint32_t);
   auto kern = bounds_kernel<DIST, C, LIST>;
   LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  kern<<<nq, kBoundThreads, smem, s>>>(cand, list, list_cap, ccnt, rows, tails, pitch, scale, n, d, q, k, kept, listed);
+  launch_next(kern, nq, kBoundThreads, smem, s, cand, list, list_cap, ccnt, rows, tails, pitch, scale, n, d, q, k, kept, listed);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 #include "profile.h"
 #include "select.cuh"
 
@@ -73,6 +74,7 @@ __global__ void __launch_bounds__(256, MINB) scan_bits_kernel(const uint32_t* __
                                                         int sbytes, const uint32_t* __restrict__ qs, int nq, int C,
                                                         int tiles_per_split, int splits, uint64_t* __restrict__ out,
                                                         const int* __restrict__ list) {
+  grid_ready();
   static_assert(KBUF >= T * kTile, "append buffer must absorb T tiles");
   constexpr int kLimit = KBUF - T * kTile;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -183,7 +185,7 @@ void launch_cfg(const uint32_t* xs, int64_t n, int wp, int words, int sbytes, co
   int ntiles = ceil_div(n, kTile);
   int tps = ceil_div(ntiles, splits);
   dim3 grid(ceil_div(nq, QB), splits);
-  kern<<<grid, 256, smem, s>>>(xs, n, wp, words, sbytes, qs, nq, C, tps, splits, out, list);
+  launch_next(kern, grid, 256, smem, s, xs, n, wp, words, sbytes, qs, nq, C, tps, splits, out, list);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

@@ -29,6 +29,7 @@
 
 #include "index.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 #include "profile.h"
 #include "tc_filter.h"
 #include "tc_ptx.cuh"
@@ -48,6 +49,7 @@ constexpr float kScoreSlack = 8e-5f;
 __global__ void unit_rows_kernel(const float* __restrict__ x, int64_t n, int d, int64_t rows_pad,
                                  __nv_bfloat16* __restrict__ out, unsigned* stat, const float* base_res,
                                  float* __restrict__ eps) {
+  grid_ready();
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -95,7 +97,7 @@ __global__ void unit_rows_kernel(const float* __restrict__ x, int64_t n, int d, 
 void launch_unit_rows(const float* x, int64_t n, int d, int64_t rows_pad, uint16_t* out, unsigned* stat,
                       const float* base_res, float* eps, cudaStream_t s) {
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((rows_pad * 32 + 255) / 256, (int64_t)num_sms() * 8));
-  unit_rows_kernel<<<blocks, 256, 0, s>>>(x, n, d, rows_pad, reinterpret_cast<__nv_bfloat16*>(out), stat, base_res,
+  launch_next(unit_rows_kernel, blocks, 256, 0, s, x, n, d, rows_pad, reinterpret_cast<__nv_bfloat16*>(out), stat, base_res,
                                           eps);
   count_launch();
   LSHG_CHECK_LAUNCH();

@@ -23,6 +23,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 #include "profile.h"
 #include "slice_filter.cuh"
 
@@ -40,6 +41,7 @@ using sf::kMaxBins;
 // `pad`) -> bit-sliced rows [rows][8 * groups]: word 8 g + i, bit s = bit i of byte 32 g + s.
 __global__ void slice_bytes_kernel(const uint32_t* __restrict__ xs, int64_t n, int wp, int groups, int64_t rows,
                                    uint32_t pad, uint32_t* __restrict__ out) {
+  grid_ready();
   const int64_t total = rows * groups * 8;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = t / (groups * 8);
@@ -59,6 +61,7 @@ __global__ void slice_bytes_kernel(const uint32_t* __restrict__ xs, int64_t n, i
 // tau[q] = the match count at which the histogram's count from the top first reaches
 // `rank` (0 -- keep everything -- when the sample holds fewer); one warp a query.
 __global__ void hist_tau_kernel(const int* __restrict__ hist, int nq, int bins, int rank, int* __restrict__ tau) {
+  grid_ready();
   const int lane = threadIdx.x & 31;
   const int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (q >= nq) return;  // warp-uniform
@@ -103,7 +106,7 @@ void launch_slice_bytes(const uint32_t* xs, int64_t n, int wp, int64_t rows, uin
   const int64_t total = rows * groups * 8;
   if (total <= 0) return;
   const int blocks = (int)std::min<int64_t>((total + 255) / 256, (int64_t)num_sms() * 16);
-  slice_bytes_kernel<<<blocks, 256, 0, s>>>(xs, n, wp, groups, rows, pad, out);
+  launch_next(slice_bytes_kernel, blocks, 256, 0, s, xs, n, wp, groups, rows, pad, out);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -129,7 +132,7 @@ bool byte_filter_plan(int64_t n, int C, int* stride, int* rank, int* cap) {
 
 void launch_hist_tau(const int* hist, int nq, int bins, int rank, int* tau, cudaStream_t s) {
   if (nq <= 0) return;
-  hist_tau_kernel<<<ceil_div(nq, 8), 256, 0, s>>>(hist, nq, bins, rank, tau);
+  launch_next(hist_tau_kernel, ceil_div(nq, 8), 256, 0, s, hist, nq, bins, rank, tau);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

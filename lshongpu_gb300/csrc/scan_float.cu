@@ -18,6 +18,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 #include "profile.h"
 #include "select.cuh"
 
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__((QB / MQ) * 32) scan_float_kernel(
     const float* __restrict__ xt, int64_t n, int d, const float* __restrict__ xnorm, const float* __restrict__ q,
     int nq, const float* __restrict__ qnorm, int C, int tiles_per_split, int splits, int nbuf,
     uint64_t* __restrict__ out) {
+  grid_ready();
   extern __shared__ __align__(16) unsigned char smem[];
   const FloatScanSmem L = float_scan_layout(d, QB, C, nbuf);
   float* xs = reinterpret_cast<float*>(smem + L.xs);
@@ -466,6 +468,7 @@ template <int DIST, int EC>
 __global__ void __launch_bounds__(256, 2) scan_float_reg_kernel(
     const float* __restrict__ xt, int64_t n, int d, const float* __restrict__ xnorm, const float* __restrict__ q,
     int nq, const float* __restrict__ qnorm, int tiles_per_split, int splits, int nbuf, uint64_t* __restrict__ out) {
+  grid_ready();
   scan_reg_block<DIST, EC>(xt, n, d, xnorm, q, nq, qnorm, tiles_per_split, splits, nbuf, out, blockIdx.x * kRegQB,
                            blockIdx.y, nullptr);
 }
@@ -477,6 +480,7 @@ __global__ void __launch_bounds__(256, 2) scan_float_listed_kernel(
     const float* __restrict__ xt, int64_t n, int d, const float* __restrict__ xnorm, const float* __restrict__ q,
     const float* __restrict__ qnorm, const int* __restrict__ list, int tiles_per_split, int splits, int nbuf,
     uint64_t* __restrict__ out) {
+  grid_ready();
   const int nq = list[0];
   const int items = (nq + kRegQB - 1) / kRegQB * splits;
   for (int it = blockIdx.x; it < items; it += gridDim.x) {
@@ -490,6 +494,7 @@ __global__ void __launch_bounds__(256, 2) scan_float_listed_kernel(
 // `out` (one block a query).
 __global__ void listed_points_kernel(const uint64_t* __restrict__ part, const int* __restrict__ list, int splits, int C,
                                      int k, lshg_point* __restrict__ out) {
+  grid_ready();
   extern __shared__ uint64_t ms[];
   const int cnt = list[0];
   for (int i = blockIdx.x; i < cnt; i += gridDim.x) {
@@ -526,7 +531,7 @@ void launch_listed(const float* xt, int64_t n, int d, const float* xnorm, const 
   auto kern = scan_float_listed_kernel<DIST, EC>;
   LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int tps = ceil_div(ceil_div(n, kTile), splits);
-  kern<<<num_sms() * 2, 256, smem, s>>>(xt, n, d, xnorm, q, qnorm, list, tps, splits, nb, part);
+  launch_next(kern, num_sms() * 2, 256, smem, s, xt, n, d, xnorm, q, qnorm, list, tps, splits, nb, part);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -541,7 +546,7 @@ void launch_reg(const float* xt, int64_t n, int d, const float* xnorm, const flo
   const int ntiles = ceil_div(n, kTile);
   const int tps = ceil_div(ntiles, splits);
   dim3 grid(ceil_div(nq, kRegQB), splits);
-  kern<<<grid, 256, smem, s>>>(xt, n, d, xnorm, q, nq, qnorm, tps, splits, nbuf, out);
+  launch_next(kern, grid, 256, smem, s, xt, n, d, xnorm, q, nq, qnorm, tps, splits, nbuf, out);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -589,7 +594,7 @@ void launch_cfg(const float* xt, int64_t n, int d, const float* xnorm, const flo
   int ntiles = ceil_div(n, kTile);
   int tps = ceil_div(ntiles, splits);
   dim3 grid(ceil_div(nq, QB), splits);
-  kern<<<grid, (QB / MQ) * 32, smem, s>>>(xt, n, d, xnorm, q, nq, qnorm, C, tps, splits, nbuf, out);
+  launch_next(kern, grid, (QB / MQ) * 32, smem, s, xt, n, d, xnorm, q, nq, qnorm, C, tps, splits, nbuf, out);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -651,7 +656,7 @@ void launch_scan_float_listed(const float* xt, int64_t n, int d, const float* xn
   else if (C == 128) LSHG_LS(4);
   else throw Error(LSHG_ERR_INVALID_ARGUMENT, "listed scan: C must be 32, 64 or 128");
 #undef LSHG_LS
-  listed_points_kernel<<<std::min(nq, num_sms() * 4), 128, (size_t)C * 8, s>>>(part, list, splits, C, k, out);
+  launch_next(listed_points_kernel, std::min(nq, num_sms() * 4), 128, (size_t)C * 8, s, part, list, splits, C, k, out);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

@@ -25,6 +25,7 @@
 
 #include "index.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 #include "profile.h"
 #include "tc_filter.h"
 
@@ -60,6 +61,7 @@ template <int ROWS>
 __global__ void __launch_bounds__(256) code_tiles_kernel(const float* __restrict__ x, int64_t n, int d, int wd, float lo,
                                                          float s, uint32_t* __restrict__ out, float4* __restrict__ tails,
                                                          int* __restrict__ bad) {
+  grid_ready();
   extern __shared__ uint32_t rows[];  // [ROWS][wd | 1]
   const int pitch = wd | 1, lane = threadIdx.x & 31;
   const int64_t row0 = (int64_t)blockIdx.x * ROWS;
@@ -113,6 +115,7 @@ __global__ void __launch_bounds__(256, 4)
                         const int* __restrict__ qbad, int nq, int ntiles, int tiles_per_split, int stride,
                         float* __restrict__ gmax, const float* __restrict__ tau, int* __restrict__ cnt,
                         uint64_t* __restrict__ cand, int cap) {
+  grid_ready();
   constexpr unsigned kOne = 0x4b000000u;  // 2^23
   extern __shared__ __align__(16) uint32_t sm[];
   uint32_t* xs = sm;               // [wd][128]
@@ -214,6 +217,7 @@ __global__ void __launch_bounds__(256, 4)
 // nothing of them to do: their candidates are emptied.
 __global__ void list_hard_kernel(const int* __restrict__ cnt, const int* __restrict__ bad, int nq, int k,
                                  int cap, uint64_t* __restrict__ cand, int* __restrict__ list) {
+  grid_ready();
   const int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (q >= nq) return;
   const int c = cnt[q];
@@ -244,7 +248,7 @@ void derive_jaccard_scan(Index& I, cudaStream_t s) {
   I.jq_scale = 255.0f / std::max(hi - lo, 1e-6f * hi);
   const size_t smem = tile_smem(wd, kTile);
   LSHG_CUDA(cudaFuncSetAttribute(code_tiles_kernel<kTile>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  code_tiles_kernel<kTile><<<tiles, 256, smem, s>>>(I.x.ptr, I.n, I.d, wd, I.jq_lo, I.jq_scale, I.jq.ptr, I.jq_tail.ptr, nullptr);
+  launch_next(code_tiles_kernel<kTile>, tiles, 256, smem, s, I.x.ptr, I.n, I.d, wd, I.jq_lo, I.jq_scale, I.jq.ptr, I.jq_tail.ptr, nullptr);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -269,7 +273,7 @@ bool query_jaccard_filtered(Index& I, const float* q, int nq, int k, lshg_point*
     LSHG_CUDA(cudaMemsetAsync(ctl.ptr, 0, ctl.bytes(), s));
     const size_t qsm = tile_smem(wd, kQB);
     LSHG_CUDA(cudaFuncSetAttribute(code_tiles_kernel<kQB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qsm));
-    code_tiles_kernel<kQB><<<qblocks, 256, qsm, s>>>(q, nq, I.d, wd, I.jq_lo, I.jq_scale, qt.ptr, qtail.ptr, bad);
+    launch_next(code_tiles_kernel<kQB>, qblocks, 256, qsm, s, q, nq, I.d, wd, I.jq_lo, I.jq_scale, qt.ptr, qtail.ptr, bad);
     count_launch();
     LSHG_CHECK_LAUNCH();
     // two rounds of four CTAs an SM where there are tiles enough, at least two tiles each
@@ -283,7 +287,7 @@ bool query_jaccard_filtered(Index& I, const float* q, int nq, int k, lshg_point*
     LSHG_CUDA(cudaFuncSetAttribute(jaccard_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     {
       ProfScope _ps("jaccard_bounds", s);
-      jaccard_scan_kernel<0><<<grid0, 256, smem, s>>>(I.jq.ptr, I.jq_tail.ptr, I.n, wd, I.d, qt.ptr, qtail.ptr, bad, nq,
+      launch_next(jaccard_scan_kernel<0>, grid0, 256, smem, s, I.jq.ptr, I.jq_tail.ptr, I.n, wd, I.d, qt.ptr, qtail.ptr, bad, nq,
                                                       stiles, tps0, S, gmax.ptr, nullptr, nullptr, nullptr, 0);
       count_launch();
       LSHG_CHECK_LAUNCH();
@@ -291,12 +295,12 @@ bool query_jaccard_filtered(Index& I, const float* q, int nq, int k, lshg_point*
     tc::launch_tau_select(gmax.ptr, nq, 4 * stiles, k, 0.0f, tau.ptr, s);
     {
       ProfScope _ps("jaccard_filter", s);
-      jaccard_scan_kernel<1><<<grid, 256, smem, s>>>(I.jq.ptr, I.jq_tail.ptr, I.n, wd, I.d, qt.ptr, qtail.ptr, bad, nq,
+      launch_next(jaccard_scan_kernel<1>, grid, 256, smem, s, I.jq.ptr, I.jq_tail.ptr, I.n, wd, I.d, qt.ptr, qtail.ptr, bad, nq,
                                                      tiles, tps, 1, nullptr, tau.ptr, cnt, cand.ptr, cap);
       count_launch();
       LSHG_CHECK_LAUNCH();
     }
-    list_hard_kernel<<<ceil_div(nq, 8), 256, 0, s>>>(cnt, bad, nq, (int)std::min<int64_t>(k, I.n), cap, cand.ptr, list);
+    launch_next(list_hard_kernel, ceil_div(nq, 8), 256, 0, s, cnt, bad, nq, (int)std::min<int64_t>(k, I.n), cap, cand.ptr, list);
     count_launch();
     LSHG_CHECK_LAUNCH();
     launch_rerank(cand.ptr, nq, cap, I.x.ptr, I.n, I.d, nullptr, q, nullptr, DIST_JACCARD, k, out, s, I.error_word(s));

@@ -27,6 +27,7 @@
 
 #include "common.cuh"
 #include "launch_count.h"
+#include "launch_next.cuh"
 #include "tc_filter.h"
 #include "tc_ptx.cuh"
 
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(kBThreads, 1)
     sliced_filter_kernel(const uint4* __restrict__ xst, int64_t n, const uint32_t* __restrict__ qsl, int nq, int NP,
                          int tstride, int chunk, const int* __restrict__ tau, int* __restrict__ hist, int bins,
                          int* __restrict__ cnt, uint64_t* __restrict__ cand, int cap, int* __restrict__ err) {
+  grid_ready();
   using LY = Layout<MODE, NG, PL>;
   constexpr int W = LY::W, NCH = W / 4, ST = LY::STAGES;
   constexpr int CPG = PL / 4;                 // chunks a group
@@ -375,7 +377,7 @@ void run_ng(const uint4* xst, int64_t n, const uint32_t* qsl, int nq, int NP, in
   const int chunk = big ? (int)std::max<int64_t>(8, std::min<int64_t>(64, items / (slots * 24))) : 0;
   const int64_t total = chunk ? (int64_t)ceil_div(nq, kBQ) * ceil_div(NP, chunk) : items;  // units or items
   const int grid = (int)std::min<int64_t>(total, slots);
-  kern<<<grid, kBThreads, smem, s>>>(xst, n, qsl, nq, NP, tstride, chunk, tau, hist, bins, cnt, cand, cap, err);
+  launch_next(kern, grid, kBThreads, smem, s, xst, n, qsl, nq, NP, tstride, chunk, tau, hist, bins, cnt, cand, cap, err);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

@@ -48,6 +48,7 @@
 // 42% of a warp's pieces, a survivor.
 #include "index.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 #include "profile.h"
 #include "select.cuh"
 #include "tc_filter.h"
@@ -129,6 +130,7 @@ template <int MODE, int GW, bool F8, int KC, int CL>
 __global__ void __launch_bounds__(F_THREADS, 1)
     tc_filter_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                      const __grid_constant__ CUtensorMap mapBhi, const FilterArgs a) {
+  grid_ready();
   using LY = FLayout<KC, CL>;
   constexpr int SBUF = LY::SBUF, F_STAGES = LY::STAGES, AB = LY::AB;
   static_assert(MODE == MODE_GROUPMAX || GW == 64, "the filter reads whole 64-column pieces");
@@ -438,6 +440,7 @@ __device__ __forceinline__ float lowered_tau(float t, float margin, const float*
 __global__ void __launch_bounds__(256) tau_select_kernel(const float* __restrict__ gmax, int nq, int M, int CT,
                                                           float margin, float* __restrict__ tau,
                                                           const float* __restrict__ eps) {
+  grid_ready();
   __shared__ unsigned hist[8][256];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q = blockIdx.x * 8 + w;
@@ -482,6 +485,7 @@ template <int R>
 __global__ void __launch_bounds__(256) tau_select_reg_kernel(const float* __restrict__ gmax, int nq, int M, int CT,
                                                               float margin, float* __restrict__ tau,
                                                               const float* __restrict__ eps) {
+  grid_ready();
   const int lane = threadIdx.x & 31;
   const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (q >= nq) return;  // warp-uniform
@@ -532,6 +536,7 @@ template <int R>
 __global__ void __launch_bounds__(256) tau_select_block_kernel(const float* __restrict__ gmax, int M, int CT,
                                                                 float margin, float* __restrict__ tau,
                                                                 const float* __restrict__ eps) {
+  grid_ready();
   __shared__ unsigned part[3][2][8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q = blockIdx.x;
   const float4* row = reinterpret_cast<const float4*>(gmax + (int64_t)q * M);
@@ -620,6 +625,7 @@ __global__ void __launch_bounds__(256) cand_select_kernel(const int* __restrict_
                                                            int nq, uint64_t* __restrict__ out,
                                                            int* __restrict__ ovf, const uint16_t* __restrict__ rows,
                                                            uint16_t* __restrict__ gathered) {
+  grid_ready();
   constexpr int CT = 32 * E;
   const int lane = threadIdx.x & 31;
   const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -655,6 +661,7 @@ __global__ void __launch_bounds__(256) exact_select_kernel(const int* __restrict
                                                             const float* __restrict__ tau,
                                                             const float* __restrict__ eps, uint64_t* __restrict__ out,
                                                             int* __restrict__ ovf) {
+  grid_ready();
   constexpr int CT = 32 * E;
   const int lane = threadIdx.x & 31;
   const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -691,6 +698,7 @@ __global__ void __launch_bounds__(256) exact_select_kernel(const int* __restrict
 // (tc_list_geometry).
 __global__ void merge_fallback_kernel(const uint64_t* __restrict__ part, const int* __restrict__ ovf, int NT,
                                       int grid, int CT, uint64_t* __restrict__ out) {
+  grid_ready();
   extern __shared__ uint64_t ms[];
   const int cntq = ovf[0];
   if (cntq == 0) return;
@@ -733,13 +741,15 @@ void run_filter_as(const FilterMaps& m, FilterArgs a, int clusters, const char* 
   cfg.blockDim = dim3(F_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = CL;
-  at.val.clusterDim.y = 1;
-  at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = CL > 1 ? 1 : 0;
+  cudaLaunchAttribute at[2]{};
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = CL;
+  at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = CL > 1 ? 2 : 1;
   ProfScope _ps(name, s);
   LSHG_CUDA(cudaLaunchKernelEx(&cfg, kern, m.a, m.b, m.bhi, a));
   count_launch();
@@ -879,13 +889,13 @@ void launch_tau_select(const float* gmax, int nq, int M, int rank, float margin,
   ProfScope _ps("tc_tau_select", s);
   // the register slots a lane walks in every bisection step: as few as cover M
   if (M <= 32 * kTauRegsFew && M % 4 == 0)
-    tau_select_reg_kernel<kTauRegsFew><<<ceil_div(nq, 8), 256, 0, s>>>(gmax, nq, M, rank, margin, tau, eps);
+    launch_next(tau_select_reg_kernel<kTauRegsFew>, ceil_div(nq, 8), 256, 0, s, gmax, nq, M, rank, margin, tau, eps);
   else if (M <= 32 * kTauRegs && M % 4 == 0)
-    tau_select_reg_kernel<kTauRegs><<<ceil_div(nq, 8), 256, 0, s>>>(gmax, nq, M, rank, margin, tau, eps);
+    launch_next(tau_select_reg_kernel<kTauRegs>, ceil_div(nq, 8), 256, 0, s, gmax, nq, M, rank, margin, tau, eps);
   else if (M <= 256 * kTauBlockRegs && M % 4 == 0)
-    tau_select_block_kernel<kTauBlockRegs><<<nq, 256, 0, s>>>(gmax, M, rank, margin, tau, eps);
+    launch_next(tau_select_block_kernel<kTauBlockRegs>, nq, 256, 0, s, gmax, M, rank, margin, tau, eps);
   else
-    tau_select_kernel<<<ceil_div(nq, 8), 256, 0, s>>>(gmax, nq, M, rank, margin, tau, eps);
+    launch_next(tau_select_kernel, ceil_div(nq, 8), 256, 0, s, gmax, nq, M, rank, margin, tau, eps);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -893,9 +903,9 @@ void launch_tau_select(const float* gmax, int nq, int M, int rank, float margin,
 void launch_cand_select(const int* cnt, const uint64_t* cand, int nq, int cap, int need, int CT, uint64_t* out,
                         int* ovf, const uint16_t* rows, uint16_t* gathered, cudaStream_t s) {
   ProfScope _ps("tc_cand_select", s);
-  if (CT == 32) cand_select_kernel<1><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf, rows, gathered);
-  else if (CT == 64) cand_select_kernel<2><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf, rows, gathered);
-  else if (CT == 128) cand_select_kernel<4><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf, rows, gathered);
+  if (CT == 32) launch_next(cand_select_kernel<1>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out, ovf, rows, gathered);
+  else if (CT == 64) launch_next(cand_select_kernel<2>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out, ovf, rows, gathered);
+  else if (CT == 128) launch_next(cand_select_kernel<4>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out, ovf, rows, gathered);
   else throw Error(LSHG_ERR_INVALID_ARGUMENT, "tensor-core scan: candidate count must be 32, 64 or 128");
   count_launch();
   LSHG_CHECK_LAUNCH();
@@ -904,8 +914,8 @@ void launch_cand_select(const int* cnt, const uint64_t* cand, int nq, int cap, i
 void launch_exact_select(const int* cnt, const uint64_t* cand, int nq, int cap, int k, int CT, const float* tau,
                          const float* eps, uint64_t* out, int* ovf, cudaStream_t s) {
   ProfScope _ps("exact_select", s);
-  if (CT == 128) exact_select_kernel<4><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, k, nq, tau, eps, out, ovf);
-  else if (CT == 256) exact_select_kernel<8><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, k, nq, tau, eps, out, ovf);
+  if (CT == 128) launch_next(exact_select_kernel<4>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, k, nq, tau, eps, out, ovf);
+  else if (CT == 256) launch_next(exact_select_kernel<8>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, k, nq, tau, eps, out, ovf);
   else throw Error(LSHG_ERR_INVALID_ARGUMENT, "exact scan: candidate count must be 128 or 256");
   count_launch();
   LSHG_CHECK_LAUNCH();
@@ -914,7 +924,7 @@ void launch_exact_select(const int* cnt, const uint64_t* cand, int nq, int cap, 
 void launch_merge_fallback(const uint64_t* part, const int* ovf, int nq, int NT, int grid, int CT, uint64_t* out,
                            cudaStream_t s) {
   const size_t smem = (size_t)CT * 8;
-  merge_fallback_kernel<<<std::min(nq, num_sms() * 4), 128, smem, s>>>(part, ovf, NT, grid, CT, out);
+  launch_next(merge_fallback_kernel, std::min(nq, num_sms() * 4), 128, smem, s, part, ovf, NT, grid, CT, out);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

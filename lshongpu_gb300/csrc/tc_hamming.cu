@@ -62,6 +62,7 @@
 // projections (below).
 #include "index.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 #include "profile.h"
 #include "select.cuh"
 #include "tc_filter.h"
@@ -162,6 +163,7 @@ template <int MODE, int GW, int KC, int CL>
 __global__ void __launch_bounds__(H_THREADS, 1)
     tc_hamming_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                       const HArgs a) {
+  grid_ready();
   using LY = HLayout<KC, CL>;
   constexpr int STAGES = LY::STAGES, SBUF = LY::SBUF;
   static_assert(MODE != MODE_FILTER || GW == HW, "the filter reads whole pieces");
@@ -452,6 +454,7 @@ template <int KC>
 __global__ void __launch_bounds__(H_THREADS, 1)
     tc_signs_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                       const SignArgs a) {
+  grid_ready();
   using LY = PLayout<KC>;
   constexpr int STAGES = LY::STAGES;
   const int U = a.NCH * a.QT;
@@ -647,6 +650,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
 // bit; nibbles past 32 * words and rows past n are 0x0.  One thread writes a word's 16 bytes.
 __global__ void expand_bits_kernel(const uint32_t* __restrict__ xs, int64_t n, int wp, int words, int kp,
                                    int64_t rows_pad, uint4* __restrict__ out) {
+  grid_ready();
   const int per_row = kp / 16;
   const int64_t total = rows_pad * per_row;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
@@ -676,6 +680,7 @@ template <int E>
 __global__ void __launch_bounds__(256) hsel_warp_kernel(const int* __restrict__ cnt, const uint64_t* __restrict__ cand,
                                                         int cap, int need, int nq, uint64_t* __restrict__ out,
                                                         int* __restrict__ ovf) {
+  grid_ready();
   constexpr int CT = 32 * E;
   const int lane = threadIdx.x & 31;
   const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -750,6 +755,7 @@ template <int T>
 __global__ void __launch_bounds__(T, 1536 / T)
     hsel_kernel(const int* __restrict__ cnt, const uint64_t* __restrict__ cand, int cap, int need, int C, int bits,
                 uint64_t* __restrict__ out, int* __restrict__ ovf) {
+  grid_ready();
   __shared__ int tie[H_TIE_MAX];  // ids at the C-th score
   __shared__ int hist[H_BINS_MAX];
   __shared__ int part[2][T / 32];
@@ -919,13 +925,15 @@ void run_hamming(const CUtensorMap& ma, const CUtensorMap& mb, HArgs a, const ch
   cfg.blockDim = dim3(H_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = CL;
-  at.val.clusterDim.y = 1;
-  at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = CL > 1 ? 1 : 0;
+  cudaLaunchAttribute at[2]{};
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = CL;
+  at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = CL > 1 ? 2 : 1;
   ProfScope _ps(name, s);
   LSHG_CUDA(cudaLaunchKernelEx(&cfg, kern, ma, mb, a));
   count_launch();
@@ -960,7 +968,7 @@ void run_signs(const CUtensorMap& ma, const CUtensorMap& mb, SignArgs a, cudaStr
   constexpr int smem = PLayout<KC>::SMEM;
   LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   ProfScope _ps("tc_project_gemm", s);
-  kern<<<grid, H_THREADS, smem, s>>>(ma, mb, a);
+  launch_next(kern, grid, H_THREADS, smem, s, ma, mb, a);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -973,6 +981,7 @@ void run_signs(const CUtensorMap& ma, const CUtensorMap& mb, SignArgs a, cudaStr
 // of the exact x.r before the FP32 accumulation's own rounding.  norms: the rows' L2 norms.
 __global__ void split_bf16_kernel(const float* __restrict__ x, int64_t n, int d, int kp, int64_t rows_pad, int order,
                                   __nv_bfloat16* __restrict__ out, float* __restrict__ norms) {
+  grid_ready();
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -1000,6 +1009,7 @@ __global__ void split_bf16_kernel(const float* __restrict__ x, int64_t n, int d,
 __global__ void sign_recheck_kernel(const uint2* __restrict__ list, const int* __restrict__ cnt, int cap, int segs,
                                     const float* __restrict__ x, const float* __restrict__ planes, int d,
                                     uint32_t* __restrict__ out32, int words, int* __restrict__ overflow) {
+  grid_ready();
   const int64_t total = (int64_t)segs * cap;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int seg = (int)(t / cap), i = (int)(t - (int64_t)seg * cap);
@@ -1026,7 +1036,7 @@ void launch_split_bf16(const float* x, int64_t n, int d, int64_t rows_pad, int o
                        cudaStream_t s) {
   LSHG_REQUIRE(d >= 1 && d <= 128, "tensor-core projections: d must be <= 128");
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((rows_pad * 32 + 255) / 256, (int64_t)num_sms() * 16));
-  split_bf16_kernel<<<blocks, 256, 0, s>>>(x, n, d, signs_part_cols(d), rows_pad, order,
+  launch_next(split_bf16_kernel, blocks, 256, 0, s, x, n, d, signs_part_cols(d), rows_pad, order,
                                            reinterpret_cast<__nv_bfloat16*>(out), norms);
   count_launch();
   LSHG_CHECK_LAUNCH();
@@ -1041,6 +1051,9 @@ void launch_tc_signs(const float* x, int64_t n, int d, const uint16_t* planes_sp
   const int64_t ppad = (int64_t)ceil_div(P, PN) * PN;
   LSHG_REQUIRE(rows_pad / BM * (ppad / PN) < (int64_t)INT_MAX, "tensor-core projections: problem too large");
   ProfScope _ps("tc_project", s);
+  const int G = num_sms();
+  DevBuf<int> cnt((size_t)G + 1, s);
+  LSHG_CUDA(cudaMemsetAsync(cnt.ptr, 0, cnt.bytes(), s));
   DevBuf<uint16_t> xa((size_t)rows_pad * 3 * kp, s);
   DevBuf<float> xn((size_t)rows_pad, s);
   launch_split_bf16(x, n, d, rows_pad, 0, xa.ptr, xn.ptr, s);
@@ -1049,12 +1062,9 @@ void launch_tc_signs(const float* x, int64_t n, int d, const uint16_t* planes_sp
   // about 0.1% of the signs of unit points and N(0, 1) planes fall inside the band; each
   // CTA's segment holds 4x its share, and the SIMT projection redoes everything if one
   // overflows
-  const int G = num_sms();
   const int64_t expect = (int64_t)n * P / 1000 / G + 1;
   const int cap = (int)std::min<int64_t>(1 << 22, std::max<int64_t>(4096, 4 * expect));
   DevBuf<uint2> list((size_t)G * cap, s);
-  DevBuf<int> cnt((size_t)G + 1, s);
-  LSHG_CUDA(cudaMemsetAsync(cnt.ptr, 0, cnt.bytes(), s));
   SignArgs a{};
   a.n = (int)n;
   a.QT = (int)(rows_pad / BM);
@@ -1076,7 +1086,7 @@ void launch_tc_signs(const float* x, int64_t n, int d, const uint16_t* planes_sp
   {
     const int64_t total = (int64_t)grid * cap;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, (int64_t)G * 16));
-    sign_recheck_kernel<<<blocks, 256, 0, s>>>(list.ptr, cnt.ptr, cap, grid, x, planes, d, out32, words, overflow);
+    launch_next(sign_recheck_kernel, blocks, 256, 0, s, list.ptr, cnt.ptr, cap, grid, x, planes, d, out32, words, overflow);
     count_launch();
     LSHG_CHECK_LAUNCH();
   }
@@ -1147,7 +1157,7 @@ void launch_expand_bits(const uint32_t* xs, int64_t n, int wp, int words, int64_
   const int64_t total = rows_pad * (kp / 16);
   if (total <= 0) return;
   const int blocks = (int)std::min<int64_t>((total + 255) / 256, (int64_t)num_sms() * 16);
-  expand_bits_kernel<<<blocks, 256, 0, s>>>(xs, n, wp, words, kp, rows_pad, reinterpret_cast<uint4*>(out));
+  launch_next(expand_bits_kernel, blocks, 256, 0, s, xs, n, wp, words, kp, rows_pad, reinterpret_cast<uint4*>(out));
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -1157,12 +1167,12 @@ void launch_int_select(const int* cnt, const uint64_t* cand, int cap, int need, 
   ProfScope _ps("tc_hamming_select", s);
   LSHG_REQUIRE(bits >= 1 && 2 * bits + 1 <= H_BINS_MAX, "integer select: scores of at most 1024 bits");
   if (C <= 128) {
-    if (C == 32) hsel_warp_kernel<1><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf);
-    else if (C == 64) hsel_warp_kernel<2><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf);
-    else hsel_warp_kernel<4><<<ceil_div(nq, 8), 256, 0, s>>>(cnt, cand, cap, need, nq, out, ovf);
+    if (C == 32) launch_next(hsel_warp_kernel<1>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out, ovf);
+    else if (C == 64) launch_next(hsel_warp_kernel<2>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out, ovf);
+    else launch_next(hsel_warp_kernel<4>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out, ovf);
   } else {
-    if (C <= 1024) hsel_kernel<256><<<nq, 256, 0, s>>>(cnt, cand, cap, need, C, bits, out, ovf);
-    else hsel_kernel<512><<<nq, 512, 0, s>>>(cnt, cand, cap, need, C, bits, out, ovf);
+    if (C <= 1024) launch_next(hsel_kernel<256>, nq, 256, 0, s, cnt, cand, cap, need, C, bits, out, ovf);
+    else launch_next(hsel_kernel<512>, nq, 512, 0, s, cnt, cand, cap, need, C, bits, out, ovf);
   }
   count_launch();
   LSHG_CHECK_LAUNCH();
@@ -1180,6 +1190,9 @@ void launch_tc_hamming(const uint8_t* xse, int64_t n, const uint32_t* xst, int w
   const HammingPlan plan = plan_hamming(n, C);
   LSHG_REQUIRE(plan.ok, "tensor-core sketch scan: C too large for this base");
   LSHG_REQUIRE((int64_t)QT * plan.NT < (int64_t)INT_MAX, "tensor-core sketch scan: problem too large");
+  DevBuf<int> ctl((size_t)nq + 1 + nq, s);  // [0, nq): survivors; [nq]: listed queries; then their list
+  int *cnt = ctl.ptr, *ovf = ctl.ptr + nq;
+  LSHG_CUDA(cudaMemsetAsync(ctl.ptr, 0, (size_t)(nq + 1) * sizeof(int), s));
   DevBuf<uint8_t> qe((size_t)qpad * kp, s);
   {
     ProfScope _ps("tc_hamming_expand", s);
@@ -1208,23 +1221,19 @@ void launch_tc_hamming(const uint8_t* xse, int64_t n, const uint32_t* xst, int w
     // scores are integers, computed the same way in both passes: no margin
     launch_tau_select(gmax.ptr, nq, plan.M, plan.rank, 0.0f, tau.ptr, s);
   }
-  DevBuf<int> cnt(nq, s);
-  LSHG_CUDA(cudaMemsetAsync(cnt.ptr, 0, cnt.bytes(), s));
   DevBuf<uint64_t> cand((size_t)nq * plan.cap, s);
   a.gmax = nullptr;
   a.M = 0;
   a.NP = plan.NT;
   a.dstride = 1;
   a.tau = plan.M > 0 ? tau.ptr : nullptr;
-  a.cnt = cnt.ptr;
+  a.cnt = cnt;
   a.cand = cand.ptr;
   a.cap = plan.cap;
   run_hamming_kc<MODE_FILTER, HW>(kc, cl, ma, mb, a, "tc_hamming", s);
-  DevBuf<int> ovf((size_t)nq + 1, s);
-  LSHG_CUDA(cudaMemsetAsync(ovf.ptr, 0, sizeof(int), s));
-  launch_int_select(cnt.ptr, cand.ptr, plan.cap, (int)std::min<int64_t>(C, n), C, 32 * words, nq, out, ovf.ptr, s);
+  launch_int_select(cnt, cand.ptr, plan.cap, (int)std::min<int64_t>(C, n), C, 32 * words, nq, out, ovf, s);
   // listed queries: exact popcount rescan written straight into their rows of `out`
-  launch_scan_bits_listed(xst, n, wp, words, 0, qs, nq, op, C, ovf.ptr, out, s);
+  launch_scan_bits_listed(xst, n, wp, words, 0, qs, nq, op, C, ovf, out, s);
 }
 
 }  // namespace tc

@@ -31,6 +31,7 @@
 // returns.
 #include "index.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 #include "profile.h"
 #include "tc_filter.h"
 #include "tc_ptx.cuh"
@@ -150,6 +151,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     tc_list_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                    const int* __restrict__ rows_dev, int64_t n, int NT, int ksteps, uint64_t* __restrict__ part,
                    int* err) {
+  grid_ready();
   constexpr TcLayout L = tc_layout(STAGES, CT);
   constexpr int fold_limit = BUFN - 8;
   const int nq = *rows_dev;  // gathered query rows (0: nothing to do)
@@ -376,6 +378,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // Unit rows in BF16, zero-padded to KD columns and to `rows_pad` rows.
 __global__ void to_unit_bf16_kernel(const float* __restrict__ x, int64_t n, int d, int64_t rows_pad,
                                     __nv_bfloat16* __restrict__ out) {
+  grid_ready();
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -396,6 +399,7 @@ __global__ void to_unit_bf16_kernel(const float* __restrict__ x, int64_t n, int 
 // Unit rows as E4M3 codes of (x / |x|) * kE4M3Scale, KD bytes a row, zero padded.
 __global__ void to_unit_e4m3_kernel(const float* __restrict__ x, int64_t n, int d, int64_t rows_pad,
                                     uint8_t* __restrict__ out) {
+  grid_ready();
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -415,7 +419,7 @@ __global__ void to_unit_e4m3_kernel(const float* __restrict__ x, int64_t n, int 
 
 void to_unit_e4m3(const float* x, int64_t n, int d, int64_t rows_pad, uint8_t* out, cudaStream_t s) {
   int blocks = (int)std::min<int64_t>((rows_pad * 32 + 255) / 256, (int64_t)num_sms() * 16);
-  to_unit_e4m3_kernel<<<std::max(blocks, 1), 256, 0, s>>>(x, n, d, rows_pad, out);
+  launch_next(to_unit_e4m3_kernel, std::max(blocks, 1), 256, 0, s, x, n, d, rows_pad, out);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -423,7 +427,7 @@ void to_unit_e4m3(const float* x, int64_t n, int d, int64_t rows_pad, uint8_t* o
 void to_unit_bf16(const float* x, int64_t n, int d, int64_t rows_pad, uint16_t* out, cudaStream_t s) {
   int64_t warps = rows_pad;
   int blocks = (int)std::min<int64_t>((warps * 32 + 255) / 256, (int64_t)num_sms() * 16);
-  to_unit_bf16_kernel<<<std::max(blocks, 1), 256, 0, s>>>(x, n, d, rows_pad, reinterpret_cast<__nv_bfloat16*>(out));
+  launch_next(to_unit_bf16_kernel, std::max(blocks, 1), 256, 0, s, x, n, d, rows_pad, reinterpret_cast<__nv_bfloat16*>(out));
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -498,7 +502,7 @@ void run_list_kernel(const CUtensorMap& ma, const CUtensorMap& mb, const int* ro
   constexpr TcLayout L = tc_layout(STAGES, CT);
   auto kern = tc_list_kernel<STAGES, CT>;
   LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total));
-  kern<<<grid, NTHREADS, L.total, s>>>(ma, mb, rows_dev, n, NT, tc_ksteps(d), part, err);
+  launch_next(kern, grid, NTHREADS, L.total, s, ma, mb, rows_dev, n, NT, tc_ksteps(d), part, err);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -547,6 +551,10 @@ void launch_tc_scan(Index& I, const float* q, int nq, int k, lshg_point* out, cu
   if (const char* e = getenv("LSHG_TC_FORCE_FALLBACK"); e && e[0] == '1') plan.cap = 0;
   const int NT = ceil_div(I.n, BN);  // 128-row tiles of the list kernel
   LSHG_REQUIRE((int64_t)QT * NT < (int64_t)INT_MAX, "tensor-core scan: problem too large");
+  DevBuf<float> tau((size_t)nq, s);
+  DevBuf<int> cnt((size_t)nq + 1 + nq, s);  // [0, nq): survivors; [nq]: overflow count; then the list
+  int* ovf = cnt.ptr + nq;
+  LSHG_CUDA(cudaMemsetAsync(cnt.ptr, 0, (size_t)(nq + 1) * sizeof(int), s));
   DevBuf<uint16_t> qbf((size_t)qpad * KD, s);
   to_unit_bf16(q, nq, I.d, qpad, qbf.ptr, s);
   const int64_t npad = (int64_t)ceil_div(I.n, FILTER_TN) * FILTER_TN;
@@ -560,10 +568,6 @@ void launch_tc_scan(Index& I, const float* q, int nq, int k, lshg_point* out, cu
                                : make_filter_maps(qbf.ptr, qpad, I.xbf.ptr, npad, I.d, false);
 
   // 1-2. thresholds and survivors
-  DevBuf<float> tau((size_t)nq, s);
-  DevBuf<int> cnt((size_t)nq + 1 + nq, s);  // [0, nq): survivors; [nq]: overflow count; then the list
-  int* ovf = cnt.ptr + nq;
-  LSHG_CUDA(cudaMemsetAsync(cnt.ptr, 0, (size_t)(nq + 1) * sizeof(int), s));
   DevBuf<uint64_t> cand((size_t)nq * plan.cap, s);
   launch_filter_scan(maps, plan, nq, I.n, I.d, QT, tau.ptr, cnt.ptr, cand.ptr, err, s);
 

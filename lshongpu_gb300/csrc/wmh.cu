@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "launch_count.h"
+#include "launch_next.cuh"
 
 namespace lshg {
 
@@ -46,6 +47,7 @@ __global__ void __launch_bounds__(256) wmh_sketch_kernel(
     int M, const float* __restrict__ rtab, const curandStateXORWOW_t* __restrict__ states, int H, int T,
     int onebit, int words, int hashBits, const uint8_t* __restrict__ bitmap, int bitmapLen,
     uint8_t* __restrict__ out8, uint32_t* __restrict__ out32, int* err) {
+  grid_ready();
   extern __shared__ int smi[];
   int* start = smi;       // [d]
   int* map = smi + d;     // [M]
@@ -125,7 +127,7 @@ void launch_wmh_sketch(const float* x, int64_t n, int d, const int* start, const
   int groups = onebit ? words : (H + 31) / 32;
   int64_t warps = n * groups;
   int blocks = (int)std::min<int64_t>((warps * 32 + 255) / 256, (int64_t)num_sms() * 16);
-  wmh_sketch_kernel<<<blocks, 256, smem, s>>>(x, n, d, start, map, M, r, (const curandStateXORWOW_t*)states, H, T,
+  launch_next(wmh_sketch_kernel, blocks, 256, smem, s, x, n, d, start, map, M, r, (const curandStateXORWOW_t*)states, H, T,
                                               onebit, words, hashBits, bitmap, bitmapLen, out8, out32, err);
   count_launch();
   LSHG_CHECK_LAUNCH();

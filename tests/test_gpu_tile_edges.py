@@ -297,3 +297,35 @@ def test_jaccard_filter_saved_index(engine, tmp_path):
     path = str(tmp_path / "jaccard.lshg")
     idx.save(path)
     assert engine.Index.load(path).query(q, 32).tobytes() == idx.query(q, 32).tobytes()
+
+
+@pytest.mark.parametrize("kw", [
+    dict(implementation=8), dict(implementation=9), dict(implementation=2, distanceFunc=1),
+    dict(implementation=2, distanceFunc=2), dict(implementation=3, sketchDim=8), dict(implementation=4, distanceFunc=2,
+                                                                                     sketchDim=64),
+], ids=["tc", "e4m3", "angular", "jaccard", "simhash", "minhash"])
+def test_batches_enqueued_back_to_back(engine, kw):
+    """Batches of several sizes down one stream without a wait, their queries written on that stream
+    just before: kernels that may start early read nothing of the batch before."""
+    import torch
+
+    n, k = 20000, 10
+    jac = kw.get("distanceFunc") == 2
+    x, q = (datasets.sparse_gamma(n, D, 121), datasets.sparse_gamma(400, D, 122)) if jac else data(n, 400)
+    idx = engine.Index(x, options=engine.make_options(candidates=128), **kw)
+    sizes = [1, 130, 3, 400, 64, 257]
+    want = [idx.query(np.roll(q, i, axis=0)[:m], k) for i, m in enumerate(sizes)]
+    st = torch.cuda.Stream()
+    host = torch.from_numpy(q).cuda()
+    torch.cuda.synchronize()
+    for _ in range(5):
+        buf, outs = torch.empty_like(host), []
+        with torch.cuda.stream(st):
+            for i, m in enumerate(sizes):
+                buf.copy_(torch.roll(host, i, 0))
+                outs.append(torch.full((m, k, 2), -7, dtype=torch.int32, device="cuda"))
+                idx.query_device_async(buf.data_ptr(), m, k, outs[-1].data_ptr(), st.cuda_stream)
+        st.synchronize()
+        idx.sync(st.cuda_stream)
+        for o, w in zip(outs, want):
+            assert o.cpu().numpy().tobytes() == w.tobytes()
