@@ -271,7 +271,8 @@ __host__ __device__ inline DirectSmem direct_layout(int S, int QB, int C, int kb
 // lanes of a warp read 32 consecutive points' chunk as one 512-byte run).  Selection as
 // in the popcount sketch scan: keys below a query's threshold go to an append buffer that
 // is folded into the sorted top-C list every T tiles when a buffer passed its limit.
-// list (optional): scan only the queries list[1 .. list[0]], results to their rows.
+// list (optional): scan only the queries list[1 .. list[0]], results to their rows, or with
+// several splits to the slots of the list.
 template <int KBUF, int T>
 __global__ void __launch_bounds__(256, 2)
     cws_direct_kernel(const uint4* __restrict__ xst, int64_t n, int S, const int2* __restrict__ qs, int nq, int C,
@@ -335,7 +336,7 @@ __global__ void __launch_bounds__(256, 2)
   for (int i = threadIdx.x; i < QB * C; i += blockDim.x) {
     const int qj = i / C, c = i - qj * C;
     if (q0 + qj < nqe) {
-      const int64_t qrow = list ? list[1 + q0 + qj] : q0 + qj;
+      const int64_t qrow = list && splits == 1 ? list[1 + q0 + qj] : q0 + qj;
       out[(qrow * splits + split) * C + c] = Sh.kept[(size_t)qj * C + c];
     }
   }
@@ -508,7 +509,15 @@ void launch_cws_scan(const uint32_t* xsl_t, const uint32_t* xst, int64_t n, int 
     DevBuf<int> list((size_t)nq + 1, s);
     if (c.pl == 8) sliced_filter_select<8>(xsl_t, n, ng, S, qsl.ptr, nq, C, out, list.ptr, err, s);
     else sliced_filter_select<16>(xsl_t, n, ng, S, qsl.ptr, nq, C, out, list.ptr, err, s);
-    launch_direct(xst, n, S, qs, nq, C, 1, out, list.ptr, s);  // listed queries: exact direct rescan
+    // listed queries: exact direct rescan
+    const int splits = listed_rescan_splits(n, nq, 2, C);
+    DevBuf<uint64_t> part;
+    if (splits > 1 && alloc_if_room(part, (size_t)nq * splits * C, s)) {
+      launch_direct(xst, n, S, qs, nq, C, splits, part.ptr, list.ptr, s);
+      launch_merge_splits(part.ptr, nq, splits, C, out, s, list.ptr);
+    } else {
+      launch_direct(xst, n, S, qs, nq, C, 1, out, list.ptr, s);
+    }
     return;
   }
   // direct scan of every query, the base split so that the grid fills the GPU

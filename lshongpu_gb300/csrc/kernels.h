@@ -143,7 +143,13 @@ int scan_listed_splits(int64_t n, int nq, int C);
 void launch_scan_float_listed(const float* xt, int64_t n, int d, const float* xnorm, const float* q, int nq,
                               const float* qnorm, int dist, const int* list, int C, int splits, uint64_t* part,
                               int k, struct ::lshg_point_s* out, cudaStream_t s);
-void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t* out, cudaStream_t s);
+void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t* out, cudaStream_t s,
+                         const int* list = nullptr);
+// Splits of the base for the exact rescan of queries listed on the device (at most nq of them, QB a
+// block): blocks enough for one or two listed queries to use the GPU, while the lists of all nq
+// would stay below 256 MB.  (One split: a query that a sampled threshold failed took 7.8 ms over
+// 1.2M 64-bit sketches, in a batch of 0.1 ms; split over 64 blocks 0.2.)
+int listed_rescan_splits(int64_t n, int nq, int QB, int C);
 // The same with the first k keys written as points; false when C or k is not one it serves.
 bool launch_merge_points(const uint64_t* in, int nq, int splits, int C, int k, struct ::lshg_point_s* out,
                          cudaStream_t s);

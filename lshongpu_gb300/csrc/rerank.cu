@@ -145,13 +145,15 @@ __device__ __forceinline__ float query_norm(const float* row, int d) {
   return __fsqrt_rn(m);
 }
 
-// One block per query: fold S sorted lists of C keys into one.
+// One block per query: fold S sorted lists of C keys into one.  list (optional): the lists of slot
+// i < list[0] go to row list[1 + i].
 __global__ void merge_splits_kernel(const uint64_t* __restrict__ in, int nq, int splits, int C,
-                                    uint64_t* __restrict__ out) {
+                                    uint64_t* __restrict__ out, const int* __restrict__ list) {
   grid_ready();
   extern __shared__ uint64_t ms[];
-  const int q = blockIdx.x;
-  const uint64_t* src = in + (int64_t)q * splits * C;
+  if (list && (int)blockIdx.x >= list[0]) return;
+  const int q = list ? list[1 + blockIdx.x] : (int)blockIdx.x;
+  const uint64_t* src = in + (int64_t)blockIdx.x * splits * C;
   for (int i = threadIdx.x; i < C; i += blockDim.x) ms[i] = src[i];
   __syncthreads();
   for (int s = 1; s < splits; ++s) {
@@ -173,12 +175,15 @@ __global__ void merge_splits_kernel(const uint64_t* __restrict__ in, int nq, int
 // in place of the keys.
 template <int E>
 __global__ void __launch_bounds__(256) merge_short_kernel(const uint64_t* __restrict__ in, int splits, int k,
-                                                           uint64_t* __restrict__ out, lshg_point* __restrict__ pts) {
+                                                           uint64_t* __restrict__ out, lshg_point* __restrict__ pts,
+                                                           const int* __restrict__ list) {
   grid_ready();
   constexpr int C = 32 * E;
   __shared__ uint64_t lists[8][C];
-  const int q = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-  const uint64_t* src = in + (int64_t)q * splits * C;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+  if (list && (int)blockIdx.x >= list[0]) return;
+  const int q = list ? list[1 + blockIdx.x] : (int)blockIdx.x;
+  const uint64_t* src = in + (int64_t)blockIdx.x * splits * C;
   uint64_t best[E], x[E];
   auto load = [&](int s) {
 #pragma unroll
@@ -663,27 +668,29 @@ __global__ void keys_to_points_kernel(const uint64_t* __restrict__ keys, int nq,
 }  // namespace
 
 namespace {
-void merge_short(const uint64_t* in, int nq, int splits, int C, int k, uint64_t* out, lshg_point* pts, cudaStream_t s) {
+void merge_short(const uint64_t* in, int nq, int splits, int C, int k, uint64_t* out, lshg_point* pts,
+                 const int* list, cudaStream_t s) {
   int W = 1;  // warps: a power of two, no more than lists
   while (W < 8 && 2 * W <= splits) W <<= 1;
-  if (C == 32) launch_next(merge_short_kernel<1>, nq, 32 * W, 0, s, in, splits, k, out, pts);
-  else if (C == 64) launch_next(merge_short_kernel<2>, nq, 32 * W, 0, s, in, splits, k, out, pts);
-  else launch_next(merge_short_kernel<4>, nq, 32 * W, 0, s, in, splits, k, out, pts);
+  if (C == 32) launch_next(merge_short_kernel<1>, nq, 32 * W, 0, s, in, splits, k, out, pts, list);
+  else if (C == 64) launch_next(merge_short_kernel<2>, nq, 32 * W, 0, s, in, splits, k, out, pts, list);
+  else launch_next(merge_short_kernel<4>, nq, 32 * W, 0, s, in, splits, k, out, pts, list);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
 }  // namespace
 
-void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t* out, cudaStream_t s) {
+void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t* out, cudaStream_t s,
+                         const int* list) {
   if (nq <= 0) return;
   ProfScope _ps("merge_splits", s);
   if (C == 32 || C == 64 || C == 128) {
-    merge_short(in, nq, splits, C, 0, out, nullptr, s);
+    merge_short(in, nq, splits, C, 0, out, nullptr, list, s);
     return;
   }
   size_t smem = (size_t)C * 8;
   LSHG_CUDA(cudaFuncSetAttribute(merge_splits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  launch_next(merge_splits_kernel, nq, 128, smem, s, in, nq, splits, C, out);
+  launch_next(merge_splits_kernel, nq, 128, smem, s, in, nq, splits, C, out, list);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -692,7 +699,7 @@ bool launch_merge_points(const uint64_t* in, int nq, int splits, int C, int k, l
   if ((C != 32 && C != 64 && C != 128) || k > C) return false;
   if (nq <= 0) return true;
   ProfScope _ps("merge_splits", s);
-  merge_short(in, nq, splits, C, k, nullptr, out, s);
+  merge_short(in, nq, splits, C, k, nullptr, out, nullptr, s);
   return true;
 }
 

@@ -12,6 +12,8 @@
 // chunk is 512 contiguous bytes; read as rows, 32 lanes a row apart would touch 32 lines
 // an instruction and the L1 data pipe, not the integer ALU, would bound the scan.  Candidates are filtered against each query's running threshold and
 // folded into a per-query sorted top-C list (select.cuh).
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "launch_count.h"
@@ -84,7 +86,8 @@ __global__ void __launch_bounds__(256, MINB) scan_bits_kernel(const uint32_t* __
                reinterpret_cast<int*>(smem + L.cnt), reinterpret_cast<uint64_t*>(smem + L.thr), C, KBUF};
 
   // list (optional): scan only the queries list[1 .. list[0]]; slot i of the list is query
-  // list[1 + i], and its result goes to that query's row
+  // list[1 + i].  Its result goes to that query's row, or with several splits to slot i (merged
+  // from there)
   const int nqe = list ? list[0] : nq;
   const int q0 = blockIdx.x * QB;
   if (q0 >= nqe) return;  // block-uniform, before any barrier
@@ -169,7 +172,7 @@ __global__ void __launch_bounds__(256, MINB) scan_bits_kernel(const uint32_t* __
   for (int i = threadIdx.x; i < QB * C; i += blockDim.x) {
     int qi = i / C, c = i - qi * C;
     if (q0 + qi < nqe) {
-      const int64_t qrow = list ? list[1 + q0 + qi] : q0 + qi;
+      const int64_t qrow = list && splits == 1 ? list[1 + q0 + qi] : q0 + qi;
       out[(qrow * splits + split) * C + c] = S.kept[(size_t)qi * C + c];
     }
   }
@@ -288,7 +291,20 @@ int launch_scan_bits(const uint32_t* xs, int64_t n, int wp, int words, int sbyte
 // the whole base, each result written to out[query][C]; blocks past the list's end exit.
 int launch_scan_bits_listed(const uint32_t* xst, int64_t n, int wp, int words, int sbytes, const uint32_t* qs, int nq,
                             int op, int C, const int* list, uint64_t* out, cudaStream_t s) {
+  const int splits = listed_rescan_splits(n, nq, C <= 128 ? 16 : (C <= 1024 ? 4 : 2), C);
+  DevBuf<uint64_t> part;
+  if (splits > 1 && alloc_if_room(part, (size_t)nq * splits * C, s)) {
+    scan_bits_dispatch(xst, n, wp, words, sbytes, qs, nq, op, C, splits, part.ptr, list, s);
+    launch_merge_splits(part.ptr, nq, splits, C, out, s, list);
+    return splits;
+  }
   return scan_bits_dispatch(xst, n, wp, words, sbytes, qs, nq, op, C, 1, out, list, s);
+}
+
+int listed_rescan_splits(int64_t n, int nq, int QB, int C) {
+  const int64_t fit = ((int64_t)256 << 20) / ((int64_t)nq * C * 8);
+  return (int)std::max<int64_t>(1, std::min<int64_t>(
+                                       {fit, 64, std::max<int64_t>(1, n / kTile / 4), (int64_t)num_sms() * 6 / ceil_div(nq, QB)}));
 }
 
 }  // namespace lshg

@@ -40,7 +40,6 @@
 
 namespace lshg {
 
-void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t* out, cudaStream_t s);
 
 namespace tc {
 

@@ -329,3 +329,36 @@ def test_batches_enqueued_back_to_back(engine, kw):
         idx.sync(st.cuda_stream)
         for o, w in zip(outs, want):
             assert o.cpu().numpy().tobytes() == w.tobytes()
+
+
+@pytest.mark.parametrize("n,nq,words,C,impl", [
+    (12000, 1, 1, 32, 3),      # one word of a chunk; one query
+    (30001, 33, 5, 128, 3),    # rows of 8 words, 5 used; the last tile partly filled
+    (120000, 64, 8, 256, 5),   # the largest batch read as packed words; a sampled prepass
+    (120000, 65, 8, 256, 5),   # beyond it: E2M1 rows
+    (150000, 7, 20, 1024, 3),  # three chunks, the last one half used; 8-point maxima
+    (40000, 64, 32, 4096, 3),  # four chunks
+])
+def test_sketch_scan_packed_words_equal_popcount(engine, n, nq, words, C, impl):
+    """Base tiles expanded from the packed sketches, and ties enough to overflow some queries, give
+    the popcount scan's results."""
+    x, q = (data(n, nq) if impl == 3 else (datasets.sparse_gamma(n, D, 131), datasets.sparse_gamma(nq, D, 132)))
+    x[: n // 3] = x[0]
+    q[0] = x[0]
+    kw = dict(implementation=impl, sketchDim=words, **({} if impl == 3 else {"distanceFunc": 2}))
+    res = [engine.Index(x, options=engine.make_options(candidates=C, sketch_scan=mode), **kw).query(q, 32)
+           for mode in (TENSOR, POPCOUNT)]
+    assert np.array_equal(res[0], res[1])
+
+
+@pytest.mark.parametrize("impl,words,C", [(3, 2, 128), (3, 4, 1024), (5, 4, 2048), (4, 64, 128), (10, 64, 512)])
+def test_listed_rescans_split_over_the_base(engine, impl, words, C):
+    """Queries that tie with half of the base are rescanned in splits of it and merged."""
+    n, nq = 50000, 5
+    x, q = data(n, nq) if impl == 3 else (datasets.sparse_gamma(n, D, 141), datasets.sparse_gamma(nq, D, 142))
+    x[: n // 2] = x[0]
+    q[1] = q[3] = x[0]
+    kw = dict(implementation=impl, sketchDim=words, **({} if impl == 3 else {"distanceFunc": 2}))
+    res = [engine.Index(x, options=engine.make_options(candidates=C, sketch_scan=mode), **kw).query(q, 32)
+           for mode in (TENSOR, POPCOUNT)]
+    assert np.array_equal(res[0], res[1])
