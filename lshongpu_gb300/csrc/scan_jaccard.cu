@@ -57,33 +57,38 @@ __device__ __forceinline__ float delta(int d) { return (2.0f * d + 7.0f) * 1.2e-
 // codes and the FP32 sums hide.  With these of a query and a point added and A = sum |u_q - u_x|,
 // A_lo = (P - A) / 2 s and A_hi = (Q - A) / 2 s bound the sum of minima.  bad[i] = 1 for a row without
 // bounds.
-template <int ROWS>
-__global__ void __launch_bounds__(256) code_tiles_kernel(const float* __restrict__ x, int64_t n, int d, int wd, float lo,
-                                                         float s, uint32_t* __restrict__ out, float4* __restrict__ tails,
-                                                         int* __restrict__ bad) {
+// A warp a row, its (at most four) loads in flight together; queries' few blocks take 32 warps
+// (one row after another by 8 warps: 17 us of a batch of 129).
+template <int ROWS, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+    code_tiles_kernel(const float* __restrict__ x, int64_t n, int d, int wd, float lo, float s,
+                      uint32_t* __restrict__ out, float4* __restrict__ tails, int* __restrict__ bad) {
   grid_ready();
   extern __shared__ uint32_t rows[];  // [ROWS][wd | 1]
   const int pitch = wd | 1, lane = threadIdx.x & 31;
   const int64_t row0 = (int64_t)blockIdx.x * ROWS;
   const float inv = 1.0f / s;
-  for (int r = threadIdx.x >> 5; r < ROWS; r += 8) {
+  for (int r = threadIdx.x >> 5; r < ROWS; r += THREADS / 32) {
     const int64_t i = row0 + r;
     uint8_t* codes = reinterpret_cast<uint8_t*>(rows + r * pitch);
+    float v[kMaxDim / 32];
+#pragma unroll
+    for (int t = 0; t < kMaxDim / 32; ++t) v[t] = i < n && 32 * t + lane < d ? x[i * d + 32 * t + lane] : 0.0f;
     float sum = 0.0f, err = 0.0f;
     unsigned total = 0;
     bool wrong = false;
-    for (int c = lane; c < 4 * wd; c += 32) {
-      const float v = i < n && c < d ? x[i * d + c] : 0.0f;
-      if (c >= d) {
-        codes[c] = 0;
-        continue;
+#pragma unroll
+    for (int t = 0; t < kMaxDim / 32; ++t) {
+      const int c = 32 * t + lane;
+      unsigned u = 0;
+      if (c < d) {
+        wrong |= !(v[t] >= 0.0f && v[t] <= 1e18f);
+        u = code(v[t] - lo, s);
+        total += u;
+        sum += v[t];
+        err += fabsf(v[t] - (lo + (float)u * inv));
       }
-      wrong |= !(v >= 0.0f && v <= 1e18f);
-      const unsigned u = code(v - lo, s);
-      codes[c] = (uint8_t)u;
-      total += u;
-      sum += v;
-      err += fabsf(v - (lo + (float)u * inv));
+      if (c < 4 * wd) codes[c] = (uint8_t)u;
     }
     total = __reduce_add_sync(0xffffffffu, total);
 #pragma unroll
@@ -101,7 +106,7 @@ __global__ void __launch_bounds__(256) code_tiles_kernel(const float* __restrict
   }
   __syncthreads();
   uint32_t* dst = out + (int64_t)blockIdx.x * wd * ROWS;
-  for (int i = threadIdx.x; i < wd * ROWS; i += 256) dst[i] = rows[(i % ROWS) * pitch + i / ROWS];
+  for (int i = threadIdx.x; i < wd * ROWS; i += THREADS) dst[i] = rows[(i % ROWS) * pitch + i / ROWS];
 }
 
 // Tiles 0, stride, 2 stride, ... (ntiles of them; tile i below is the i-th).
@@ -247,8 +252,8 @@ void derive_jaccard_scan(Index& I, cudaStream_t s) {
   I.jq_lo = lo;
   I.jq_scale = 255.0f / std::max(hi - lo, 1e-6f * hi);
   const size_t smem = tile_smem(wd, kTile);
-  LSHG_CUDA(cudaFuncSetAttribute(code_tiles_kernel<kTile>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  launch_next(code_tiles_kernel<kTile>, tiles, 256, smem, s, I.x.ptr, I.n, I.d, wd, I.jq_lo, I.jq_scale, I.jq.ptr, I.jq_tail.ptr, nullptr);
+  launch_next(code_tiles_kernel<kTile, 256>, tiles, 256, smem, s, I.x.ptr, I.n, I.d, wd, I.jq_lo, I.jq_scale, I.jq.ptr,
+              I.jq_tail.ptr, nullptr);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -272,8 +277,8 @@ bool query_jaccard_filtered(Index& I, const float* q, int nq, int k, lshg_point*
     int *cnt = ctl.ptr, *bad = ctl.ptr + nq, *list = ctl.ptr + 2 * nq;
     LSHG_CUDA(cudaMemsetAsync(ctl.ptr, 0, ctl.bytes(), s));
     const size_t qsm = tile_smem(wd, kQB);
-    LSHG_CUDA(cudaFuncSetAttribute(code_tiles_kernel<kQB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qsm));
-    launch_next(code_tiles_kernel<kQB>, qblocks, 256, qsm, s, q, nq, I.d, wd, I.jq_lo, I.jq_scale, qt.ptr, qtail.ptr, bad);
+    launch_next(code_tiles_kernel<kQB, 1024>, qblocks, 1024, qsm, s, q, nq, I.d, wd, I.jq_lo, I.jq_scale, qt.ptr, qtail.ptr,
+                bad);
     count_launch();
     LSHG_CHECK_LAUNCH();
     // two rounds of four CTAs an SM where there are tiles enough, at least two tiles each
