@@ -79,19 +79,6 @@ struct DevBuf {
   size_t bytes() const { return n * sizeof(T); }
 };
 
-// False, with nothing allocated, when there is no room: for buffers that only make a step faster.
-template <typename T>
-bool alloc_if_room(DevBuf<T>& b, size_t count, cudaStream_t s) {
-  try {
-    b.alloc(count, s);
-  } catch (const Error& e) {
-    if (e.status != LSHG_ERR_OUT_OF_MEMORY) throw;
-    cudaGetLastError();
-    return false;
-  }
-  return true;
-}
-
 // ---------------------------------------------------------------------------------
 // Keys.
 // ---------------------------------------------------------------------------------

@@ -507,17 +507,13 @@ void launch_cws_scan(const uint32_t* xsl_t, const uint32_t* xst, int64_t n, int 
     DevBuf<uint32_t> qsl((size_t)nq * ng * c.pl, s);
     launch_cws_slice(qs, nq, S, d, c, true, qsl.ptr, s);
     DevBuf<int> list((size_t)nq + 1, s);
-    if (c.pl == 8) sliced_filter_select<8>(xsl_t, n, ng, S, qsl.ptr, nq, C, out, list.ptr, err, s);
-    else sliced_filter_select<16>(xsl_t, n, ng, S, qsl.ptr, nq, C, out, list.ptr, err, s);
+    DevBuf<uint64_t> cand;
+    const int cap = c.pl == 8 ? sliced_filter_select<8>(xsl_t, n, ng, S, qsl.ptr, nq, C, out, list.ptr, &cand, err, s)
+                              : sliced_filter_select<16>(xsl_t, n, ng, S, qsl.ptr, nq, C, out, list.ptr, &cand, err, s);
     // listed queries: exact direct rescan
-    const int splits = listed_rescan_splits(n, nq, 2, C);
-    DevBuf<uint64_t> part;
-    if (splits > 1 && alloc_if_room(part, (size_t)nq * splits * C, s)) {
-      launch_direct(xst, n, S, qs, nq, C, splits, part.ptr, list.ptr, s);
-      launch_merge_splits(part.ptr, nq, splits, C, out, s, list.ptr);
-    } else {
-      launch_direct(xst, n, S, qs, nq, C, 1, out, list.ptr, s);
-    }
+    const int splits = listed_rescan_splits(n, nq, 2, C, cap);
+    launch_direct(xst, n, S, qs, nq, C, splits, splits > 1 ? cand.ptr : out, list.ptr, s);
+    if (splits > 1) launch_merge_splits(cand.ptr, nq, splits, C, out, s, list.ptr);
     return;
   }
   // direct scan of every query, the base split so that the grid fills the GPU

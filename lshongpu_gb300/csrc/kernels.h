@@ -146,10 +146,14 @@ void launch_scan_float_listed(const float* xt, int64_t n, int d, const float* xn
 void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t* out, cudaStream_t s,
                          const int* list = nullptr);
 // Splits of the base for the exact rescan of queries listed on the device (at most nq of them, QB a
-// block): blocks enough for one or two listed queries to use the GPU, while the lists of all nq
-// would stay below 256 MB.  (One split: a query that a sampled threshold failed took 7.8 ms over
-// 1.2M 64-bit sketches, in a batch of 0.1 ms; split over 64 blocks 0.2.)
-int listed_rescan_splits(int64_t n, int nq, int QB, int C);
+// block): blocks enough for one or two listed queries to use the GPU, as far as the lists of all nq
+// fit `room` keys a query (the filter's survivor arrays, free by then).  With one split, a query
+// that ties with half of 1.2M 64-bit sketches took 10.7 ms; split over 64 blocks 0.34 (the popcount
+// scan of the same batch: 0.29).  In a batch of 1,000 queries: 13.7 -> 1.7 ms.
+int listed_rescan_splits(int64_t n, int nq, int QB, int C, int room);
+// Keys a query of the survivor arrays: `cap`, or room for up to 64 splits' lists within 4 MB.  (32
+// MB cost batches of 100 queries 20 to 40 us in the allocator.)
+int survivor_room(int nq, int cap, int C);
 // The same with the first k keys written as points; false when C or k is not one it serves.
 bool launch_merge_points(const uint64_t* in, int nq, int splits, int C, int k, struct ::lshg_point_s* out,
                          cudaStream_t s);

@@ -289,22 +289,24 @@ int launch_scan_bits(const uint32_t* xs, int64_t n, int wp, int words, int sbyte
 
 // The queries list[1 .. list[0]] (a device-side list, at most nq of them) scanned over
 // the whole base, each result written to out[query][C]; blocks past the list's end exit.
+// scratch: `room` keys a query that the scan may overwrite.
 int launch_scan_bits_listed(const uint32_t* xst, int64_t n, int wp, int words, int sbytes, const uint32_t* qs, int nq,
-                            int op, int C, const int* list, uint64_t* out, cudaStream_t s) {
-  const int splits = listed_rescan_splits(n, nq, C <= 128 ? 16 : (C <= 1024 ? 4 : 2), C);
-  DevBuf<uint64_t> part;
-  if (splits > 1 && alloc_if_room(part, (size_t)nq * splits * C, s)) {
-    scan_bits_dispatch(xst, n, wp, words, sbytes, qs, nq, op, C, splits, part.ptr, list, s);
-    launch_merge_splits(part.ptr, nq, splits, C, out, s, list);
-    return splits;
-  }
-  return scan_bits_dispatch(xst, n, wp, words, sbytes, qs, nq, op, C, 1, out, list, s);
+                            int op, int C, const int* list, uint64_t* out, uint64_t* scratch, int room,
+                            cudaStream_t s) {
+  const int splits = listed_rescan_splits(n, nq, C <= 128 ? 16 : (C <= 1024 ? 4 : 2), C, room);
+  if (splits == 1) return scan_bits_dispatch(xst, n, wp, words, sbytes, qs, nq, op, C, 1, out, list, s);
+  scan_bits_dispatch(xst, n, wp, words, sbytes, qs, nq, op, C, splits, scratch, list, s);
+  launch_merge_splits(scratch, nq, splits, C, out, s, list);
+  return splits;
 }
 
-int listed_rescan_splits(int64_t n, int nq, int QB, int C) {
-  const int64_t fit = ((int64_t)256 << 20) / ((int64_t)nq * C * 8);
-  return (int)std::max<int64_t>(1, std::min<int64_t>(
-                                       {fit, 64, std::max<int64_t>(1, n / kTile / 4), (int64_t)num_sms() * 6 / ceil_div(nq, QB)}));
+int survivor_room(int nq, int cap, int C) {
+  return std::max<int>(cap, (int)std::min<int64_t>(64 * C, ((int64_t)4 << 20) / 8 / nq));
+}
+
+int listed_rescan_splits(int64_t n, int nq, int QB, int C, int room) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>({room / C, 64, n / kTile / 4,
+                                                      (int64_t)num_sms() * 6 / ceil_div(nq, QB)}));
 }
 
 }  // namespace lshg

@@ -30,7 +30,8 @@
 namespace lshg {
 
 int launch_scan_bits_listed(const uint32_t* xst, int64_t n, int wp, int words, int sbytes, const uint32_t* qs, int nq,
-                            int op, int C, const int* list, uint64_t* out, cudaStream_t s);
+                            int op, int C, const int* list, uint64_t* out, uint64_t* scratch, int room,
+                            cudaStream_t s);
 
 namespace {
 
@@ -146,8 +147,10 @@ void launch_byte_filter_scan(const uint32_t* xsl_t, const uint32_t* xst, int64_t
   launch_slice_bytes(qs, nq, wp, nq, 0xFF, qsl.ptr, s);
   DevBuf<int> list((size_t)nq + 1, s);
   // match counts 0..4 wp (the padding bytes of a packed row never match)
-  sliced_filter_select<8>(xsl_t, n, ng, 4 * wp, qsl.ptr, nq, C, out, list.ptr, err, s);
-  launch_scan_bits_listed(xst, n, wp, (sbytes + 3) / 4, sbytes, qs, nq, OP_BYTE_JACCARD, C, list.ptr, out, s);
+  DevBuf<uint64_t> cand;
+  const int cap = sliced_filter_select<8>(xsl_t, n, ng, 4 * wp, qsl.ptr, nq, C, out, list.ptr, &cand, err, s);
+  launch_scan_bits_listed(xst, n, wp, (sbytes + 3) / 4, sbytes, qs, nq, OP_BYTE_JACCARD, C, list.ptr, out, cand.ptr, cap,
+                          s);
 }
 
 }  // namespace lshg

@@ -416,11 +416,11 @@ bool byte_filter_plan(int64_t n, int C, int* stride, int* rank, int* cap);
 // The whole threshold-filter selection over PL-plane sliced codes: prepass histograms,
 // thresholds, filter, exact integer select into out [nq][C].  Queries whose survivors are
 // fewer than C or overflow their array are listed in `list` (count, then query indices)
-// for the caller's exact rescan.  `samples` is the number of real samples a row (match
+// for the caller's exact rescan, which may use the survivors' arrays (returns their keys a query).  `samples` is the number of real samples a row (match
 // counts 0..samples).
 template <int PL>
-void sliced_filter_select(const uint32_t* base_t, int64_t n, int ng, int samples, const uint32_t* qsl, int nq, int C,
-                          uint64_t* out, int* list, int* err, cudaStream_t s) {
+int sliced_filter_select(const uint32_t* base_t, int64_t n, int ng, int samples, const uint32_t* qsl, int nq, int C,
+                         uint64_t* out, int* list, DevBuf<uint64_t>* survivors, int* err, cudaStream_t s) {
   int stride = 0, rank = 0, cap = 0;
   LSHG_REQUIRE(byte_filter_plan(n, C, &stride, &rank, &cap), "sliced filter scan: base too small for C");
   LSHG_REQUIRE(samples >= 1 && samples < sf::kMaxBins && samples <= 32 * ng, "sliced filter scan: bad sample count");
@@ -435,11 +435,14 @@ void sliced_filter_select(const uint32_t* base_t, int64_t n, int ng, int samples
   launch_hist_tau(hist.ptr, nq, bins, rank, tau.ptr, s);
   DevBuf<int> cnt((size_t)nq, s);
   LSHG_CUDA(cudaMemsetAsync(cnt.ptr, 0, cnt.bytes(), s));
-  DevBuf<uint64_t> cand((size_t)nq * cap, s);
+  DevBuf<uint64_t>& cand = *survivors;
+  const int room = survivor_room(nq, cap, C);
+  cand.alloc((size_t)nq * room, s);
   sf::run_pass<1, PL>(ng, base, n, qsl, nq, NT, 1, tau.ptr, nullptr, bins, cnt.ptr, cand.ptr, cap, err, s);
   LSHG_CUDA(cudaMemsetAsync(list, 0, sizeof(int), s));
   // scores are match counts 0..samples: the integer select with "bits" = samples
   tc::launch_int_select(cnt.ptr, cand.ptr, cap, (int)std::min<int64_t>(C, n), C, samples, nq, out, list, s);
+  return room;
 }
 
 }  // namespace lshg

@@ -73,7 +73,8 @@
 namespace lshg {
 
 int launch_scan_bits_listed(const uint32_t* xst, int64_t n, int wp, int words, int sbytes, const uint32_t* qs, int nq,
-                            int op, int C, const int* list, uint64_t* out, cudaStream_t s);
+                            int op, int C, const int* list, uint64_t* out, uint64_t* scratch, int room,
+                            cudaStream_t s);
 
 namespace tc {
 
@@ -1221,7 +1222,8 @@ void launch_tc_hamming(const uint8_t* xse, int64_t n, const uint32_t* xst, int w
     // scores are integers, computed the same way in both passes: no margin
     launch_tau_select(gmax.ptr, nq, plan.M, plan.rank, 0.0f, tau.ptr, s);
   }
-  DevBuf<uint64_t> cand((size_t)nq * plan.cap, s);
+  const int room = survivor_room(nq, plan.cap, C);
+  DevBuf<uint64_t> cand((size_t)nq * room, s);
   a.gmax = nullptr;
   a.M = 0;
   a.NP = plan.NT;
@@ -1233,7 +1235,7 @@ void launch_tc_hamming(const uint8_t* xse, int64_t n, const uint32_t* xst, int w
   run_hamming_kc<MODE_FILTER, HW>(kc, cl, ma, mb, a, "tc_hamming", s);
   launch_int_select(cnt, cand.ptr, plan.cap, (int)std::min<int64_t>(C, n), C, 32 * words, nq, out, ovf, s);
   // listed queries: exact popcount rescan written straight into their rows of `out`
-  launch_scan_bits_listed(xst, n, wp, words, 0, qs, nq, op, C, ovf, out, s);
+  launch_scan_bits_listed(xst, n, wp, words, 0, qs, nq, op, C, ovf, out, cand.ptr, room, s);
 }
 
 }  // namespace tc
