@@ -88,7 +88,7 @@ int64_t hamming_rows(int64_t n);
 void launch_expand_bits(const uint32_t* xs, int64_t n, int wp, int words, int64_t rows_pad, uint8_t* out,
                         cudaStream_t s);
 // Top-C keys [nq][C] of each query by (hamming asc, id asc); xse: the base's E2M1 rows
-// (launch_expand_bits, hamming_rows(n) of them), xst: the tiled sketches (listed rescans), qs:
+// (launch_expand_bits, hamming_rows(n) of them), xst: the tiled sketches (small batches, listed rescans), qs:
 // query sketches [nq][wp].  op: OP_HAMMING or OP_ONEBIT_JACCARD.
 void launch_tc_hamming(const uint8_t* xse, int64_t n, const uint32_t* xst, int wp, int words, const uint32_t* qs,
                        int nq, int op, int C, uint64_t* out, int* err, cudaStream_t s);

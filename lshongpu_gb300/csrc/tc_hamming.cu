@@ -89,6 +89,11 @@ constexpr int H_ACC_COL = 256;
 constexpr int H_SF_COL = HN;
 constexpr int H_MAX_CH = 36;      // base tiles a unit: 36 * 224 column offsets fit the staging's 13 bits
 constexpr int H_EPI_WARPS = 16;
+// Batches whose base tiles are expanded from packed sketches: those that leave half of the epilogue
+// warps without query rows to read.  They are bounded by the base's bytes where it does not fit in L2
+// (16 queries of 1,024 bits: 1.2M points, filter pass 97 -> 82 us, batch 185 -> 165; 400k, batch 163 ->
+// 145; 256 bits, 1.2M, 161 -> 151), and as fast either way where it does (100k: 87 and 87).
+constexpr int H_BITS_MAX_Q = 64;
 constexpr int H_SEL_MAX = 16384;  // survivor slots a query of a filtered base, at most
 constexpr int PN = 256;           // planes a tile of the projections' GEMM (UMMA N)
 constexpr int P_NACC = 2;         // its TMEM accumulators of PN columns
@@ -131,6 +136,8 @@ struct HArgs {
   uint64_t* cand;   // [nq][cap] survivor keys
   int cap;
   int* err;
+  const uint4* xst;  // BITS: the packed sketches, [ceil(n/128)][wq][128] 16-byte words
+  int wq;
 };
 
 // Survivor staging: a thread's entries lie BM words apart in its warpgroup's [SBUF][BM]
@@ -160,7 +167,21 @@ __device__ __noinline__ void h_flush(int* cnt, uint64_t* dst, int cap, uint32_t 
   }
 }
 
-template <int MODE, int GW, int KC, int CL>
+// A sketch word as the E2M1 values of its bits, sign bit = sketch bit: value j of word e is bit
+// 4 j + 3 - e.  Any order does, as long as queries and points have the same.
+__device__ __forceinline__ uint4 expand_word(uint32_t b) {
+  constexpr uint32_t S = 0x88888888u, ONE = 0x22222222u;
+  return make_uint4((b & S) | ONE, ((b << 1) & S) | ONE, ((b << 2) & S) | ONE, ((b << 3) & S) | ONE);
+}
+
+// BITS (CL = 1, batches of at most H_BITS_MAX_Q queries): the base tile is read as packed
+// sketches, a quarter of the E2M1 rows' bytes, and expanded into the ring by the epilogue warps
+// that have no query rows (TMEM lanes 64 and up): thread r takes row r, its next tile's words in
+// flight while this one's are expanded, and its 16-byte stores of a chunk fall into distinct banks
+// by the rows' swizzle.  Bounded by shared memory (114 KB written and 176 KB of operands read a
+// tile) and by the expanding warps' chain of wait, store, fence and arrive; a quarter of the stores
+// alone would take 27 us off the 82.
+template <int MODE, int GW, int KC, int CL, bool BITS>
 __global__ void __launch_bounds__(H_THREADS, 1)
     tc_hamming_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                       const HArgs a) {
@@ -169,6 +190,8 @@ __global__ void __launch_bounds__(H_THREADS, 1)
   constexpr int STAGES = LY::STAGES, SBUF = LY::SBUF;
   static_assert(MODE != MODE_FILTER || GW == HW, "the filter reads whole pieces");
   static_assert(GW == HW || GW == 8, "group width");
+  static_assert(!BITS || CL == 1, "one query tile");
+  constexpr int EPI_WARPS = BITS ? H_EPI_WARPS / 2 : H_EPI_WARPS;  // those with query rows
   const int U = a.NCH * a.QP;
   const int cid = blockIdx.x / CL, ncl = gridDim.x / CL;  // cluster, clusters
   if (cid >= U) return;  // no unit for this cluster: leave before any barrier or TMEM use
@@ -193,14 +216,14 @@ __global__ void __launch_bounds__(H_THREADS, 1)
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(FULL(s), 1);
+      mbar_init(FULL(s), BITS ? HN / 32 : 1);
       mbar_init(EMPTY(s), 1);
     }
     mbar_init(A_FULL, 1);
     mbar_init(A_EMPTY, 1);
     for (int b = 0; b < 2; ++b) {
       mbar_init(ACC_FULL(b), 1);
-      mbar_init(ACC_EMPTY(b), CL * H_EPI_WARPS);  // a pair's even CTA waits for both
+      mbar_init(ACC_EMPTY(b), CL * EPI_WARPS);  // a pair's even CTA waits for both
     }
     mbar_init(DONE, 1);
     *abort_flag = 0;
@@ -241,7 +264,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         // while those MMAs finish.  The query tile is reloaded once the previous unit's MMAs
         // have completed, and kept when the next unit has the same one.  (A tile past the
         // last one, where the query tiles do not fill the cluster, reads as zeros.)
-        const int total = (p1 - p0) * KC, pre = min(STAGES, total);
+        const int total = BITS ? 0 : (p1 - p0) * KC, pre = min(STAGES, total);
         for (int ci = 0; ci <= total; ++ci) {
           if (ci == pre && qp != have) {
             if (!mbar_wait(A_EMPTY, (na & 1) ^ 1, abort_flag)) { ok = false; break; }
@@ -327,6 +350,55 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     }
     // drain: all issued MMAs complete before TMEM is released
     mbar_wait(DONE, 0, abort_flag, true);
+    __syncwarp();
+  } else if (BITS && warp >= 4 && (warp & 2)) {
+    // ---------------- expansion of the base tiles' words ----------------
+    const int r = (((warp - 4) >> 2) * 2 + (warp & 1)) * 32 + lane;  // row of the tile
+    if (r < HN) {  // warp-uniform: HN / 32 of the eight warps
+      uint4 w[2 * KC];
+      auto fetch = [&](int p, int i) {
+        const int64_t row = (int64_t)p * a.dstride * HN + r;
+        w[i] = row < a.n && i < a.wq ? __ldg(a.xst + ((row >> 7) * a.wq + i) * 128 + (row & 127)) : make_uint4(0, 0, 0, 0);
+      };
+      auto first = [&](int u) { return u / a.QP * a.CH; };
+#pragma unroll
+      for (int i = 0; i < 2 * KC; ++i) fetch(first(cid), i);
+      int st = 0;
+      uint32_t ph = 1;
+      bool ok = true;
+      for (int u = cid; u < U && ok; u += ncl) {
+        const int p0 = first(u), p1 = min(a.NP, p0 + a.CH);
+        for (int p = p0; p < p1 && ok; ++p) {
+          const int next = p + 1 < p1 ? p + 1 : u + ncl < U ? first(u + ncl) : -1;
+#pragma unroll
+          for (int kc = 0; kc < KC; ++kc) {
+            if (!mbar_wait_warp(EMPTY(st), ph, abort_flag)) { ok = false; break; }
+            const uint32_t dst = s0 + LY::B_OFF + st * LY::B_BYTES + (uint32_t)r * H_CHUNK;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const uint4 c = w[2 * kc + i];
+              if (next >= 0) fetch(next, 2 * kc + i);
+              const uint32_t bits[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const uint4 o = expand_word(bits[e]);
+                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(
+                                 dst + (uint32_t)(((4 * i + e) ^ (r & 7)) * 16)),
+                             "r"(o.x), "r"(o.y), "r"(o.z), "r"(o.w)
+                             : "memory");
+              }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMAs read what was stored
+            __syncwarp();
+            if (lane == 0) mbar_arrive(FULL(st));
+            if (++st == STAGES) {
+              st = 0;
+              ph ^= 1u;
+            }
+          }
+        }
+      }
+    }
     __syncwarp();
   } else if (warp >= 4) {
     // ---------------- epilogue ----------------
@@ -646,9 +718,9 @@ __global__ void __launch_bounds__(H_THREADS, 1)
   if (threadIdx.x == 0) a.list_cnt[blockIdx.x] = *reinterpret_cast<int*>(tmem_slot + 2);
 }
 
-// Sketch rows of wp words (the first `words` real) -> E2M1 rows of kp bytes: bit b of word w
-// (LSB first) -> nibble 32w + b (low nibble first) = 0x2 (+1) for a 0 bit, 0xA (-1) for a 1
-// bit; nibbles past 32 * words and rows past n are 0x0.  One thread writes a word's 16 bytes.
+// Sketch rows of wp words (the first `words` real) -> E2M1 rows of kp bytes: 16 bytes a word
+// (expand_word), 0x2 (+1) for a 0 bit, 0xA (-1) for a 1 bit; nibbles past 32 * words and rows past n
+// are 0x0.
 __global__ void expand_bits_kernel(const uint32_t* __restrict__ xs, int64_t n, int wp, int words, int kp,
                                    int64_t rows_pad, uint4* __restrict__ out) {
   grid_ready();
@@ -658,19 +730,7 @@ __global__ void expand_bits_kernel(const uint32_t* __restrict__ xs, int64_t n, i
     const int64_t i = t / per_row;
     const int w = (int)(t - i * per_row);
     uint4 o = make_uint4(0, 0, 0, 0);
-    if (i < n && w < words) {
-      const uint32_t bits = xs[i * wp + w];
-      uint32_t r[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        uint32_t b = (bits >> (8 * e)) & 0xFFu;  // bit j of the byte -> bit 3 of nibble j (the sign of +-1.0)
-        b = (b | (b << 12)) & 0x000F000Fu;
-        b = (b | (b << 6)) & 0x03030303u;
-        b = (b | (b << 3)) & 0x11111111u;
-        r[e] = 0x22222222u | (b << 3);
-      }
-      o = make_uint4(r[0], r[1], r[2], r[3]);
-    }
+    if (i < n && w < words) o = expand_word(xs[i * wp + w]);
     out[t] = o;
   }
 }
@@ -909,7 +969,7 @@ CUtensorMap map_sketch_rows(const void* base, int64_t rows, int kp, int box_rows
   return make_map_bytes(base, rows, kp, box_rows);
 }
 
-template <int MODE, int GW, int KC, int CL>
+template <int MODE, int GW, int KC, int CL, bool BITS>
 void run_hamming(const CUtensorMap& ma, const CUtensorMap& mb, HArgs a, const char* name, cudaStream_t s) {
   // units: long enough to amortise the query tile's reload, at least 8 a cluster
   const int G = std::max(1, num_sms() / CL);
@@ -918,7 +978,7 @@ void run_hamming(const CUtensorMap& ma, const CUtensorMap& mb, HArgs a, const ch
   a.CH = (int)std::max<int64_t>(1, std::min<int64_t>(H_MAX_CH, (work + 8 * G - 1) / (8 * G)));
   a.NCH = ceil_div(a.NP, a.CH);
   const int grid = CL * std::min(G, a.NCH * a.QP);
-  auto kern = tc_hamming_kernel<MODE, GW, KC, CL>;
+  auto kern = tc_hamming_kernel<MODE, GW, KC, CL, BITS>;
   constexpr int smem = HLayout<KC, CL>::SMEM;
   LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   cudaLaunchConfig_t cfg{};
@@ -940,19 +1000,24 @@ void run_hamming(const CUtensorMap& ma, const CUtensorMap& mb, HArgs a, const ch
   count_launch();
 }
 
-// cl: CTAs a cluster; mb's boxes hold a CTA's share of a base tile (HN / cl rows).
+// cl: CTAs a cluster (1 when a.xst is set); mb's boxes hold a CTA's share of a base tile (HN / cl rows).
 template <int MODE, int GW>
 void run_hamming_kc(int kc, int cl, const CUtensorMap& ma, const CUtensorMap& mb, const HArgs& a, const char* name,
                     cudaStream_t s) {
-  switch (kc * 2 + (cl - 1)) {
-    case 2: run_hamming<MODE, GW, 1, 1>(ma, mb, a, name, s); break;
-    case 3: run_hamming<MODE, GW, 1, 2>(ma, mb, a, name, s); break;
-    case 4: run_hamming<MODE, GW, 2, 1>(ma, mb, a, name, s); break;
-    case 5: run_hamming<MODE, GW, 2, 2>(ma, mb, a, name, s); break;
-    case 6: run_hamming<MODE, GW, 3, 1>(ma, mb, a, name, s); break;
-    case 7: run_hamming<MODE, GW, 3, 2>(ma, mb, a, name, s); break;
-    case 8: run_hamming<MODE, GW, 4, 1>(ma, mb, a, name, s); break;
-    case 9: run_hamming<MODE, GW, 4, 2>(ma, mb, a, name, s); break;
+  const int form = a.xst ? 2 : cl - 1;
+  switch (kc * 3 + form) {
+    case 3: run_hamming<MODE, GW, 1, 1, false>(ma, mb, a, name, s); break;
+    case 4: run_hamming<MODE, GW, 1, 2, false>(ma, mb, a, name, s); break;
+    case 5: run_hamming<MODE, GW, 1, 1, true>(ma, mb, a, name, s); break;
+    case 6: run_hamming<MODE, GW, 2, 1, false>(ma, mb, a, name, s); break;
+    case 7: run_hamming<MODE, GW, 2, 2, false>(ma, mb, a, name, s); break;
+    case 8: run_hamming<MODE, GW, 2, 1, true>(ma, mb, a, name, s); break;
+    case 9: run_hamming<MODE, GW, 3, 1, false>(ma, mb, a, name, s); break;
+    case 10: run_hamming<MODE, GW, 3, 2, false>(ma, mb, a, name, s); break;
+    case 11: run_hamming<MODE, GW, 3, 1, true>(ma, mb, a, name, s); break;
+    case 12: run_hamming<MODE, GW, 4, 1, false>(ma, mb, a, name, s); break;
+    case 13: run_hamming<MODE, GW, 4, 2, false>(ma, mb, a, name, s); break;
+    case 14: run_hamming<MODE, GW, 4, 1, true>(ma, mb, a, name, s); break;
     default: throw Error(LSHG_ERR_INVALID_ARGUMENT, "tensor-core sketch scan: rows of 1..4 chunks of 256 bits");
   }
 }
@@ -1210,6 +1275,10 @@ void launch_tc_hamming(const uint8_t* xse, int64_t n, const uint32_t* xst, int w
   a.QT = QT;
   a.ksteps = (words + 1) / 2;
   a.err = err;
+  if (nq <= H_BITS_MAX_Q) {
+    a.xst = reinterpret_cast<const uint4*>(xst);
+    a.wq = wp / 4;
+  }
   DevBuf<float> tau(nq, s);
   if (plan.M > 0) {
     DevBuf<float> gmax((size_t)nq * plan.M, s);
