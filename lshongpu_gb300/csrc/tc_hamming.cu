@@ -24,9 +24,9 @@
 //   filter   on the whole base keeps the points whose score reaches tau[q], staged per row
 //            in shared memory and moved to the query's candidate array with one atomicAdd
 //            a batch;
-//   select   keeps each query's first C survivors by (score desc, id asc): a warp sort for
-//            C <= 128, bisection over the integer scores and over the ids at the C-th score
-//            beyond.
+//   select   keeps each query's first C survivors by (score desc, id asc): bisection
+//            over the integer scores and over the ids at the C-th score by a block, or a warp
+//            sort for C <= 128 and many queries.
 //            A query with fewer than C survivors (tau above its C-th best score: the
 //            sample was unrepresentative) or more than its array holds (massive ties) is
 //            listed and rescanned exactly by the popcount scan on the device, so the result
@@ -1232,7 +1232,11 @@ void launch_int_select(const int* cnt, const uint64_t* cand, int cap, int need, 
                        int* ovf, cudaStream_t s) {
   ProfScope _ps("tc_hamming_select", s);
   LSHG_REQUIRE(bits >= 1 && 2 * bits + 1 <= H_BINS_MAX, "integer select: scores of at most 1024 bits");
-  if (C <= 128) {
+  // Short lists: a warp a query, or a block while every query's block is resident at once (6 an SM).  A
+  // warp's chain of sorts is the longer one; blocks pay their barriers where the grid is full.  Batch
+  // over 20,000 x 256 bits, C = 128, warps and blocks: 16 queries 79 and 70 us, 300 101 and 90, 1,000
+  // 120 and 117, 5,000 262 and 261 (C = 32: 190 and 208).
+  if (C <= 128 && nq > 6 * num_sms()) {
     if (C == 32) launch_next(hsel_warp_kernel<1>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out, ovf);
     else if (C == 64) launch_next(hsel_warp_kernel<2>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out, ovf);
     else launch_next(hsel_warp_kernel<4>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out, ovf);

@@ -362,3 +362,13 @@ def test_listed_rescans_split_over_the_base(engine, impl, words, C):
     res = [engine.Index(x, options=engine.make_options(candidates=C, sketch_scan=mode), **kw).query(q, 32)
            for mode in (TENSOR, POPCOUNT)]
     assert np.array_equal(res[0], res[1])
+
+
+@pytest.mark.parametrize("nq", [3, 1500])
+@pytest.mark.parametrize("C", [32, 64, 128])
+def test_sketch_scan_short_lists_by_block_and_by_warp(engine, nq, C):
+    x, q = data(20000, nq)
+    res = [engine.Index(x, implementation=3, sketchDim=4,
+                        options=engine.make_options(candidates=C, sketch_scan=mode)).query(q, 32)
+           for mode in (TENSOR, POPCOUNT)]
+    assert np.array_equal(res[0], res[1])
