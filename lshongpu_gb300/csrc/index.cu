@@ -23,7 +23,7 @@ namespace lshg {
 // 128-query tile is mostly padding for a few queries, but the scan then costs little more than
 // reading the base once, where the popcount scan folds each query's candidates by itself.
 // Measured, popcount against tensor cores: 1.2M x 1,024 bits, C = 128: one query 325 / 199 us, 16
-// 1,141 / 214; C = 1,024: one 827 / 203, 63 3,061 / 231; 10k points, C = 128: one 95 / 100, four
+// 1,141 / 156; C = 1,024: one 827 / 203, 63 3,061 / 231; 10k points, C = 128: one 95 / 100, four
 // 106 / 107, 16 155 / 114; C = 1,024: one 180 / 94.
 constexpr int kTcSketchLongList = 128;       // candidates above which every batch takes it
 constexpr int64_t kTcSketchMinPairs = 65536; // (query, point) pairs from which every list does
@@ -32,6 +32,11 @@ constexpr int64_t kTcSketchMinPairs = 65536; // (query, point) pairs from which 
 // filter, 256 samples: 500k points, C = 4,096: one query 1,339 / 341 us, 64 2,301 / 450; C = 128:
 // one 334 / 313, 64 1,374 / 388; 10k points: C = 128 one 114 / 114, C = 32 one 102 / 114, 16 215 / 175.
 constexpr int64_t kByteFilterMinPairs = 16384;
+// SimHash signs of a batch up to which one SIMT kernel is shorter than the tensor cores' chain of
+// five (split, product, recheck, its fallback, and a memset).  Batch on 20,000 points, chain and
+// SIMT: 1,024 planes: one query 77 / 60 us, 300 148 / 129, 1,000 159 / 147, 1,500 159 / 163, 5,000 303
+// / 332; 256 planes: 300 109 / 97, 5,000 271 / 265.
+constexpr int64_t kSignsMinSigns = 1 << 20;
 bool tensor_sketch_batch(int64_t n, int nq, int C) {
   return C > kTcSketchLongList || (int64_t)nq * n >= kTcSketchMinPairs;
 }
@@ -198,7 +203,8 @@ void make_sketch(const Index& idx, const float* v, int64_t rows, uint8_t padbyte
   switch (idx.sk_kind) {
     case 3: {
       DevBuf<uint32_t> raw(rows * idx.words, s);
-      if (idx.sk_split.ptr)  // tensor cores, bit-identical (exact recheck of the near-zero signs)
+      if (idx.sk_split.ptr && rows * idx.words * 32 > kSignsMinSigns)
+        // tensor cores, bit-identical (exact recheck of the near-zero signs)
         tc::launch_tc_signs(v, rows, d, idx.sk_split.ptr, idx.sk_pnorm.ptr, idx.sk_planes.ptr, idx.words * 32,
                             idx.words, raw.ptr, err, s);
       else

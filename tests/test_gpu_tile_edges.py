@@ -372,3 +372,11 @@ def test_sketch_scan_short_lists_by_block_and_by_warp(engine, nq, C):
                         options=engine.make_options(candidates=C, sketch_scan=mode)).query(q, 32)
            for mode in (TENSOR, POPCOUNT)]
     assert np.array_equal(res[0], res[1])
+
+
+@pytest.mark.parametrize("nq", [1, 1024, 1025])  # the largest batch of SIMT signs at 32 words, the smallest beyond
+def test_simhash_signs_by_batch_size_equal_oracle(engine, orc, nq):
+    x, q = data(3000, nq)
+    idx = engine.Index(x, implementation=3, sketchDim=32)
+    sk, _ = idx.sketch_queries(q, np.uint32, 32)
+    assert np.array_equal(sk, orc.simhash(q, engine.random_normals(D * 32 * 32), 32, 32))
