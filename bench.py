@@ -224,14 +224,16 @@ def algorithmic(path: str, prof: dict, nq: int, lsh_counts=None):
     if path == "wmh1":
         return "scan_bits", "popc", nq * N_BASE * 8 / 1e9, "Gword/s"
     # LSH gather: bytes the query kernel must move -- every bucket entry walked (4 B id),
-    # every distinct candidate's row and norm, the queries and the results -- from the
-    # kernel's own counters over the timed launches
+    # every distinct candidate's 8-bit row with its scale and residual, the FP32 rows of at
+    # least the results, the queries and the results -- from the kernel's own counters over the
+    # timed launches
     if lsh_counts is None:
         return "lsh_query", "gather", None, None
     entries, distinct = lsh_counts
     dims = d + PAD_DIM
     return ("lsh_query", "gather",
-            (entries * 4 + distinct * (4 * dims + 4) + nq * (4 * dims + 8 * K)) / 1e9, "GB/s")
+            (entries * 4 + distinct * (-(-dims // 16) * 16 + 8 + 4) +
+             nq * (K * (4 * dims + 4) + 4 * dims + 8 * K)) / 1e9, "GB/s")
 
 
 def dram_traffic(kernel: str, workload: str):
@@ -365,7 +367,7 @@ def workload_text(args) -> str:
     data = ("sparse Gamma(2,1) values, 30% nonzero" if DATA == "sparse"
             else "clustered unit vectors (1000 clusters, sigma 0.05)")
     what = {"tc": "tensor-core exact scan", "tc8": "tensor-core exact scan, E4M3 (FP8) scores",
-            "exact": "FP32 SIMT exact scan",
+            "exact": "exact scan, FP32 distances",
             "simhash": f"1024-bit SimHash, {CAND} candidates re-ranked",
             "cplsh": f"cross-polytope LSH, L={CP_TABLES}, K={CP_HASHES}, 3 rounds, exact angular on candidates",
             "wmh": "weighted MinHash, 256 byte samples, Jaccard scan + generalized-Jaccard re-rank",

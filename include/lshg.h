@@ -100,9 +100,9 @@ typedef struct lshg_options_s {
                             re-ranked scan (3-6, 8, 9).  The exact scan (2) returns the
                             reference's FP32 order. */
   int sketch_scan;       /* Hamming / one-bit Jaccard sketch scans (3, 5) with rows of at most
-                            1024 bits: 0 (default) = tensor cores for batches of 64 queries or
-                            more, XOR/popcount otherwise; 1 = always XOR/popcount (and no E4M3
-                            copy of the sketches is kept); 2 = tensor cores whenever the base
+                            1024 bits: 0 (default) = tensor cores, but for a few queries on
+                            candidate lists of at most 128 in a small base; 1 = always
+                            XOR/popcount (and no expanded copy of the sketches is kept); 2 = tensor cores whenever the base
                             allows.  Both give the same candidates (ties: lower index). */
 } lshg_options;
 

@@ -205,7 +205,8 @@ void launch_row_norms(const float* x, int64_t n, int d, float* norms, cudaStream
   size_t smem = staged_smem(kRowsPerBlock, d);
   LSHG_REQUIRE(smem <= 200 * 1024, "dimension too large for row_norms");
   LSHG_CUDA(cudaFuncSetAttribute(row_norm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  launch_next(row_norm_kernel<false>, ceil_div(n, kRowsPerBlock), kNormThreads, smem, s, const_cast<float*>(x), n, d, norms);
+  launch_next(row_norm_kernel<false>, ceil_div(n, kRowsPerBlock), kNormThreads, smem, s, const_cast<float*>(x), n, d,
+              norms);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

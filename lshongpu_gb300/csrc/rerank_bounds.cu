@@ -424,7 +424,8 @@ void launch_bounds(const uint64_t* cand, const int* list, int list_cap, const in
   constexpr int smem = C * (int)sizeof(uint32_t);
   auto kern = bounds_kernel<DIST, C, LIST>;
   LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  launch_next(kern, nq, kBoundThreads, smem, s, cand, list, list_cap, ccnt, rows, tails, pitch, scale, n, d, q, k, kept, listed);
+  launch_next(kern, nq, kBoundThreads, smem, s, cand, list, list_cap, ccnt, rows, tails, pitch, scale, n, d, q, k,
+              kept, listed);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

@@ -1,5 +1,4 @@
-// Threshold-filter scan of byte weighted-MinHash samples (implementation 4) for long
-// candidate lists: the reference's scanJaccardDistance (sketchedDistanceScanners.cuh:
+// Threshold-filter scan of byte weighted-MinHash samples (implementation 4): the reference's scanJaccardDistance (sketchedDistanceScanners.cuh:
 // 194-274) with the byte distance 1 - (#equal samples) / sketchDim (distanceFunctions.cuh:
 // 102-116).
 //

@@ -305,7 +305,8 @@ bool query_jaccard_filtered(Index& I, const float* q, int nq, int k, lshg_point*
       count_launch();
       LSHG_CHECK_LAUNCH();
     }
-    launch_next(list_hard_kernel, ceil_div(nq, 8), 256, 0, s, cnt, bad, nq, (int)std::min<int64_t>(k, I.n), cap, cand.ptr, list);
+    launch_next(list_hard_kernel, ceil_div(nq, 8), 256, 0, s, cnt, bad, nq, (int)std::min<int64_t>(k, I.n), cap,
+                cand.ptr, list);
     count_launch();
     LSHG_CHECK_LAUNCH();
     launch_rerank(cand.ptr, nq, cap, I.x.ptr, I.n, I.d, nullptr, q, nullptr, DIST_JACCARD, k, out, s, I.error_word(s));

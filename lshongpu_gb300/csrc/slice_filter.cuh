@@ -377,7 +377,8 @@ void run_ng(const uint4* xst, int64_t n, const uint32_t* qsl, int nq, int NP, in
   const int chunk = big ? (int)std::max<int64_t>(8, std::min<int64_t>(64, items / (slots * 24))) : 0;
   const int64_t total = chunk ? (int64_t)ceil_div(nq, kBQ) * ceil_div(NP, chunk) : items;  // units or items
   const int grid = (int)std::min<int64_t>(total, slots);
-  launch_next(kern, grid, kBThreads, smem, s, xst, n, qsl, nq, NP, tstride, chunk, tau, hist, bins, cnt, cand, cap, err);
+  launch_next(kern, grid, kBThreads, smem, s, xst, n, qsl, nq, NP, tstride, chunk, tau, hist, bins, cnt, cand, cap,
+              err);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

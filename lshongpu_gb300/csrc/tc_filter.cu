@@ -11,7 +11,7 @@
 //   pass 1 (MODE_FILTER) runs on the whole base.  The epilogue compares each score with
 //     its row's tau; the (rare) survivors are staged per row in shared memory and moved
 //     to the query's candidate array in global memory with one atomicAdd a batch (at the
-//     end of each work unit, or when the 8-entry staging is full).  There is no per-row
+//     end of each work unit, or when the 16-entry staging is full).  There is no per-row
 //     selection state on chip, so the common case is a 64-wide maximum and a warp vote.
 //
 // cand_select_kernel then sorts each query's survivors and keeps the first CT keys
@@ -903,9 +903,12 @@ void launch_tau_select(const float* gmax, int nq, int M, int rank, float margin,
 void launch_cand_select(const int* cnt, const uint64_t* cand, int nq, int cap, int need, int CT, uint64_t* out,
                         int* ovf, const uint16_t* rows, uint16_t* gathered, cudaStream_t s) {
   ProfScope _ps("tc_cand_select", s);
-  if (CT == 32) launch_next(cand_select_kernel<1>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out, ovf, rows, gathered);
-  else if (CT == 64) launch_next(cand_select_kernel<2>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out, ovf, rows, gathered);
-  else if (CT == 128) launch_next(cand_select_kernel<4>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out, ovf, rows, gathered);
+  if (CT == 32) launch_next(cand_select_kernel<1>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out, ovf,
+                            rows, gathered);
+  else if (CT == 64) launch_next(cand_select_kernel<2>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out,
+                                 ovf, rows, gathered);
+  else if (CT == 128) launch_next(cand_select_kernel<4>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, need, nq, out,
+                                  ovf, rows, gathered);
   else throw Error(LSHG_ERR_INVALID_ARGUMENT, "tensor-core scan: candidate count must be 32, 64 or 128");
   count_launch();
   LSHG_CHECK_LAUNCH();
@@ -914,8 +917,10 @@ void launch_cand_select(const int* cnt, const uint64_t* cand, int nq, int cap, i
 void launch_exact_select(const int* cnt, const uint64_t* cand, int nq, int cap, int k, int CT, const float* tau,
                          const float* eps, uint64_t* out, int* ovf, cudaStream_t s) {
   ProfScope _ps("exact_select", s);
-  if (CT == 128) launch_next(exact_select_kernel<4>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, k, nq, tau, eps, out, ovf);
-  else if (CT == 256) launch_next(exact_select_kernel<8>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, k, nq, tau, eps, out, ovf);
+  if (CT == 128) launch_next(exact_select_kernel<4>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, k, nq, tau, eps,
+                             out, ovf);
+  else if (CT == 256) launch_next(exact_select_kernel<8>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, k, nq, tau,
+                                  eps, out, ovf);
   else throw Error(LSHG_ERR_INVALID_ARGUMENT, "exact scan: candidate count must be 128 or 256");
   count_launch();
   LSHG_CHECK_LAUNCH();

@@ -1152,7 +1152,8 @@ void launch_tc_signs(const float* x, int64_t n, int d, const uint16_t* planes_sp
   {
     const int64_t total = (int64_t)grid * cap;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, (int64_t)G * 16));
-    launch_next(sign_recheck_kernel, blocks, 256, 0, s, list.ptr, cnt.ptr, cap, grid, x, planes, d, out32, words, overflow);
+    launch_next(sign_recheck_kernel, blocks, 256, 0, s, list.ptr, cnt.ptr, cap, grid, x, planes, d, out32, words,
+                overflow);
     count_launch();
     LSHG_CHECK_LAUNCH();
   }

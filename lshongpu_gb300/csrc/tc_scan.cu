@@ -426,7 +426,8 @@ void to_unit_e4m3(const float* x, int64_t n, int d, int64_t rows_pad, uint8_t* o
 void to_unit_bf16(const float* x, int64_t n, int d, int64_t rows_pad, uint16_t* out, cudaStream_t s) {
   int64_t warps = rows_pad;
   int blocks = (int)std::min<int64_t>((warps * 32 + 255) / 256, (int64_t)num_sms() * 16);
-  launch_next(to_unit_bf16_kernel, std::max(blocks, 1), 256, 0, s, x, n, d, rows_pad, reinterpret_cast<__nv_bfloat16*>(out));
+  launch_next(to_unit_bf16_kernel, std::max(blocks, 1), 256, 0, s, x, n, d, rows_pad,
+              reinterpret_cast<__nv_bfloat16*>(out));
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
