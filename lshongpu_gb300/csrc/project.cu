@@ -35,14 +35,24 @@ __global__ void __launch_bounds__(256) project_kernel(const float* __restrict__ 
   const int np = (int)imin<int64_t>(kTP, n - p0);
   const int nl = min(kTL, nplanes - l0);
 
-  for (int i = threadIdx.x; i < kTP * d; i += blockDim.x) {
-    int p = i / d, j = i - p * d;
-    xs[j * kPitch + p] = (p < np) ? x[(p0 + p) * d + j] : 0.0f;
-  }
-  for (int i = threadIdx.x; i < kTL * d; i += blockDim.x) {
-    int l = i / d, j = i - l * d;
-    rs[j * kPitch + l] = (l < nl) ? planes[(int64_t)(l0 + l) * d + j] : 0.0f;
-  }
+  // rows are contiguous: eight loads of a thread in flight, then their transposed stores (one after the
+  // other they were most of a small batch's 21 us)
+  auto stage = [&](const float* src, int rows, float* dst) {
+    const int have = rows * d, all = kTP * d;
+    for (int i0 = threadIdx.x; i0 < all; i0 += 8 * 256) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = i0 + 256 * u < have ? src[i0 + 256 * u] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int i = i0 + 256 * u, r = i / d;
+        if (i < all) dst[(i - r * d) * kPitch + r] = v[u];
+      }
+    }
+  };
+  static_assert(kTP == kTL, "one staging form");
+  stage(x + p0 * d, np, xs);
+  stage(planes + (int64_t)l0 * d, nl, rs);
   __syncthreads();
 
   const int tl = threadIdx.x & 15;  // planes 4*tl .. 4*tl+3
