@@ -72,7 +72,7 @@ void tile_sketches(Index& I, cudaStream_t s) {
   if ((I.sk_kind == 3 || I.sk_kind == 5) && I.words <= 32 && I.p.opt.sketch_scan != 1) {
     const int64_t rows = tc::hamming_rows(I.n);
     I.xse.alloc((size_t)rows * 128 * tc::hamming_chunks(I.words), s);
-    tc::launch_expand_bits(I.xs.ptr, I.n, I.wp, I.words, rows, I.xse.ptr, s);
+    tc::launch_expand_bits(I.xs.ptr, I.n, I.wp, I.words, rows, I.xse.ptr, nullptr, 0, s);
   }
 }
 

@@ -19,6 +19,13 @@ namespace lshg {
 
 __device__ __forceinline__ void grid_ready() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Counters of a later kernel, zeroed by the first kernel of a batch: a memset of its own costs an ordinary
+// launch's gaps on both sides (5 us).
+__device__ __forceinline__ void zero_counters(int* c, int n) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) c[i] = 0;
+}
+
 template <typename... P, typename... A>
 void launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
   cudaLaunchConfig_t cfg{};

@@ -48,8 +48,9 @@ constexpr float kScoreSlack = 8e-5f;
 // row against a base of largest residual *base_res, infinite for a row out of range.
 __global__ void unit_rows_kernel(const float* __restrict__ x, int64_t n, int d, int64_t rows_pad,
                                  __nv_bfloat16* __restrict__ out, unsigned* stat, const float* base_res,
-                                 float* __restrict__ eps) {
+                                 float* __restrict__ eps, int* counters, int ncounters) {
   grid_ready();
+  zero_counters(counters, ncounters);
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -95,10 +96,10 @@ __global__ void unit_rows_kernel(const float* __restrict__ x, int64_t n, int d, 
 }
 
 void launch_unit_rows(const float* x, int64_t n, int d, int64_t rows_pad, uint16_t* out, unsigned* stat,
-                      const float* base_res, float* eps, cudaStream_t s) {
+                      const float* base_res, float* eps, int* counters, int ncounters, cudaStream_t s) {
   const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((rows_pad * 32 + 255) / 256, (int64_t)num_sms() * 8));
-  launch_next(unit_rows_kernel, blocks, 256, 0, s, x, n, d, rows_pad, reinterpret_cast<__nv_bfloat16*>(out), stat, base_res,
-                                          eps);
+  launch_next(unit_rows_kernel, blocks, 256, 0, s, x, n, d, rows_pad, reinterpret_cast<__nv_bfloat16*>(out), stat,
+              base_res, eps, counters, ncounters);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -130,7 +131,7 @@ void derive_exact(Index& I, cudaStream_t s) {
   }
   LSHG_CUDA(cudaMemsetAsync(I.ebf_res.ptr, 0, I.ebf_res.bytes(), s));
   unsigned* stat = reinterpret_cast<unsigned*>(I.ebf_res.ptr);
-  launch_unit_rows(I.x.ptr, I.n, I.d, npad, I.ebf.ptr, stat, nullptr, nullptr, s);
+  launch_unit_rows(I.x.ptr, I.n, I.d, npad, I.ebf.ptr, stat, nullptr, nullptr, nullptr, 0, s);
   LSHG_CUDA(cudaMemcpyAsync(&bad, stat + 1, sizeof(bad), cudaMemcpyDeviceToHost, s));
   LSHG_CUDA(cudaStreamSynchronize(s));
   if (bad) I.ebf.release();
@@ -154,8 +155,7 @@ bool query_exact_filtered(Index& I, const float* q, int nq, int k, lshg_point* o
     DevBuf<uint64_t> cand((size_t)nq * std::max(plan.cap, 1), s), best((size_t)nq * CT, s);
     DevBuf<uint64_t> part((size_t)nq * splits * C, s);
     int* ovf = cnt.ptr + nq;
-    LSHG_CUDA(cudaMemsetAsync(cnt.ptr, 0, (size_t)(nq + 1) * sizeof(int), s));
-    launch_unit_rows(q, nq, I.d, qpad, qbf.ptr, nullptr, I.ebf_res.ptr, eps.ptr, s);
+    launch_unit_rows(q, nq, I.d, qpad, qbf.ptr, nullptr, I.ebf_res.ptr, eps.ptr, cnt.ptr, nq + 1, s);
     const FilterMaps maps = make_filter_maps(qbf.ptr, qpad, I.ebf.ptr, npad, I.d, false);
     launch_filter_scan(maps, plan, nq, I.n, I.d, (int)(qpad / BM), tau.ptr, cnt.ptr, cand.ptr, I.error_word(s), s,
                        eps.ptr);
@@ -163,7 +163,8 @@ bool query_exact_filtered(Index& I, const float* q, int nq, int k, lshg_point* o
                         plan.M > 0 ? tau.ptr : nullptr, eps.ptr, best.ptr, ovf, s);
     launch_rerank(best.ptr, nq, CT, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, nullptr, DIST_ANGULAR, k, out, s,
                   I.error_word(s), false, nullptr, nullptr, qnorm.ptr);
-    launch_scan_float_listed(I.xt.ptr, I.n, I.d, I.xnorm.ptr, q, nq, qnorm.ptr, DIST_ANGULAR, ovf, C, splits, part.ptr, k, out, s);
+    launch_scan_float_listed(I.xt.ptr, I.n, I.d, I.xnorm.ptr, q, nq, qnorm.ptr, DIST_ANGULAR, ovf, C, splits, part.ptr,
+                             k, out, s);
   } catch (const Error& e) {
     if (e.status != LSHG_ERR_OUT_OF_MEMORY) throw;
     cudaGetLastError();  // temporaries that do not fit: the FP32 scan needs fewer

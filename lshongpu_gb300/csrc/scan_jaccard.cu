@@ -62,8 +62,9 @@ __device__ __forceinline__ float delta(int d) { return (2.0f * d + 7.0f) * 1.2e-
 template <int ROWS, int THREADS>
 __global__ void __launch_bounds__(THREADS)
     code_tiles_kernel(const float* __restrict__ x, int64_t n, int d, int wd, float lo, float s,
-                      uint32_t* __restrict__ out, float4* __restrict__ tails, int* __restrict__ bad) {
+                      uint32_t* __restrict__ out, float4* __restrict__ tails, int* __restrict__ bad, int* counters, int ncounters) {
   grid_ready();
+  zero_counters(counters, ncounters);
   extern __shared__ uint32_t rows[];  // [ROWS][wd | 1]
   const int pitch = wd | 1, lane = threadIdx.x & 31;
   const int64_t row0 = (int64_t)blockIdx.x * ROWS;
@@ -253,7 +254,7 @@ void derive_jaccard_scan(Index& I, cudaStream_t s) {
   I.jq_scale = 255.0f / std::max(hi - lo, 1e-6f * hi);
   const size_t smem = tile_smem(wd, kTile);
   launch_next(code_tiles_kernel<kTile, 256>, tiles, 256, smem, s, I.x.ptr, I.n, I.d, wd, I.jq_lo, I.jq_scale, I.jq.ptr,
-              I.jq_tail.ptr, nullptr);
+              I.jq_tail.ptr, nullptr, nullptr, 0);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -271,14 +272,13 @@ bool query_jaccard_filtered(Index& I, const float* q, int nq, int k, lshg_point*
   try {
     DevBuf<uint32_t> qt((size_t)qblocks * wd * kQB, s);
     DevBuf<float4> qtail((size_t)qblocks * kQB, s);
-    DevBuf<int> ctl((size_t)3 * nq + 1, s);  // [0, nq): candidates; [nq, 2 nq): no bounds; then count and list
+    DevBuf<int> ctl((size_t)3 * nq + 1, s);  // [0, nq): candidates; [nq]: listed, then their list; then no bounds
     DevBuf<float> gmax((size_t)nq * 4 * stiles, s), tau((size_t)nq, s);
     DevBuf<uint64_t> cand((size_t)nq * cap, s), part((size_t)nq * lsplits * C, s);
-    int *cnt = ctl.ptr, *bad = ctl.ptr + nq, *list = ctl.ptr + 2 * nq;
-    LSHG_CUDA(cudaMemsetAsync(ctl.ptr, 0, ctl.bytes(), s));
+    int *cnt = ctl.ptr, *list = ctl.ptr + nq, *bad = ctl.ptr + 2 * nq + 1;
     const size_t qsm = tile_smem(wd, kQB);
-    launch_next(code_tiles_kernel<kQB, 1024>, qblocks, 1024, qsm, s, q, nq, I.d, wd, I.jq_lo, I.jq_scale, qt.ptr, qtail.ptr,
-                bad);
+    launch_next(code_tiles_kernel<kQB, 1024>, qblocks, 1024, qsm, s, q, nq, I.d, wd, I.jq_lo, I.jq_scale, qt.ptr,
+                qtail.ptr, bad, cnt, nq + 1);
     count_launch();
     LSHG_CHECK_LAUNCH();
     // two rounds of four CTAs an SM where there are tiles enough, at least two tiles each

@@ -85,8 +85,9 @@ HammingPlan plan_hamming(int64_t n, int C);
 int hamming_chunks(int words);
 int64_t hamming_rows(int64_t n);
 // Sketch rows [n][wp] (first `words` real) -> E2M1 +-1 rows [rows_pad][128 * chunks].
+// (counters: zeroed by the same launch)
 void launch_expand_bits(const uint32_t* xs, int64_t n, int wp, int words, int64_t rows_pad, uint8_t* out,
-                        cudaStream_t s);
+                        int* counters, int ncounters, cudaStream_t s);
 // Top-C keys [nq][C] of each query by (hamming asc, id asc); xse: the base's E2M1 rows
 // (launch_expand_bits, hamming_rows(n) of them), xst: the tiled sketches (small batches, listed rescans), qs:
 // query sketches [nq][wp].  op: OP_HAMMING or OP_ONEBIT_JACCARD.

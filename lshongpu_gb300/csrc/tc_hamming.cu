@@ -722,8 +722,9 @@ __global__ void __launch_bounds__(H_THREADS, 1)
 // (expand_word), 0x2 (+1) for a 0 bit, 0xA (-1) for a 1 bit; nibbles past 32 * words and rows past n
 // are 0x0.
 __global__ void expand_bits_kernel(const uint32_t* __restrict__ xs, int64_t n, int wp, int words, int kp,
-                                   int64_t rows_pad, uint4* __restrict__ out) {
+                                   int64_t rows_pad, uint4* __restrict__ out, int* counters, int ncounters) {
   grid_ready();
+  zero_counters(counters, ncounters);
   const int per_row = kp / 16;
   const int64_t total = rows_pad * per_row;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
@@ -1219,12 +1220,13 @@ int hamming_chunks(int words) { return (words + 7) / 8; }
 int64_t hamming_rows(int64_t n) { return (int64_t)ceil_div(n, HN) * HN; }
 
 void launch_expand_bits(const uint32_t* xs, int64_t n, int wp, int words, int64_t rows_pad, uint8_t* out,
-                        cudaStream_t s) {
+                        int* counters, int ncounters, cudaStream_t s) {
   const int kp = hamming_chunks(words) * H_CHUNK;
   const int64_t total = rows_pad * (kp / 16);
   if (total <= 0) return;
   const int blocks = (int)std::min<int64_t>((total + 255) / 256, (int64_t)num_sms() * 16);
-  launch_next(expand_bits_kernel, blocks, 256, 0, s, xs, n, wp, words, kp, rows_pad, reinterpret_cast<uint4*>(out));
+  launch_next(expand_bits_kernel, blocks, 256, 0, s, xs, n, wp, words, kp, rows_pad, reinterpret_cast<uint4*>(out),
+              counters, ncounters);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -1263,11 +1265,10 @@ void launch_tc_hamming(const uint8_t* xse, int64_t n, const uint32_t* xst, int w
   LSHG_REQUIRE((int64_t)QT * plan.NT < (int64_t)INT_MAX, "tensor-core sketch scan: problem too large");
   DevBuf<int> ctl((size_t)nq + 1 + nq, s);  // [0, nq): survivors; [nq]: listed queries; then their list
   int *cnt = ctl.ptr, *ovf = ctl.ptr + nq;
-  LSHG_CUDA(cudaMemsetAsync(ctl.ptr, 0, (size_t)(nq + 1) * sizeof(int), s));
   DevBuf<uint8_t> qe((size_t)qpad * kp, s);
   {
     ProfScope _ps("tc_hamming_expand", s);
-    launch_expand_bits(qs, nq, wp, words, qpad, qe.ptr, s);
+    launch_expand_bits(qs, nq, wp, words, qpad, qe.ptr, cnt, nq + 1, s);
   }
   const CUtensorMap ma = map_sketch_rows(qe.ptr, qpad, kp, BM);
   // clusters of two query tiles share each base tile's fetch; one tile alone would leave the

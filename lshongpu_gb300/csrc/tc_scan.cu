@@ -376,8 +376,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 
 // Unit rows in BF16, zero-padded to KD columns and to `rows_pad` rows.
 __global__ void to_unit_bf16_kernel(const float* __restrict__ x, int64_t n, int d, int64_t rows_pad,
-                                    __nv_bfloat16* __restrict__ out) {
+                                    __nv_bfloat16* __restrict__ out, int* counters, int ncounters) {
   grid_ready();
+  zero_counters(counters, ncounters);
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -423,11 +424,13 @@ void to_unit_e4m3(const float* x, int64_t n, int d, int64_t rows_pad, uint8_t* o
   LSHG_CHECK_LAUNCH();
 }
 
-void to_unit_bf16(const float* x, int64_t n, int d, int64_t rows_pad, uint16_t* out, cudaStream_t s) {
+void to_unit_bf16(const float* x, int64_t n, int d, int64_t rows_pad, uint16_t* out, int* counters, int ncounters,
+                  cudaStream_t s) {
   int64_t warps = rows_pad;
   int blocks = (int)std::min<int64_t>((warps * 32 + 255) / 256, (int64_t)num_sms() * 16);
   launch_next(to_unit_bf16_kernel, std::max(blocks, 1), 256, 0, s, x, n, d, rows_pad,
-              reinterpret_cast<__nv_bfloat16*>(out));
+              reinterpret_cast<__nv_bfloat16*>(out), counters,
+              ncounters);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }
@@ -517,7 +520,7 @@ void tc_prepare(Index& I, cudaStream_t s) {
   I.dp = KD;
   const int64_t npad = (int64_t)ceil_div(I.n, FILTER_TN) * FILTER_TN;  // whole filter tiles
   I.xbf.alloc((size_t)npad * KD, s);
-  to_unit_bf16(I.x.ptr, I.n, I.d, npad, I.xbf.ptr, s);
+  to_unit_bf16(I.x.ptr, I.n, I.d, npad, I.xbf.ptr, nullptr, 0, s);
   if (I.p.implementation == 9) {  // E4M3 operands for the filter (BF16 stays for the fallback)
     I.xf8.alloc((size_t)npad * KD, s);
     to_unit_e4m3(I.x.ptr, I.n, I.d, npad, I.xf8.ptr, s);
@@ -554,9 +557,8 @@ void launch_tc_scan(Index& I, const float* q, int nq, int k, lshg_point* out, cu
   DevBuf<float> tau((size_t)nq, s);
   DevBuf<int> cnt((size_t)nq + 1 + nq, s);  // [0, nq): survivors; [nq]: overflow count; then the list
   int* ovf = cnt.ptr + nq;
-  LSHG_CUDA(cudaMemsetAsync(cnt.ptr, 0, (size_t)(nq + 1) * sizeof(int), s));
   DevBuf<uint16_t> qbf((size_t)qpad * KD, s);
-  to_unit_bf16(q, nq, I.d, qpad, qbf.ptr, s);
+  to_unit_bf16(q, nq, I.d, qpad, qbf.ptr, cnt.ptr, nq + 1, s);
   const int64_t npad = (int64_t)ceil_div(I.n, FILTER_TN) * FILTER_TN;
   const CUtensorMap mb = make_map(I.xbf.ptr, npad);  // list kernel: 128-row boxes
   DevBuf<uint8_t> qf8;
