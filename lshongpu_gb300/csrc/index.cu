@@ -23,7 +23,7 @@ namespace lshg {
 // 128-query tile is mostly padding for a few queries, but the scan then costs little more than
 // reading the base once, where the popcount scan folds each query's candidates by itself.
 // Measured, popcount against tensor cores: 1.2M x 1,024 bits, C = 128: one query 325 / 199 us, 16
-// 1,141 / 156; C = 1,024: one 827 / 203, 63 3,061 / 231; 10k points, C = 128: one 95 / 100, four
+// 1,141 / 139; C = 1,024: one 827 / 203, 63 3,061 / 231; 10k points, C = 128: one 95 / 100, four
 // 106 / 107, 16 155 / 114; C = 1,024: one 180 / 94.
 constexpr int kTcSketchLongList = 128;       // candidates above which every batch takes it
 constexpr int64_t kTcSketchMinPairs = 65536; // (query, point) pairs from which every list does

@@ -23,7 +23,7 @@
 //
 // r(x) is about 8e-4 for vectors of 100 comparable components, so 2 eps is about 0.004 and the
 // candidates are a handful more than k.  Measured (100k x 100, 1,000 queries, k = 32): the
-// FP32 scan 886 us, this 82; 1.2M x 100: one query 1,065 -> 110 us, 1,000 queries 6.62 -> 0.30
+// FP32 scan 886 us, this 78; 1.2M x 100: one query 1,065 -> 110 us, 1,000 queries 6.62 -> 0.30
 // ms.
 #include <algorithm>
 

@@ -17,10 +17,10 @@
 //
 // scan kernel: a CTA takes 64 queries and a run of 128-point tiles, warp w queries 8w .. 8w + 7,
 // lane l points 4l .. 4l + 3: 32 sums a thread, three shared 16-byte loads a four-dimension step.
-// Measured (60,013 x 100, 129 queries, k = 10): the FP32 scan 413 us, this 120 (the two
-// passes 19 + 31; the rest is launches and latency); 1M x 100, one query 2,140 -> 246, 100 queries,
-// k = 32, 2,640 -> 1,000.  The divisions of every bound instead of the linear form below: 49 us for
-// the second pass.
+// Measured (60,013 x 100, 129 queries, k = 10): the FP32 scan 413 us, this 85 (the two passes 15 + 27,
+// the re-rank 14; the rest is launches and latency); 1M x 100, one query 2,140 -> 246, 100 queries, k =
+// 32, 2,640 -> 1,000.  With the divisions of every bound in place of the linear form below the second
+// pass took 49 us against 31.
 #include <algorithm>
 
 #include "index.h"
