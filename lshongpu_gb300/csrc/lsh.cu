@@ -683,15 +683,26 @@ static void launch_split(const LshQueryArgs& a, int cap, size_t fused_smem, lshg
   // 100, 16 tables, 49: one query 55 / 61 us, 64 75 / 68; 1M x 128, 488: one 87 / 71).
   const int64_t avg = a.n * a.tables / a.tableSize;
   const int* only = nullptr;
+  DevBuf<uint64_t> kept;
   DevBuf<int> hard;
-  if (DV == DIST_ANGULAR && a.xq8 && a.k <= 128 && cap <= kListBounds && 2 * avg <= cap && avg * a.nq >= 400) {
-    DevBuf<uint64_t> kept((size_t)a.nq * kBoundsKeep, s);
-    hard.alloc((size_t)a.nq + 1, s);
+  bool bounds = DV == DIST_ANGULAR && a.xq8 && a.k <= 128 && cap <= kListBounds && 2 * avg <= cap && avg * a.nq >= 400;
+  if (bounds) {
+    try {
+      kept.alloc((size_t)a.nq * kBoundsKeep, s);
+      hard.alloc((size_t)a.nq + 1, s);
+    } catch (const Error& e) {  // no room for the kept candidates: every one is scored
+      if (e.status != LSHG_ERR_OUT_OF_MEMORY) throw;
+      cudaGetLastError();
+      bounds = false;
+    }
+  }
+  if (bounds) {
     LSHG_CUDA(cudaMemsetAsync(hard.ptr, 0, sizeof(int), s));
     launch_list_bounds(cand.ptr, cap, ccnt.ptr, a.xq8, a.xq8_tail, a.n, a.d, a.q, a.nq, a.k, kept.ptr, hard.ptr, s);
     launch_rerank(kept.ptr, a.nq, kBoundsKeep, a.x, a.n, a.d, a.xnorm, a.q, a.qnorm, DIST_ANGULAR, a.k, out, s, a.err);
     only = hard.ptr;
   }
+  kept.release();
   launch_next(lsh_score_kernel<DV>, sgrid, kQThreads, ssmem, s, a, cand.ptr, cap, ccnt.ptr, out, ctl.ptr + 1, only);
   count_launch();
   LSHG_CHECK_LAUNCH();

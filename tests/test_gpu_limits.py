@@ -1,0 +1,87 @@
+"""Queries at the limits of a device's memory and of several host threads: what a batch allocates,
+what it does where its optional temporaries do not fit, and indexes of different dimensions
+queried at the same time.
+
+Memory is limited by a pool with a maximum size of its own, in place of the device's default
+pool, so the device itself is never filled.
+"""
+import contextlib
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+from lshongpu_gb300 import datasets
+
+pytestmark = pytest.mark.gpu
+
+USED_HIGH = 0x8  # cudaMemPoolAttrUsedMemHigh
+
+
+class PoolProps(C.Structure):
+    """struct cudaMemPoolProps."""
+    _fields_ = [("alloc_type", C.c_int), ("handle_types", C.c_int), ("location_type", C.c_int),
+                ("location_id", C.c_int), ("security", C.c_void_p), ("max_size", C.c_size_t),
+                ("usage", C.c_ushort), ("reserved", C.c_ubyte * 54)]
+
+
+def cudart():
+    import torch
+
+    torch.cuda.synchronize()
+    rt = C.CDLL("libcudart.so.13")
+    rt.cudaMemPoolDestroy.argtypes = [C.c_void_p]
+    rt.cudaDeviceSetMemPool.argtypes = [C.c_int, C.c_void_p]
+    for f in ("cudaMemPoolGetAttribute", "cudaMemPoolSetAttribute"):
+        getattr(rt, f).argtypes = [C.c_void_p, C.c_int, C.c_void_p]
+    return rt
+
+
+@contextlib.contextmanager
+def memory_pool(max_bytes=0):
+    """The device's allocations come from a pool of at most max_bytes (0: no limit of its own);
+    yields a function that returns, and resets, the most bytes in use since its last call."""
+    rt = cudart()
+    old, pool = C.c_void_p(), C.c_void_p()
+    assert rt.cudaDeviceGetMemPool(C.byref(old), 0) == 0
+    props = PoolProps(alloc_type=1, location_type=1, location_id=0, max_size=max_bytes)
+    assert rt.cudaMemPoolCreate(C.byref(pool), C.byref(props)) == 0
+    assert rt.cudaDeviceSetMemPool(0, pool) == 0
+
+    def high():
+        v = C.c_uint64()
+        assert rt.cudaDeviceSynchronize() == 0
+        assert rt.cudaMemPoolGetAttribute(pool, USED_HIGH, C.byref(v)) == 0
+        zero = C.c_uint64(0)
+        assert rt.cudaMemPoolSetAttribute(pool, USED_HIGH, C.byref(zero)) == 0
+        return v.value
+
+    try:
+        yield high
+    finally:
+        rt.cudaDeviceSynchronize()
+        assert rt.cudaDeviceSetMemPool(0, old) == 0
+        assert rt.cudaMemPoolDestroy(pool) == 0
+
+
+def test_lsh_batch_without_room_for_the_bounds(engine):
+    """An LSH batch whose candidate lists fit, but not the 2 KB a query its bounds keep, is scored
+    without them, with the same results."""
+    n, d, nq = 20000, 16, 43000
+    x = datasets.clustered(n, d, 151, count=200)
+    q = np.tile(datasets.clustered(1000, d, 152, count=200), (nq // 1000, 1))
+    kw = dict(implementation=2, distanceFunc=1, framework=1, keysImplementation=7, bucketKeyBits=10, tables=4,
+              options=engine.make_options(cp_hashes=2))
+    with memory_pool() as high:
+        idx = engine.Index(x, **kw)
+        high()
+        want = idx.query(q, 32)
+        full = high()
+        idx.close()
+    kept = nq * 2048
+    with memory_pool(full - kept // 2) as high:
+        idx = engine.Index(x, **kw)
+        got = idx.query(q, 32)
+        idx.close()
+    assert got.tobytes() == want.tobytes()
