@@ -124,7 +124,8 @@ void derive_exact(Index& I, cudaStream_t s) {
   try {
     I.ebf.alloc((size_t)npad * tc::KD, s);
     I.ebf_res.alloc(2, s);
-  } catch (const Error&) {  // no room for the filter's rows: the FP32 scan needs none
+  } catch (const Error& e) {  // no room for the filter's rows: the FP32 scan needs none
+    if (e.status != LSHG_ERR_OUT_OF_MEMORY) throw;
     cudaGetLastError();
     I.ebf.release();
     return;
@@ -134,7 +135,10 @@ void derive_exact(Index& I, cudaStream_t s) {
   launch_unit_rows(I.x.ptr, I.n, I.d, npad, I.ebf.ptr, stat, nullptr, nullptr, nullptr, 0, s);
   LSHG_CUDA(cudaMemcpyAsync(&bad, stat + 1, sizeof(bad), cudaMemcpyDeviceToHost, s));
   LSHG_CUDA(cudaStreamSynchronize(s));
-  if (bad) I.ebf.release();
+  if (bad) {
+    I.ebf.release();
+    I.ebf_res.release();
+  }
 }
 
 bool query_exact_filtered(Index& I, const float* q, int nq, int k, lshg_point* out, cudaStream_t s) {
