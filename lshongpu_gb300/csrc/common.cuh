@@ -119,6 +119,16 @@ constexpr float kEmptyDistance = 2147483648.0f;
 inline int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
 int num_sms();
+
+// A launch with `bytes` of dynamic shared memory is allowed from here on.  The limit belongs to the
+// kernel, not to a launch: it is only ever raised, so that host threads whose calls need different
+// sizes (indexes of different dimensions) cannot lower it between another's call and its launch.
+void raise_smem_limit(const void* kernel, size_t bytes);
+template <typename... P>
+void raise_smem_limit(void (*kernel)(P...), size_t bytes) {
+  raise_smem_limit(reinterpret_cast<const void*>(kernel), bytes);
+}
+
 void keep_pool_memory();  // keep the default mempool's reserve between query batches
 
 template <typename T>

@@ -347,7 +347,7 @@ void launch_direct_cfg(const uint32_t* xst, int64_t n, int S, const uint32_t* qs
                        uint64_t* out, const int* list, cudaStream_t s) {
   const size_t smem = direct_layout(S, 2, C, KBUF).total;
   auto kern = cws_direct_kernel<KBUF, T>;
-  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(kern, smem);
   const int ntiles = ceil_div(n, kTile);
   const int tps = ceil_div(ntiles, splits);
   dim3 grid(ceil_div(nq, 2), splits);
@@ -411,7 +411,7 @@ void launch_cws_sketch(const float* x, int64_t rows, int d, int S, const float* 
   if (rows <= 0) return;
   LSHG_REQUIRE(d >= 1 && d <= 4096, "CWS: d must be in [1, 4096]");
   const size_t smem = (size_t)8 * d * sizeof(float);
-  LSHG_CUDA(cudaFuncSetAttribute(cws_sketch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(cws_sketch_kernel, smem);
   const int blocks = (int)std::min<int64_t>((rows + 7) / 8, (int64_t)num_sms() * 8);
   launch_next(cws_sketch_kernel, blocks, 256, smem, s, x, rows, d, S, reinterpret_cast<const float4*>(tab),
                                               reinterpret_cast<int2*>(out));

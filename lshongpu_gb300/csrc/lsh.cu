@@ -622,7 +622,7 @@ size_t lsh_query_smem(const LshQueryArgs& a) {
 
 template <int DV>
 static int lsh_ctas_per_sm(size_t smem) {
-  LSHG_CUDA(cudaFuncSetAttribute(lsh_query_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(lsh_query_kernel<DV>, smem);
   int per = 0;
   LSHG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, lsh_query_kernel<DV>, kQThreads, smem));
   return per;
@@ -652,7 +652,7 @@ void lsh_query_plan(LshQueryArgs& a, int max_grid) {
   a.walk_grid = 0;
   if (a.split_cap > 0) {
     constexpr int wsmem = kWalkSlots * 4;
-    LSHG_CUDA(cudaFuncSetAttribute(lsh_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wsmem));
+    raise_smem_limit(lsh_walk_kernel, wsmem);
     int wper = 0;
     LSHG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wper, lsh_walk_kernel, kQThreads, wsmem));
     a.walk_grid = std::max(1, std::min(a.nq, num_sms() * std::max(1, wper)));
@@ -670,7 +670,7 @@ static void launch_split(const LshQueryArgs& a, int cap, size_t fused_smem, lshg
   count_launch();
   LSHG_CHECK_LAUNCH();
   const size_t ssmem = lsh_stage_bytes(a.d) + (size_t)(a.C + kQBuf) * 8 + (size_t)((a.d + 3) & ~3) * 4 + 16;
-  LSHG_CUDA(cudaFuncSetAttribute(lsh_score_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem));
+  raise_smem_limit(lsh_score_kernel<DV>, ssmem);
   int per = 0;
   LSHG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, lsh_score_kernel<DV>, kQThreads, ssmem));
   const int sgrid = std::max(1, std::min(a.nq, num_sms() * std::max(1, per)));
@@ -712,7 +712,7 @@ static void launch_split(const LshQueryArgs& a, int cap, size_t fused_smem, lshg
   f.qctr = ctl.ptr + 2;
   DevBuf<int> lists((size_t)a.grid * kListCap, s);
   f.lists = lists.ptr;
-  LSHG_CUDA(cudaFuncSetAttribute(lsh_query_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem));
+  raise_smem_limit(lsh_query_kernel<DV>, fused_smem);
   launch_next(lsh_query_kernel<DV>, a.grid, kQThreads, fused_smem, s, f, out);
   count_launch();
   LSHG_CHECK_LAUNCH();
@@ -744,7 +744,7 @@ void launch_lsh_query(const LshQueryArgs& a, lshg_point* out, cudaStream_t s) {
   f.qctr = qctr.ptr;
 #define LSHG_LQ(DV)                                                                                        \
   do {                                                                                                     \
-    LSHG_CUDA(cudaFuncSetAttribute(lsh_query_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+    raise_smem_limit(lsh_query_kernel<DV>, smem); \
     launch_next(lsh_query_kernel<DV>, a.grid, kQThreads, smem, s, f, out);                                          \
   } while (0)
   switch (a.dist) {

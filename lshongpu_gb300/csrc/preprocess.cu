@@ -7,6 +7,7 @@
 // (processingUtils.cuh:48-67, distanceFunctions.cuh:23-40).  Rows are staged through
 // shared memory so global reads stay coalesced while each thread walks its own row.
 #include <mutex>
+#include <unordered_map>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -180,6 +181,16 @@ int num_sms() {
   return sms;
 }
 
+void raise_smem_limit(const void* kernel, size_t bytes) {
+  static std::mutex mu;
+  static std::unordered_map<const void*, size_t> largest;
+  std::lock_guard<std::mutex> g(mu);
+  size_t& most = largest[kernel];
+  const size_t v = std::max(most, bytes);
+  LSHG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v));
+  most = v;  // a size that was refused is not kept
+}
+
 // Query batches allocate their temporaries (hundreds of MB for large batches) with
 // cudaMallocAsync.  The default pool returns unused memory to the driver at every
 // synchronisation, so each batch would map its temporaries again; keeping what the
@@ -204,7 +215,7 @@ void launch_row_norms(const float* x, int64_t n, int d, float* norms, cudaStream
   if (n <= 0) return;
   size_t smem = staged_smem(kRowsPerBlock, d);
   LSHG_REQUIRE(smem <= 200 * 1024, "dimension too large for row_norms");
-  LSHG_CUDA(cudaFuncSetAttribute(row_norm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(row_norm_kernel<false>, smem);
   launch_next(row_norm_kernel<false>, ceil_div(n, kRowsPerBlock), kNormThreads, smem, s, const_cast<float*>(x), n, d,
               norms);
   count_launch();
@@ -215,7 +226,7 @@ void launch_normalize(float* x, int64_t n, int d, cudaStream_t s) {
   if (n <= 0) return;
   size_t smem = staged_smem(kRowsPerBlock, d);
   LSHG_REQUIRE(smem <= 200 * 1024, "dimension too large for normalize");
-  LSHG_CUDA(cudaFuncSetAttribute(row_norm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(row_norm_kernel<true>, smem);
   launch_next(row_norm_kernel<true>, ceil_div(n, kRowsPerBlock), kNormThreads, smem, s, x, n, d, nullptr);
   count_launch();
   LSHG_CHECK_LAUNCH();
@@ -225,7 +236,7 @@ void launch_tile_transpose(const float* x, int64_t n, int d, float* xt, cudaStre
   if (n <= 0) return;
   size_t smem = staged_smem(128, d);
   LSHG_REQUIRE(smem <= 220 * 1024, "dimension too large for the tiled layout");
-  LSHG_CUDA(cudaFuncSetAttribute(tile_transpose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(tile_transpose_kernel, smem);
   tile_transpose_kernel<<<ceil_div(n, 128), 256, smem, s>>>(x, n, d, xt);
   count_launch();
   LSHG_CHECK_LAUNCH();

@@ -128,7 +128,7 @@ void launch_project(const float* x, int64_t n, int d, const float* planes, int n
   size_t smem = (size_t)2 * d * kPitch * sizeof(float);
   LSHG_REQUIRE(smem <= 220 * 1024, "dimension too large for projection");
   ProfScope _ps(mode == 1 ? "project_jl" : "project_simhash", s);
-  LSHG_CUDA(cudaFuncSetAttribute(project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(project_kernel, smem);
   dim3 grid(ceil_div(n, kTP), ceil_div(nplanes, kTL));
   launch_next(project_kernel, grid, 256, smem, s, x, n, d, planes, nplanes, mode, bits, words, out32, out_f, nullptr);
   count_launch();
@@ -140,7 +140,7 @@ void launch_project_gated(const float* x, int64_t n, int d, const float* planes,
   if (n <= 0 || nplanes <= 0) return;
   size_t smem = (size_t)2 * d * kPitch * sizeof(float);
   LSHG_REQUIRE(smem <= 220 * 1024 && nplanes == 32 * words, "bad projection shape");
-  LSHG_CUDA(cudaFuncSetAttribute(project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(project_kernel, smem);
   dim3 grid(ceil_div(n, kTP), ceil_div(nplanes, kTL));
   launch_next(project_kernel, grid, 256, smem, s, x, n, d, planes, nplanes, 0, 32, words, out32, nullptr, gate);
   count_launch();

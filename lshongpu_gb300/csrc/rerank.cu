@@ -689,7 +689,7 @@ void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t
     return;
   }
   size_t smem = (size_t)C * 8;
-  LSHG_CUDA(cudaFuncSetAttribute(merge_splits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(merge_splits_kernel, smem);
   launch_next(merge_splits_kernel, nq, 128, smem, s, in, nq, splits, C, out, list);
   count_launch();
   LSHG_CHECK_LAUNCH();
@@ -751,8 +751,7 @@ void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t 
     }
 #define LSHG_RR2(DV)                                                                                            \
   do {                                                                                                          \
-    LSHG_CUDA(cudaFuncSetAttribute(rerank_gather_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
-                                   (int)gather_smem));                                                          \
+    raise_smem_limit(rerank_gather_kernel<DV>, gather_smem);                                                          \
     launch_next(rerank_gather_kernel<DV>, dim3(nq, C / 128), 128, gather_smem, s, gin, C, x, n, d, xnorm, q, qnorm,      \
                                                                          gk.ptr, err);                          \
     count_launch();                                                                                             \
@@ -767,8 +766,7 @@ void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t 
       launch_next(rerank_top_kernel<DV, 2>, nq, 512, (size_t)d * 4, s, gk.ptr, C, x, d, q, k, out, band_abs, band_rel,   \
                                                               xn64, kb);                                        \
     else {                                                                                                      \
-      LSHG_CUDA(cudaFuncSetAttribute(rerank_select_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                                     (int)select_smem));                                                        \
+      raise_smem_limit(rerank_select_kernel<DV>, select_smem);                                                        \
       launch_next(rerank_select_kernel<DV>, nq, 512, select_smem, s, gk.ptr, C, x, d, q, k, out, band_abs, band_rel,     \
                                                             xn64, kb);                                          \
     }                                                                                                           \
@@ -788,8 +786,7 @@ void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t 
   if (stageable && staged_smem <= 96 * 1024) {
 #define LSHG_RRS(DV)                                                                                           \
   do {                                                                                                         \
-    LSHG_CUDA(cudaFuncSetAttribute(rerank_staged_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
-                                   (int)staged_smem));                                                         \
+    raise_smem_limit(rerank_staged_kernel<DV>, staged_smem);                                                         \
     launch_next(rerank_staged_kernel<DV>, nq, CH, staged_smem, s, cand, nq, C, x, n, d, xnorm, q, qnorm, qnorm_out, k,  \
                                                          out, err, band_abs, band_rel, xn64, test_stall, kb); \
   } while (0)
@@ -810,7 +807,7 @@ void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t 
   int threads = C >= 256 ? 256 : 128;
 #define LSHG_RR(DV)                                                                                       \
   do {                                                                                                    \
-    LSHG_CUDA(cudaFuncSetAttribute(rerank_kernel<DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+    raise_smem_limit(rerank_kernel<DV>, smem); \
     launch_next(rerank_kernel<DV>, nq, threads, smem, s, cand, nq, C, x, n, d, xnorm, q, qnorm, qnorm_out, k, out,      \
                                                 band_abs, band_rel, xn64, kb);                            \
   } while (0)
@@ -834,7 +831,7 @@ void launch_rerank_listed(const uint64_t* cand, int C, const float* x, int64_t n
   ProfScope _ps("rerank_listed", s);
   const size_t smem = (size_t)C * 8 + (size_t)d * 4 + 16;
   auto kern = dist == DIST_JACCARD ? rerank_listed_kernel<DIST_JACCARD> : rerank_listed_kernel<DIST_ANGULAR>;
-  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(kern, smem);
   kern<<<std::min(nq, num_sms() * 4), 512, smem, s>>>(cand, C, x, n, d, xnorm, q, qnorm, listed, k, out);
   count_launch();
   LSHG_CHECK_LAUNCH();

@@ -423,7 +423,7 @@ void launch_bounds(const uint64_t* cand, const int* list, int list_cap, const in
   ProfScope _ps("rerank_bounds", s);
   constexpr int smem = C * (int)sizeof(uint32_t);
   auto kern = bounds_kernel<DIST, C, LIST>;
-  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  raise_smem_limit(kern, smem);
   launch_next(kern, nq, kBoundThreads, smem, s, cand, list, list_cap, ccnt, rows, tails, pitch, scale, n, d, q, k,
               kept, listed);
   count_launch();

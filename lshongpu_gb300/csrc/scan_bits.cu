@@ -184,7 +184,7 @@ void launch_cfg(const uint32_t* xs, int64_t n, int wp, int words, int sbytes, co
   ProfScope _ps(list ? "scan_bits_listed" : "scan_bits", s);
   size_t smem = bits_layout(wp, QB, C, KBUF).total;
   auto kern = scan_bits_kernel<OP, QB, KBUF, T, NC, MINB>;
-  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(kern, smem);
   int ntiles = ceil_div(n, kTile);
   int tps = ceil_div(ntiles, splits);
   dim3 grid(ceil_div(nq, QB), splits);

@@ -529,7 +529,7 @@ void launch_listed(const float* xt, int64_t n, int d, const float* xnorm, const 
   smem = reg_scan_smem(d, 32 * EC, nb);
   LSHG_REQUIRE(smem <= 220 * 1024, "listed scan: dimension too large");
   auto kern = scan_float_listed_kernel<DIST, EC>;
-  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(kern, smem);
   const int tps = ceil_div(ceil_div(n, kTile), splits);
   launch_next(kern, num_sms() * 2, 256, smem, s, xt, n, d, xnorm, q, qnorm, list, tps, splits, nb, part);
   count_launch();
@@ -542,7 +542,7 @@ void launch_reg(const float* xt, int64_t n, int d, const float* xnorm, const flo
   ProfScope _ps("scan_float", s);
   const size_t smem = reg_scan_smem(d, 32 * EC, nbuf);
   auto kern = scan_float_reg_kernel<DIST, EC>;
-  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(kern, smem);
   const int ntiles = ceil_div(n, kTile);
   const int tps = ceil_div(ntiles, splits);
   dim3 grid(ceil_div(nq, kRegQB), splits);
@@ -590,7 +590,7 @@ void launch_cfg(const float* xt, int64_t n, int d, const float* xnorm, const flo
   ProfScope _ps("scan_float", s);
   size_t smem = float_scan_layout(d, QB, C, nbuf).total;
   auto kern = scan_float_kernel<DIST, QB, MQ>;
-  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(kern, smem);
   int ntiles = ceil_div(n, kTile);
   int tps = ceil_div(ntiles, splits);
   dim3 grid(ceil_div(nq, QB), splits);

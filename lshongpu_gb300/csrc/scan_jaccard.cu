@@ -288,8 +288,8 @@ bool query_jaccard_filtered(Index& I, const float* q, int nq, int k, lshg_point*
     const int tps0 = split(stiles), tps = split(tiles);
     const dim3 grid0(qblocks, ceil_div(stiles, tps0)), grid(qblocks, ceil_div(tiles, tps));
     const size_t smem = (size_t)wd * (kTile + kQB) * 4;
-    LSHG_CUDA(cudaFuncSetAttribute(jaccard_scan_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    LSHG_CUDA(cudaFuncSetAttribute(jaccard_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    raise_smem_limit(jaccard_scan_kernel<0>, smem);
+    raise_smem_limit(jaccard_scan_kernel<1>, smem);
     {
       ProfScope _ps("jaccard_bounds", s);
       launch_next(jaccard_scan_kernel<0>, grid0, 256, smem, s, I.jq.ptr, I.jq_tail.ptr, I.n, wd, I.d, qt.ptr, qtail.ptr, bad, nq,

@@ -368,7 +368,7 @@ void run_ng(const uint4* xst, int64_t n, const uint32_t* qsl, int nq, int NP, in
             int bins, int* cnt, uint64_t* cand, int cap, int* err, cudaStream_t s) {
   constexpr int smem = Layout<MODE, NG, PL>::SMEM;
   auto kern = sliced_filter_kernel<MODE, NG, PL>;
-  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  raise_smem_limit(kern, smem);
   int per_sm = 0;
   LSHG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBThreads, smem));
   const int64_t slots = (int64_t)num_sms() * std::max(1, per_sm);

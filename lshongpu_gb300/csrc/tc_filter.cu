@@ -735,7 +735,7 @@ void run_filter_as(const FilterMaps& m, FilterArgs a, int clusters, const char* 
   const int grid = CL * std::min(clusters, a.NCH * a.QP);
   auto kern = tc_filter_kernel<MODE, GW, F8, KC, CL>;
   constexpr int smem = FLayout<KC, CL>::SMEM;
-  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  raise_smem_limit(kern, smem);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(F_THREADS);

@@ -981,7 +981,7 @@ void run_hamming(const CUtensorMap& ma, const CUtensorMap& mb, HArgs a, const ch
   const int grid = CL * std::min(G, a.NCH * a.QP);
   auto kern = tc_hamming_kernel<MODE, GW, KC, CL, BITS>;
   constexpr int smem = HLayout<KC, CL>::SMEM;
-  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  raise_smem_limit(kern, smem);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(H_THREADS);
@@ -1033,7 +1033,7 @@ void run_signs(const CUtensorMap& ma, const CUtensorMap& mb, SignArgs a, cudaStr
   *grid_out = grid;
   auto kern = tc_signs_kernel<KC>;
   constexpr int smem = PLayout<KC>::SMEM;
-  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  raise_smem_limit(kern, smem);
   ProfScope _ps("tc_project_gemm", s);
   launch_next(kern, grid, H_THREADS, smem, s, ma, mb, a);
   count_launch();

@@ -504,7 +504,7 @@ void run_list_kernel(const CUtensorMap& ma, const CUtensorMap& mb, const int* ro
                      int grid, uint64_t* part, int* err, cudaStream_t s) {
   constexpr TcLayout L = tc_layout(STAGES, CT);
   auto kern = tc_list_kernel<STAGES, CT>;
-  LSHG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.total));
+  raise_smem_limit(kern, L.total);
   launch_next(kern, grid, NTHREADS, L.total, s, ma, mb, rows_dev, n, NT, tc_ksteps(d), part, err);
   count_launch();
   LSHG_CHECK_LAUNCH();

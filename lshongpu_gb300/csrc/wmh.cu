@@ -123,7 +123,7 @@ void launch_wmh_sketch(const float* x, int64_t n, int d, const int* start, const
   LSHG_REQUIRE(!onebit || (hashBits >= 1 && hashBits <= 32 && words * hashBits == H), "one-bit WMH: bad shape");
   size_t smem = (size_t)(d + M) * sizeof(int);
   LSHG_REQUIRE(smem <= 200 * 1024, "weighted MinHash: index map too large");
-  LSHG_CUDA(cudaFuncSetAttribute(wmh_sketch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  raise_smem_limit(wmh_sketch_kernel, smem);
   int groups = onebit ? words : (H + 31) / 32;
   int64_t warps = n * groups;
   int blocks = (int)std::min<int64_t>((warps * 32 + 255) / 256, (int64_t)num_sms() * 16);

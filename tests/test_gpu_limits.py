@@ -85,3 +85,40 @@ def test_lsh_batch_without_room_for_the_bounds(engine):
         got = idx.query(q, 32)
         idx.close()
     assert got.tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("dist,k", [(1, 32), (2, 10), (1, 200)])
+def test_two_threads_of_different_dimensions(engine, dist, k):
+    """Host threads that query indexes of 20 and of 128 dimensions at the same time: the kernels they
+    share are launched with different amounts of shared memory."""
+    import torch
+
+    batches, nq = 3000, 8
+    jobs = []
+    for d in (20, 128):
+        rows = datasets.sparse_gamma if dist == 2 else datasets.clustered
+        x, q = rows(4200, d, 161), rows(nq, d, 162)
+        idx = engine.Index(x, implementation=2, distanceFunc=dist)
+        jobs.append((idx, idx.query(q, k), torch.from_numpy(q).cuda(), torch.cuda.Stream(),
+                     torch.empty((nq, k, 2), dtype=torch.int32, device="cuda")))
+    torch.cuda.synchronize()
+    failed = []
+    start = threading.Barrier(len(jobs))
+
+    def work(idx, want, q, stream, out):
+        start.wait()
+        try:
+            for _ in range(batches):
+                idx.query_device_async(q.data_ptr(), nq, k, out.data_ptr(), stream=stream.cuda_stream)
+            idx.sync(stream.cuda_stream)
+            if out.cpu().numpy().tobytes() != want.tobytes():
+                failed.append("results differ")
+        except engine.LshgError as e:
+            failed.append(str(e))
+
+    threads = [threading.Thread(target=work, args=job) for job in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
