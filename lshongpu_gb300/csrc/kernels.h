@@ -135,14 +135,18 @@ void launch_cws_scan(const uint32_t* xsl_t, const uint32_t* xst, int64_t n, int 
                      const uint32_t* qs, int nq, int C, uint64_t* out, int* err, cudaStream_t s);
 
 // ---- rerank.cu -------------------------------------------------------------------
-// Merge per-split sorted lists into one sorted list of C keys per query.
 // The exact top-k (angular or Jaccard) of the queries listed on the device (list[0] = count, list[1..] =
-// rows of q), written to their rows of `out`; k <= 128.  part: nq * listed_splits(n, nq, C) * C
-// keys, C = the power of two >= max(32, k).
-int scan_listed_splits(int64_t n, int nq, int C);
+// rows of q), written to their rows of `out`; k <= 128.  lim[q]: a distance that k points have at most
+// (infinite: none known).  part: `room` >= nq * C keys, C = the power of two >= max(32, k); the more
+// room, the further few listed queries spread over the GPU.
 void launch_scan_float_listed(const float* xt, int64_t n, int d, const float* xnorm, const float* q, int nq,
-                              const float* qnorm, int dist, const int* list, int C, int splits, uint64_t* part,
-                              int k, struct ::lshg_point_s* out, cudaStream_t s);
+                              const float* qnorm, int dist, const int* list, const float* lim, int C, uint64_t* part,
+                              int64_t room, int k, struct ::lshg_point_s* out, cudaStream_t s);
+// Keys to allocate for survivor arrays of `have` keys that the listed scan uses after them: up to 10 MB
+// where listed queries could use them (128 splits each).
+int64_t listed_scan_room(int nq, int C, int64_t have);
+// Merge per-split sorted lists into one sorted list of C keys per query.  list (optional): the lists of
+// slot i < list[0] go to row list[1 + i].
 void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t* out, cudaStream_t s,
                          const int* list = nullptr);
 // Splits of the base for the exact rescan of queries listed on the device (at most nq of them, QB a

@@ -151,24 +151,24 @@ bool query_exact_filtered(Index& I, const float* q, int nq, int k, lshg_point* o
   if (const char* e = getenv("LSHG_TC_FORCE_FALLBACK"); e && e[0] == '1') plan.cap = 0;
   int C = 32;
   while (C < k) C <<= 1;
-  const int splits = scan_listed_splits(I.n, nq, C);
+  const int64_t room = listed_scan_room(nq, C, (int64_t)nq * plan.cap);
   try {
     DevBuf<uint16_t> qbf((size_t)qpad * KD, s);
     DevBuf<float> eps((size_t)nq, s), tau((size_t)nq, s), qnorm((size_t)nq, s);
     DevBuf<int> cnt((size_t)nq + 1 + nq, s);  // [0, nq): survivors; [nq]: listed; then the list
-    DevBuf<uint64_t> cand((size_t)nq * std::max(plan.cap, 1), s), best((size_t)nq * CT, s);
-    DevBuf<uint64_t> part((size_t)nq * splits * C, s);
+    // survivors, then (the re-rank reads `best`) the lists of the FP32 scan
+    DevBuf<uint64_t> cand((size_t)room, s), best((size_t)nq * CT, s);
     int* ovf = cnt.ptr + nq;
     launch_unit_rows(q, nq, I.d, qpad, qbf.ptr, nullptr, I.ebf_res.ptr, eps.ptr, cnt.ptr, nq + 1, s);
     const FilterMaps maps = make_filter_maps(qbf.ptr, qpad, I.ebf.ptr, npad, I.d, false);
     launch_filter_scan(maps, plan, nq, I.n, I.d, (int)(qpad / BM), tau.ptr, cnt.ptr, cand.ptr, I.error_word(s), s,
                        eps.ptr);
     launch_exact_select(cnt.ptr, cand.ptr, nq, plan.cap, (int)std::min<int64_t>(k, I.n), CT,
-                        plan.M > 0 ? tau.ptr : nullptr, eps.ptr, best.ptr, ovf, s);
+                        plan.M > 0 ? tau.ptr : nullptr, eps.ptr, best.ptr, ovf, tau.ptr, s);
     launch_rerank(best.ptr, nq, CT, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, nullptr, DIST_ANGULAR, k, out, s,
                   I.error_word(s), false, nullptr, nullptr, qnorm.ptr);
-    launch_scan_float_listed(I.xt.ptr, I.n, I.d, I.xnorm.ptr, q, nq, qnorm.ptr, DIST_ANGULAR, ovf, C, splits, part.ptr,
-                             k, out, s);
+    launch_scan_float_listed(I.xt.ptr, I.n, I.d, I.xnorm.ptr, q, nq, qnorm.ptr, DIST_ANGULAR, ovf, tau.ptr, C, cand.ptr,
+                             room, k, out, s);
   } catch (const Error& e) {
     if (e.status != LSHG_ERR_OUT_OF_MEMORY) throw;
     cudaGetLastError();  // temporaries that do not fit: the FP32 scan needs fewer

@@ -305,12 +305,13 @@ __device__ __noinline__ uint64_t merge_candidates(uint64_t* list, uint64_t k0, u
 }
 
 // The scan of query block q0 .. q0 + 63 over the tiles of one split.  rows: the queries' rows of
-// q (nullptr: themselves).
+// q (nullptr: themselves).  lim (with rows; by row of q): a distance that k points of the base
+// have at most, infinite where none is known.
 template <int DIST, int EC>
 __device__ __forceinline__ void scan_reg_block(
     const float* __restrict__ xt, int64_t n, int d, const float* __restrict__ xnorm, const float* __restrict__ q,
     int nq, const float* __restrict__ qnorm, int tiles_per_split, int splits, int nbuf, uint64_t* __restrict__ out,
-    int q0, int split, const int* __restrict__ rows) {
+    int q0, int split, const int* __restrict__ rows, const float* __restrict__ lim) {
   constexpr int C = 32 * EC;
   extern __shared__ __align__(16) unsigned char smem[];
   size_t off = 0;
@@ -340,7 +341,13 @@ __device__ __forceinline__ void scan_reg_block(
   for (int a = 0; a < 8; ++a) {
     thr[a] = kEmptyKey;
     bcnt[a] = 0;
+    if (lim && q0 + 8 * w + a < nq) {
+      const float t = lim[rows[q0 + 8 * w + a]];
+      if (t < 1e30f) thr[a] = ((uint64_t)float_to_ordered(t) + 1) << 32;  // false for NaN
+    }
   }
+  // the threshold after a merge into a list that may not be full
+  auto lower = [&](uint64_t t, uint64_t merged) { return lim && t < merged ? t : merged; };
   const unsigned lt_mask = (1u << lane) - 1u;
 
   const int tile_f4 = kTile * d / 4;
@@ -427,7 +434,7 @@ __device__ __forceinline__ void scan_reg_block(
       }
       if (bcnt[a] + nc > kRegBuf) {
         if (bcnt[a] > 0) {  // make room: merge the buffer, then re-filter with the new threshold
-          thr[a] = fold_candidates<EC>(lists + (size_t)qi * C, qbuf, bcnt[a]);
+          thr[a] = lower(thr[a], fold_candidates<EC>(lists + (size_t)qi * C, qbuf, bcnt[a]));
           bcnt[a] = 0;
           nc = 0;
 #pragma unroll
@@ -437,7 +444,8 @@ __device__ __forceinline__ void scan_reg_block(
           }
         }
         if (nc > kRegBuf) {  // more than a buffer's worth in one tile: merge them directly
-          thr[a] = merge_candidates<EC>(lists + (size_t)qi * C, k[0], k[1], k[2], k[3], thr[a], scratch + w * 32);
+          thr[a] = lower(thr[a], merge_candidates<EC>(lists + (size_t)qi * C, k[0], k[1], k[2], k[3], thr[a],
+                                                      scratch + w * 32));
           continue;
         }
       }
@@ -470,7 +478,30 @@ __global__ void __launch_bounds__(256, 2) scan_float_reg_kernel(
     int nq, const float* __restrict__ qnorm, int tiles_per_split, int splits, int nbuf, uint64_t* __restrict__ out) {
   grid_ready();
   scan_reg_block<DIST, EC>(xt, n, d, xnorm, q, nq, qnorm, tiles_per_split, splits, nbuf, out, blockIdx.x * kRegQB,
-                           blockIdx.y, nullptr);
+                           blockIdx.y, nullptr, nullptr);
+}
+
+// Splits of the base's ntiles tiles for `cnt` > 0 listed queries: enough that the (query block,
+// split) items fill the `slots` CTAs in whole rounds, within `room` keys of lists.  How many
+// queries are listed is only known on the device, and one split count for any number of them serves
+// neither end: with 128, a batch of 1,000 that are all listed (100k x 100 in tight clusters, k = 32)
+// took 2,057 us, as each item fills its lists anew, and lists of up to 256 MB that most calls leave
+// empty.  This way 770, the FP32 scan of all 887; one listed query keeps its 128.
+__device__ __forceinline__ int listed_splits(int cnt, int ntiles, int slots, int C, int64_t room) {
+  const int qb = (cnt + kRegQB - 1) / kRegQB;
+  const int most = max(1, min(min(128, ntiles / 4), (int)min((int64_t)128, room / ((int64_t)cnt * C))));
+  const int want = min(most, max(1, slots / qb));
+  int best = want;
+  int64_t best_eff = 0;  // permille of the CTAs' rounds; whole numbers, as two kernels have to agree
+  for (int sp = want; sp <= min(most, max(8, 2 * want)); ++sp) {
+    const int64_t items = (int64_t)qb * sp, rounds = (items + slots - 1) / slots;
+    const int64_t eff = items * 1000 / (rounds * slots);
+    if (eff > best_eff + 10) {
+      best_eff = eff;
+      best = sp;
+    }
+  }
+  return best;
 }
 
 // The listed queries (list[0] of them): CTAs take (query block, split) items in turn, so that a
@@ -478,25 +509,31 @@ __global__ void __launch_bounds__(256, 2) scan_float_reg_kernel(
 template <int DIST, int EC>
 __global__ void __launch_bounds__(256, 2) scan_float_listed_kernel(
     const float* __restrict__ xt, int64_t n, int d, const float* __restrict__ xnorm, const float* __restrict__ q,
-    const float* __restrict__ qnorm, const int* __restrict__ list, int tiles_per_split, int splits, int nbuf,
-    uint64_t* __restrict__ out) {
+    const float* __restrict__ qnorm, const int* __restrict__ list, const float* __restrict__ lim, int64_t room,
+    int nbuf, uint64_t* __restrict__ out) {
   grid_ready();
   const int nq = list[0];
+  if (nq == 0) return;
+  const int ntiles = (int)((n + kTile - 1) / kTile);
+  const int splits = listed_splits(nq, ntiles, gridDim.x, 32 * EC, room);
+  const int tiles_per_split = (ntiles + splits - 1) / splits;
   const int items = (nq + kRegQB - 1) / kRegQB * splits;
   for (int it = blockIdx.x; it < items; it += gridDim.x) {
     scan_reg_block<DIST, EC>(xt, n, d, xnorm, q, nq, qnorm, tiles_per_split, splits, nbuf, out,
-                             it / splits * kRegQB, it % splits, list + 1);
+                             it / splits * kRegQB, it % splits, list + 1, lim);
     __syncthreads();  // the item's shared memory is done with
   }
 }
 
-// The first k of each listed query's `splits` sorted lists of C keys, as points into its row of
-// `out` (one block a query).
-__global__ void listed_points_kernel(const uint64_t* __restrict__ part, const int* __restrict__ list, int splits, int C,
-                                     int k, lshg_point* __restrict__ out) {
+// The first k of each listed query's sorted lists of C keys, as points into its row of `out` (one
+// block a query).  slots: the scan's CTAs.
+__global__ void listed_points_kernel(const uint64_t* __restrict__ part, const int* __restrict__ list, int64_t n,
+                                     int slots, int64_t room, int C, int k, lshg_point* __restrict__ out) {
   grid_ready();
   extern __shared__ uint64_t ms[];
   const int cnt = list[0];
+  if (cnt == 0) return;
+  const int splits = listed_splits(cnt, (int)((n + kTile - 1) / kTile), slots, C, room);
   for (int i = blockIdx.x; i < cnt; i += gridDim.x) {
     const uint64_t* src = part + (int64_t)i * splits * C;
     for (int j = threadIdx.x; j < C; j += blockDim.x) ms[j] = src[j];
@@ -520,9 +557,10 @@ __global__ void listed_points_kernel(const uint64_t* __restrict__ part, const in
   }
 }
 
+// Returns the CTAs launched: as many as are resident at once.
 template <int DIST, int EC>
-void launch_listed(const float* xt, int64_t n, int d, const float* xnorm, const float* q, const float* qnorm,
-                   const int* list, int splits, uint64_t* part, cudaStream_t s) {
+int launch_listed(const float* xt, int64_t n, int d, const float* xnorm, const float* q, const float* qnorm,
+                  const int* list, const float* lim, int64_t room, uint64_t* part, cudaStream_t s) {
   const int nbuf = reg_scan_smem(d, 32 * EC, 1) <= kRegTwoCtaSmem ? 1 : 2;
   size_t smem = reg_scan_smem(d, 32 * EC, nbuf);
   const int nb = smem <= 220 * 1024 ? nbuf : 1;
@@ -530,10 +568,11 @@ void launch_listed(const float* xt, int64_t n, int d, const float* xnorm, const 
   LSHG_REQUIRE(smem <= 220 * 1024, "listed scan: dimension too large");
   auto kern = scan_float_listed_kernel<DIST, EC>;
   raise_smem_limit(kern, smem);
-  const int tps = ceil_div(ceil_div(n, kTile), splits);
-  launch_next(kern, num_sms() * 2, 256, smem, s, xt, n, d, xnorm, q, qnorm, list, tps, splits, nb, part);
+  const int grid = num_sms() * (smem <= kRegTwoCtaSmem ? 2 : 1);
+  launch_next(kern, grid, 256, smem, s, xt, n, d, xnorm, q, qnorm, list, lim, room, nb, part);
   count_launch();
   LSHG_CHECK_LAUNCH();
+  return grid;
 }
 
 template <int DIST, int EC>
@@ -635,28 +674,29 @@ int scan_float_splits(int64_t n, int nq, int C) {
   return best;
 }
 
-int scan_listed_splits(int64_t n, int nq, int C) {
-  // as many as spread one 64-query block over the SMs, while the lists stay below 256 MB
-  const int64_t fit = ((int64_t)256 << 20) / ((int64_t)nq * C * 8);
-  return (int)std::max<int64_t>(1, std::min<int64_t>({fit, 128, std::max(1, ceil_div(n, kTile) / 4)}));
+int64_t listed_scan_room(int nq, int C, int64_t have) {
+  // one item a CTA: 64 queries' lists each, 304 CTAs of lists of 32 or 64 keys or 152 of lists of 128
+  return std::max<int64_t>({have, (int64_t)nq * C, std::min<int64_t>((int64_t)nq * C * 128, (int64_t)5 << 18)});
 }
 
 void launch_scan_float_listed(const float* xt, int64_t n, int d, const float* xnorm, const float* q, int nq,
-                              const float* qnorm, int dist, const int* list, int C, int splits, uint64_t* part,
-                              int k, lshg_point* out, cudaStream_t s) {
+                              const float* qnorm, int dist, const int* list, const float* lim, int C, uint64_t* part,
+                              int64_t room, int k, lshg_point* out, cudaStream_t s) {
   ProfScope _ps("scan_float_listed", s);
   const bool jac = dist == DIST_JACCARD;
+  int slots = 0;
 #define LSHG_LS(EC)                                                                                          \
   do {                                                                                                       \
-    if (jac) launch_listed<DIST_JACCARD, EC>(xt, n, d, xnorm, q, qnorm, list, splits, part, s);              \
-    else launch_listed<DIST_ANGULAR, EC>(xt, n, d, xnorm, q, qnorm, list, splits, part, s);                  \
+    if (jac) slots = launch_listed<DIST_JACCARD, EC>(xt, n, d, xnorm, q, qnorm, list, lim, room, part, s);   \
+    else slots = launch_listed<DIST_ANGULAR, EC>(xt, n, d, xnorm, q, qnorm, list, lim, room, part, s);       \
   } while (0)
   if (C == 32) LSHG_LS(1);
   else if (C == 64) LSHG_LS(2);
   else if (C == 128) LSHG_LS(4);
   else throw Error(LSHG_ERR_INVALID_ARGUMENT, "listed scan: C must be 32, 64 or 128");
 #undef LSHG_LS
-  launch_next(listed_points_kernel, std::min(nq, num_sms() * 4), 128, (size_t)C * 8, s, part, list, splits, C, k, out);
+  launch_next(listed_points_kernel, std::min(nq, num_sms() * 4), 128, (size_t)C * 8, s, part, list, n, slots, room, C, k,
+              out);
   count_launch();
   LSHG_CHECK_LAUNCH();
 }

@@ -220,16 +220,20 @@ __global__ void __launch_bounds__(256, 4)
 }
 
 // Queries to scan in full: more candidates than places, fewer than k, or no bounds.  The re-rank has
-// nothing of them to do: their candidates are emptied.
+// nothing of them to do: their candidates are emptied, and tau becomes the full scan's distance limit T.
 __global__ void list_hard_kernel(const int* __restrict__ cnt, const int* __restrict__ bad, int nq, int k,
-                                 int cap, uint64_t* __restrict__ cand, int* __restrict__ list) {
+                                 int cap, uint64_t* __restrict__ cand, int* __restrict__ list,
+                                 float* __restrict__ tau) {
   grid_ready();
   const int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (q >= nq) return;
   const int c = cnt[q];
   const bool hard = bad[q] || c > cap || c < k;
   for (int i = lane + (hard ? 0 : c); i < cap; i += 32) cand[(int64_t)q * cap + i] = kEmptyKey;
-  if (hard && lane == 0) list[1 + atomicAdd(list, 1)] = q;
+  if (hard && lane == 0) {
+    list[1 + atomicAdd(list, 1)] = q;
+    tau[q] = bad[q] || c < k ? INFINITY : -tau[q];
+  }
 }
 
 size_t tile_smem(int wd, int rows) { return (size_t)rows * (wd | 1) * 4; }
@@ -268,13 +272,13 @@ bool query_jaccard_filtered(Index& I, const float* q, int nq, int k, lshg_point*
   const int S = std::max(1, std::min({8, cap / 16 / k, tiles / k})), stiles = ceil_div(tiles, S);
   int C = 32;
   while (C < k) C <<= 1;
-  const int lsplits = scan_listed_splits(I.n, nq, C);
+  const int64_t room = listed_scan_room(nq, C, (int64_t)nq * cap);
   try {
     DevBuf<uint32_t> qt((size_t)qblocks * wd * kQB, s);
     DevBuf<float4> qtail((size_t)qblocks * kQB, s);
     DevBuf<int> ctl((size_t)3 * nq + 1, s);  // [0, nq): candidates; [nq]: listed, then their list; then no bounds
     DevBuf<float> gmax((size_t)nq * 4 * stiles, s), tau((size_t)nq, s);
-    DevBuf<uint64_t> cand((size_t)nq * cap, s), part((size_t)nq * lsplits * C, s);
+    DevBuf<uint64_t> cand((size_t)room, s);  // candidates, then the lists of the FP32 scan
     int *cnt = ctl.ptr, *list = ctl.ptr + nq, *bad = ctl.ptr + 2 * nq + 1;
     const size_t qsm = tile_smem(wd, kQB);
     launch_next(code_tiles_kernel<kQB, 1024>, qblocks, 1024, qsm, s, q, nq, I.d, wd, I.jq_lo, I.jq_scale, qt.ptr,
@@ -306,12 +310,12 @@ bool query_jaccard_filtered(Index& I, const float* q, int nq, int k, lshg_point*
       LSHG_CHECK_LAUNCH();
     }
     launch_next(list_hard_kernel, ceil_div(nq, 8), 256, 0, s, cnt, bad, nq, (int)std::min<int64_t>(k, I.n), cap,
-                cand.ptr, list);
+                cand.ptr, list, tau.ptr);
     count_launch();
     LSHG_CHECK_LAUNCH();
     launch_rerank(cand.ptr, nq, cap, I.x.ptr, I.n, I.d, nullptr, q, nullptr, DIST_JACCARD, k, out, s, I.error_word(s));
-    launch_scan_float_listed(I.xt.ptr, I.n, I.d, nullptr, q, nq, nullptr, DIST_JACCARD, list, C, lsplits, part.ptr, k,
-                             out, s);
+    launch_scan_float_listed(I.xt.ptr, I.n, I.d, nullptr, q, nq, nullptr, DIST_JACCARD, list, tau.ptr, C, cand.ptr,
+                             room, k, out, s);
   } catch (const Error& e) {
     if (e.status != LSHG_ERR_OUT_OF_MEMORY) throw;
     cudaGetLastError();  // temporaries that do not fit: the FP32 scan needs fewer

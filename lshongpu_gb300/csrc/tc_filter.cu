@@ -658,9 +658,9 @@ __global__ void __launch_bounds__(256) cand_select_kernel(const int* __restrict_
 template <int E>
 __global__ void __launch_bounds__(256) exact_select_kernel(const int* __restrict__ cnt,
                                                             const uint64_t* __restrict__ cand, int cap, int k, int nq,
-                                                            const float* __restrict__ tau,
-                                                            const float* __restrict__ eps, uint64_t* __restrict__ out,
-                                                            int* __restrict__ ovf) {
+                                                            const float* tau, const float* __restrict__ eps,
+                                                            uint64_t* __restrict__ out, int* __restrict__ ovf,
+                                                            float* lim) {
   grid_ready();
   constexpr int CT = 32 * E;
   const int lane = threadIdx.x & 31;
@@ -674,6 +674,9 @@ __global__ void __launch_bounds__(256) exact_select_kernel(const int* __restrict
 #pragma unroll
   for (int e = 0; e < E; ++e) best[e] = kEmptyKey;
   float cut = 0.0f;
+  // a score that k points reach (none: -inf); it bounds their distances by 1 - reach + eps
+  const float t = tau ? tau[q] : -INFINITY;
+  float reach = c >= k ? t : -INFINITY;
   if (!listed) {
     warp_top<E>(cand + (int64_t)q * cap, c, lane, best);
     uint64_t kth = kEmptyKey, last = kEmptyKey;
@@ -684,13 +687,18 @@ __global__ void __launch_bounds__(256) exact_select_kernel(const int* __restrict
       last = best[e];
     }
     last = __shfl_sync(0xffffffffu, last, 31);
-    cut = -key_dist(kth) - e2;  // scores from here up
-    listed = (tau && tau[q] > cut) || (last != kEmptyKey && c > CT && -key_dist(last) >= cut);
+    reach = -key_dist(kth);
+    cut = reach - e2;  // scores from here up
+    listed = (tau && t > cut) || (last != kEmptyKey && c > CT && -key_dist(last) >= cut);
   }
 #pragma unroll
   for (int e = 0; e < E; ++e)
     dst[e * 32 + lane] = !listed && best[e] != kEmptyKey && -key_dist(best[e]) >= cut ? best[e] : kEmptyKey;
-  if (listed && lane == 0) ovf[1 + atomicAdd(ovf, 1)] = q;
+  __syncwarp();  // every lane has read tau[q], which may be lim[q]
+  if (listed && lane == 0) {
+    ovf[1 + atomicAdd(ovf, 1)] = q;
+    lim[q] = e2 < 1e30f ? 1.0f - reach + 0.5f * e2 + 1e-6f : INFINITY;
+  }
 }
 
 // Merge the list kernel's per-CTA partial lists of every listed query and write the
@@ -915,12 +923,12 @@ void launch_cand_select(const int* cnt, const uint64_t* cand, int nq, int cap, i
 }
 
 void launch_exact_select(const int* cnt, const uint64_t* cand, int nq, int cap, int k, int CT, const float* tau,
-                         const float* eps, uint64_t* out, int* ovf, cudaStream_t s) {
+                         const float* eps, uint64_t* out, int* ovf, float* lim, cudaStream_t s) {
   ProfScope _ps("exact_select", s);
   if (CT == 128) launch_next(exact_select_kernel<4>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, k, nq, tau, eps,
-                             out, ovf);
+                             out, ovf, lim);
   else if (CT == 256) launch_next(exact_select_kernel<8>, ceil_div(nq, 8), 256, 0, s, cnt, cand, cap, k, nq, tau,
-                                  eps, out, ovf);
+                                  eps, out, ovf, lim);
   else throw Error(LSHG_ERR_INVALID_ARGUMENT, "exact scan: candidate count must be 128 or 256");
   count_launch();
   LSHG_CHECK_LAUNCH();

@@ -63,9 +63,10 @@ void launch_cand_select(const int* cnt, const uint64_t* cand, int nq, int cap, i
 // within 2 eps[q] of the k-th best one, out of the top-CT (CT = 128 or 256; the rest of the row
 // is empty keys).  Listed in ovf instead: queries with more survivors than cap or fewer than
 // k, with more than CT candidates, whose threshold tau[q] (nullptr: none) does not reach that
-// far down, or whose eps is not finite.
+// far down, or whose eps is not finite.  lim[q] (may be tau) of a listed query: a distance that k
+// points have at most, infinite where the scores give none.
 void launch_exact_select(const int* cnt, const uint64_t* cand, int nq, int cap, int k, int CT, const float* tau,
-                         const float* eps, uint64_t* out, int* ovf, cudaStream_t s);
+                         const float* eps, uint64_t* out, int* ovf, float* lim, cudaStream_t s);
 
 // Tensor-core sketch scan (tc_hamming.cu): threshold plan for a base of n points and the
 // top-C of each query.  ok = false: no prepass shape bounds C well (use the popcount scan).

@@ -122,3 +122,43 @@ def test_two_threads_of_different_dimensions(engine, dist, k):
     for t in threads:
         t.join()
     assert not failed
+
+
+@pytest.mark.parametrize("dist", [1, 2])
+def test_exact_batches_allocate_by_the_query(engine, dist):
+    """A filtered exact batch takes less than 32 KB a query and 16 MB: the rescan of listed queries
+    has no lists of its own, whose number was as large as if every query were listed alone."""
+    n, d, nq = 60000, 16, 1000
+    rows = datasets.sparse_gamma if dist == 2 else datasets.clustered
+    x, q = rows(n, d, 171), rows(nq, d, 172)
+    with memory_pool() as high:
+        idx = engine.Index(x, implementation=2, distanceFunc=dist)
+        high()
+        held = high()
+        idx.query(q, 100)
+        used = high() - held
+        idx.close()
+    assert used <= nq * 32768 + (16 << 20)
+
+
+@pytest.mark.parametrize("dist", [1, 2])
+@pytest.mark.parametrize("n,nq,listed,d,k", [
+    (4096, 4, 1, 16, 1),          # one listed query, one neighbour; few tiles a split
+    (9000, 200, 3, 37, 64),       # listed queries anywhere in the batch; lists of 64
+    (20011, 70, 65, 100, 32),     # a second block of one query
+    (30000, 1500, 1500, 20, 10),  # every query: few splits
+    (50000, 300, 299, 128, 128),  # lists of 128, one CTA an SM
+])
+def test_listed_queries_equal_fp32_scan(engine, dist, n, nq, listed, d, k):
+    """Queries that tie with a third of the base, or (angular) have no direction, are scanned in full within
+    the limits their scores give: ids and distances of the FP32 scan, bit for bit."""
+    rows = datasets.sparse_gamma if dist == 2 else datasets.clustered
+    x, q = rows(n, d, 181), rows(nq, d, 182)
+    x[1::3] = x[0]
+    at = np.random.default_rng(5).permutation(nq)[:listed]
+    q[at] = x[0]
+    q[at[1::3]] *= np.float32(1.0003)
+    q[at[2::7]] = 0 if dist == 1 else q[at[2::7]]
+    idx = engine.Index(x, implementation=2, distanceFunc=dist)
+    want = idx.query(q, 129)[:, :k]  # k beyond the filter: the FP32 scan
+    assert idx.query(q, k).tobytes() == want.tobytes()
