@@ -114,11 +114,21 @@ constexpr int64_t kExactFilterMinPairs = 16384;
 // has more points within 2 eps of the k-th (1.2M x 32, 1,000 queries, k = 10: with 128 places
 // 901 us, with 256 292; 100k x 100, k = 32: 108 against 116).
 constexpr int64_t kExactFewCandidatesBase = 1 << 18;
+// The largest base that is filtered at few dimensions: on a sphere of d - 1 dimensions the points
+// within 2 eps of the k-th fill a fixed share of it, more than the places hold beyond about these
+// sizes, and the batch is then scanned twice.  Uniform points, filtered / FP32, us: d = 3, 20,000
+// points, 16 queries 106 / 90, 1,000 154 / 242; 100,000 points 213 / 149; d = 4, 100,000 190 / 149
+// and 303 / 638, 1M, one 329 / 214; d = 5, 1M, one 103 / 220, 1,000 656 / 2,922, 3M, one 703 /
+// 588; d = 6, 3M, one 180 / 612.  Below d = 3 every size lost (d = 2, 100,000 points, 200 queries
+// 339 / 259).
+int64_t exact_filter_max_base(int d) {
+  return d < 3 ? 0 : d == 3 ? 1 << 15 : d == 4 ? 1 << 17 : d == 5 ? 1 << 20 : INT_MAX;
+}
 
 }  // namespace
 
 void derive_exact(Index& I, cudaStream_t s) {
-  if (I.dist != DIST_ANGULAR || I.d > tc::KD || I.n < kExactFilterMinBase) return;
+  if (I.dist != DIST_ANGULAR || I.d > tc::KD || I.n < kExactFilterMinBase || I.n > exact_filter_max_base(I.d)) return;
   const int64_t npad = (int64_t)ceil_div(I.n, tc::FILTER_TN) * tc::FILTER_TN;
   unsigned bad = 0;
   try {

@@ -162,3 +162,22 @@ def test_listed_queries_equal_fp32_scan(engine, dist, n, nq, listed, d, k):
     idx = engine.Index(x, implementation=2, distanceFunc=dist)
     want = idx.query(q, 129)[:, :k]  # k beyond the filter: the FP32 scan
     assert idx.query(q, k).tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("n,d,filtered", [
+    (5000, 1, False), (5000, 2, False), (32768, 3, True), (32769, 3, False), (131072, 4, True), (131073, 4, False),
+    (200000, 5, True), (200000, 6, True),
+])
+def test_exact_filter_at_few_dimensions(engine, n, d, filtered):
+    """On a sphere of few dimensions the scores' error holds more points than the filter has places from
+    some base size on: the FP32 scan answers those, with the same results."""
+    rng = np.random.default_rng(7)
+    x, q = (rng.standard_normal((m, d)).astype(np.float32) for m in (n, 70))
+    idx = engine.Index(x, implementation=2, distanceFunc=1)
+    engine.profile_enable(True)
+    engine.profile_report()
+    got = idx.query(q, 32)
+    ran = engine.profile_report()
+    engine.profile_enable(False)
+    assert ("tc_filter" in ran) == filtered
+    assert got.tobytes() == idx.query(q, 129)[:, :32].tobytes()  # k beyond the filter: the FP32 scan
