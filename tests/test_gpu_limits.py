@@ -181,3 +181,29 @@ def test_exact_filter_at_few_dimensions(engine, n, d, filtered):
     engine.profile_enable(False)
     assert ("tc_filter" in ran) == filtered
     assert got.tobytes() == idx.query(q, 129)[:, :32].tobytes()  # k beyond the filter: the FP32 scan
+
+
+@pytest.mark.parametrize("case,filtered", [("sparse", True), ("dense", True), ("copies of 1000", True),
+                                           ("a third copies", True), ("copies of 10", False), ("near rows", False)])
+def test_jaccard_filter_by_the_bases_resolution(engine, case, filtered):
+    """A base whose rows have, mostly, more points within the codes' resolution than a query has places
+    is left to the FP32 scan; results are its either way."""
+    n, d, nq, k = 60013, 100, 40, 10
+    rng = np.random.default_rng(9)
+    x, q = datasets.sparse_gamma(n, d, 191), datasets.sparse_gamma(nq, d, 192)
+    if case == "dense":
+        x, q = rng.random((n, d), dtype=np.float32), rng.random((nq, d), dtype=np.float32)
+    elif case == "a third copies":
+        x[::3] = x[0]
+    elif case.startswith("copies of"):
+        x = x[rng.integers(0, int(case.split()[-1]), n)]
+    elif case == "near rows":
+        x, q = (x[:1] + 1e-4 * rng.random((m, d), dtype=np.float32) for m in (n, nq))
+    idx = engine.Index(x, implementation=2, distanceFunc=2)
+    engine.profile_enable(True)
+    engine.profile_report()
+    got = idx.query(q, k)
+    ran = engine.profile_report()
+    engine.profile_enable(False)
+    assert ("jaccard_filter" in ran) == filtered
+    assert got.tobytes() == idx.query(q, 129)[:, :k].tobytes()  # k beyond the filter: the FP32 scan
