@@ -39,6 +39,10 @@ constexpr int kMinDim = 16;   // 8-bit codes of fewer dimensions leave too many 
 constexpr int kMaxDim = 128;  // the listed FP32 scan's shared memory
 constexpr int kMinBase = 4096;
 constexpr int64_t kMinPairs = 16384;
+// Group maxima a query at most: groups span several tiles on bases that have more.  (1.2M points, k
+// = 32, had 37,500, 150 KB a query, which also took the threshold select's slowest form; any group
+// bounds as well, and with 48 groups or more for each of the k the threshold hardly moves.)
+constexpr int kMaxGroups = 6144;
 
 __device__ __forceinline__ unsigned code(float v, float s) {
   return (unsigned)__float2int_rn(fminf(fmaxf(v * s, 0.0f), 255.0f));
@@ -112,13 +116,14 @@ __global__ void __launch_bounds__(THREADS)
 
 // Tiles 0, stride, 2 stride, ... (ntiles of them; tile i below is the i-th).
 // MODE 0: gmax[q][4 i + g] = -(smallest upper bound of tile i's 32 points of group g).
+// MODE 2: the same with groups over the tiles i gt .. i gt + gt - 1 (tiles_per_split is a multiple of gt).
 // MODE 1: points with a lower bound <= T = -tau[q] appended to cand[q][0..cap) (cnt[q] counts
 // all).  The sums start at 2^23 as a float's bits, so they are read as floats without conversions.
 template <int MODE>
 __global__ void __launch_bounds__(256, 4)
     jaccard_scan_kernel(const uint32_t* __restrict__ xt, const float4* __restrict__ xtail, int64_t n, int wd, int d,
                         const uint32_t* __restrict__ qt, const float4* __restrict__ qtail,
-                        const int* __restrict__ qbad, int nq, int ntiles, int tiles_per_split, int stride,
+                        const int* __restrict__ qbad, int nq, int ntiles, int tiles_per_split, int stride, int gt,
                         float* __restrict__ gmax, const float* __restrict__ tau, int* __restrict__ cnt,
                         uint64_t* __restrict__ cand, int cap) {
   grid_ready();
@@ -127,6 +132,7 @@ __global__ void __launch_bounds__(256, 4)
   uint32_t* xs = sm;               // [wd][128]
   uint32_t* qs = sm + wd * kTile;  // [wd][64]
   __shared__ float2 xl[kTile], ql[kQB];
+  __shared__ float runs[MODE == 2 ? kQB : 1][4];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int q0 = blockIdx.x * kQB;
   const int t0 = blockIdx.y * tiles_per_split, t1 = min(ntiles, t0 + tiles_per_split);
@@ -135,7 +141,7 @@ __global__ void __launch_bounds__(256, 4)
   if (tid < kQB) {
     const int q = q0 + tid;
     const float4 v = qtail[q];
-    if (MODE == 0) {
+    if (MODE != 1) {
       ql[tid] = make_float2(v.x, v.y);
     } else {
       // 1 - A_hi / (S - A_hi) - delta <= T  <=>  A_hi >= S c / (1 + c), c = 1 - delta - T
@@ -158,7 +164,7 @@ __global__ void __launch_bounds__(256, 4)
       reinterpret_cast<uint4*>(xs)[i] = __ldg(reinterpret_cast<const uint4*>(xt + row0 * wd) + i);
     if (tid < kTile) {
       const float4 v = __ldg(xtail + row0 + tid);
-      xl[tid] = make_float2(v.x, MODE == 0 ? v.y : v.z);
+      xl[tid] = make_float2(v.x, MODE != 1 ? v.y : v.z);
     }
     __syncthreads();
     if (q0 + 8 * w >= nq) continue;  // no query of this warp: it only copies
@@ -187,7 +193,7 @@ __global__ void __launch_bounds__(256, 4)
     for (int a = 0; a < 8; ++a) {
       const float2 qv = ql[8 * w + a];
       const int q = q0 + 8 * w + a;
-      if (MODE == 0) {
+      if (MODE != 1) {
         float best = 0.0f;  // the largest A_lo / S
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
@@ -199,9 +205,19 @@ __global__ void __launch_bounds__(256, 4)
         best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, 2));
         best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, 4));
         // a group without points bounds nothing
-        if ((lane & 7) == 0 && q < nq)
-          gmax[(int64_t)q * 4 * ntiles + 4 * t + (lane >> 3)] =
-              left > 0 ? __fdividef(best, 1.0f - best) - 1.0f - delta(d) : -INFINITY;
+        if ((lane & 7) == 0 && q < nq) {
+          float up = left > 0 ? __fdividef(best, 1.0f - best) - 1.0f - delta(d) : -INFINITY;
+          if (MODE == 0) {
+            gmax[(int64_t)q * 4 * ntiles + 4 * t + (lane >> 3)] = up;
+          } else {
+            float* run = &runs[8 * w + a][lane >> 3];  // this thread's own
+            const int in = t % gt;
+            if (in) up = fmaxf(up, *run);
+            *run = up;
+            if (in == gt - 1 || t == ntiles - 1)
+              gmax[(int64_t)q * 4 * ((ntiles + gt - 1) / gt) + 4 * (t / gt) + (lane >> 3)] = up;
+          }
+        }
       } else {
         unsigned hits = 0;
 #pragma unroll
@@ -326,6 +342,7 @@ bool query_jaccard_filtered(Index& I, const float* q, int nq, int k, lshg_point*
   // Every S-th tile for the thresholds: the bounds pass about 5 S k candidates (60,013 sparse rows of
   // 100: 150 at S k = 32, at most 255), within the places, and never fewer than 4 k groups.
   const int S = std::max(1, std::min({8, cap / 16 / k, tiles / k})), stiles = ceil_div(tiles, S);
+  const int gt = ceil_div(4 * (int64_t)stiles, kMaxGroups), groups = 4 * ceil_div(stiles, gt);
   int C = 32;
   while (C < k) C <<= 1;
   const int64_t room = listed_scan_room(nq, C, (int64_t)nq * cap);
@@ -333,7 +350,7 @@ bool query_jaccard_filtered(Index& I, const float* q, int nq, int k, lshg_point*
     DevBuf<uint32_t> qt((size_t)qblocks * wd * kQB, s);
     DevBuf<float4> qtail((size_t)qblocks * kQB, s);
     DevBuf<int> ctl((size_t)3 * nq + 1, s);  // [0, nq): candidates; [nq]: listed, then their list; then no bounds
-    DevBuf<float> gmax((size_t)nq * 4 * stiles, s), tau((size_t)nq, s);
+    DevBuf<float> gmax((size_t)nq * groups, s), tau((size_t)nq, s);
     DevBuf<uint64_t> cand((size_t)room, s);  // candidates, then the lists of the FP32 scan
     int *cnt = ctl.ptr, *list = ctl.ptr + nq, *bad = ctl.ptr + 2 * nq + 1;
     const size_t qsm = tile_smem(wd, kQB);
@@ -345,23 +362,24 @@ bool query_jaccard_filtered(Index& I, const float* q, int nq, int k, lshg_point*
     auto split = [&](int nt) {
       return ceil_div(nt, std::max(1, std::min(ceil_div(nt, 2), ceil_div(num_sms() * 8, qblocks))));
     };
-    const int tps0 = split(stiles), tps = split(tiles);
+    const int tps0 = ceil_div(split(stiles), gt) * gt, tps = split(tiles);
     const dim3 grid0(qblocks, ceil_div(stiles, tps0)), grid(qblocks, ceil_div(tiles, tps));
     const size_t smem = (size_t)wd * (kTile + kQB) * 4;
-    raise_smem_limit(jaccard_scan_kernel<0>, smem);
+    auto bounds = gt == 1 ? jaccard_scan_kernel<0> : jaccard_scan_kernel<2>;
+    raise_smem_limit(bounds, smem);
     raise_smem_limit(jaccard_scan_kernel<1>, smem);
     {
       ProfScope _ps("jaccard_bounds", s);
-      launch_next(jaccard_scan_kernel<0>, grid0, 256, smem, s, I.jq.ptr, I.jq_tail.ptr, I.n, wd, I.d, qt.ptr, qtail.ptr, bad, nq,
-                                                      stiles, tps0, S, gmax.ptr, nullptr, nullptr, nullptr, 0);
+      launch_next(bounds, grid0, 256, smem, s, I.jq.ptr, I.jq_tail.ptr, I.n, wd, I.d, qt.ptr, qtail.ptr, bad, nq,
+                                                      stiles, tps0, S, gt, gmax.ptr, nullptr, nullptr, nullptr, 0);
       count_launch();
       LSHG_CHECK_LAUNCH();
     }
-    tc::launch_tau_select(gmax.ptr, nq, 4 * stiles, k, 0.0f, tau.ptr, s);
+    tc::launch_tau_select(gmax.ptr, nq, groups, k, 0.0f, tau.ptr, s);
     {
       ProfScope _ps("jaccard_filter", s);
       launch_next(jaccard_scan_kernel<1>, grid, 256, smem, s, I.jq.ptr, I.jq_tail.ptr, I.n, wd, I.d, qt.ptr, qtail.ptr, bad, nq,
-                                                     tiles, tps, 1, nullptr, tau.ptr, cnt, cand.ptr, cap);
+                                                     tiles, tps, 1, 1, nullptr, tau.ptr, cnt, cand.ptr, cap);
       count_launch();
       LSHG_CHECK_LAUNCH();
     }

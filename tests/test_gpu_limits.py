@@ -124,11 +124,12 @@ def test_two_threads_of_different_dimensions(engine, dist, k):
     assert not failed
 
 
-@pytest.mark.parametrize("dist", [1, 2])
-def test_exact_batches_allocate_by_the_query(engine, dist):
-    """A filtered exact batch takes less than 32 KB a query and 16 MB: the rescan of listed queries
-    has no lists of its own, whose number was as large as if every query were listed alone."""
-    n, d, nq = 60000, 16, 1000
+@pytest.mark.parametrize("n,dist", [(60000, 1), (60000, 2), (1000000, 2)])
+def test_exact_batches_allocate_by_the_query(engine, n, dist):
+    """A filtered exact batch takes less than 32 KB a query and 16 MB, also on a large base: the rescan of
+    listed queries has no lists of its own, whose number was as large as if every query were listed
+    alone, and the Jaccard scan's group maxima are bounded."""
+    d, nq = 16, 1000
     rows = datasets.sparse_gamma if dist == 2 else datasets.clustered
     x, q = rows(n, d, 171), rows(nq, d, 172)
     with memory_pool() as high:
@@ -207,3 +208,16 @@ def test_jaccard_filter_by_the_bases_resolution(engine, case, filtered):
     engine.profile_enable(False)
     assert ("jaccard_filter" in ran) == filtered
     assert got.tobytes() == idx.query(q, 129)[:, :k].tobytes()  # k beyond the filter: the FP32 scan
+
+
+@pytest.mark.parametrize("n,nq,k", [
+    (196608, 9, 100),  # 6,144 group maxima: a tile a group
+    (196609, 70, 32),  # one point more: two tiles a group, the last group of one tile
+    (450000, 33, 128),  # three
+    (700000, 5, 10),   # a sampled pass of them
+])
+def test_jaccard_filter_groups_of_tiles(engine, n, nq, k):
+    """Bases with more group maxima than the threshold select takes: the FP32 scan's results."""
+    x, q = datasets.sparse_gamma(n, 20, 201), datasets.sparse_gamma(nq, 20, 202)
+    idx = engine.Index(x, implementation=2, distanceFunc=2)
+    assert idx.query(q, k).tobytes() == idx.query(q, 129)[:, :k].tobytes()  # k beyond the filter
