@@ -177,7 +177,7 @@ struct RerankBounds {
 // (listed[0] of them, then their rows), into their rows of `out`.
 void launch_rerank_listed(const uint64_t* cand, int C, const float* x, int64_t n, int d, const float* xnorm,
                           const float* q, const float* qnorm, int dist, const int* listed, int nq, int k,
-                          struct ::lshg_point_s* out, cudaStream_t s);
+                          struct ::lshg_point_s* out, cudaStream_t s, int* err);
 // Angular candidates (lists of at most cap <= kListBounds ids, ccnt[q] of them) reduced by bounds to
 // those that can be in the top-k: kept[nq][kBoundsKeep] keys; listed: count, then the queries to score
 // in full (rerank_bounds.cu).  Queries with more than cap ids are left out (their kept is empty).

@@ -524,7 +524,8 @@ bool rerank_by_bounds(Index& I, const uint64_t* cand, int nq, int C, const float
   }
 #undef LSHG_RB
   launch_rerank(kept.ptr, nq, kKeep, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, qnorm, I.dist, k, out, s, I.error_word(s));
-  launch_rerank_listed(cand, C, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, qnorm, I.dist, listed.ptr, nq, k, out, s);
+  launch_rerank_listed(cand, C, I.x.ptr, I.n, I.d, I.xnorm.ptr, q, qnorm, I.dist, listed.ptr, nq, k, out, s,
+                       I.error_word(s));
   return true;
 }
 

@@ -221,3 +221,28 @@ def test_jaccard_filter_groups_of_tiles(engine, n, nq, k):
     x, q = datasets.sparse_gamma(n, 20, 201), datasets.sparse_gamma(nq, 20, 202)
     idx = engine.Index(x, implementation=2, distanceFunc=2)
     assert idx.query(q, k).tobytes() == idx.query(q, 129)[:, :k].tobytes()  # k beyond the filter
+
+
+@pytest.mark.parametrize("impl,n,nq,d,C,k", [
+    (3, 20000, 40, 64, 1024, 10),     # rows staged in shared memory
+    (3, 20000, 33, 128, 4096, 128),   # the widest rows, the longest list and k
+    (3, 20000, 700, 37, 2048, 32),    # rows read directly; several queries a block
+    (6, 20000, 20, 100, 1024, 1),
+    (10, 20000, 400, 40, 4096, 32),   # Jaccard
+    (10, 20000, 17, 33, 1024, 100),   # Jaccard, read directly
+])
+def test_listed_rerank_equals_full_rerank(engine, impl, n, nq, d, C, k):
+    """Lists that the 8-bit bounds cannot separate (near-equal rows), all of a batch and some of one: what
+    scoring every candidate returns."""
+    rng = np.random.default_rng(11)
+    rows = datasets.sparse_gamma if impl == 10 else datasets.clustered
+    x, q = rows(n, d, 211), rows(nq, d, 212)
+    near = lambda m: np.abs(x[:1] + 1e-4 * rng.standard_normal((m, d))).astype(np.float32) if impl == 10 else \
+        (x[:1] + 1e-4 * rng.standard_normal((m, d))).astype(np.float32)
+    x[: n // 2] = near(n // 2)
+    kw = dict(implementation=impl, sketchDim=64 if impl == 10 else 8, options=engine.make_options(candidates=C))
+    idx = engine.Index(x, **kw, **({"distanceFunc": 2} if impl == 10 else {}))
+    for some in (q, near(nq)):
+        some[::3] = near(len(some[::3]))
+        want = idx.query(some, 129)[:, :k]  # k beyond the bounds: every candidate is scored
+        assert idx.query(some, k).tobytes() == want.tobytes()
