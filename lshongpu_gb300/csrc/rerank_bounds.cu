@@ -174,6 +174,29 @@ __global__ void quantise_angular_kernel(const float* __restrict__ x, int64_t n, 
   if (wrong) atomicExch(bad, 1u);
 }
 
+// near[b]: of kProbePoints points spread over the base (all of a smaller one), those within the codes'
+// resolution of row b of kProbeRows: a distance that the residuals of both may hide.
+constexpr int kProbeRows = 64, kProbePoints = 8192;
+__global__ void __launch_bounds__(256) near_rows_kernel(const uint8_t* __restrict__ rows,
+                                                        const float2* __restrict__ tails, int64_t n, int pitch,
+                                                        int points, unsigned* __restrict__ near) {
+  const int64_t step = n / points;  // at least 1
+  const int64_t i = (2 * blockIdx.x + 1) * n / (2 * kProbeRows);
+  const unsigned t = blockIdx.y * blockDim.x + threadIdx.x;
+  bool in = false;
+  if ((int)t < points) {
+    const int64_t j = t * n / points + ((t + 1) * 2654435761u >> 8) % (unsigned)step;  // no period
+    int dot = 0;
+    for (int w = 0; w < pitch / 4; ++w)
+      dot = __dp4a(*reinterpret_cast<const int*>(rows + i * pitch + 4 * w),
+                   *reinterpret_cast<const int*>(rows + j * pitch + 4 * w), dot);
+    const float2 ti = tails[i], tj = tails[j];
+    in = i != j && 1.0f - (float)dot * (ti.x * tj.x) <= ti.y + tj.y;
+  }
+  const int c = __syncthreads_count(in);
+  if (threadIdx.x == 0 && c) atomicAdd(near + blockIdx.x, (unsigned)c);
+}
+
 // Bounds are kept as 16-bit steps of a distance in [-0.0625, 2.0625), rounded outwards (a step is
 // 3.2e-5, a tenth of the narrowest bounds); kEmptyStep: none.
 constexpr float kBase = -0.0625f, kStepsPer = 65000.0f / 2.125f;
@@ -443,18 +466,32 @@ void derive_jaccard(Index& I, cudaStream_t s) {
 
 void derive_angular(Index& I, cudaStream_t s) {
   const int pitch = angular_pitch(I.d);
-  DevBuf<unsigned> bad(1, s);
-  LSHG_CUDA(cudaMemsetAsync(bad.ptr, 0, bad.bytes(), s));
+  DevBuf<unsigned> stat(1 + kProbeRows, s);  // a row without bounds; the probe's counts
+  LSHG_CUDA(cudaMemsetAsync(stat.ptr, 0, stat.bytes(), s));
   I.xq8.alloc((size_t)I.n * pitch, s);
   I.xq8_tail.alloc((size_t)I.n, s);
   quantise_angular_kernel<<<(int)std::min<int64_t>((I.n * 32 + 255) / 256, (int64_t)num_sms() * 16), 256, 0, s>>>(
-      I.x.ptr, I.n, I.d, pitch, reinterpret_cast<int8_t*>(I.xq8.ptr), I.xq8_tail.ptr, bad.ptr);
+      I.x.ptr, I.n, I.d, pitch, reinterpret_cast<int8_t*>(I.xq8.ptr), I.xq8_tail.ptr, stat.ptr);
   count_launch();
   LSHG_CHECK_LAUNCH();
-  unsigned h = 0;
-  LSHG_CUDA(cudaMemcpyAsync(&h, bad.ptr, sizeof(h), cudaMemcpyDeviceToHost, s));
+  const int points = (int)std::min<int64_t>(kProbePoints, I.n);
+  near_rows_kernel<<<dim3(kProbeRows, ceil_div(points, 256)), 256, 0, s>>>(I.xq8.ptr, I.xq8_tail.ptr, I.n, pitch, points,
+                                                                          stat.ptr + 1);
+  count_launch();
+  LSHG_CHECK_LAUNCH();
+  unsigned h[1 + kProbeRows];
+  LSHG_CUDA(cudaMemcpyAsync(h, stat.ptr, sizeof(h), cudaMemcpyDeviceToHost, s));
   LSHG_CUDA(cudaStreamSynchronize(s));
-  if (h) I.xq8.release();  // a row without bounds: every candidate is scored
+  // A row without bounds, or a base whose rows mostly have more points within the codes' resolution
+  // than a query may keep: every candidate is scored.  Bounds on top of that took a fifth more
+  // (300,000 x 128, 32 tables, clusters of 1,500 within 0.013, 2,000 queries: 607 us without, 727
+  // with).
+  int crowded = 0;
+  for (int b = 0; b < kProbeRows; ++b) crowded += (int64_t)h[1 + b] * I.n > (int64_t)kKeep * points ? 1 : 0;
+  if (h[0] || 2 * crowded > kProbeRows) {
+    I.xq8.release();
+    I.xq8_tail.release();
+  }
 }
 
 }  // namespace

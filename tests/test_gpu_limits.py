@@ -246,3 +246,22 @@ def test_listed_rerank_equals_full_rerank(engine, impl, n, nq, d, C, k):
         some[::3] = near(len(some[::3]))
         want = idx.query(some, 129)[:, :k]  # k beyond the bounds: every candidate is scored
         assert idx.query(some, k).tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("sigma,copies,used", [(0.05, 1, True), (0.05, 50, True), (0.01, 1, False), (0.05, 2000, False)])
+def test_lsh_bounds_by_the_bases_resolution(engine, sigma, copies, used):
+    """LSH candidates go through bounds unless the base's rows mostly have more points within the codes'
+    resolution than a query may keep; results are those of scoring every candidate either way."""
+    n, d, nq, k = 100000, 100, 200, 32
+    x = datasets.clustered(n // copies, d, 221, count=50, sigma=sigma)
+    q = datasets.clustered(nq, d, 222, count=50, sigma=sigma)
+    x = np.ascontiguousarray(np.repeat(x, copies, axis=0))
+    idx = engine.Index(x, implementation=2, distanceFunc=1, framework=1, keysImplementation=7, bucketKeyBits=16,
+                       tables=16, options=engine.make_options(cp_hashes=2))
+    engine.profile_enable(True)
+    engine.profile_report()
+    got = idx.query(q, k)
+    ran = engine.profile_report()
+    engine.profile_enable(False)
+    assert ("rerank_bounds" in ran) == used
+    assert got.tobytes() == idx.query(q, 129)[:, :k].tobytes()  # k beyond the bounds
