@@ -677,15 +677,19 @@ static void launch_split(const LshQueryArgs& a, int cap, size_t fused_smem, lshg
   // Angular: the candidates that can be in the top-k, by bounds from 8-bit rows, then the
   // re-rank of those; the scoring kernel keeps the queries whose bounds leave too many.
   // 10,000 queries on 1M x 128, 1,900 distinct candidates each: scoring every row 1.31 ms, this way
-  // 0.66.  By the average bucket (entries a query if keys were spread evenly; clustered data
-  // has several times as many): not where most lists would overflow to the fused kernel (50k x
-  // 64, one hash a key, 7,800: one query 204 / 213 us), nor for a handful of candidates (200k x
-  // 100, 16 tables, 49: one query 55 / 61 us, 64 75 / 68; 1M x 128, 488: one 87 / 71).
+  // 0.66.  The rule goes by the average bucket, the entries a query has if keys were spread evenly
+  // (clustered data has three to five times as many): two launches more are won back by lists of
+  // about 120 entries, at four queries or more, or one query's 400.  us a batch, with bounds / without:
+  // 97 entries (100k x 64) 16 queries 52 / 48, 1,000 86 / 81; 100 (150k x 100) 16 56 / 54, 1,000 115 /
+  // 125; 122 (1M x 128) one 51 / 51, four 54 / 58, 1,000 121 / 147; 585 (300k x 48) one 60 / 65, 1,000
+  // 134 / 192; two (20k x 100) 256 queries 53 / 40.  Nor where most lists would overflow to the fused
+  // kernel (50k x 64, one hash a key, 6,250 entries: one query 204 / 213).
   const int64_t avg = a.n * a.tables / a.tableSize;
   const int* only = nullptr;
   DevBuf<uint64_t> kept;
   DevBuf<int> hard;
-  bool bounds = DV == DIST_ANGULAR && a.xq8 && a.k <= 128 && cap <= kListBounds && 2 * avg <= cap && avg * a.nq >= 400;
+  bool bounds = DV == DIST_ANGULAR && a.xq8 && a.k <= 128 && cap <= kListBounds && avg >= 120 && 2 * avg <= cap &&
+                avg * a.nq >= 400;
   if (bounds) {
     try {
       kept.alloc((size_t)a.nq * kBoundsKeep, s);

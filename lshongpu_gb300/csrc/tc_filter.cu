@@ -68,7 +68,9 @@ constexpr int F_TMEM_COLS = F_NACC * TN;  // 512 = all of TMEM (one CTA per SM)
 constexpr int F_EPI_WARPS = 16;      // four warpgroups, one 64-column piece each
 constexpr int kTauRegs = 80;  // group maxima a lane holds in the register threshold select
 constexpr int kTauBlockRegs = 24;  // and a thread of the block form: 6,144 maxima
-constexpr int kTauRegsFew = 44;  // and its smaller form: 1,408 maxima, what a base of 1.2M points leaves
+// and its smaller form, 1,408 maxima (59 registers, four blocks an SM).  One query on 1.2M points, the
+// batch: 87 us with 44, 89 with 40, 90 with 48.
+constexpr int kTauRegsFew = 44;
 
 // Shared-memory layout of a CTA in a cluster of CL: CL buffers of its query tile (rows of KC
 // chunks; a pair loads its next query tiles while these are in use, a CTA alone has but one

@@ -71,7 +71,7 @@ def test_lsh_batch_without_room_for_the_bounds(engine):
     n, d, nq = 20000, 16, 43000
     x = datasets.clustered(n, d, 151, count=200)
     q = np.tile(datasets.clustered(1000, d, 152, count=200), (nq // 1000, 1))
-    kw = dict(implementation=2, distanceFunc=1, framework=1, keysImplementation=7, bucketKeyBits=10, tables=4,
+    kw = dict(implementation=2, distanceFunc=1, framework=1, keysImplementation=7, bucketKeyBits=10, tables=7,
               options=engine.make_options(cp_hashes=2))
     with memory_pool() as high:
         idx = engine.Index(x, **kw)
@@ -257,7 +257,31 @@ def test_lsh_bounds_by_the_bases_resolution(engine, sigma, copies, used):
     q = datasets.clustered(nq, d, 222, count=50, sigma=sigma)
     x = np.ascontiguousarray(np.repeat(x, copies, axis=0))
     idx = engine.Index(x, implementation=2, distanceFunc=1, framework=1, keysImplementation=7, bucketKeyBits=16,
-                       tables=16, options=engine.make_options(cp_hashes=2))
+                       tables=80, options=engine.make_options(cp_hashes=2))
+    engine.profile_enable(True)
+    engine.profile_report()
+    got = idx.query(q, k)
+    ran = engine.profile_report()
+    engine.profile_enable(False)
+    assert ("rerank_bounds" in ran) == used
+    assert got.tobytes() == idx.query(q, 129)[:, :k].tobytes()  # k beyond the bounds
+
+
+@pytest.mark.parametrize("n,nq,k,d,tables,used", [
+    (80000, 200, 32, 100, 98, False),  # 119 entries a query on average
+    (80000, 200, 32, 100, 99, True),   # 120
+    (8000, 3, 128, 16, 16, False),     # 125, 375 in the batch
+    (8000, 4, 128, 16, 16, True),      # 500
+    (4000, 1, 1, 128, 256, False),     # 15
+    (27000, 1, 10, 16, 16, True),      # 421, one query
+    (200000, 50, 10, 16, 16, False),   # 3,125: more than half of the list's places
+])
+def test_lsh_bounds_rule(engine, n, nq, k, d, tables, used):
+    """Where LSH candidates go through bounds, and that the results do not depend on it."""
+    x, q = datasets.clustered(n, d, 231, count=500), datasets.clustered(nq, d, 232, count=500)
+    P = 1 << (d - 1).bit_length()
+    idx = engine.Index(x, implementation=2, distanceFunc=1, framework=1, keysImplementation=7,
+                       bucketKeyBits=2 * P.bit_length(), tables=tables, options=engine.make_options(cp_hashes=2))
     engine.profile_enable(True)
     engine.profile_report()
     got = idx.query(q, k)
