@@ -134,7 +134,7 @@ void launch_cws_slice(const uint32_t* smp, int64_t rows, int S, int d, const Cws
 void launch_cws_scan(const uint32_t* xsl_t, const uint32_t* xst, int64_t n, int S, int d, const CwsCodes& c,
                      const uint32_t* qs, int nq, int C, uint64_t* out, int* err, cudaStream_t s);
 
-// ---- rerank.cu -------------------------------------------------------------------
+// ---- rescans of queries listed on the device -------------------------------------------
 // The exact top-k (angular or Jaccard) of the queries listed on the device (list[0] = count, list[1..] =
 // rows of q), written to their rows of `out`; k <= 128.  lim[q]: a distance that k points have at most
 // (infinite: none known).  part: `room` >= nq * C keys, C = the power of two >= max(32, k); the more
@@ -145,10 +145,6 @@ void launch_scan_float_listed(const float* xt, int64_t n, int d, const float* xn
 // Keys to allocate for survivor arrays of `have` keys that the listed scan uses after them: up to 10 MB
 // where listed queries could use them (128 splits each).
 int64_t listed_scan_room(int nq, int C, int64_t have);
-// Merge per-split sorted lists into one sorted list of C keys per query.  list (optional): the lists of
-// slot i < list[0] go to row list[1 + i].
-void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t* out, cudaStream_t s,
-                         const int* list = nullptr);
 // Splits of the base for the exact rescan of queries listed on the device (at most nq of them, QB a
 // block): blocks enough for one or two listed queries to use the GPU, as far as the lists of all nq
 // fit `room` keys a query (the filter's survivor arrays, free by then).  With one split, a query
@@ -158,6 +154,12 @@ int listed_rescan_splits(int64_t n, int nq, int QB, int C, int room);
 // Keys a query of the survivor arrays: `cap`, or room for up to 64 splits' lists within 4 MB.  (32
 // MB cost batches of 100 queries 20 to 40 us in the allocator.)
 int survivor_room(int nq, int cap, int C);
+
+// ---- rerank.cu -------------------------------------------------------------------
+// Merge per-split sorted lists into one sorted list of C keys per query.  list (optional): the lists of
+// slot i < list[0] go to row list[1 + i].
+void launch_merge_splits(const uint64_t* in, int nq, int splits, int C, uint64_t* out, cudaStream_t s,
+                         const int* list = nullptr);
 // The same with the first k keys written as points; false when C or k is not one it serves.
 bool launch_merge_points(const uint64_t* in, int nq, int splits, int C, int k, struct ::lshg_point_s* out,
                          cudaStream_t s);
@@ -173,6 +175,12 @@ struct RerankBounds {
 // fp64_recheck: re-score, in double precision, the run of candidates around the k-th
 // place whose FP32 distances lie within the FP32 error bound of one another (among the
 // first 128) and order that run by the FP64 distance.
+// qnorm == nullptr (angular, C < 1024): the kernel computes the query norms itself, and writes
+// them to qnorm_out where given.
+void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t n, int d,
+                   const float* xnorm, const float* q, const float* qnorm, int dist, int k,
+                   struct ::lshg_point_s* out, cudaStream_t s, int* err = nullptr, bool fp64_recheck = false,
+                   const double* xn64 = nullptr, const RerankBounds* extra_dev = nullptr, float* qnorm_out = nullptr);
 // The re-rank (k <= 128, C = 1024, 2048 or 4096; Jaccard or angular) of the listed queries alone
 // (listed[0] of them, then their rows), into their rows of `out`.
 void launch_rerank_listed(const uint64_t* cand, int C, const float* x, int64_t n, int d, const float* xnorm,
@@ -185,12 +193,6 @@ constexpr int kBoundsKeep = 256;
 constexpr int kListBounds = 6144;
 void launch_list_bounds(const int* list, int cap, const int* ccnt, const uint8_t* rows, const float2* tails, int64_t n,
                         int d, const float* q, int nq, int k, uint64_t* kept, int* listed, cudaStream_t s);
-// qnorm == nullptr (angular, C < 1024): the kernel computes the query norms itself, and writes
-// them to qnorm_out where given.
-void launch_rerank(const uint64_t* cand, int nq, int C, const float* x, int64_t n, int d,
-                   const float* xnorm, const float* q, const float* qnorm, int dist, int k,
-                   struct ::lshg_point_s* out, cudaStream_t s, int* err = nullptr, bool fp64_recheck = false,
-                   const double* xn64 = nullptr, const RerankBounds* extra_dev = nullptr, float* qnorm_out = nullptr);
 // Row norms in double precision (sum of squares in dimension order, then sqrt): the FP64
 // re-check's base magnitudes.
 void launch_row_norms_fp64(const float* x, int64_t n, int d, double* out, cudaStream_t s);

@@ -4,10 +4,13 @@
 // process whose free HBM is already owned by another allocator (a framework's caching
 // allocator reserves it up front), or a latency-critical thread that must not enter the
 // CUDA allocator at all (growing the stream-ordered pool can block).  For them,
-// lshg_index_query_noalloc runs the same kernels as lshg_index_query for an exact
-// angular index (implementation 2, linear scan) but takes every temporary -- query
+// lshg_index_query_noalloc answers queries of an exact angular index (implementation 2,
+// linear scan) by the FP32 scan of scan_float.cu and takes every temporary -- query
 // magnitudes, the per-split candidate lists and their merge -- from one file-scope
 // device array of kNoAllocScratchBytes.  Nothing is allocated or freed on any call.
+// lshg_index_query goes through the tensor-core filter of scan_exact.cu where that serves
+// (k <= 128, d <= 128, bases and batches large enough), whose survivor arrays would not fit
+// the array; the results are the same, bit for bit.
 //
 // Properties the caller must respect:
 //  * the array exists once per GPU that loads this library and stays allocated until

@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kBoundThreads, 5) bounds_kernel(
   grid_ready();
   constexpr bool JAC = DIST == DIST_JACCARD;
   constexpr int W = kBoundThreads / 32, PER = C / kBoundThreads;
-  extern __shared__ uint32_t bnd[];  // [C] lower bound << 16 | upper bound, in steps of kStep from kBase
+  extern __shared__ uint32_t bnd[];  // [C] lower bound << 16 | upper bound, in steps of 1 / kStepsPer from kBase
   __shared__ int wcnt[2][W];
   __shared__ int total;
   const int qi = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

@@ -105,14 +105,16 @@ void launch_unit_rows(const float* x, int64_t n, int d, int64_t rows_pad, uint16
 }
 
 // Bases below kExactFilterMinBase points and batches below kExactFilterMinPairs (query, point)
-// pairs stay with the FP32 scan: the filter's nine launches take 60 us whatever the sizes, the
-// FP32 scan 46 to 60 us for one query on 4,096 points, 72 to 89 on 20,000 and 99 to 120 for 16
-// queries on 4,096.
+// pairs stay with the FP32 scan: the filter's eight launches take 39 to 52 us whatever the sizes.
+// FP32 scan and filter, us, k = 10: one query on 20,000 x 100 53 / 41, two on 8,192 53 / 40, four
+// on 4,096 67 / 40; below the line one on 8,192 and on 4,096 46.  At 16 dimensions the FP32 scan is
+// shorter for one query up to 60,000 points (20,000: 30 / 40) and longer from four on (4,096: 48 / 39).
 constexpr int64_t kExactFilterMinBase = 4096;
 constexpr int64_t kExactFilterMinPairs = 16384;
-// Candidates re-scored a query at most.  Queries with more go to the FP32 scan, and a large base
-// has more points within 2 eps of the k-th (1.2M x 32, 1,000 queries, k = 10: with 128 places
-// 901 us, with 256 292; 100k x 100, k = 32: 108 against 116).
+// The base from which a query re-scores 256 candidates at most instead of 128 (k <= 32): queries with
+// more go to the FP32 scan, and a large base has more points within 2 eps of the k-th.  1.2M x 32,
+// 1,000 queries, k = 10: with 128 places 595 us, with 256 261; 100k x 100, k = 32: 81 and
+// 90.
 constexpr int64_t kExactFewCandidatesBase = 1 << 18;
 // The largest base that is filtered at few dimensions: on a sphere of d - 1 dimensions the points
 // within 2 eps of the k-th fill a fixed share of it, more than the places hold beyond about these

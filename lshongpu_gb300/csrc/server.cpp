@@ -426,7 +426,9 @@ int lshg_server_submit(lshg_server* s, int index_id, const float* queries, int N
       return LSHG_ERR_BUSY;
     }
   }
-  // admission by free HBM: the request's buffers plus scratch must fit above the reserve
+  // admission by free HBM: the request's buffers plus scratch must fit above the reserve.  32 KB a
+  // query: an exact scan's survivors, candidates and group maxima take 10 to 30 (on bases of up to
+  // 5M points); its rescan of listed queries uses the survivors' arrays.
   size_t free_b = 0, total_b = 0;
   cudaSetDevice(s->device);
   if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {

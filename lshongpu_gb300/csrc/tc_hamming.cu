@@ -406,8 +406,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     const int r = (warp & 3) * 32 + lane;  // query row within the tile = TMEM lane
     const uint32_t tbase = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g * HW);
     const uint32_t at0 = s0 + LY::S_OFF + (uint32_t)(g * SBUF * BM + r) * 4u;
-    constexpr int GRP = SBUF >= 16 ? 8 : 4;                            // columns pushed between two room checks
-    const uint32_t at_lim = at0 + (uint32_t)(SBUF - GRP) * (BM * 4u);  // beyond: no room for GRP more
+    const uint32_t at_lim = at0 + (uint32_t)(SBUF - 8) * (BM * 4u);  // beyond: no room for a group of 8 more
     uint32_t at = at0;
     int ia = 0;
     bool ok = true;
@@ -466,16 +465,13 @@ __global__ void __launch_bounds__(H_THREADS, 1)
 #pragma unroll
           for (int gg = 0; gg < 7; ++gg) {
             if (!__any_sync(0xffffffffu, m[gg] >= tau)) continue;
+            if (__any_sync(0xffffffffu, at > at_lim)) flush();
 #pragma unroll
-            for (int h = 0; h < 8; h += GRP) {
-              if (__any_sync(0xffffffffu, at > at_lim)) flush();
-#pragma unroll
-              for (int jj = h; jj < h + GRP; ++jj) h_push(v[8 * gg + jj], tau, at, off + (uint32_t)(8 * gg + jj));
-            }
+            for (int jj = 0; jj < 8; ++jj) h_push(v[8 * gg + jj], tau, at, off + (uint32_t)(8 * gg + jj));
           }
         }
       }
-      if (MODE == MODE_FILTER) flush();  // the next unit is another query tile
+      if (MODE == MODE_FILTER) flush();  // the next unit counts its offsets from another tile, often for another query
     }
   }
 
