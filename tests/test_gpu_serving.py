@@ -198,3 +198,30 @@ def test_cws_index_same_alone_and_in_the_mix(engine):
         assert np.array_equal(out, cws.query(q, k))
     assert srv.stats()["completed"] == len(reqs)
     srv.close()
+
+
+@pytest.mark.parametrize("hard", [False, True])
+def test_jaccard_index_same_alone_and_in_the_mix(engine, hard):
+    """The filtered exact Jaccard scan recorded in graphs and replayed: requests of every size and k, with
+    queries that the replays have to rescan (ties with a third of the base) in some of them only."""
+    x = datasets.sparse_gamma(20000, D, 73)
+    if hard:
+        x[::3] = x[0]
+    idx = engine.Index(x, implementation=2, distanceFunc=2)
+    rng = np.random.default_rng(13)
+    srv = engine.Server(max_batch=512, streams=2, use_graphs=True)
+    srv.add_index(0, idx)
+    reqs = []
+    for t in range(40):
+        nq = int(np.exp(rng.uniform(0, np.log(200))))
+        k = int(rng.choice([10, 32, 100]))
+        q = datasets.sparse_gamma(nq, D, 4000 + t)
+        if hard and t % 2:
+            q[:: 1 + t % 3] = x[0]
+        reqs.append((q, k, srv.submit(0, q, k)))
+    for q, k, tk in reqs:
+        out, _ = srv.wait(tk)
+        assert np.array_equal(out, idx.query(q, k))
+    st = srv.stats()
+    assert st["completed"] == len(reqs) and st["graph_replays"] >= 1
+    srv.close()

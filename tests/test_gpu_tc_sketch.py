@@ -134,3 +134,31 @@ def test_byte_minhash_filter_ties_rescanned(engine, orc):
     ids, ds = orc.sketch_scan(xp, orc.normalize(q), 4, skx, skq, S, C, 2, 32)
     assert np.array_equal(res["ID"], ids)
     assert np.array_equal(res["distance"], ds)
+
+
+@pytest.mark.parametrize("impl,n,nq,C,kernel", [
+    (3, 16384, 3, 128, "scan_bits"),            # 49,152 (query, point) pairs
+    (3, 16384, 4, 128, "tc_hamming"),           # 65,536: the tensor cores
+    (3, 16383, 4, 128, "scan_bits"),
+    (3, 5000, 1, 256, "tc_hamming"),            # longer lists: any batch
+    (5, 16384, 3, 32, "scan_bits"),
+    (5, 16384, 4, 32, "tc_hamming"),
+    (4, 8192, 1, 32, "scan_bits"),              # byte samples: 8,192 pairs
+    (4, 8192, 2, 32, "scan_bytes_filter"),      # 16,384: the threshold filter
+    (4, 5000, 1, 64, "scan_bytes_filter"),      # longer lists: any batch
+])
+def test_automatic_choice_of_the_sketch_scan(engine, impl, n, nq, C, kernel):
+    """Which scan a batch takes by default, on both sides of each line; the results are the popcount
+    scan's."""
+    rows = datasets.clustered if impl == 3 else datasets.sparse_gamma
+    x, q = rows(n, D, 61), rows(nq, D, 62)
+    kw = dict(implementation=impl, sketchDim=64 if impl == 4 else 4, **({} if impl == 3 else {"distanceFunc": 2}))
+    auto = engine.Index(x, options=engine.make_options(candidates=C), **kw)
+    want = engine.Index(x, options=engine.make_options(candidates=C, sketch_scan=POPCOUNT), **kw).query(q, 10)
+    engine.profile_enable(True)
+    engine.profile_report()
+    got = auto.query(q, 10)
+    ran = engine.profile_report()
+    engine.profile_enable(False)
+    assert [k for k in ("scan_bits", "tc_hamming", "scan_bytes_filter") if k in ran] == [kernel]
+    assert np.array_equal(got, want)
