@@ -164,7 +164,19 @@ typedef struct lshg_index_params_s {
   lshg_options opt;
 } lshg_index_params;
 
-/* Build an index over N_data points (host pointer unless data_on_device). */
+/* Build an index over N_data points (host pointer unless data_on_device).  Device memory it keeps, bytes a
+ * point: 4 d for the rows, and
+ *   exact scan (2)            4 d tiled rows; angular 4 + 256 where d <= 128 and N >= 4,096 (BF16 rows of
+ *                             128 columns whatever d is; not for few dimensions on large bases);
+ *                             Jaccard 4 ceil(d / 4) + 16 where 16 <= d <= 128 and N >= 4,096
+ *   tensor-core scans (8, 9)  4 + 256 + 8, and 128 more for 9
+ *   sketches (3, 4, 5, 10)    the sketch twice, and an expanded or bit-sliced copy unless sketch_scan = 1
+ *   LSH (framework 1)         6 a table
+ *   re-rank by bounds         d rounded up to 16, + 8 (angular: SimHash and JL with 1,024 candidates or
+ *                             more, and LSH with d a multiple of 4), or d + 8 rounded up to 32 (Jaccard:
+ *                             MinHash and CWS with 1,024 or more), where d <= 128 (120)
+ * The BF16, 8-bit and expanded rows are derived at build and at load, and not kept where a base has no use for
+ * them; without room for the BF16 or 8-bit rows the index is built without them. */
 int lshg_index_build(const lshg_index_params* p, const float* data, int64_t N_data, int data_on_device,
                      lshg_index** out);
 /* Query: `queries` [N_query][d], `results` [N_query][k]; both host pointers unless

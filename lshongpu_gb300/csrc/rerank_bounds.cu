@@ -26,7 +26,8 @@
 // A row of 100 dimensions is 128 bytes here against 400 (angular, 128 dimensions: 160 against
 // 512), and about 60 of 4,096 Jaccard candidates, 130 of 1,900 of an LSH query, are left at k =
 // 32.  Eight lanes read a row, 16 bytes each.  The Jaccard kernel is bounded by its instructions
-// (minima as packed 16-bit pairs: 1.15 ms, 28 a row), the LSH lists' by latency: bounds of 4
+// (minima as packed 16-bit pairs: 1.15 ms, 28 a row), the LSH lists' by instructions and gathers
+// together (600k x 128: 75% of the issue slots, waiting for rows otherwise): bounds of 4
 // bytes a candidate and 48 registers let five CTAs share an SM (8 bytes and 58: 0.66 ms).
 // Measured (10,000 queries): Jaccard, C = 4,096,
 // 500k x 100: partition, gather of every row and select 2.77 ms; this way 0.74 + 0.15 ms.

@@ -11,7 +11,8 @@
 //                         within 2^-18 of u;
 //   the accumulation      of at most 128 products of magnitude <= 1 (in total, by
 //                         Cauchy-Schwarz) in the tensor core: 2^-15 allowed, 64 times what
-//                         eight FP32 additions with truncation lose;
+//                         eight FP32 additions with truncation lose (an allowance: how the
+//                         tensor core adds is not documented);
 //   the FP32 distance     within (2 d + 7) 2^-24 of 1 - cos (fp64_band in rerank.cu) while
 //                         both norms are in [2^-40, 2^40], so that nothing over- or underflows.
 // Let s_k be the k-th best score.  The k points that reach it have D <= 1 - s_k + eps, so every
@@ -23,7 +24,7 @@
 //
 // r(x) is about 8e-4 for vectors of 100 comparable components, so 2 eps is about 0.004 and the
 // candidates are a handful more than k.  Measured (100k x 100, 1,000 queries, k = 32): the
-// FP32 scan 886 us, this 78; 1.2M x 100: one query 1,065 -> 110 us, 1,000 queries 6.62 -> 0.30
+// FP32 scan 886 us, this 78; 1M x 100, one query 915 -> 100 us; 1.2M, 1,000 queries 6.62 -> 0.28
 // ms.
 #include <algorithm>
 

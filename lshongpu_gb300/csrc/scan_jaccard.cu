@@ -13,14 +13,15 @@
 //   candidates  points whose lower bound is at most T -- every point of the top-k -- are listed
 //               (at most 512 or 1,024 a query) and scored with the reference's formula (launch_rerank).
 // Queries with more candidates, or with a negative or non-finite value, are scanned by the FP32
-// scan from a list on the device.  A base with such a value always takes it.
+// scan from a list on the device, starting from T.  A base with such a value, or whose rows lie too
+// close for the codes (crowded_rows_kernel), always takes it.
 //
 // scan kernel: a CTA takes 64 queries and a run of 128-point tiles, warp w queries 8w .. 8w + 7,
 // lane l points 4l .. 4l + 3: 32 sums a thread, three shared 16-byte loads a four-dimension step.
 // Measured (60,013 x 100, 129 queries, k = 10): the FP32 scan 413 us, this 85 (the two passes 15 + 27,
-// the re-rank 14; the rest is launches and latency); 1M x 100, one query 2,140 -> 246, 100 queries, k =
-// 32, 2,640 -> 1,000.  With the divisions of every bound in place of the linear form below the second
-// pass took 49 us against 31.
+// the re-rank 14; the rest is launches and latency); 1M x 100, one query 2,140 -> 117, 100 queries, k =
+// 32, 2,640 -> 631.  Both passes are bounded by the integer ALU (77 and 83% busy, memory idle).  With
+// the divisions of every bound in place of the linear form below the second pass took 49 us against 31.
 #include <algorithm>
 
 #include "index.h"
